@@ -95,6 +95,8 @@ struct hmc_system {
     int32_t variant[2] = {-1, -1};  // launch variant per precision; -1: the cached choice or the default
     bool pdl = true;                // colour passes launch while the previous one finishes
     uint32_t rounds_guess = 2;      // colour sets enqueued before the sweep's count is known
+    uint64_t flow_entries = 0;      // trials the draw buffers of dataflow launches hold
+    uint32_t flow_cells = 0;        // spaces that progress holds
     // serial sweep grid (allocated on first use)
     uint32_t serial_nc[3] = {0, 0, 0};
     double serial_w[3] = {0, 0, 0};
@@ -230,10 +232,17 @@ void lj_setup_for(int dim, const Geometry& geom, Pair& P, double eps, double sig
         wmax = std::max(wmax, geom.width[a]);
         Lmax = std::max(Lmax, geom.L[a]);
     }
-    // the FP32 sigma^2 and 4 eps carry one rounding each; fold them into E generously
-    const double E = (8.0 * u32 * wmax + 16.0 * u64 * (Lmax + wmax) + 4.0 * u32 * sigma) * fp32_band_scale();
+    // The FP32 displacement of two fixed-point sites (fixed_dist2) is off by at most E on each axis
+    // (their roundings, half a unit of L / 2^32 each; the FP64 site's and difference's own) plus
+    // three FP32 roundings of itself, r^2 by three more, and sigma^2 in FP32 by one: as an r^2 error
+    // (1 + 2 * 3 + 3) u32 r^2, here 10.4.
+    const double scale = fp32_band_scale();
+    const double E = (std::ldexp(1.1 * Lmax, -32) + 16.0 * u64 * (Lmax + wmax)) * scale;
+    const double rel = 10.4 * u32 * scale;
+    for (int a = 0; a < 3; ++a) P.lj_fix[a] = a < dim ? (float)std::ldexp(geom.L[a], -32) : 0.f;
     P.lj_disp_err = (float)(E * 1.01);
-    const double band = 2.0 * (3.5 * E * (rcut + E) + 3.1 * u32 * rcut * rcut);
+    P.lj_rel_err = (float)(rel * 1.01);
+    const double band = 2.0 * (3.5 * E * (rcut + E) + rel * rcut * rcut);
     P.lj_rcut2_lo32 = std::nextafter((float)(P.lj_rcut2 - band), -INFINITY);
     P.lj_rcut2_hi32 = std::nextafter((float)(P.lj_rcut2 + band), INFINITY);
     double e_lo = lj_energy_host(P.lj_four_eps, sigma, std::sqrt(std::max(P.lj_rcut2 - 2.0 * band, 0.0))) - P.lj_e_shift;
@@ -294,6 +303,7 @@ void pair_setup(hmc_system* s) {
 // 97-107) and HypercuboidCheckerboard::compute_dimensions (hypercuboid.rs:188-228). The
 // checkerboard arrays grow when the box needs more spaces than they hold.
 hmc_status setup_geometry(hmc_system* s, const double* L) {
+    s->arr.fixed_sites = s->soft_fp32() ? 1u : 0u;
     Geometry g = s->geom;
     for (int a = 0; a < 3; ++a) g.L[a] = a < s->dim ? L[a] : 1.0;
     double min_l = g.L[0];
@@ -340,7 +350,7 @@ hmc_status setup_geometry(hmc_system* s, const double* L) {
         if ((st = dalloc(s, &A.cell_count, cells)) || (st = dalloc(s, &A.cell_start, cells + 1)) ||
             (st = dalloc(s, &A.block_sums, (size_t)scan_blocks * 9)) || (st = dalloc(s, &A.color_cells, cells)))
             return st;
-        if (s->soft() || s->oriented()) {  // the rounds' trial moves of the passes with lanes per trial
+        if (s->oriented()) {  // the rounds' trial moves of the passes with lanes per trial
             dfree(s, &A.trial_t);
             dfree(s, &A.trial_o);
             dfree(s, &A.trial_k);
@@ -370,7 +380,47 @@ hmc_status check_flags(hmc_system* s) {
     if (f & kErrAngleRange) return fail(HMC_INVALID_ARGUMENT, "a 2-D orientation angle reached 2^19 rad");
     if (f & kErrCellOverflow) return fail(HMC_CELL_OVERFLOW, "a cell of the serial sweep's grid is full");
     if (f & kErrIterationCap) return fail(HMC_ITERATION_CAP, "an approximate separation ran past its step bound");
+    if (f & kErrFlowTimeout) return fail(HMC_TIMEOUT, "a trial waited for its neighbours past the time limit");
     return HMC_OK;
+}
+
+// The draw buffers of a system's dataflow launches (hmc_flow.cuh): one launch per sweep needs one
+// entry per trial, rounds x non-empty spaces < bodies + spaces. Where they would take more than a
+// quarter of the free memory the launches run one colour set each.
+hmc_status flow_buffers(hmc_system* s) {
+    Arrays& A = s->arr;
+    const uint64_t cells = s->geom.n_cells;
+    hmc_status st;
+    if (s->flow_cells < cells) {
+        dfree(s, &A.progress);
+        if ((st = dalloc(s, &A.progress, cells))) return st;
+        s->flow_cells = (uint32_t)cells;
+    }
+    const uint64_t want = s->capacity + cells;
+    if (s->flow_entries >= want) return HMC_OK;
+    const size_t entry = sizeof(*A.draw_d) + sizeof(*A.draw_i);
+    size_t free_bytes = 0, total_bytes = 0;
+    HMC_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+    uint64_t n = want;
+    // HMC_B200_FLOW_SETS=1 (tests): one colour set per launch, as where memory is short
+    const char* sets = std::getenv("HMC_B200_FLOW_SETS");
+    if (sets && std::atoi(sets) == 1) n = cells;
+    if (entry * want > (free_bytes + entry * s->flow_entries) / 4) n = cells;
+    if (s->flow_entries >= n) return HMC_OK;
+    dfree(s, &A.draw_d);
+    dfree(s, &A.draw_i);
+    s->flow_entries = 0;
+    if ((st = dalloc(s, &A.draw_d, n)) || (st = dalloc(s, &A.draw_i, n))) return st;
+    s->flow_entries = n;
+    return HMC_OK;
+}
+
+// Whether the system's sweeps run in dataflow order, and the colour sets one launch then holds.
+bool flow_of(const hmc_system* s) { return s->soft(); }
+uint32_t flow_sets(const hmc_system* s) {
+    const uint64_t cells = s->geom.n_cells;
+    if (s->flow_entries >= s->n + cells) return UINT32_MAX;
+    return (uint32_t)std::max<uint64_t>(1, s->flow_entries / cells);
 }
 
 // ---- launch variants -------------------------------------------------------------------------
@@ -975,6 +1025,10 @@ static SweepPlan sweep_plan(const hmc_system* s, const hmc_sweep_params* p) {
 // The cell-list rebuild of the current sweep; shapes read S in both modes, and the colour passes
 // do not read slot_of_body.
 static hmc_status sweep_rebuild(hmc_system* s, const SweepPlan& sp) {
+    if (flow_of(s)) {
+        hmc_status st = flow_buffers(s);
+        if (st) return st;
+    }
     return rebuild(s, !sp.fp32 || s->oriented() || (s->soft() && !s->soft_fp32()), false);
 }
 
@@ -995,13 +1049,23 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
                                uint32_t r1) {
     const bool fp32 = sp.fp32;
     const uint32_t colors = 1u << s->dim;
+    if (flow_of(s)) {
+        const uint32_t sets = flow_sets(s);
+        L.substep = s->substep;  // the kernels add the colour set
+        for (uint32_t r = r0; r < r1; r += std::min(sets, r1 - r)) {
+            L.round = r;
+            L.round_end = r + std::min(sets, r1 - r);
+            // the overlap penalty and Isotropic have no FP32 path: FP64 in both modes
+            HMC_CUDA(launch_flow_lj(s->dim, fp32 && s->soft_fp32(), !s->soft_fp32(), s->geom, s->arr, s->pair, L,
+                                    s->stream, sp.variant));
+            s->prof.kernel_launches += 2;
+        }
+        return HMC_OK;
+    }
     for (uint32_t r = r0; r < r1; ++r) {
         L.substep = s->substep + r;  // increment_substep after every full colour set
         L.round = r;
-        if (s->soft()) {
-            HMC_CUDA(launch_propose_lj(s->dim, fp32 && s->soft_fp32(), s->geom, s->arr, L, s->stream));
-            s->prof.kernel_launches += 1;
-        } else if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON) {
+        if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON) {
             HMC_CUDA(launch_propose_poly(fp32 && !s->shape_soft, s->geom, s->arr, L, p->move == HMC_ROTATE,
                                          s->shape_soft, s->stream));
             s->prof.kernel_launches += 1;
@@ -1015,11 +1079,8 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
             L.overlap_previous = (r > 0 || c > 0) && s->pdl ? 1u : 0u;
             // the first pass after the rebuild (or after a round's proposals): launch early, wait
             // for it before reading anything
-            L.early_wait = (r == 0 || s->soft() || s->oriented()) && c == 0 && s->pdl ? 1u : 0u;
-            if (s->soft())  // the overlap penalty has no FP32 path: FP64 in both modes
-                HMC_CUDA(launch_sweep_lj(s->dim, fp32 && s->soft_fp32(), !s->soft_fp32(), s->geom, s->arr, s->pair, L,
-                                         s->stream, sp.variant));
-            else if (s->shape_soft && s->dim == 3)  // FP64 in both modes
+            L.early_wait = (r == 0 || s->oriented()) && c == 0 && s->pdl ? 1u : 0u;
+            if (s->shape_soft && s->dim == 3)  // FP64 in both modes
                 HMC_CUDA(launch_sweep_poly3_soft(s->geom, s->arr, s->verts, s->n_vertices, s->so, L, s->stream));
             else if (s->shape_soft)
                 HMC_CUDA(launch_sweep_poly2_soft(s->sat(), s->geom, s->arr, s->verts, s->n_vertices, s->so, L,
@@ -1037,6 +1098,12 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
         }
     }
     return HMC_OK;
+}
+
+// The colour sets the host enqueues before it knows a sweep's count: the last sweep's, or all of
+// them where one dataflow launch runs however many there are.
+static uint32_t guessed_sets(const hmc_system* s) {
+    return flow_of(s) && flow_sets(s) == UINT32_MAX ? UINT32_MAX : std::max(1u, s->rounds_guess);
 }
 
 // A finished sweep into the call's Count and the system's Counter.
@@ -1078,10 +1145,9 @@ static hmc_status sweep_pipelined(hmc_system* s, const hmc_sweep_params* p, hmc_
         s->slots_cap = kPipelineSweeps;
     }
     const SweepPlan sp = sweep_plan(s, p);
-    uint32_t done = 0;
+    uint32_t done = 0, guess = 1;
     while (done < p->n_sweeps) {
         const uint32_t chunk = std::min(p->n_sweeps - done, kPipelineSweeps);
-        const uint32_t guess = std::max(1u, s->rounds_guess);
         const uint64_t step0 = s->step;
         const uint32_t substep0 = s->substep;
         hmc_status st = HMC_OK;
@@ -1089,6 +1155,7 @@ static hmc_status sweep_pipelined(hmc_system* s, const hmc_sweep_params* p, hmc_
             s->step = step0 + j;
             s->substep = j == 0 ? substep0 : 0u;
             if ((st = sweep_rebuild(s, sp))) break;
+            if (j == 0) guess = guessed_sets(s);
             Launch L = sweep_launch(s, p);
             if ((st = enqueue_sets(s, p, sp, L, 0, guess))) break;
             cudaError_t e = launch_sweep_guard(s->arr.stats, guess, s->arr.abort_word, s->stream);
@@ -1169,7 +1236,7 @@ hmc_status hmc_sweep(hmc_system* s, const hmc_sweep_params* p, hmc_count* out) {
         // The rounds (while count.total() < N, :402-418) are known on the device after the
         // rebuild; the host enqueues the previous sweep's number of colour sets without
         // waiting, the kernels skip sets beyond the true count, and any missing sets follow.
-        const uint32_t guess = s->n == 0 ? 0u : s->rounds_guess;
+        const uint32_t guess = s->n == 0 ? 0u : guessed_sets(s);
         if ((st = enqueue_sets(s, p, sp, L, 0, guess))) return st;
         // the passes' end is recorded before the host waits for the counts, so that profiling adds
         // no host round trip to the sweep
@@ -1190,7 +1257,9 @@ hmc_status hmc_sweep(hmc_system* s, const hmc_sweep_params* p, hmc_count* out) {
             s->prof.rebuild_ms += t_rebuild;
             s->prof.rebuild_launches += rebuild_kernels(s);
             s->prof.sweep_ms += t_sweep;
-            s->prof.sweep_launches += (uint64_t)std::max(rounds, guess) * colors;
+            // a dataflow launch holds several colour passes
+            s->prof.sweep_launches += flow_of(s) ? (guess == UINT32_MAX ? 1u : std::max(rounds, guess))
+                                                 : (uint64_t)std::max(rounds, guess) * colors;
             s->prof.sweeps += 1;
         }
         account_sweep(s, p, *s->host_stats, total);
@@ -2267,6 +2336,7 @@ struct hmc_batch {
     uint64_t kernel_launches = 0;
     int32_t variant[2] = {-1, -1};  // launch variant of the hard-sphere replica pass per precision
     uint32_t rounds_guess = 2;
+    uint64_t flow_entries = 0;               // trials the draw buffers of dataflow launches hold
     uint32_t interaction = HMC_HARD_SPHERE;  // the same for every replica
     std::vector<double> body_range;          // [R] ParallelSweep range of each replica
     // captured sweeps (hmc_batch_set_captured_sweeps): one sweep as a CUDA graph, built for a
@@ -2332,24 +2402,32 @@ hmc_status batch_read(hmc_batch* bt) {
     const uint32_t f = bt->host_stats->error_flags;
     if (f & kErrNonFinite) return fail(HMC_NAN_STATE, "a body position is not finite");
     if (f & kErrOutsideCheckerboard) return fail(HMC_OUTSIDE_CHECKERBOARD, "a body maps to no checkerboard space");
+    if (f & kErrFlowTimeout) return fail(HMC_TIMEOUT, "a trial waited for its neighbours past the time limit");
     return HMC_OK;
 }
 
-// The colour passes of one set of a batch sweep, every colour, on stream s.
-hmc_status batch_enqueue_colours(hmc_batch* bt, bool fp32, uint32_t round, bool first, uint32_t variant,
-                                 cudaStream_t s) {
-    const uint32_t colors = 1u << bt->dim;
-    for (uint32_t c = 0; c < colors; ++c) {
-        const bool overlap = !first || c > 0, early = first && c == 0;
-        if (bt->interaction == HMC_LENNARD_JONES)
-            HMC_CUDA(launch_sweep_batch_lj(bt->dim, fp32, bt->b, bt->arr, c, round, bt->b.color_stride, overlap, early,
-                                           s, variant));
-        else
-            HMC_CUDA(launch_sweep_batch(bt->dim, fp32, bt->b, bt->arr, c, round, bt->b.color_stride, overlap, early, s,
-                                        variant));
+// The colour sets one batch_enqueue_sets runs: those the draw buffers of a Lennard-Jones batch's
+// dataflow launches hold (a replica's last colour sets leave entries empty), else one.
+uint32_t batch_sets(const hmc_batch* bt) {
+    if (bt->interaction != HMC_LENNARD_JONES) return 1;
+    return (uint32_t)std::max<uint64_t>(1, bt->flow_entries / std::max(1u, bt->cells));
+}
+
+// batch_sets colour sets of a batch sweep from set `round` on stream s.
+hmc_status batch_enqueue_sets(hmc_batch* bt, bool fp32, uint32_t round, bool first, uint32_t variant, cudaStream_t s) {
+    if (bt->interaction == HMC_LENNARD_JONES) {
+        const uint32_t sets = batch_sets(bt);
+        HMC_CUDA(launch_flow_batch_lj(bt->dim, fp32, bt->b, bt->arr, round, round == kRoundFromDevice ? sets : round + sets,
+                                      s, variant));
+        return HMC_OK;
     }
+    const uint32_t colors = 1u << bt->dim;
+    for (uint32_t c = 0; c < colors; ++c)
+        HMC_CUDA(launch_sweep_batch(bt->dim, fp32, bt->b, bt->arr, c, round, bt->b.color_stride, !first || c > 0,
+                                    first && c == 0, s, variant));
     return HMC_OK;
 }
+uint32_t batch_set_kernels(const hmc_batch* bt) { return bt->interaction == HMC_LENNARD_JONES ? 2u : 1u << bt->dim; }
 
 void batch_drop_graph(hmc_batch* bt) {
     if (bt->graph_exec) cudaGraphExecDestroy(bt->graph_exec);
@@ -2409,13 +2487,14 @@ hmc_status batch_build_graph(hmc_batch* bt, bool fp32, uint32_t variant, bool in
         HMC_CUDA(cudaStreamBeginCaptureToGraph(bt->body_stream, body, nullptr, nullptr, 0,
                                                cudaStreamCaptureModeThreadLocal));
         hmc_status sb = capture(bt->body_stream, [&]() -> hmc_status {
-            hmc_status r = batch_enqueue_colours(bt, fp32, kRoundFromDevice, true, variant, bt->body_stream);
+            hmc_status r = batch_enqueue_sets(bt, fp32, kRoundFromDevice, true, variant, bt->body_stream);
             if (r) return r;
-            HMC_CUDA(launch_batch_round_next(h, bt->arr.stats, bt->round_dev, bt->body_stream));
+            HMC_CUDA(launch_batch_round_next(h, bt->arr.stats, bt->round_dev, batch_sets(bt), bt->body_stream));
             return HMC_OK;
         });
         if (sb) return sb;
-        HMC_CUDA(launch_batch_sweep_end(bt->b, rep, bt->arr.stats, bt->rep_counts, bt->totals, increment_step, cs));
+        HMC_CUDA(launch_batch_sweep_end(bt->b, rep, bt->arr.stats, bt->rep_counts, bt->totals, increment_step,
+                                        batch_sets(bt), cs));
         return HMC_OK;
     });
     if (st) {
@@ -2460,10 +2539,11 @@ hmc_status batch_sweep_captured(hmc_batch* bt, const hmc_sweep_params& p0, bool 
     // kernels: origins, the rebuild's six, rounds, the first test and the end per sweep; the
     // colour passes and the step per colour set
     const uint64_t per_sweep = bt->n > 0 ? 10 : 6;
-    bt->kernel_launches += per_sweep * p0.n_sweeps + t.colour_sets * ((1u << bt->dim) + 1);
+    bt->kernel_launches += per_sweep * p0.n_sweeps + t.set_launches * (batch_set_kernels(bt) + 1);
     const uint32_t f = t.error_flags;
     if (f & kErrNonFinite) return fail(HMC_NAN_STATE, "a body position is not finite");
     if (f & kErrOutsideCheckerboard) return fail(HMC_OUTSIDE_CHECKERBOARD, "a body maps to no checkerboard space");
+    if (f & kErrFlowTimeout) return fail(HMC_TIMEOUT, "a trial waited for its neighbours past the time limit");
     hmc_count tot{};
     for (uint32_t k = 0; k < bt->n_rep; ++k) {
         const uint64_t acc = bt->host_rep_counts[2 * k], rej = bt->host_rep_counts[2 * k + 1];
@@ -2655,6 +2735,16 @@ hmc_status hmc_batch_create(hmc_context* ctx, uint32_t n_replicas, const hmc_sys
         (st = balloc(bt, &bt->first_bad, 1)) || (st = balloc(bt, &bt->round_dev, 1)) ||
         (st = balloc(bt, &bt->rep_counts, 2 * (size_t)n_replicas)) || (st = balloc(bt, &bt->totals, 1)))
         return destroy_fail(st);
+    A.fixed_sites = lj ? 1u : 0u;
+    if (lj) {  // the draws of all colour sets of equal replicas, or of one set where memory is short
+        size_t free_bytes = 0, total_bytes = 0;
+        cudaMemGetInfo(&free_bytes, &total_bytes);
+        const size_t entry = sizeof(*A.draw_d) + sizeof(*A.draw_i);
+        bt->flow_entries = entry * (n + cells) <= free_bytes / 4 ? n + cells : cells;
+        if ((st = balloc(bt, &A.draw_d, bt->flow_entries)) || (st = balloc(bt, &A.draw_i, bt->flow_entries)) ||
+            (st = balloc(bt, &A.progress, cells)))
+            return destroy_fail(st);
+    }
     bt->b.round_dev = bt->round_dev;
     A.body_ori = nullptr;
     A.sorted_q = nullptr;
@@ -2665,6 +2755,7 @@ hmc_status hmc_batch_create(hmc_context* ctx, uint32_t n_replicas, const hmc_sys
     bt->b.body_rep = d_body_rep;
     bt->b.n_replicas = n_replicas;
     bt->b.n_cells = cells;
+    bt->b.n_bodies = (uint32_t)n;
     bt->b.color_stride = cells >> dim;
     // Microstate::add_body (microstate.rs:777-835): each body keeps wrap(input).
     std::vector<double4> host(n);
@@ -2728,8 +2819,7 @@ hmc_status hmc_batch_sweep(hmc_batch* bt, const hmc_sweep_params* params, hmc_co
     }
     HMC_CUDA(cudaSetDevice(bt->ctx->device));
     const bool fp32 = p0.precision == HMC_FP32_RECHECK;
-    const uint32_t colors = 1u << bt->dim;
-    const uint32_t variant = batch_variant_of(bt, fp32);
+    const uint32_t variant = batch_variant_of(bt, fp32), sets = batch_sets(bt);
     if (counts) std::memset(counts, 0, sizeof(hmc_count) * bt->n_rep);
     if (bt->captured) return batch_sweep_captured(bt, p0, fp32, variant, counts, total);
     hmc_count tot{};
@@ -2740,20 +2830,14 @@ hmc_status hmc_batch_sweep(hmc_batch* bt, const hmc_sweep_params* params, hmc_co
         bt->kernel_launches += 1;
         HMC_CUDA(cudaMemsetAsync(bt->b.accepted, 0, sizeof(unsigned long long) * bt->n_rep, bt->stream));
         auto enqueue = [&](uint32_t r0, uint32_t r1) -> hmc_status {
-            for (uint32_t round = r0; round < r1; ++round)
-                for (uint32_t c = 0; c < colors; ++c) {
-                    if (bt->interaction == HMC_LENNARD_JONES)
-                        HMC_CUDA(launch_sweep_batch_lj(bt->dim, fp32, bt->b, bt->arr, c, round, bt->b.color_stride,
-                                                       round > 0 || c > 0, round == 0 && c == 0, bt->stream,
-                                                       variant));
-                    else
-                        HMC_CUDA(launch_sweep_batch(bt->dim, fp32, bt->b, bt->arr, c, round, bt->b.color_stride,
-                                                    round > 0 || c > 0, round == 0 && c == 0, bt->stream, variant));
-                    bt->kernel_launches += 1;
-                }
+            for (uint32_t round = r0; round < r1; round += sets) {
+                hmc_status se = batch_enqueue_sets(bt, fp32, round, round == 0, variant, bt->stream);
+                if (se) return se;
+                bt->kernel_launches += batch_set_kernels(bt);
+            }
             return HMC_OK;
         };
-        const uint32_t guess = bt->rounds_guess;
+        const uint32_t guess = (bt->rounds_guess + sets - 1) / sets * sets;
         if ((st = enqueue(0, guess))) return st;
         if ((st = batch_read(bt))) return st;
         const uint32_t max_rounds = bt->host_stats->rounds;

@@ -17,6 +17,7 @@ enum : uint32_t {
     kErrCellOverflow = 1u << 3,  // a cell of the serial sweep's grid is full
     kErrIterationCap = 1u << 4,  // an approximate separation loop ran past ShapeOverlap::max_steps
     kErrAborted = 1u << 5,       // a sweep of a pipelined call after one that stopped the call
+    kErrFlowTimeout = 1u << 6,   // a dataflow launch's wait ran past its time limit (hmc_flow.cuh)
 };
 
 // Counters written by the kernels. Zeroed by the host before a sweep.
@@ -32,6 +33,7 @@ struct DeviceStats {
     unsigned int rounds;              // full colour sets of the sweep: ceil(N / non-empty spaces)
     unsigned long long ambiguous;     // soft-potential trials whose decision the order of the
                                       // FP64 pair-energy sum could change (order_ambiguous)
+    unsigned int ticket;              // the next trial of the running dataflow launch (hmc_flow.cuh)
 };
 
 // The checkerboard (hoomd-mc/src/hypercuboid.rs) together with the periodic box.
@@ -58,7 +60,8 @@ struct Arrays {
     double4* body_ori;       // [n] body versors (s, x, y, z), body order; may be null
     double4* sorted_b;       // [n] body positions B in cell order (proposal source)
     double4* sorted_s;       // [n] site positions S = wrap(B) in cell order (neighbour tests)
-    float4* sorted_off;      // [n] FP32 offsets of S from its cell corner; .w = fast-axis cell index bits
+    float4* sorted_off;      // [n] FP32 offsets of S from its cell corner; .w = fast-axis cell index bits;
+                             // or (fixed_sites) the bits of S's fixed-point coordinates (fixed_site)
     double4* sorted_q;       // [n] versors in cell order; may be null
     uint32_t* sorted_body;   // [n] cell-order slot -> body index
     uint32_t* slot_of_body;  // [n] body index -> cell-order slot
@@ -73,14 +76,21 @@ struct Arrays {
     uint32_t* abort_word;    // pipelined sweeps: nonzero once a sweep stopped the call (may be null)
     const double* zig_x;     // ziggurat tables (257 each)
     const double* zig_f;
-    // A round's trial moves, one per colour-list entry (soft potentials: k_propose_lj writes them
-    // before the round's colour passes, which give each trial a warp): trial site T = wrap(W1) and
+    // A round's trial moves, one per colour-list entry (shapes: k_propose_poly3/2 write them
+    // before the round's colour passes, which give each trial several lanes): trial site T = wrap(W1) and
     // the Metropolis uniform in trial_t, T's FP32 offsets in trial_o, the chosen slot in trial_k
     // (kNoTrial when the move leaves its space or the entry is empty).
     double4* trial_t;        // [cells]
     float4* trial_o;         // [cells]
     uint32_t* trial_k;       // [cells]
     double4* trial_q;        // [cells] shapes: the proposed versor (2-D: the angle in .x)
+    // Dataflow launches (hmc_flow.cuh): what the random streams of a launch's trials give, by trial
+    // number (draw_d: displacement and uniform, draw_i: slot, space, uniform's bounds), and the
+    // colour sets each space has finished (~0 for an empty space).
+    double4* draw_d;
+    uint4* draw_i;
+    uint32_t* progress;      // [cells]
+    uint32_t fixed_sites;    // Lennard-Jones: sorted_off holds fixed-point sites
 };
 constexpr uint32_t kNoTrial = 0xffffffffu;
 
@@ -101,6 +111,8 @@ struct Pair {
     float lj_rcut2_lo32;  // r_cut^2 minus the r^2 error bound: below, the pair is inside for certain
     float lj_rcut2_hi32;  // r_cut^2 plus the bound: at or above, outside for certain
     float lj_disp_err;    // per-axis FP32 displacement error bound E
+    float lj_rel_err;     // the part of the FP32 r^2 error that grows with r^2, as a fraction of it
+    float lj_fix[3];      // L / 2^32 per axis (fixed_site)
     float lj_band_energy; // bound on |pair energy| for a pair inside the cut-off band
     // Isotropic<Expanded<OverlapPenalty>> (overlap_penalty.rs:109-115, expanded.rs:64-66):
     // r^2 >= r_cut^2 -> 0; x = sqrt(r^2) - delta; x < -d_max -> inf; x < 0 -> (0.5 k) x^2 + eps
@@ -236,6 +248,7 @@ struct Launch {
     uint32_t n_active;    // upper bound of the colour's list length (grid size); the kernels read
                           // the length itself from DeviceStats::color_count
     uint32_t round;       // colour set within the sweep; kernels skip it when >= DeviceStats::rounds
+    uint32_t round_end;   // dataflow launches run the colour sets [round, round_end)
     double max_move;      // Translate maximum distance
     double kt;            // Isothermal temperature
     uint32_t n_bodies;
@@ -297,24 +310,25 @@ struct LaunchShape {
 };
 constexpr LaunchShape kSphereDirectShapes[] = {{6, 1, 0}, {5, 1, 0}, {7, 1, 0}};
 constexpr LaunchShape kSphereCoopShapes[] = {{6, 1, 2}, {6, 1, 1}, {6, 1, 3}, {5, 1, 2}, {7, 1, 2}};
-// Lennard-Jones and Isotropic passes; own_steps 2: two candidates per lane and step
-constexpr LaunchShape kLjShapes[] = {{9, 1, 0}, {7, 1, 0}, {11, 1, 0}, {7, 1, 2}, {9, 1, 2}};
+// Lennard-Jones and Isotropic trials; own_steps: warps per trial (variant 0: by the trials of a
+// colour)
+constexpr LaunchShape kLjShapes[] = {{0, 1, 0}, {6, 1, 1}, {12, 1, 2}, {6, 1, 4}, {3, 1, 8}};
 constexpr LaunchShape kPolyShapes[] = {{5, 4, 0}, {5, 2, 0}, {5, 8, 0}};
 constexpr LaunchShape kBatchShapes[] = {{4, 1, 0}, {3, 1, 0}, {5, 1, 0}, {6, 1, 0}, {7, 1, 0}, {8, 1, 0}};
 // The polygon pass: one compiled shape; in the FP32 mode, variant 1 runs the FP64 pass instead
 // of the FP32 prefilter (the same decisions; the prefilter saves little where the FP64
 // circumsphere test is cheap against the separating-axis or XenoCollide test behind it).
 constexpr LaunchShape kPoly2Shapes[] = {{8, 4, 0}, {8, 4, 0}};
-// the Lennard-Jones replica passes; own_steps 2: two candidates per lane and step
-constexpr LaunchShape kBatchLjShapes[] = {{7, 1, 0}, {9, 1, 0}, {5, 1, 0}, {7, 1, 2}, {9, 1, 2}};
+// the Lennard-Jones replicas, as kLjShapes
+constexpr LaunchShape kBatchLjShapes[] = {{0, 1, 0}, {6, 1, 1}, {12, 1, 2}, {6, 1, 4}, {3, 1, 8}};
 template <size_t N>
 constexpr uint32_t n_shapes(const LaunchShape (&)[N]) {
     return (uint32_t)N;
 }
 
-// Blocks in one resident wave of a 128-thread kernel on the current device (SMs x resident
-// blocks per SM), cached per kernel.
-int resident_wave(const void* kernel);
+// Blocks in one resident wave of a kernel with `threads` per block on the current device (SMs x
+// resident blocks per SM), cached per kernel.
+int resident_wave(const void* kernel, int threads = 128);
 
 // Launch configuration of a colour pass: 128 threads per block; overlap = programmatic
 // dependent launch after the previous colour pass of the same sweep (the kernel waits with
@@ -369,6 +383,7 @@ struct Batch {
     const uint32_t* round_dev;      // the colour set a pass launched with kRoundFromDevice runs
     uint32_t n_replicas;
     uint32_t n_cells;               // all replicas
+    uint32_t n_bodies;              // all replicas
     uint32_t color_stride;          // capacity of one colour's list
 };
 // The round argument of a batch pass that reads its colour set from Batch::round_dev (the passes
@@ -384,7 +399,7 @@ struct BatchSweepTotals {
     unsigned long long ambiguous;
     unsigned long long max_err_bits;
     unsigned long long sweeps;
-    unsigned long long colour_sets;  // the colour sets (rounds) run, summed over the sweeps
+    unsigned long long set_launches;  // passes of the rounds loop's body, summed over the sweeps
     unsigned int error_flags;
     unsigned int pad;
 };
@@ -408,33 +423,33 @@ cudaError_t launch_batch_origins(int dim, const Batch& b, Replica* rep, cudaStre
 cudaError_t launch_batch_round_first(cudaGraphConditionalHandle h, const DeviceStats* stats, uint32_t* round_dev,
                                      const BatchSweepTotals* totals, cudaStream_t s);
 cudaError_t launch_batch_round_next(cudaGraphConditionalHandle h, const DeviceStats* stats, uint32_t* round_dev,
-                                    cudaStream_t s);
+                                    uint32_t step, cudaStream_t s);
 cudaError_t launch_batch_sweep_end(const Batch& b, Replica* rep, const DeviceStats* stats,
                                    unsigned long long* rep_counts, BatchSweepTotals* totals, bool increment_step,
-                                   cudaStream_t s);
+                                   uint32_t sets, cudaStream_t s);
 // Batches of replicas: the rebuild and the hard-sphere colour pass over all replicas at once.
 cudaError_t launch_rebuild_batch(int dim, const Batch& b, const Arrays& a, uint32_t n, bool write_s, cudaStream_t s);
 cudaError_t launch_sweep_batch(int dim, bool fp32, const Batch& b, const Arrays& a, uint32_t color, uint32_t round,
                                uint32_t max_active, bool overlap_previous, bool early_wait, cudaStream_t s,
                                uint32_t variant = 0);
 cudaError_t launch_overlap_batch(int dim, const Batch& b, const Arrays& a, uint32_t n, cudaStream_t s);
-// Batches of Lennard-Jones replicas: one warp per trial over every replica's colour list (hmc_lj.cu).
-cudaError_t launch_sweep_batch_lj(int dim, bool fp32, const Batch& b, const Arrays& a, uint32_t color, uint32_t round,
-                                  uint32_t max_active, bool overlap_previous, bool early_wait, cudaStream_t s,
-                                  uint32_t variant = 0);
+// Batches of Lennard-Jones replicas (hmc_lj.cu): the colour sets [round, round_end) of every replica
+// (round = kRoundFromDevice: round_end sets from Batch::round_dev), two kernels: the trials' random
+// draws, then the trials in dataflow order.
+cudaError_t launch_flow_batch_lj(int dim, bool fp32, const Batch& b, const Arrays& a, uint32_t round,
+                                 uint32_t round_end, cudaStream_t s, uint32_t variant = 0);
 // coop selects the warp-cooperative pass (the per-lane pass otherwise).
 cudaError_t launch_sweep_sphere(int dim, bool fp32, const Geometry& g, const Arrays& a, const Pair& p,
                                 const Launch& l, bool coop, cudaStream_t s, uint32_t variant = 0);
 cudaError_t launch_overlap_sphere(int dim, const Geometry& g, const Arrays& a, const Pair& p, uint32_t n,
                                   cudaStream_t s);
 // generic: the system's energy is not Shifted Lennard-Jones (the overlap penalty, Isotropic).
-cudaError_t launch_sweep_lj(int dim, bool fp32, bool generic, const Geometry& g, const Arrays& a, const Pair& p,
-                            const Launch& l,
-                            cudaStream_t s, uint32_t variant = 0);
+// The colour sets [l.round, l.round_end), two kernels as in launch_flow_batch_lj.
+cudaError_t launch_flow_lj(int dim, bool fp32, bool generic, const Geometry& g, const Arrays& a, const Pair& p,
+                           const Launch& l, cudaStream_t s, uint32_t variant = 0);
 // The trial moves of round l.round for every colour list at once (Arrays::trial_*), one thread
 // per trial; launched in stream order before the round's colour passes of the passes that give a
-// trial several lanes (LJ and the overlap penalty, convex polyhedra, convex polygons).
-cudaError_t launch_propose_lj(int dim, bool fp32, const Geometry& g, const Arrays& a, const Launch& l, cudaStream_t s);
+// trial several lanes (convex polyhedra, convex polygons).
 // soft: the trial also draws the Metropolis uniform after the move (trial_t.w in 3-D, .z in 2-D).
 cudaError_t launch_propose_poly(bool fp32, const Geometry& g, const Arrays& a, const Launch& l, bool rotate,
                                 bool soft, cudaStream_t s);

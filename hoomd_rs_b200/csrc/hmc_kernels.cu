@@ -772,16 +772,77 @@ __device__ __forceinline__ uint32_t color_of(const uint32_t* m) {
 }
 
 
+// The colours of a thread's kScanItems consecutive spaces from space c, walked along the fast axis.
+template <int DIM>
+struct ColourWalk {
+    uint32_t m[3] = {0, 0, 0};
+    __device__ __forceinline__ ColourWalk(const Geometry& g, uint32_t c) {
+#pragma unroll
+        for (int a = DIM - 1; a >= 0; --a) {
+            m[a] = c % g.shape[a];
+            c /= g.shape[a];
+        }
+    }
+    __device__ __forceinline__ uint32_t color() const { return color_of<DIM>(m); }
+    __device__ __forceinline__ void next(const Geometry& g) {
+#pragma unroll
+        for (int a = DIM - 1; a >= 0; --a) {
+            if (++m[a] < g.shape[a]) return;
+            m[a] = 0;
+        }
+    }
+};
+// Eight 16-bit counters (a tile has 2048 spaces), one per colour.
+struct ColourCounts {
+    uint64_t lo = 0, hi = 0;
+    __device__ __forceinline__ void add(uint32_t color) {
+        if (color < 4)
+            lo += 1ull << (16u * color);
+        else
+            hi += 1ull << (16u * (color - 4u));
+    }
+    __device__ __forceinline__ uint32_t get(uint32_t color) const {
+        return (uint32_t)((color < 4 ? lo >> (16u * color) : hi >> (16u * (color - 4u))) & 0xffffu);
+    }
+};
+
 // Exclusive scan of the space counts into cell_start: per-block totals, then each block's scan
 // offset by the sum of the totals before it.
+// LISTS = DIM: the two kernels also write the colour lists, sorted by space (block totals per
+// colour, then each block's places), for sweeps in dataflow order, whose trials find the spaces
+// around theirs finished when neighbours are started close together (flow_rotated). LISTS = 0: k_cells
+// appends them in the order its blocks run.
+template <int LISTS>
 __global__ void __launch_bounds__(kScanThreads) k_count_reduce(const uint32_t* __restrict__ count, uint32_t n_cells,
-                                                               uint32_t* block_sums) {
+                                                               uint32_t* block_sums, Geometry g) {
     grid_dependency_wait();  // rebuild kernels run back to back: the previous one has ended here
     allow_dependent_launch();
     const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     uint32_t sum = 0;
+    if constexpr (LISTS > 0) {
+        __shared__ uint32_t s_color[8];
+        if (threadIdx.x < 8) s_color[threadIdx.x] = 0;
+        __syncthreads();
+        ColourWalk<LISTS> walk(g, base);
+        ColourCounts cc;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) sum += base + k < n_cells ? count[base + k] : 0u;
+        for (int k = 0; k < kScanItems; ++k) {
+            const uint32_t v = base + k < n_cells ? count[base + k] : 0u;
+            sum += v;
+            if (v) cc.add(walk.color());
+            walk.next(g);
+        }
+#pragma unroll
+        for (uint32_t c = 0; c < 1u << LISTS; ++c) {
+            const uint32_t t = __reduce_add_sync(0xffffffffu, cc.get(c));
+            if ((threadIdx.x & 31) == 0 && t) atomicAdd(&s_color[c], t);
+        }
+        __syncthreads();
+        if (threadIdx.x < 8) block_sums[gridDim.x + blockIdx.x * 8u + threadIdx.x] = s_color[threadIdx.x];
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) sum += base + k < n_cells ? count[base + k] : 0u;
+    }
     sum = __reduce_add_sync(0xffffffffu, sum);
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = sum;
@@ -838,9 +899,11 @@ __global__ void __launch_bounds__(1024) k_scan_block_sums(uint32_t* block_sums, 
     }
 }
 
+template <int LISTS>
 __global__ void __launch_bounds__(kScanThreads) k_count_apply(const uint32_t* __restrict__ count, uint32_t n_cells,
                                                               const uint32_t* __restrict__ block_sums,
-                                                              uint32_t* cell_start, uint32_t scanned) {
+                                                              uint32_t* cell_start, uint32_t scanned, Geometry g,
+                                                              Arrays A) {
     grid_dependency_wait();  // rebuild kernels run back to back: the previous one has ended here
     allow_dependent_launch();
     const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
@@ -875,6 +938,45 @@ __global__ void __launch_bounds__(kScanThreads) k_count_apply(const uint32_t* __
         run += v[k];
         if (c + 1 == n_cells) cell_start[n_cells] = run;
     }
+    if constexpr (LISTS > 0) {
+        // the earlier blocks' spaces per colour, then this thread's place in the block
+        __shared__ uint32_t s_color[8];
+        if (threadIdx.x < 8) s_color[threadIdx.x] = 0;
+        __syncthreads();
+        uint32_t before = 0;  // colour threadIdx.x & 7
+        for (uint32_t i = threadIdx.x; i < blockIdx.x * 8u; i += kScanThreads) before += block_sums[gridDim.x + i];
+        if (before) atomicAdd(&s_color[threadIdx.x & 7u], before);
+        ColourCounts cc;
+        const ColourWalk<LISTS> start(g, base);
+        ColourWalk<LISTS> walk = start;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            if (v[k]) cc.add(walk.color());
+            walk.next(g);
+        }
+        ColourCounts all;
+        cc.lo = block_exclusive_scan(cc.lo, &all.lo);
+        cc.hi = LISTS == 3 ? block_exclusive_scan(cc.hi, &all.hi) : 0ull;
+        __syncthreads();
+        walk = start;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            const uint32_t c = base + k;
+            if (v[k]) {
+                const uint32_t color = walk.color();
+                A.color_cells[(size_t)color * g.color_stride + s_color[color] + cc.get(color)] = pack_m<LISTS>(walk.m);
+                cc.add(color);
+            } else if (c < n_cells) {
+                A.progress[c] = 0xffffffffu;  // nothing waits for an empty space
+            }
+            walk.next(g);
+        }
+        if (blockIdx.x + 1 == gridDim.x && threadIdx.x < 8) {
+            const uint32_t total_c = s_color[threadIdx.x] + all.get(threadIdx.x);
+            A.stats->color_count[threadIdx.x] = total_c;
+            if (total_c) atomicAdd(&A.stats->nonempty, total_c);
+        }
+    }
 }
 
 // Colour-list positions for one block: each lane with an entry gets a slot in its colour's
@@ -908,10 +1010,10 @@ __device__ __forceinline__ uint32_t append_by_color(DeviceStats* stats, bool has
 constexpr int kCellThreads = 512;  // 1024: 71.7 us per 2^20-sphere rebuild, 512: 70.7 us
 
 // Per space: order its bodies by index (the order update_checkerboard pushes them,
-// parallel_sweep.rs:194-200, which IndexedRandom::choose indexes), and list it under its
+// parallel_sweep.rs:194-200, which IndexedRandom::choose indexes), and (lists) list it under its
 // colour when it is not empty.
 template <int DIM>
-__global__ void __launch_bounds__(kCellThreads) k_cells(Geometry g, Arrays A) {
+__global__ void __launch_bounds__(kCellThreads) k_cells(Geometry g, Arrays A, uint32_t lists) {
     grid_dependency_wait();  // rebuild kernels run back to back: the previous one has ended here
     allow_dependent_launch();
     __shared__ uint32_t s_count[8], s_base[8], s_nonempty;
@@ -930,7 +1032,10 @@ __global__ void __launch_bounds__(kCellThreads) k_cells(Geometry g, Arrays A) {
             A.sorted_body[j] = v;
         }
     }
+    if (!lists) return;  // block-uniform: the count scan wrote the colour lists
     const bool has = e > s;
+    // dataflow launches: nothing waits for an empty space (the others start with the draws)
+    if (A.progress && !has && c < g.n_cells) A.progress[c] = 0xffffffffu;
     uint32_t packed = 0, col = 0;
     if (has) {
         uint32_t m[3] = {0, 0, 0};
@@ -977,7 +1082,7 @@ __global__ void k_gather(Geometry g, Arrays A, uint32_t n) {
     if (WRITE_S) A.sorted_s[k] = make_double4(sv[0], sv[1], sv[2], 0.0);
     uint32_t m[3] = {0, 0, 0};
     unpack_m<DIM>(A.body_m[i], m);
-    A.sorted_off[k] = cell_offsets<DIM>(g, sv, m);
+    A.sorted_off[k] = site32<DIM>(g, A, sv, m);
     if (A.sorted_q) A.sorted_q[k] = A.body_ori[i];
 }
 
@@ -1200,6 +1305,7 @@ __global__ void __launch_bounds__(kCellThreads) k_cells_batch(Batch B, Arrays A)
         }
     }
     const bool has = e > s;
+    if (A.progress && !has && c < B.n_cells) A.progress[c] = 0xffffffffu;
     uint32_t packed = 0, col = 0, r = 0xffffffffu;
     if (has) {
         const uint32_t first = A.sorted_body[s];
@@ -1247,7 +1353,7 @@ __global__ void k_gather_batch(Batch B, Arrays A, uint32_t n) {
     if (WRITE_S) A.sorted_s[k] = make_double4(sv[0], sv[1], sv[2], 0.0);
     uint32_t m[3] = {0, 0, 0};
     unpack_m<DIM>(A.body_m[i], m);
-    A.sorted_off[k] = cell_offsets<DIM>(g, sv, m);
+    A.sorted_off[k] = site32<DIM>(g, A, sv, m);
 }
 
 // Accepted moves per replica from one warp: the lanes of each replica in the warp add up.
@@ -1365,10 +1471,12 @@ __global__ void k_batch_round_first(cudaGraphConditionalHandle h, const DeviceSt
 }
 
 // The end of one colour set of a captured sweep: the next runs while the sweep has rounds left.
-__global__ void k_batch_round_next(cudaGraphConditionalHandle h, const DeviceStats* stats, uint32_t* round_dev) {
-    const uint32_t next = *round_dev + 1u;
+// (step: the colour sets the body runs)
+__global__ void k_batch_round_next(cudaGraphConditionalHandle h, const DeviceStats* stats, uint32_t* round_dev,
+                                   uint32_t step) {
+    const uint32_t next = *round_dev + step;
     *round_dev = next;
-    cudaGraphSetConditional(h, next < stats->rounds);
+    cudaGraphSetConditional(h, next < stats->rounds && stats->error_flags == 0u);
 }
 
 // The host's bookkeeping after a batch sweep, on the device: per replica its trials
@@ -1377,7 +1485,7 @@ __global__ void k_batch_round_next(cudaGraphConditionalHandle h, const DeviceSta
 // A sweep whose rebuild flagged an error (or that follows one) ran no pass and changes nothing
 // but the flags.
 __global__ void k_batch_sweep_end(Batch B, Replica* rep, const DeviceStats* stats, unsigned long long* rep_counts,
-                                  BatchSweepTotals* totals, uint32_t increment_step) {
+                                  BatchSweepTotals* totals, uint32_t increment_step, uint32_t sets) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     // (thread 0 adds only this sweep's flags, which every thread reads itself)
     const bool failed = stats->error_flags != 0u || totals->error_flags != 0u;
@@ -1389,7 +1497,7 @@ __global__ void k_batch_sweep_end(Batch B, Replica* rep, const DeviceStats* stat
             totals->ambiguous += stats->ambiguous;
             if (stats->max_err_bits > totals->max_err_bits) totals->max_err_bits = stats->max_err_bits;
             totals->sweeps += 1;
-            totals->colour_sets += stats->rounds;
+            totals->set_launches += (stats->rounds + sets - 1) / sets;
         }
     }
     if (failed || r >= B.n_replicas) return;
@@ -1652,15 +1760,20 @@ cudaError_t launch_chained(void (*kernel)(K...), uint32_t grid, uint32_t block, 
     return cudaLaunchKernelEx(&pl.cfg, kernel, args...);
 }
 
-cudaError_t launch_count_scan(const Arrays& a, uint32_t n_cells, cudaStream_t s, bool chained = true) {
+// lists: 0, or the dimension where the scan also writes the colour lists (at most kScanDirectBlocks
+// blocks).
+cudaError_t launch_count_scan(const Arrays& a, uint32_t n_cells, cudaStream_t s, bool chained = true, int lists = 0,
+                              const Geometry& g = Geometry{}) {
     const uint32_t nb = blocks_for(n_cells, kScanTile);
-    cudaError_t e = launch_chained(k_count_reduce, nb, kScanThreads, chained, s, (const uint32_t*)a.cell_count,
-                                   n_cells, a.block_sums);
+    cudaError_t e = launch_chained(lists == 0 ? k_count_reduce<0> : (lists == 2 ? k_count_reduce<2> : k_count_reduce<3>),
+                                   nb, kScanThreads, chained, s, (const uint32_t*)a.cell_count, n_cells, a.block_sums,
+                                   g);
     const uint32_t scanned = nb > kScanDirectBlocks ? 1u : 0u;
     if (e == cudaSuccess && scanned) e = launch_chained(k_scan_block_sums, 1, 1024, true, s, a.block_sums, nb);
     if (e == cudaSuccess)
-        e = launch_chained(k_count_apply, nb, kScanThreads, true, s, (const uint32_t*)a.cell_count, n_cells,
-                           (const uint32_t*)a.block_sums, a.cell_start, scanned);
+        e = launch_chained(lists == 0 ? k_count_apply<0> : (lists == 2 ? k_count_apply<2> : k_count_apply<3>), nb,
+                           kScanThreads, true, s, (const uint32_t*)a.cell_count, n_cells, (const uint32_t*)a.block_sums,
+                           a.cell_start, scanned, g, a);
     return e;
 }
 }  // namespace
@@ -1681,17 +1794,21 @@ cudaError_t launch_rebuild(int dim, const Geometry& g, const Arrays& a, uint32_t
         else
             k_bin<3><<<blocks_for(n, kBodyThreads), kBodyThreads, 0, s>>>(g, a, n);
     }
-    if ((e = launch_count_scan(a, g.n_cells, s, n > 0)) != cudaSuccess) return e;
+    // sorted colour lists for sweeps in dataflow order; beyond kScanDirectBlocks blocks the lists'
+    // order of arrival is close enough to sorted (few of their blocks run at a time)
+    const bool sorted = a.progress && blocks_for(g.n_cells, kScanTile) <= kScanDirectBlocks;
+    const uint32_t lists = sorted ? 0u : 1u;
+    if ((e = launch_count_scan(a, g.n_cells, s, n > 0, sorted ? dim : 0, g)) != cudaSuccess) return e;
     if (n == 0) return cudaSuccess;
     if ((e = launch_chained(k_scatter, blocks_for(n, kBodyThreads), kBodyThreads, true, s, a, n)) != cudaSuccess) return e;
     const uint32_t cb = blocks_for(g.n_cells, kCellThreads), gb = blocks_for(n, kBodyThreads);
     if (dim == 2) {
-        if ((e = launch_chained(k_cells<2>, cb, kCellThreads, true, s, g, a)) != cudaSuccess) return e;
+        if ((e = launch_chained(k_cells<2>, cb, kCellThreads, true, s, g, a, lists)) != cudaSuccess) return e;
         return launch_chained(write_slots ? (write_s ? k_gather<2, true, true> : k_gather<2, false, true>)
                                           : (write_s ? k_gather<2, true, false> : k_gather<2, false, false>),
                               gb, kBodyThreads, true, s, g, a, n);
     }
-    if ((e = launch_chained(k_cells<3>, cb, kCellThreads, true, s, g, a)) != cudaSuccess) return e;
+    if ((e = launch_chained(k_cells<3>, cb, kCellThreads, true, s, g, a, lists)) != cudaSuccess) return e;
     return launch_chained(write_slots ? (write_s ? k_gather<3, true, true> : k_gather<3, false, true>)
                                       : (write_s ? k_gather<3, true, false> : k_gather<3, false, false>),
                           gb, kBodyThreads, true, s, g, a, n);
@@ -1774,16 +1891,16 @@ cudaError_t launch_batch_round_first(cudaGraphConditionalHandle h, const DeviceS
 }
 
 cudaError_t launch_batch_round_next(cudaGraphConditionalHandle h, const DeviceStats* stats, uint32_t* round_dev,
-                                    cudaStream_t s) {
-    k_batch_round_next<<<1, 1, 0, s>>>(h, stats, round_dev);
+                                    uint32_t step, cudaStream_t s) {
+    k_batch_round_next<<<1, 1, 0, s>>>(h, stats, round_dev, step);
     return cudaGetLastError();
 }
 
 cudaError_t launch_batch_sweep_end(const Batch& b, Replica* rep, const DeviceStats* stats,
                                    unsigned long long* rep_counts, BatchSweepTotals* totals, bool increment_step,
-                                   cudaStream_t s) {
+                                   uint32_t sets, cudaStream_t s) {
     k_batch_sweep_end<<<blocks_for(b.n_replicas, 128), 128, 0, s>>>(b, rep, stats, rep_counts, totals,
-                                                                      increment_step ? 1u : 0u);
+                                                                      increment_step ? 1u : 0u, sets);
     return cudaGetLastError();
 }
 
@@ -1831,7 +1948,7 @@ SphereKernel coop_kernel(int dim, bool fp32, uint32_t v) {
 
 }  // namespace
 
-int resident_wave(const void* kernel) {
+int resident_wave(const void* kernel, int threads) {
     static std::mutex mu;
     static std::unordered_map<const void*, int> cache;
     int dev = 0;
@@ -1842,7 +1959,7 @@ int resident_wave(const void* kernel) {
     if (it != cache.end()) return it->second;
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess) {
         cudaGetLastError();
         per_sm = 1;
     }

@@ -1,44 +1,40 @@
-// Lennard-Jones Metropolis sweep: PairwiseCutoff<Isotropic<Shifted<LennardJones>>>.
+// Lennard-Jones Metropolis sweep: PairwiseCutoff<Isotropic<Shifted<LennardJones>>> (and the overlap
+// penalty and the other isotropic potentials, in FP64).
 //
 // delta_energy_one (hoomd-interaction/src/pairwise_cutoff.rs:919-941) sums the pair energy of
 // the trial site and of the current site over every other site within r_cut; the Metropolis
 // test (hoomd-mc/src/parallel_sweep.rs:267-268) accepts when dH <= 0, else draws u and accepts
 // when u < exp(-dH / kT). At rho = 0.8 with r_cut = 2.5 a space holds ~13 bodies, so a colour
-// pass has few trials (~5k for 2^19 bodies) with ~340 candidates each: one warp per trial,
-// which takes the candidates of all stencil rows 32 at a time (FlatStencil: ~11 steps instead
-// of two per row), and warp reductions of the sums.
+// pass has few trials (~5k for 2^19 bodies) with ~340 candidates each, and a sweep 112 passes. All of
+// them run in one launch in dataflow order (hmc_flow.cuh): a trial's latency then no longer adds
+// up to a pass's, and the launches are gone.
 //
-// FP32 + recheck: the warp sums FP32 pair energies together with a rigorous bound B on
-// |dU32 - dU64| (r^2 error from the FP32 offsets, propagated through dE/dr^2; rounding of the
-// energy formula; summation chains; the FP64 sum's own error). A decision that B cannot
-// change is taken from the FP32 sums; otherwise the warp recomputes dU in FP64 with exactly
-// the lane assignment and reduction order of the plain FP64 pass, so decisions equal it.
+// FP32 + recheck: FP32 pair energies together with a rigorous bound B on |dU32 - dU64| (r^2 error
+// from the fixed-point sites, propagated through dE/dr^2; rounding of the energy formula;
+// summation chains; the FP64 sum's own error). A decision that B cannot change is taken from the
+// FP32 sums; otherwise the warp recomputes dU in FP64. Any FP64 sum that another order could
+// decide differently is counted (order_ambiguous), so decisions equal the FP64 pass.
+//
+// Bound: the dependent chain of a trial (L2 latency of the staging copies, the acquire and release
+// of the progress words, FP64 wraps) and issue slots; DRAM is idle (the state stays in L2).
+// Measured, ten sweeps with the frame's copy: 2^19 sites FP32 29.3 -> 14.0 ms, 20,011 sites FP64
+// 18.3 -> 7.8 ms, 64 replicas of 8,192 FP32 43.7 -> 21.8 ms, against one launch per colour pass
+// with a warp per trial.
 #include <cuda_runtime.h>
 
-#include "hmc_device.cuh"
+#include <type_traits>
+
+#include "hmc_flow.cuh"
 
 namespace hmc {
 namespace {
-
-// Resident blocks per SM the sweep pass is compiled for: 9 caps it at 56 registers, so that a
-// colour pass of the 2^19-body LJ system (4,913 trials of one warp) runs in one wave; measured
-// 1.32e8 (FP32) and 1.83e8 (FP64) trial moves/s there, against 1.01e8 and 1.24e8 uncapped.
-#ifndef HMC_LJ_MIN_BLOCKS
-#define HMC_LJ_MIN_BLOCKS 9
-#endif
-// The same for the batch passes: 7 (72 registers) still runs a colour pass of 64 replicas of
-// 8192 bodies (4,096 trials) in one wave and spills less: 1.34e8 (FP32) and 1.15e8 (FP64)
-// trial moves/s there, against 1.18e8 and 1.07e8 at 56 registers and 1.01e8 and 7.1e7 at 80.
-#ifndef HMC_LJ_BATCH_MIN_BLOCKS
-#define HMC_LJ_BATCH_MIN_BLOCKS 7
-#endif
 
 constexpr float kU32 = 5.9604645e-8f;  // 2^-24
 
 // FP32 pair energy and a bound on its error against the exact energy of the FP64 sites, for
 // a pair with r2 below the band's upper end (the caller skips pairs outside the cut-off).
 // The r^2 error is bounded without a square root: sum |d_a| <= sqrt(3) r and
-// r <= (r^2 + 1) / 2, so |r2_32 - r2| <= 3.5 E ((r^2 + 1)/2 + E) + 3.1 u32 r^2.
+// r <= (r^2 + 1) / 2, so |r2_32 - r2| <= 3.5 E ((r^2 + 1)/2 + E) + lj_rel_err r^2 (lj_setup_for).
 __device__ __forceinline__ void lj_pair32(const Pair& P, float r2, float& e, float& err) {
     if (r2 >= P.lj_rcut2_lo32) {  // the FP64 pass may or may not count this pair
         e = 0.f;
@@ -46,7 +42,7 @@ __device__ __forceinline__ void lj_pair32(const Pair& P, float r2, float& e, flo
         return;
     }
     const float E = P.lj_disp_err;
-    const float dr2 = 3.5f * E * (0.5f * (r2 + 1.f) + E) + 3.1f * kU32 * r2;
+    const float dr2 = 3.5f * E * (0.5f * (r2 + 1.f) + E) + P.lj_rel_err * r2;
     const float inv = __frcp_rn(r2);
     const float sr2 = P.lj_sigma2_32 * inv;
     const float sr6 = sr2 * sr2 * sr2;
@@ -54,8 +50,8 @@ __device__ __forceinline__ void lj_pair32(const Pair& P, float r2, float& e, flo
     const float a = b * sr6;                // 4 eps (sigma/r)^12
     e = (a - b) - P.lj_e_shift32;
     // |dE/dr^2| <= (6a + 3b) / r^2; 1.1 covers its variation over [r2 - dr2, r2 + dr2] and the
-    // FP32 evaluation of this bound; 24 u32 covers the roundings of the energy formula.
-    err = 1.1f * ((6.f * a + 3.f * b) * (dr2 * inv) + 24.f * kU32 * (a + b + fabsf(P.lj_e_shift32)));
+    // FP32 evaluation of this bound; 25 u32 covers the roundings of the energy formula and of 4 eps.
+    err = 1.1f * ((6.f * a + 3.f * b) * (dr2 * inv) + 25.f * kU32 * (a + b + fabsf(P.lj_e_shift32)));
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -74,111 +70,60 @@ __device__ __forceinline__ uint32_t warp_maxu(uint32_t v) {
     return v;
 }
 
-// FP64 energy of site ta (and, when TWO, of site tb in the same space) against the stencil
-// fs, skipping slot self: the warp takes the stencil's candidates 32 at a time, each lane sums
-// its own in that order, then a butterfly reduction (every lane ends with the same values).
-// S of a candidate comes from sorted_s when have_s, else from wrap(sorted_b). The two sums of
-// one call equal two calls of one sum each over the same stencil.
-// mag receives sum |e| over both sums (for order_ambiguous).
-// U: candidates a lane loads per step (U = 2 keeps two loads in flight); a lane still adds its
-// terms in increasing candidate order, so the sums are the same bits for every U.
-template <int DIM, bool TWO, bool GENERIC = true, int U = 1>
+// FP64 energy of site ta against the stencil fs, skipping slot self: the warp takes the stencil's
+// candidates 32 at a time, each lane sums its own in that order, then a butterfly reduction (every
+// lane ends with the same values). mag receives sum |e| (for order_ambiguous). For injected moves
+// and the tuner, whose sites may lie in different spaces.
+template <int DIM>
 __device__ __forceinline__ void lj_energy64(const Geometry& g, const Arrays& A, const Pair& P, const double* ta,
-                                            const double* tb, const FlatStencil& fs, uint32_t self, bool have_s,
-                                            uint32_t lane, double& ea, double& eb, double& mag) {
-    double a = 0.0, b = 0.0, am = 0.0;
+                                            const FlatStencil& fs, uint32_t self, uint32_t lane, double& ea,
+                                            double& mag) {
+    double a = 0.0, am = 0.0;
 #pragma unroll 1
-    for (uint32_t j0 = 0; j0 < fs.total; j0 += 32u * U) {
-        double4 v[U];
-        bool ok[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint32_t j = j0 + 32u * u + lane;
-            uint32_t part;
-            const uint32_t q = flat_slot(fs, j, part);
-            ok[u] = j < fs.total && q != self;
-            v[u] = ok[u] ? ldg4((have_s ? A.sorted_s : A.sorted_b) + q) : make_double4(0.0, 0.0, 0.0, 0.0);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (!ok[u]) continue;
-            double sv[3] = {v[u].x, v[u].y, v[u].z};
-            if (!have_s) wrap_inv<DIM>(g.L, g.invL, sv);
-            const double ra = ref_dist2<DIM>(g, ta, sv);
-            const double x = soft_pair64<GENERIC>(P, ra);
-            a = dadd(a, x);
-            am += GENERIC ? soft_pair_mag(P, ra, x) : fabs(x);
-            if (TWO) {
-                const double rb = ref_dist2<DIM>(g, tb, sv);
-                const double y = soft_pair64<GENERIC>(P, rb);
-                b = dadd(b, y);
-                am += GENERIC ? soft_pair_mag(P, rb, y) : fabs(y);
-            }
-        }
+    for (uint32_t j0 = 0; j0 < fs.total; j0 += 32u) {
+        const uint32_t j = j0 + lane;
+        uint32_t part;
+        const uint32_t q = flat_slot(fs, j, part);
+        if (j >= fs.total || q == self) continue;
+        const double4 v = ldg4(A.sorted_s + q);
+        const double sv[3] = {v.x, v.y, v.z};
+        const double ra = ref_dist2<DIM>(g, ta, sv);
+        const double x = soft_pair64<true>(P, ra);
+        a = dadd(a, x);
+        am += soft_pair_mag(P, ra, x);
     }
     ea = warp_sum(a);
-    eb = TWO ? warp_sum(b) : 0.0;
     mag = warp_sum(am);
 }
 
 struct Sums32 {
     float e_new, e_old, err, mag;
-    uint32_t terms, pairs;
+    uint32_t terms;
 };
 
-// FP32 energies of the trial site (offsets t32) and the current site (offsets c32) against
-// the stencil fs of their common space, with error bounds. Each lane takes U candidates per
-// step (loads issued together); the order of a lane's terms does not enter the bound.
-template <int DIM, int U = 1>
-__device__ __forceinline__ Sums32 lj_energy32(const Geometry& g, const Arrays& A, const Pair& P, float4 t32,
-                                               float4 c32, int mf, const FlatStencil& fs, uint32_t self,
-                                               uint32_t lane) {
-    Sums32 s{0.f, 0.f, 0.f, 0.f, 0u, 0u};
-    const uint32_t sf = g.shape[DIM - 1];
+// FP32 energies of the trial site t32 and the current site c32 (fixed_site) against the stencil fs
+// of their common space, with error bounds (hmc_eval_moves).
+template <int DIM>
+__device__ __forceinline__ Sums32 lj_energy32(const Arrays& A, const Pair& P, const int4& t32, const int4& c32,
+                                               const FlatStencil& fs, uint32_t self, uint32_t lane) {
+    Sums32 s{0.f, 0.f, 0.f, 0.f, 0u};
 #pragma unroll 1
-    for (uint32_t j0 = 0; j0 < fs.total; j0 += 32u * U) {
-        float4 o[U];
-        float s0[U], s1[U];
-        bool ok[U];
+    for (uint32_t j0 = 0; j0 < fs.total; j0 += 32u) {
+        const uint32_t j = j0 + lane;
+        uint32_t part;
+        const uint32_t q = flat_slot(fs, j, part);
+        if (j >= fs.total || q == self) continue;
+        const int4 o = __ldg(reinterpret_cast<const int4*>(A.sorted_off) + q);
+        const float r2[2] = {fixed_dist2<DIM>(P, t32, o), fixed_dist2<DIM>(P, c32, o)};
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint32_t j = j0 + 32u * u + lane;
-            uint32_t part;
-            const uint32_t q = flat_slot(fs, j, part);
-            s0[u] = __shfl_sync(0xffffffffu, fs.s0, part);
-            s1[u] = __shfl_sync(0xffffffffu, fs.s1, part);
-            ok[u] = j < fs.total && q != self;
-            o[u] = ok[u] ? __ldg(A.sorted_off + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (!ok[u]) continue;
-            int dm = __float_as_int(o[u].w) - mf;
-            if (sf >= 4) {
-                if (dm > 1)
-                    dm -= (int)sf;
-                else if (dm < -1)
-                    dm += (int)sf;
-            }
-            const float r2n = fp32_dist2<DIM>(g, t32, o[u], s0[u], s1[u], dm);
-            const float r2o = fp32_dist2<DIM>(g, c32, o[u], s0[u], s1[u], dm);
-            s.pairs += 2;
-            if (r2n < P.lj_rcut2_hi32) {
-                float e, err;
-                lj_pair32(P, r2n, e, err);
-                s.e_new += e;
-                s.err += err;
-                s.mag += fabsf(e);
-                s.terms += 1;
-            }
-            if (r2o < P.lj_rcut2_hi32) {
-                float e, err;
-                lj_pair32(P, r2o, e, err);
-                s.e_old += e;
-                s.err += err;
-                s.mag += fabsf(e);
-                s.terms += 1;
-            }
+        for (int i = 0; i < 2; ++i) {
+            if (!(r2[i] < P.lj_rcut2_hi32)) continue;
+            float e, err;
+            lj_pair32(P, r2[i], e, err);
+            (i == 0 ? s.e_new : s.e_old) += e;
+            s.err += err;
+            s.mag += fabsf(e);
+            s.terms += 1;
         }
     }
     s.e_new = warp_sumf(s.e_new);
@@ -189,557 +134,568 @@ __device__ __forceinline__ Sums32 lj_energy32(const Geometry& g, const Arrays& A
     return s;
 }
 
-// Metropolis decision from the FP32 sums: 1 accept, 0 reject, -1 needs the FP64 sums. u is the
-// uniform the reference draws only when dU > 0 (parallel_sweep.rs:267-268): the next value of
-// the trial's stream, which nothing else draws from, so the kernel draws it up front.
-__device__ __forceinline__ int decide32(const Sums32& s, double kt, double u) {
-    const float d32 = s.e_new - s.e_old;
-    // summation chains (per lane + 5 reduction levels + the final difference), FP64's own error
-    const float b = s.err + (float)(s.terms + 7) * kU32 * s.mag * 1.01f + kU32 * fabsf(d32) + 1e-9f * (s.mag + 1.f);
-    if (!isfinite(d32) || !isfinite(b)) return -1;
-    const double lo = (double)d32 - (double)b, hi = (double)d32 + (double)b;
-    if (hi <= 0.0) return 1;  // dU64 <= 0 for certain: accepted without a uniform
-    if (lo <= 0.0) return -1;
-    const double t_hi = exp(-lo / kt) * (1.0 + 1e-12);  // dU64 > 0 for certain
-    const double t_lo = exp(-hi / kt) * (1.0 - 1e-12);
-    if (u < t_lo) return 1;
-    if (u >= t_hi) return 0;
-    return -1;
+// ---- the sweep --------------------------------------------------------------------------------
+// What the random streams of the trials of colour sets [L.round, L.round_end) give, one thread per
+// trial (generate_trial_moves, parallel_sweep.rs:231-278): the body (IndexedRandom::choose), the
+// displacement (Ball::sample) and the Metropolis uniform, from Counter(step, substep + set,
+// seed).index(space). None of it depends on a site, so it is computed for all of a launch's trials
+// at once with every lane busy, and k_flow_lj, which gives a trial a warp, does not repeat it in
+// 32 lanes. The FP32 pass also gets -kT ln u as a pair of FP32 bounds (metropolis_bounds), which
+// spares its decision two exponentials.
+// Each space's progress is set to the first colour set; the ticket starts at 0.
+struct DrawRecord {
+    uint32_t k;      // the chosen body's slot; kNoTrial: the replica runs no such colour set
+    uint32_t m;      // packed multi-index of the space
+    float w_lo, w_hi;
+};
+
+// Bounds around w = -kT ln u, the energy below which u < exp(-dU / kT): dU < w_lo accepts and
+// dU > w_hi rejects for certain. The exponent's slack of 1e-11 covers the rounding of dU / kT
+// (|dU / kT| <= 37 where u >= 2^-53 decides), of the reference's exp and of log here (each a few
+// ulp). u = 0 is left to the FP64 sums.
+__device__ __forceinline__ void metropolis_bounds(double u, double kt, float& lo, float& hi) {
+    const double x = -log(u);
+    lo = u > 0.0 ? __double2float_rd(kt * (x - 1e-11)) : -INFINITY;
+    hi = u > 0.0 ? __double2float_ru(kt * (x + 1e-11)) : INFINITY;
 }
 
-// The trial moves of one round for all colour lists (generate_trial_moves, parallel_sweep.rs:
-// 231-278, up to the Metropolis test): thread i takes entry i of the colour lists, draws the
-// body (IndexedRandom::choose), the displacement (Ball::sample) and the uniform from
-// Counter(step, substep + round, seed).index(space), wraps (W1) and checks that W1 stays in the
-// space; the passes then give each trial a warp and read the move from here instead of having
-// every lane of the warp compute it. A trial reads only the rebuild's arrays and the bodies of its
-// own colour, which the previous colours of the round do not move.
-template <int DIM, bool FP32>
-__global__ void __launch_bounds__(128) k_propose_lj(Geometry g, Arrays A, Launch L) {
-    const DeviceStats* st = A.stats;
-    if (st->error_flags != 0u || L.round >= st->rounds) return;
-    const uint32_t colors = 1u << DIM;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < colors * g.color_stride;
-         i += gridDim.x * blockDim.x) {
-        const uint32_t c = i / g.color_stride, w = i - c * g.color_stride;
-        if (w >= st->color_count[c]) continue;
+template <int DIM, bool BATCH>
+__global__ void __launch_bounds__(128) k_draw_lj(Geometry g, Arrays A, Launch L, Batch B) {
+    grid_dependency_wait();
+    allow_dependent_launch();
+    if (BATCH && L.round == kRoundFromDevice) {  // a captured sweep's rounds loop
+        L.round = *B.round_dev;
+        L.round_end += L.round;
+    }
+    const FlowRange f = flow_range(A.stats, L.round, L.round_end, 1u << DIM);
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.stats->ticket = 0;
+    const uint32_t stride = BATCH ? B.color_stride : g.color_stride;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += gridDim.x * blockDim.x) {
+        uint32_t round, color, entry;
+        flow_item(f, i, round, color, entry);
+        if (!BATCH) entry = flow_rotated(f, A.stats->color_count[color], round, color, 1u << DIM, g.shape[0], entry);
+        const size_t e = (size_t)color * stride + entry;
+        const uint32_t packed = __ldg(A.color_cells + e);
         uint32_t m[3] = {0, 0, 0};
-        unpack_m<DIM>(__ldg(A.color_cells + i), m);
-        const uint32_t cell = cell_index<DIM>(g, m);
-        const uint32_t start = __ldg(A.cell_start + cell);
-        const uint32_t count = __ldg(A.cell_start + cell + 1) - start;
-        Sfc64 rng = make_rng(L.step, L.substep, L.seed, (uint64_t)cell);
-        const uint32_t k = start + canon_range_u32(rng, count);
-        const double4 b4 = A.sorted_b[k];
-        double x[3] = {b4.x, b4.y, b4.z};
-        double dv[3];
-        ball_sample<DIM>(rng, L.max_move, A.zig_x, A.zig_f, dv);
-        const double u = uniform01(rng);
-#pragma unroll
-        for (int a = 0; a < DIM; ++a) x[a] = dadd(x[a], dv[a]);
-        wrap_inv<DIM>(g.L, g.invL, x);  // W1 = wrap(propose(..))
-        uint32_t mt[3];
-        if (!(point_to_space<DIM>(g, x, mt) && cell_index<DIM>(g, mt) == cell)) {
-            A.trial_k[i] = kNoTrial;  // leaves its space: rejected before delta_energy_one
+        unpack_m<DIM>(packed, m);
+        const Replica* R = BATCH ? B.rep + __ldg(B.color_rep + e) : nullptr;
+        const Geometry& G = BATCH ? R->g : g;
+        const uint32_t cell = cell_index<DIM>(G, m), base = BATCH ? R->cell_base : 0u;
+        if (round == f.r0) A.progress[base + cell] = f.r0;
+        if (BATCH && round >= R->rounds) {
+            A.draw_i[i] = make_uint4(kNoTrial, packed, 0u, 0u);
             continue;
         }
-        double t[3] = {x[0], x[1], DIM == 3 ? x[2] : 0.0};
-        wrap_inv<DIM>(g.L, g.invL, t);  // the trial site T = wrap(W1)
-        A.trial_t[i] = make_double4(t[0], t[1], t[2], u);
-        if (FP32) A.trial_o[i] = cell_offsets<DIM>(g, t, m);
-        A.trial_k[i] = k;
+        const uint32_t start = __ldg(A.cell_start + base + cell);
+        const uint32_t count = __ldg(A.cell_start + base + cell + 1) - start;
+        Sfc64 rng = make_rng(BATCH ? R->step : L.step, (BATCH ? R->substep : L.substep) + round,
+                             BATCH ? R->seed : L.seed, (uint64_t)cell);
+        const uint32_t k = start + canon_range_u32(rng, count);
+        double dv[3];
+        ball_sample<DIM>(rng, BATCH ? R->max_move : L.max_move, A.zig_x, A.zig_f, dv);
+        const double u = uniform01(rng);
+        float lo, hi;
+        metropolis_bounds(u, BATCH ? R->kt : L.kt, lo, hi);
+        A.draw_d[i] = make_double4(dv[0], dv[1], DIM == 3 ? dv[2] : 0.0, u);
+        A.draw_i[i] = make_uint4(k, packed, __float_as_uint(lo), __float_as_uint(hi));
     }
 }
 
-// Injected trial w of the probe mode (Injected) in a warp-per-trial pass: the body's slot and
-// space, W1 and u from the list. The colour pass evaluates only trials that stay in their body's
-// space; the others are rejected as in the sweep (kTrialOutsideSpace).
-template <int DIM>
-__device__ __forceinline__ void lj_inject(const Arrays& A, const Injected& J, uint32_t w, uint32_t* m, uint32_t& k,
-                                          double* x, double& u) {
-    const uint64_t body = J.bodies[w];
-    k = A.slot_of_body[body];
-    unpack_m<DIM>(A.body_m[body], m);
-    const double4 w4 = J.trial[w];
-    x[0] = w4.x;
-    x[1] = w4.y;
-    x[2] = DIM == 3 ? w4.z : 0.0;
-    u = J.u[w];
+// The team of W warps that decides one trial shares this: the non-empty parts of the trial's
+// stencil (stencil_part) as ranges of the candidate number j (slot = base + j for j < end), the
+// staged sites of the candidates (FP32: fixed point), the trial, and per warp the pairs inside the
+// cut-off that wait for their energies and the partial sums. Batches: the trial's replica too, since
+// its fields would else come from L2 after every acquire.
+struct StencilPart {
+    uint32_t base, end;
+};
+constexpr uint32_t kStage = 384;  // candidates staged at a time (a stencil of 2^19 sites at 0.8 holds ~345)
+template <bool FP32, bool BATCH, int W>
+struct alignas(16) Team {
+    using Site = typename std::conditional<FP32, int4, double4>::type;
+    Site site[kStage];
+    union {
+        float2 q32[64];
+        double2 q64[64];
+    } list[W];
+    StencilPart part[18];
+    unsigned long long bar;
+    double sum64[W][3];
+    float2 sum32[W];
+    double t[3], s[3];  // the trial site and (FP64) the current site
+    int4 t32, s32;      // the same in fixed point (FP32)
+    uint32_t n_parts, total, self, valid;
+    typename std::conditional<BATCH, Replica, uint32_t>::type rep;
+};
+
+template <int W>
+__device__ __forceinline__ void team_sync() {
+    if (W == 1)
+        __syncwarp();
+    else
+        __syncthreads();  // a block is one team
 }
 
-// The FP64 pass: one warp per trial. INJ: the probe mode (decisions instead of commits).
-template <int DIM, bool INJ = false, int MINB = HMC_LJ_MIN_BLOCKS, bool GENERIC = true, int U = 1>
-__global__ void __launch_bounds__(128, MINB) k_sweep_lj(Geometry g, Arrays A, Pair P, Launch L, Injected J) {
-    if (L.early_wait) grid_dependency_wait();  // first pass: the rebuild's arrays are read at once
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
-    uint32_t n_accepted = 0;
-    PairStats pst;
-    const uint32_t n_active = INJ ? J.n : active_count(A, L.color, L.round);
-    for (uint32_t w = warp; w < n_active; w += n_warps) {
-        uint32_t m[3] = {0, 0, 0};
-        uint32_t k = 0;
-        double x[3] = {0.0, 0.0, 0.0};
-        double u = 0.0;
-        double t[3] = {0.0, 0.0, 0.0};
-        if constexpr (INJ) {
-            lj_inject<DIM>(A, J, w, m, k, x, u);
-        } else {
-            // the round's trial from k_propose_lj
-            const size_t e = (size_t)L.color * g.color_stride + w;
-            k = __ldg(A.trial_k + e);
-            if (k == kNoTrial) continue;  // warp-uniform: the move left its space
-            unpack_m<DIM>(__ldg(A.color_cells + e), m);
-            const double4 t4 = ldg4(A.trial_t + e);
-            t[0] = t4.x;
-            t[1] = t4.y;
-            t[2] = t4.z;
-            u = t4.w;
+// The stencil around space m into the team's scratch, by one warp, with the candidate number of slot k.
+template <int DIM, typename T>
+__device__ __forceinline__ void team_parts(const Geometry& g, const uint32_t* __restrict__ cs, const uint32_t* m,
+                                           uint32_t k, uint32_t lane, T& S) {
+    const unsigned full = 0xffffffffu;
+    uint32_t lo = 0, len = 0;
+    float s0, s1;
+    if (lane < 2u * kRows<DIM>) stencil_part<DIM>(g, cs, m, (int)(lane >> 1), (lane & 1u) != 0, lo, len, s0, s1);
+    uint32_t x = len;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(full, x, o);
+        if (lane >= o) x += y;
+    }
+    const unsigned has = __ballot_sync(full, len > 0);
+    if (len > 0) {
+        S.part[__popc(has & ((1u << lane) - 1u))] = {lo - (x - len), x};
+        if (k - lo < len) S.self = k - lo + (x - len);
+    }
+    if (lane == 31) {
+        S.total = x;
+        S.n_parts = __popc(has);
+    }
+    __syncwarp();
+}
+
+// Candidates [c0, c0 + kStage) into the team's staging buffer by one warp, one bulk copy per part:
+// every copy is in flight at once, where a walk over the candidates in global memory waits for a
+// load per step or two.
+template <bool FP32, typename T>
+__device__ __forceinline__ void team_stage(const Arrays& A, uint32_t c0, uint32_t lane, T& S) {
+    using Site = typename T::Site;
+    const Site* src;
+    if constexpr (FP32)
+        src = reinterpret_cast<const Site*>(A.sorted_off);
+    else
+        src = A.sorted_s;
+    const uint32_t c1 = min(c0 + kStage, S.total);
+    if (lane == 0) mbar_expect(&S.bar, (c1 - c0) * (uint32_t)sizeof(Site));
+    __syncwarp();
+    if (lane < S.n_parts) {
+        const StencilPart p = S.part[lane];
+        const uint32_t b = max(lane == 0 ? 0u : S.part[lane - 1].end, c0), e = min(p.end, c1);
+        if (b < e) bulk_copy(S.site + (b - c0), src + (p.base + b), (e - b) * (uint32_t)sizeof(Site), &S.bar);
+    }
+}
+
+// dU in FP32 of the team's trial with a bound on its error against the FP64 sums: its warps take
+// the staged candidates 32 at a time and list the pairs inside the cut-off band (1 in 6); the pair
+// energies are evaluated 32 listed pairs at a time, so that those ~60 instructions run with every
+// lane busy (two evaluations per trial instead of one per 32 candidates with five lanes). `phase`:
+// the parity of the staging barrier, the first chunk already on its way.
+template <int DIM, int W, typename T>
+__device__ __forceinline__ void lj_delta32(const Arrays& A, const Pair& P, uint32_t lane, uint32_t warp, T& S,
+                                           uint32_t& phase, float& d32, float& bound) {
+    const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+    float2* list = S.list[warp].q32;
+    const uint32_t total = S.total;
+    const int4 t32 = S.t32, s32 = S.s32;
+    const float cut2 = P.lj_rcut2_hi32;
+    float d = 0.f, err = 0.f, mag = 0.f;
+    uint32_t listed = 0, rounds = 1;
+    auto evaluate = [&](uint32_t at) {
+        const float2 r2 = list[at];
+        float e, x;
+        if (r2.x < cut2) {
+            lj_pair32(P, r2.x, e, x);
+            d += e;
+            err += x;
+            mag += fabsf(e);
         }
-        const uint32_t cell = cell_index<DIM>(g, m);
-        const FlatStencil fs = flat_stencil<DIM>(g, A.cell_start, m, lane);
+        if (r2.y < cut2) {
+            lj_pair32(P, r2.y, e, x);
+            d -= e;
+            err += x;
+            mag += fabsf(e);
+        }
+    };
+#pragma unroll 1
+    for (uint32_t c0 = 0; c0 < total; c0 += kStage) {
+        if (c0 > 0) {
+            team_sync<W>();  // the chunk before has been read
+            if (warp == 0) team_stage<true>(A, c0, lane, S);
+        }
+        mbar_wait(&S.bar, phase, A.stats);
+        phase ^= 1u;
+        const uint32_t n = min(kStage, total - c0), self = S.self - c0;
+#pragma unroll 2
+        for (uint32_t j0 = 32u * warp; j0 < n; j0 += 32u * W) {
+            const uint32_t j = j0 + lane;
+            const int4 o = S.site[j];  // (j < kStage; stale beyond n)
+            const float rn = fixed_dist2<DIM>(P, t32, o), ro = fixed_dist2<DIM>(P, s32, o);
+            const bool need = fminf(rn, ro) < cut2 && j < n && j != self;
+            const unsigned b = __ballot_sync(full, need);
+            if (need) list[listed + __popc(b & below)] = make_float2(rn, ro);
+            listed += __popc(b);
+            if (listed >= 32u) {
+                __syncwarp();
+                listed -= 32u;
+                evaluate(listed + lane);
+                rounds += 1;
+                __syncwarp();
+            }
+        }
+    }
+    __syncwarp();
+    if (lane < listed) evaluate(lane);
+    // summation chains (per lane, the reduction, the warps' sums, the final difference), FP64's own
+    // error
+    const float chain = (float)(2u * rounds + 7u + W) * kU32 * 1.01f + 1e-9f;
+    d32 = warp_sumf(d);
+    bound = warp_sumf(err + chain * mag);
+    if (W > 1) {
+        if (lane == 0) S.sum32[warp] = make_float2(d32, bound);
+        team_sync<W>();
+        d32 = bound = 0.f;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            d32 += S.sum32[w].x;
+            bound += S.sum32[w].y;
+        }
+    }
+    bound += kU32 * fabsf(d32) + 1e-9f;
+}
+
+// FP64 energies of the trial site ta and of the current site tb against the stencil's candidates,
+// and sum |e| over both (order_ambiguous), by the team. Like lj_delta32 the pairs inside the
+// cut-off are listed first and their energies evaluated 32 at a time; a pair outside adds an exact
+// zero and is left out. STAGED: S of the candidates comes from the staging buffer; else it is
+// wrap(sorted_b) (the recheck of the FP32 pass, which does not keep S).
+// INTERIOR: no space of the stencil is the first of an axis (which straddles the box boundary) or
+// reached across the wrap, and an axis has six spaces or more: every site of the stencil then lies
+// within 2 w <= L / 3 of the trial on each axis and any image at least 4 w away, so
+// ref_dist2 would choose the site itself.
+template <int DIM, bool GENERIC, bool INTERIOR, bool STAGED, int W, typename T>
+__device__ __forceinline__ void lj_energies64(const Geometry& g, const Arrays& A, const Pair& P, const double* ta,
+                                              const double* tb, uint32_t lane, uint32_t warp, T& S, uint32_t& phase,
+                                              double& ea, double& eb, double& mag) {
+    const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+    const double cut2 = !GENERIC || P.penalty == 0u ? P.lj_rcut2 : (P.penalty == 1u ? P.op_rcut2 : P.uv_rcut2);
+    double2* list = S.list[warp].q64;
+    const uint32_t total = S.total;
+    double a = 0.0, b = 0.0, am = 0.0;
+    uint32_t listed = 0, part = 0;
+    auto evaluate = [&](uint32_t at) {
+        const double2 r2 = list[at];
+        const double x = soft_pair64<GENERIC>(P, r2.x), y = soft_pair64<GENERIC>(P, r2.y);
+        a = dadd(a, x);
+        b = dadd(b, y);
+        am += GENERIC ? soft_pair_mag(P, r2.x, x) : fabs(x);
+        am += GENERIC ? soft_pair_mag(P, r2.y, y) : fabs(y);
+    };
+    auto dist2 = [&](const double* t, const double* s) -> double {
+        if (!INTERIOR) return ref_dist2<DIM>(g, t, s);
+        double r2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) {
+            const double x = dsub(t[k], s[k]);
+            r2 = dadd(r2, dmul(x, x));
+        }
+        return r2;
+    };
+#pragma unroll 1
+    for (uint32_t c0 = 0; c0 < total; c0 += kStage) {
+        if constexpr (STAGED) {
+            if (c0 > 0) {
+                team_sync<W>();  // the chunk before has been read
+                if (warp == 0) team_stage<false>(A, c0, lane, S);
+            }
+            mbar_wait(&S.bar, phase, A.stats);
+            phase ^= 1u;
+        }
+        const uint32_t n = min(kStage, total - c0), self = S.self - c0;
+#pragma unroll 1
+        for (uint32_t j0 = 32u * warp; j0 < n; j0 += 32u * W) {
+            const uint32_t j = j0 + lane;
+            double rn = cut2, ro = cut2;
+            if (j < n && j != self) {
+                double sv[3];
+                if constexpr (STAGED) {
+                    const double4 v = S.site[j];
+                    sv[0] = v.x, sv[1] = v.y, sv[2] = v.z;
+                } else {
+                    while (c0 + j >= S.part[part].end) ++part;
+                    const double4 v = ldcg4(A.sorted_b + (S.part[part].base + c0 + j));
+                    sv[0] = v.x, sv[1] = v.y, sv[2] = v.z;
+                    wrap_inv<DIM>(g.L, g.invL, sv);
+                }
+                rn = dist2(ta, sv);
+                ro = dist2(tb, sv);
+            }
+            const bool need = rn < cut2 || ro < cut2;
+            const unsigned h = __ballot_sync(full, need);
+            if (need) list[listed + __popc(h & below)] = make_double2(rn, ro);
+            listed += __popc(h);
+            if (listed >= 32u) {
+                __syncwarp();
+                listed -= 32u;
+                evaluate(listed + lane);
+                __syncwarp();
+            }
+        }
+    }
+    __syncwarp();
+    if (lane < listed) evaluate(lane);
+    ea = warp_sum(a);
+    eb = warp_sum(b);
+    mag = warp_sum(am);
+    if (W > 1) {
+        if (lane == 0) {
+            S.sum64[warp][0] = ea;
+            S.sum64[warp][1] = eb;
+            S.sum64[warp][2] = mag;
+        }
+        team_sync<W>();
+        ea = eb = mag = 0.0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            ea = dadd(ea, S.sum64[w][0]);
+            eb = dadd(eb, S.sum64[w][1]);
+            mag += S.sum64[w][2];
+        }
+    }
+}
+
+// The Metropolis test of the team's trial, slot k in space m (parallel_sweep.rs:267-268): FP32 sums
+// first (FP32), the FP64 sums when their bound could change the decision. The candidates of
+// the stencil in the team's scratch are on their way into its staging buffer.
+template <int DIM, bool FP32, bool GENERIC, int W, typename T>
+__device__ __forceinline__ bool lj_decide(const Geometry& g, const Arrays& A, const Pair& P, double kt,
+                                          const uint32_t* m, uint32_t k, double u, float w_lo, float w_hi,
+                                          uint32_t lane, uint32_t warp, T& S, uint32_t& phase, PairStats& pst,
+                                          uint8_t& flags) {
+    float d32 = 0.f;
+    if constexpr (FP32) {
+        float b;
+        lj_delta32<DIM, W>(A, P, lane, warp, S, phase, d32, b);
+        if (lane == 0 && warp == 0) pst.checks += 2u * (S.total - 1u);
+        const float lo = __fsub_rd(d32, b), hi = __fadd_ru(d32, b);
+        if (hi <= 0.f) return true;  // dU64 <= 0 for certain: accepted without a uniform
+        if (lo > 0.f && hi < w_lo) return true;
+        if (lo > 0.f && lo > w_hi) return false;
+        flags |= kTrialRechecked;  // (also where a sum is not finite: every comparison is false)
+    }
+    const double t[3] = {S.t[0], S.t[1], DIM == 3 ? S.t[2] : 0.0};
+    double si[3] = {S.s[0], S.s[1], DIM == 3 ? S.s[2] : 0.0};
+    bool interior = !FP32;
+    if (FP32) {
+        const double4 b4 = ldcg4(A.sorted_b + k);
+        si[0] = b4.x, si[1] = b4.y, si[2] = b4.z;
+        wrap_inv<DIM>(g.L, g.invL, si);
+    }
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) interior = interior && g.shape[a] >= 6 && m[a] >= 2 && m[a] + 2 <= g.shape[a];
+    double e_new, e_old, mag;
+    if (!FP32 && interior)
+        lj_energies64<DIM, GENERIC, !FP32, !FP32, W>(g, A, P, t, si, lane, warp, S, phase, e_new, e_old, mag);
+    else
+        lj_energies64<DIM, GENERIC, false, !FP32, W>(g, A, P, t, si, lane, warp, S, phase, e_new, e_old, mag);
+    const double du = dsub(e_new, e_old);
+    const double e0 = exp(ddiv(-du, kt));
+    if (order_ambiguous(du, mag, S.total, u, kt, e0)) flags |= kTrialAmbiguous;
+    if (lane == 0 && warp == 0) {
+        if (FP32) {
+            pst.rechecks++;
+            const double err = fabs((double)d32 - du);
+            pst.max_err = err > pst.max_err ? err : pst.max_err;
+        }
+        if (flags & kTrialAmbiguous) pst.ambiguous++;
+    }
+    return du <= 0.0 || u < e0;
+}
+
+// The sweep: one team of W warps per trial in dataflow order (hmc_flow.cuh), all colour passes of
+// colour sets [L.round, L.round_end) in one launch. BATCH: over every replica of a batch, with the
+// box, checkerboard, pair parameters and kT of the trial's replica. INJ: the probe mode, team w
+// decides injected trial w against the unchanged state (no order, no commit).
+// The proposal (B + displacement, W1 = wrap, the space check, T = wrap(W1), fixed-point site) and the
+// commit run on one lane per axis of the team's first warp; the proposal needs the own space's
+// last colour set only and is done before the wait for the neighbours.
+template <int DIM, bool FP32, bool GENERIC, bool BATCH, bool INJ, int WARPS, int MINB, int W>
+__global__ void __launch_bounds__(32 * WARPS, MINB)
+    k_flow_lj(Geometry g0, Arrays A, Pair P0, Launch L, Batch B, Injected J) {
+    static_assert(W == 1 || W == WARPS, "a team is a warp or a block");
+    constexpr unsigned full = 0xffffffffu;
+    constexpr uint32_t kTeams = WARPS / W, kNear = DIM == 3 ? 27u : 9u, kOwn = kNear / 2;
+    using TeamT = Team<FP32, BATCH, W>;
+    __shared__ TeamT s_team[kTeams];
+    __shared__ FlowRange s_range;
+    __shared__ uint32_t s_item[2];
+    const uint32_t lane = threadIdx.x & 31u, axis = lane < DIM ? lane : 0u;
+    const uint32_t warp = W == 1 ? 0u : threadIdx.x >> 5;  // within the team
+    TeamT& S = s_team[W == 1 ? threadIdx.x >> 5 : 0u];
+    if (lane == 0 && warp == 0) mbar_init(&S.bar);
+    if (!INJ) {
+        grid_dependency_wait();
+        if (threadIdx.x == 0) {
+            uint32_t round = L.round, round_end = L.round_end;
+            if (BATCH && round == kRoundFromDevice) {
+                round = *B.round_dev;
+                round_end += round;
+            }
+            s_range = flow_range(A.stats, round, round_end, 1u << DIM);
+        }
+    }
+    __syncthreads();
+    const uint32_t n = INJ ? J.n : s_range.n;
+    const uint32_t team = blockIdx.x * kTeams + (W == 1 ? threadIdx.x >> 5 : 0u), n_teams = gridDim.x * kTeams;
+    auto take = [&]() -> uint32_t { return lane == 0 && warp == 0 ? atomicAdd(&A.stats->ticket, 1u) : 0u; };
+    uint32_t n_accepted = 0, phase = 0, turn = 0;
+    PairStats pst;
+    uint32_t next = INJ ? team : take();
+    for (;;) {
+        uint32_t item = next;
+        if (!INJ) {
+            item = __shfl_sync(full, next, 0);
+            if (W > 1) {
+                // (two words: a thread may still read the last one's when a replica's entry is skipped)
+                if (threadIdx.x == 0) s_item[turn] = item;
+                __syncthreads();
+                item = s_item[turn];
+                turn ^= 1u;
+            }
+        }
+        if (item >= n) break;
+        next = INJ ? item + n_teams : take();  // in flight while this trial runs
+        uint32_t m[3] = {0, 0, 0}, k, r = 0, round = 0;
+        uint8_t flags = 0;
         if constexpr (INJ) {
+            const uint64_t body = J.bodies[item];
+            k = A.slot_of_body[body];
+            unpack_m<DIM>(A.body_m[body], m);
+            const double4 w4 = J.trial[item];
+            double x[3] = {w4.x, w4.y, DIM == 3 ? w4.z : 0.0};
             uint32_t mt[3];
-            if (!(point_to_space<DIM>(g, x, mt) && cell_index<DIM>(g, mt) == cell)) {
+            if (!(point_to_space<DIM>(g0, x, mt) && cell_index<DIM>(g0, mt) == cell_index<DIM>(g0, m))) {
                 if (lane == 0) {
-                    J.decisions[w] = 0;
-                    J.flags[w] = kTrialOutsideSpace;
+                    J.decisions[item] = 0;
+                    J.flags[item] = kTrialOutsideSpace;
                 }
                 continue;
             }
-            t[0] = x[0];
-            t[1] = x[1];
-            t[2] = DIM == 3 ? x[2] : 0.0;
-            wrap_inv<DIM>(g.L, g.invL, t);
-        }
-        grid_dependency_wait();  // the previous colour's moves are visible from here on
-        allow_dependent_launch();
-        const double4 s4 = ldg4(A.sorted_s + k);
-        const double si[3] = {s4.x, s4.y, s4.z};
-        double e_new, e_old, mag;
-        lj_energy64<DIM, true, GENERIC, U>(g, A, P, t, si, fs, k, true, lane, e_new, e_old, mag);
-        const double du = dsub(e_new, e_old);
-        const double e0 = exp(ddiv(-du, L.kt));
-        const bool amb = order_ambiguous(du, mag, fs.total, u, L.kt, e0);
-        if constexpr (INJ) {
+            wrap_inv<DIM>(g0.L, g0.invL, x);
+            const double4 s4 = ldg4(A.sorted_s + k);
             if (lane == 0) {
-                J.decisions[w] = du <= 0.0 || u < e0;
-                J.flags[w] = amb ? kTrialAmbiguous : 0;
+                S.t[0] = x[0], S.t[1] = x[1], S.t[2] = x[2];
+                S.s[0] = s4.x, S.s[1] = s4.y, S.s[2] = s4.z;
+                S.t32 = fixed_site<DIM>(g0, x);
+                S.s32 = __ldg(reinterpret_cast<const int4*>(A.sorted_off) + k);
             }
-            continue;
+            const double u = J.u[item];
+            float w_lo, w_hi;
+            metropolis_bounds(u, L.kt, w_lo, w_hi);
+            team_parts<DIM>(g0, A.cell_start, m, k, lane, S);
+            team_stage<FP32>(A, 0, lane, S);
+            const bool ok = lj_decide<DIM, FP32, GENERIC, W>(g0, A, P0, L.kt, m, k, u, w_lo, w_hi, lane, warp, S, phase,
+                                                             pst, flags);
+            if (lane == 0) {
+                J.decisions[item] = ok;
+                J.flags[item] = flags;
+            }
+            __syncwarp();
+        } else {
+            const uint4 di = __ldg(A.draw_i + item);
+            if (BATCH) {
+                if (di.x == kNoTrial) continue;  // the replica has finished its colour sets
+                uint32_t color, entry;
+                flow_item(s_range, item, round, color, entry);
+                r = __ldg(B.color_rep + (size_t)color * B.color_stride + entry);
+            } else {
+                round = s_range.r0 + item / s_range.per_set;
+            }
+            const double u = __ldg(reinterpret_cast<const double*>(A.draw_d + item) + 3);
+            k = di.x;
+            unpack_m<DIM>(di.y, m);
+            if constexpr (BATCH) {
+                if (warp == 0) {
+                    static_assert(sizeof(Replica) % 8 == 0, "copied in 8-byte words");
+                    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(B.rep + r);
+                    unsigned long long* dst = reinterpret_cast<unsigned long long*>(&S.rep);
+#pragma unroll
+                    for (uint32_t i = 0; i < (sizeof(Replica) / 8 + 31) / 32; ++i)
+                        if (i * 32 + lane < sizeof(Replica) / 8) dst[i * 32 + lane] = __ldg(src + i * 32 + lane);
+                    __syncwarp();
+                }
+            }
+            const Replica* R;
+            if constexpr (BATCH)
+                R = &S.rep;
+            else
+                R = nullptr;
+            const Geometry& g = BATCH ? R->g : g0;
+            const Pair& P = BATCH ? R->p : P0;
+            const uint32_t ma = axis == 0 ? m[0] : (axis == 1 ? m[1] : m[2]);
+            double ta = 0.0;
+            if (warp == 0) {
+                const uint32_t base = BATCH ? R->cell_base : 0u;
+                const double dv = __ldg(reinterpret_cast<const double*>(A.draw_d + item) + axis);
+                uint32_t color = 0;
+#pragma unroll
+                for (int a = 0; a < DIM; ++a) color = (color << 1) | (m[a] & 1u);
+                uint32_t space = 0, need = 0;
+                if (lane < kNear) flow_need<DIM>(g, m, color, round, lane, space, need);
+                const uint32_t* word = A.progress + base + space;
+                bool ok = lane >= kNear;
+                team_parts<DIM>(g, A.cell_start + base, m, k, lane, S);
+                bool going = flow_wait(word, need, 1u << kOwn, ok, A.stats);
+                __syncwarp();
+                const AxisGeometry ax = axis_geometry<DIM>(g, axis);
+                const double b = __ldcg(reinterpret_cast<const double*>(A.sorted_b + k) + axis);
+                // the current site
+                if constexpr (FP32) {
+                    const int s = __ldcg(reinterpret_cast<const int*>(A.sorted_off + k) + axis);
+                    if (lane < DIM) reinterpret_cast<int*>(&S.s32)[lane] = s;
+                } else {
+                    const double s = __ldcg(reinterpret_cast<const double*>(A.sorted_s + k) + axis);
+                    if (lane < DIM) S.s[lane] = s;
+                }
+                const double w1 = wrap_axis(ax.L, ax.invL, dadd(b, dv));  // W1 = wrap(propose(..))
+                const bool inside = __all_sync(full, axis_in_space(ax.origin, ax.width, ax.invW, ax.shape, ma, w1));
+                ta = wrap_axis(ax.L, ax.invL, w1);  // the trial site T = wrap(W1)
+                if (lane < DIM) {
+                    S.t[lane] = ta;
+                    if (FP32) reinterpret_cast<int*>(&S.t32)[lane] = fixed_axis(ax.invL, ta);
+                }
+                if (inside && going) going = flow_wait(word, need, full, ok, A.stats);
+                if (lane == 0) S.valid = going ? (inside ? 1u : 0u) : 2u;
+                __syncwarp();
+                if (inside && going) {
+                    fence_proxy_async();
+                    team_stage<FP32>(A, 0, lane, S);
+                }
+            }
+            team_sync<W>();
+            const uint32_t valid = S.valid;
+            if (valid == 2u) break;  // the launch is given up
+            if (valid == 1u) {
+                if (lj_decide<DIM, FP32, GENERIC, W>(g, A, P, BATCH ? R->kt : L.kt, m, k, u, __uint_as_float(di.z),
+                                                     __uint_as_float(di.w), lane, warp, S, phase, pst, flags) &&
+                    warp == 0) {
+                    // update_body_properties: body = T, site = wrap(body)
+                    const AxisGeometry ax = axis_geometry<DIM>(g, axis);
+                    const double sv = wrap_axis(ax.L, ax.invL, ta);
+                    if (lane < DIM) {
+                        reinterpret_cast<double*>(A.sorted_b + k)[lane] = ta;
+                        if (FP32)
+                            reinterpret_cast<int*>(A.sorted_off + k)[lane] = fixed_axis(ax.invL, sv);
+                        else
+                            reinterpret_cast<double*>(A.sorted_s + k)[lane] = sv;
+                        reinterpret_cast<double*>(A.body_pos + A.sorted_body[k])[lane] = ta;
+                    }
+                    n_accepted += lane == 0;
+                    if (BATCH && lane == 0) atomicAdd(B.accepted + r, 1ull);
+                }
+            }
+            __syncwarp();
+            if (lane == 0 && warp == 0)
+                store_release(A.progress + (BATCH ? R->cell_base : 0u) + cell_index<DIM>(g, m), round + 1u);
         }
-        if (amb && lane == 0) pst.ambiguous++;
-        if ((du <= 0.0 || u < e0) && lane == 0) {
-            n_accepted++;
-            double sv[3] = {t[0], t[1], t[2]};
-            wrap_inv<DIM>(g.L, g.invL, sv);
-            A.sorted_b[k] = make_double4(t[0], t[1], t[2], 0.0);
-            A.sorted_s[k] = make_double4(sv[0], sv[1], sv[2], 0.0);
-            A.sorted_off[k] = cell_offsets<DIM>(g, sv, m);
-            A.body_pos[A.sorted_body[k]] = make_double4(t[0], t[1], t[2], 0.0);
-        }
-        __syncwarp();
     }
-    grid_dependency_wait();
-    allow_dependent_launch();
-    flush_stats(A.stats, pst, n_accepted);
-}
-
-// A trial's stencil and sites published in shared memory for the block-cooperative recheck.
-struct SharedTrial {
-    uint32_t lo[32], pre[32];  // the owner warp's FlatStencil parts
-    double t[3], si[3];        // trial site and current site
-    uint32_t total, self;
-};
-
-// Slot of candidate j of a published stencil (the FlatStencil search over shared memory).
-__device__ __forceinline__ uint32_t shared_slot(const SharedTrial& st, uint32_t j) {
-    uint32_t s = 0;
-#pragma unroll
-    for (uint32_t step = 16; step > 0; step >>= 1)
-        if (st.pre[s + step] <= j) s += step;
-    return st.lo[s] + (j - st.pre[s]);
-}
-
-constexpr uint32_t kRecheckChunks = 8;  // 32-candidate chunks per shared-memory round
-
-// The FP32 + recheck pass. One warp per trial as in the FP64 pass, the block's four warps
-// taking four trials at a time. A trial whose FP32 sums cannot decide is rechecked by the whole
-// block: each warp evaluates every fourth 32-candidate chunk of the FP64 walk into shared
-// memory, and the trial's own warp adds them per lane in chunk order, which gives the FP64
-// pass's sums bit for bit (lj_energy64: the same candidates per lane in the same order, the
-// same butterfly; an empty slot adds +0, which leaves a sum that starts at +0 unchanged). A
-// lone warp walking the stencil in FP64 would otherwise set the duration of a pass whose
-// trials all run in one wave.
-template <int DIM, bool INJ = false, int MINB = HMC_LJ_MIN_BLOCKS, int U = 1>
-__global__ void __launch_bounds__(128, MINB) k_sweep_lj32(Geometry g, Arrays A, Pair P, Launch L, Injected J) {
-    if (L.early_wait) grid_dependency_wait();  // first pass: the rebuild's arrays are read at once
-    __shared__ double s_e[kRecheckChunks][2][32];
-    __shared__ SharedTrial s_trial;
-    __shared__ uint32_t s_active;
-    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    uint32_t n_accepted = 0;
-    PairStats pst;
-    if (threadIdx.x == 0) s_active = INJ ? J.n : active_count(A, L.color, L.round);
-    __syncthreads();
-    const uint32_t n_active = s_active;  // block-uniform: the loop below holds barriers
-    for (uint32_t base = blockIdx.x * 4u; base < n_active; base += gridDim.x * 4u) {
-        const uint32_t w = base + wib;
-        uint32_t m[3] = {0, 0, 0};
-        uint32_t k = 0;
-        double t[3] = {0.0, 0.0, 0.0};
-        double u = 0.0;
-        bool trial = false;
-        FlatStencil fs{0u, 0u, 0u, 0.f, 0.f};
-        bool outside = false;
-        float4 t32p = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (INJ && w < n_active) {  // warp-uniform
-            double x[3];
-            lj_inject<DIM>(A, J, w, m, k, x, u);
-            const uint32_t cell = cell_index<DIM>(g, m);
-            fs = flat_stencil<DIM>(g, A.cell_start, m, lane);
-            uint32_t mt[3];
-            trial = point_to_space<DIM>(g, x, mt) && cell_index<DIM>(g, mt) == cell;
-            outside = !trial;
-            t[0] = x[0];
-            t[1] = x[1];
-            t[2] = x[2];
-            wrap_inv<DIM>(g.L, g.invL, t);
-        } else if (w < n_active) {  // warp-uniform: the round's trial from k_propose_lj
-            const size_t e = (size_t)L.color * g.color_stride + w;
-            k = __ldg(A.trial_k + e);
-            trial = k != kNoTrial;
-            if (trial) {
-                unpack_m<DIM>(__ldg(A.color_cells + e), m);
-                fs = flat_stencil<DIM>(g, A.cell_start, m, lane);
-                const double4 t4 = ldg4(A.trial_t + e);
-                t[0] = t4.x;
-                t[1] = t4.y;
-                t[2] = t4.z;
-                u = t4.w;
-                t32p = __ldg(A.trial_o + e);
-            }
-        }
-        grid_dependency_wait();  // the previous colour's moves are visible from here on
-        allow_dependent_launch();
-        int decision = 0;
-        float d32 = 0.f;
-        if (trial) {
-            const float4 t32 = INJ ? cell_offsets<DIM>(g, t, m) : t32p;
-            const float4 c32 = __ldg(A.sorted_off + k);
-            const Sums32 s = lj_energy32<DIM, U>(g, A, P, t32, c32, (int)m[DIM - 1], fs, k, lane);
-            pst.checks += s.pairs;
-            decision = decide32(s, L.kt, u);
-            d32 = s.e_new - s.e_old;
-        }
-        const bool unsure = decision < 0;
-        bool amb = false;
-        if (__syncthreads_or(unsure)) {
-            for (uint32_t o = 0; o < 4u; ++o) {
-                const bool mine = unsure && wib == o;
-                if (mine) {
-                    s_trial.lo[lane] = fs.lo;
-                    s_trial.pre[lane] = fs.pre;
-                    if (lane == 0) {
-                        const double4 c4 = ldg4(A.sorted_b + k);
-                        double si[3] = {c4.x, c4.y, c4.z};
-                        wrap_inv<DIM>(g.L, g.invL, si);
-#pragma unroll
-                        for (int a = 0; a < 3; ++a) {
-                            s_trial.t[a] = t[a];
-                            s_trial.si[a] = si[a];
-                        }
-                        s_trial.total = fs.total;
-                        s_trial.self = k;
-                    }
-                }
-                if (!__syncthreads_or(mine)) continue;  // also publishes s_trial
-                const uint32_t total = s_trial.total, self = s_trial.self;
-                const uint32_t n_chunks = (total + 31u) / 32u;
-                double ea = 0.0, eb = 0.0, em = 0.0;
-                for (uint32_t c0 = 0; c0 < n_chunks; c0 += kRecheckChunks) {
-                    const uint32_t c1 = min(c0 + kRecheckChunks, n_chunks);
-                    for (uint32_t c = c0 + wib; c < c1; c += 4u) {
-                        const uint32_t j = c * 32u + lane;
-                        double en = 0.0, eo = 0.0;
-                        if (j < total) {
-                            const uint32_t q = shared_slot(s_trial, j);
-                            if (q != self) {
-                                const double4 b4 = ldg4(A.sorted_b + q);
-                                double sv[3] = {b4.x, b4.y, b4.z};
-                                wrap_inv<DIM>(g.L, g.invL, sv);
-                                en = lj_only64(P, ref_dist2<DIM>(g, s_trial.t, sv));
-                                eo = lj_only64(P, ref_dist2<DIM>(g, s_trial.si, sv));
-                            }
-                        }
-                        s_e[c - c0][0][lane] = en;
-                        s_e[c - c0][1][lane] = eo;
-                    }
-                    __syncthreads();
-                    if (wib == o) {
-                        for (uint32_t c = c0; c < c1; ++c) {
-                            ea = dadd(ea, s_e[c - c0][0][lane]);
-                            eb = dadd(eb, s_e[c - c0][1][lane]);
-                            em += fabs(s_e[c - c0][0][lane]) + fabs(s_e[c - c0][1][lane]);
-                        }
-                    }
-                    __syncthreads();
-                }
-                if (wib == o) {
-                    const double du = dsub(warp_sum(ea), warp_sum(eb));
-                    const double mag = warp_sum(em);
-                    const double e0 = exp(ddiv(-du, L.kt));
-                    amb = order_ambiguous(du, mag, total, u, L.kt, e0);
-                    if (lane == 0) {
-                        pst.rechecks++;
-                        pst.ambiguous += amb ? 1u : 0u;
-                        const double err = fabs((double)d32 - du);
-                        pst.max_err = err > pst.max_err ? err : pst.max_err;
-                    }
-                    decision = (du <= 0.0 || u < e0) ? 1 : 0;
-                }
-            }
-        }
-        if constexpr (INJ) {
-            if (w < n_active && lane == 0) {
-                J.decisions[w] = decision == 1;
-                J.flags[w] = (outside ? kTrialOutsideSpace : 0) | (unsure ? kTrialRechecked : 0) |
-                             (amb ? kTrialAmbiguous : 0);
-            }
-        } else if (decision == 1 && lane == 0) {
-            n_accepted++;
-            double sv[3] = {t[0], t[1], t[2]};
-            wrap_inv<DIM>(g.L, g.invL, sv);
-            A.sorted_b[k] = make_double4(t[0], t[1], t[2], 0.0);
-            A.sorted_off[k] = cell_offsets<DIM>(g, sv, m);
-            A.body_pos[A.sorted_body[k]] = make_double4(t[0], t[1], t[2], 0.0);
-        }
-        __syncwarp();
-    }
-    grid_dependency_wait();
-    allow_dependent_launch();
-    flush_stats(A.stats, pst, n_accepted);
-}
-
-// One colour pass over every replica of a batch that still runs round `round` of this sweep,
-// FP64: one warp per trial as in k_sweep_lj, with the box, checkerboard, pair parameters,
-// Counter, move size and kT of the trial's replica from the replica table.
-template <int DIM, int MINB = HMC_LJ_BATCH_MIN_BLOCKS, int U = 1>
-__global__ void __launch_bounds__(128, MINB)
-    k_sweep_batch_lj(Batch B, Arrays A, uint32_t color, uint32_t round, uint32_t early_wait) {
-    if (early_wait) grid_dependency_wait();  // first pass: the rebuild's arrays are read at once
-    if (round == kRoundFromDevice) round = *B.round_dev;  // a captured sweep's rounds loop
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
-    uint32_t n_accepted = 0;
-    PairStats pst;
-    const uint32_t n_active = active_count(A, color, round);
-    for (uint32_t w = warp; w < n_active; w += n_warps) {
-        const size_t e = (size_t)color * B.color_stride + w;
-        const uint32_t r = __ldg(B.color_rep + e);
-        const Replica& R = B.rep[r];
-        if (round >= R.rounds) continue;  // warp-uniform
-        const Geometry& g = R.g;
-        const uint32_t* cs = A.cell_start + R.cell_base;
-        uint32_t m[3] = {0, 0, 0};
-        unpack_m<DIM>(__ldg(A.color_cells + e), m);
-        const uint32_t cell = cell_index<DIM>(g, m);
-        const FlatStencil fs = flat_stencil<DIM>(g, cs, m, lane);
-        const uint32_t start = __ldg(cs + cell);
-        const uint32_t count = __ldg(cs + cell + 1) - start;
-        Sfc64 rng = make_rng(R.step, R.substep + round, R.seed, (uint64_t)cell);
-        const uint32_t k = start + canon_range_u32(rng, count);
-        const double4 b4 = A.sorted_b[k];
-        double x[3] = {b4.x, b4.y, b4.z};
-        double dv[3];
-        ball_sample<DIM>(rng, R.max_move, A.zig_x, A.zig_f, dv);
-        const double u = uniform01(rng);
-#pragma unroll
-        for (int a = 0; a < DIM; ++a) x[a] = dadd(x[a], dv[a]);
-        wrap_inv<DIM>(g.L, g.invL, x);
-        uint32_t mt[3];
-        if (!(point_to_space<DIM>(g, x, mt) && cell_index<DIM>(g, mt) == cell)) continue;
-        double t[3] = {x[0], x[1], DIM == 3 ? x[2] : 0.0};
-        wrap_inv<DIM>(g.L, g.invL, t);
-        grid_dependency_wait();  // the previous colour's moves are visible from here on
-        allow_dependent_launch();
-        const double4 s4 = ldg4(A.sorted_s + k);
-        const double si[3] = {s4.x, s4.y, s4.z};
-        double e_new, e_old, mag;
-        lj_energy64<DIM, true, false, U>(g, A, R.p, t, si, fs, k, true, lane, e_new, e_old, mag);
-        const double du = dsub(e_new, e_old);
-        const double e0 = exp(ddiv(-du, R.kt));
-        if (lane == 0 && order_ambiguous(du, mag, fs.total, u, R.kt, e0)) pst.ambiguous++;
-        if ((du <= 0.0 || u < e0) && lane == 0) {
-            n_accepted++;
-            atomicAdd(B.accepted + r, 1ull);
-            double sv[3] = {t[0], t[1], t[2]};
-            wrap_inv<DIM>(g.L, g.invL, sv);
-            A.sorted_b[k] = make_double4(t[0], t[1], t[2], 0.0);
-            A.sorted_s[k] = make_double4(sv[0], sv[1], sv[2], 0.0);
-            A.sorted_off[k] = cell_offsets<DIM>(g, sv, m);
-            A.body_pos[A.sorted_body[k]] = make_double4(t[0], t[1], t[2], 0.0);
-        }
-        __syncwarp();
-    }
-    grid_dependency_wait();
-    allow_dependent_launch();
-    flush_stats(A.stats, pst, n_accepted);
-}
-
-// The FP32 + recheck pass over a batch: k_sweep_lj32 (four trials per block, an undecided
-// trial rechecked by the whole block in the FP64 pass's order) with each trial's geometry and
-// parameters from its replica; the owner also publishes its replica for the helping warps.
-template <int DIM, int MINB = HMC_LJ_BATCH_MIN_BLOCKS, int U = 1>
-__global__ void __launch_bounds__(128, MINB)
-    k_sweep_batch_lj32(Batch B, Arrays A, uint32_t color, uint32_t round, uint32_t early_wait) {
-    if (early_wait) grid_dependency_wait();  // first pass: the rebuild's arrays are read at once
-    if (round == kRoundFromDevice) round = *B.round_dev;  // a captured sweep's rounds loop
-    __shared__ double s_e[kRecheckChunks][2][32];
-    __shared__ SharedTrial s_trial;
-    __shared__ uint32_t s_active, s_rep;
-    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    uint32_t n_accepted = 0;
-    PairStats pst;
-    if (threadIdx.x == 0) s_active = active_count(A, color, round);
-    __syncthreads();
-    const uint32_t n_active = s_active;  // block-uniform: the loop below holds barriers
-    for (uint32_t base = blockIdx.x * 4u; base < n_active; base += gridDim.x * 4u) {
-        const uint32_t w = base + wib;
-        uint32_t m[3] = {0, 0, 0};
-        uint32_t k = 0, r = 0;
-        double t[3] = {0.0, 0.0, 0.0};
-        double u = 0.0;
-        bool trial = false;
-        FlatStencil fs{0u, 0u, 0u, 0.f, 0.f};
-        if (w < n_active) {  // warp-uniform
-            const size_t e = (size_t)color * B.color_stride + w;
-            r = __ldg(B.color_rep + e);
-            const Replica& R = B.rep[r];
-            if (round < R.rounds) {
-                const Geometry& g = R.g;
-                const uint32_t* cs = A.cell_start + R.cell_base;
-                unpack_m<DIM>(__ldg(A.color_cells + e), m);
-                const uint32_t cell = cell_index<DIM>(g, m);
-                fs = flat_stencil<DIM>(g, cs, m, lane);
-                const uint32_t start = __ldg(cs + cell);
-                const uint32_t count = __ldg(cs + cell + 1) - start;
-                Sfc64 rng = make_rng(R.step, R.substep + round, R.seed, (uint64_t)cell);
-                k = start + canon_range_u32(rng, count);
-                const double4 b4 = A.sorted_b[k];
-                double x[3] = {b4.x, b4.y, b4.z};
-                double dv[3];
-                ball_sample<DIM>(rng, R.max_move, A.zig_x, A.zig_f, dv);
-                u = uniform01(rng);
-#pragma unroll
-                for (int a = 0; a < DIM; ++a) x[a] = dadd(x[a], dv[a]);
-                wrap_inv<DIM>(g.L, g.invL, x);
-                uint32_t mt[3];
-                trial = point_to_space<DIM>(g, x, mt) && cell_index<DIM>(g, mt) == cell;
-                t[0] = x[0];
-                t[1] = x[1];
-                t[2] = DIM == 3 ? x[2] : 0.0;
-                wrap_inv<DIM>(g.L, g.invL, t);
-            }
-        }
-        grid_dependency_wait();  // the previous colour's moves are visible from here on
-        allow_dependent_launch();
-        int decision = 0;
-        float d32 = 0.f;
-        if (trial) {
-            const Replica& R = B.rep[r];
-            const float4 t32 = cell_offsets<DIM>(R.g, t, m);
-            const float4 c32 = __ldg(A.sorted_off + k);
-            const Sums32 s = lj_energy32<DIM, U>(R.g, A, R.p, t32, c32, (int)m[DIM - 1], fs, k, lane);
-            pst.checks += s.pairs;
-            decision = decide32(s, R.kt, u);
-            d32 = s.e_new - s.e_old;
-        }
-        const bool unsure = decision < 0;
-        if (__syncthreads_or(unsure)) {
-            for (uint32_t o = 0; o < 4u; ++o) {
-                const bool mine = unsure && wib == o;
-                if (mine) {
-                    s_trial.lo[lane] = fs.lo;
-                    s_trial.pre[lane] = fs.pre;
-                    if (lane == 0) {
-                        const Geometry& g = B.rep[r].g;
-                        const double4 c4 = ldg4(A.sorted_b + k);
-                        double si[3] = {c4.x, c4.y, c4.z};
-                        wrap_inv<DIM>(g.L, g.invL, si);
-#pragma unroll
-                        for (int a = 0; a < 3; ++a) {
-                            s_trial.t[a] = t[a];
-                            s_trial.si[a] = si[a];
-                        }
-                        s_trial.total = fs.total;
-                        s_trial.self = k;
-                        s_rep = r;
-                    }
-                }
-                if (!__syncthreads_or(mine)) continue;  // also publishes s_trial and s_rep
-                const Replica& RO = B.rep[s_rep];
-                const uint32_t total = s_trial.total, self = s_trial.self;
-                const uint32_t n_chunks = (total + 31u) / 32u;
-                double ea = 0.0, eb = 0.0, em = 0.0;
-                for (uint32_t c0 = 0; c0 < n_chunks; c0 += kRecheckChunks) {
-                    const uint32_t c1 = min(c0 + kRecheckChunks, n_chunks);
-                    for (uint32_t c = c0 + wib; c < c1; c += 4u) {
-                        const uint32_t j = c * 32u + lane;
-                        double en = 0.0, eo = 0.0;
-                        if (j < total) {
-                            const uint32_t q = shared_slot(s_trial, j);
-                            if (q != self) {
-                                const double4 b4 = ldg4(A.sorted_b + q);
-                                double sv[3] = {b4.x, b4.y, b4.z};
-                                wrap_inv<DIM>(RO.g.L, RO.g.invL, sv);
-                                en = lj_only64(RO.p, ref_dist2<DIM>(RO.g, s_trial.t, sv));
-                                eo = lj_only64(RO.p, ref_dist2<DIM>(RO.g, s_trial.si, sv));
-                            }
-                        }
-                        s_e[c - c0][0][lane] = en;
-                        s_e[c - c0][1][lane] = eo;
-                    }
-                    __syncthreads();
-                    if (wib == o) {
-                        for (uint32_t c = c0; c < c1; ++c) {
-                            ea = dadd(ea, s_e[c - c0][0][lane]);
-                            eb = dadd(eb, s_e[c - c0][1][lane]);
-                            em += fabs(s_e[c - c0][0][lane]) + fabs(s_e[c - c0][1][lane]);
-                        }
-                    }
-                    __syncthreads();
-                }
-                if (wib == o) {
-                    const double du = dsub(warp_sum(ea), warp_sum(eb));
-                    const double mag = warp_sum(em);
-                    const double e0 = exp(ddiv(-du, RO.kt));
-                    if (lane == 0) {
-                        pst.rechecks++;
-                        pst.ambiguous += order_ambiguous(du, mag, total, u, RO.kt, e0) ? 1u : 0u;
-                        const double err = fabs((double)d32 - du);
-                        pst.max_err = err > pst.max_err ? err : pst.max_err;
-                    }
-                    decision = (du <= 0.0 || u < e0) ? 1 : 0;
-                }
-            }
-        }
-        if (decision == 1 && lane == 0) {
-            const Geometry& g = B.rep[r].g;
-            n_accepted++;
-            atomicAdd(B.accepted + r, 1ull);
-            double sv[3] = {t[0], t[1], t[2]};
-            wrap_inv<DIM>(g.L, g.invL, sv);
-            A.sorted_b[k] = make_double4(t[0], t[1], t[2], 0.0);
-            A.sorted_off[k] = cell_offsets<DIM>(g, sv, m);
-            A.body_pos[A.sorted_body[k]] = make_double4(t[0], t[1], t[2], 0.0);
-        }
-        __syncwarp();
-    }
-    grid_dependency_wait();
-    allow_dependent_launch();
     flush_stats(A.stats, pst, n_accepted);
 }
 
@@ -767,10 +723,10 @@ __global__ void __launch_bounds__(128) k_eval_lj(Geometry g, Arrays A, Pair P, c
         if (ok) {
             const FlatStencil ft = flat_stencil<DIM>(g, A.cell_start, mt, lane);
             const FlatStencil fi = flat_stencil<DIM>(g, A.cell_start, mi, lane);
-            double e_new, e_old, unused;
+            double e_new, e_old;
             double mag_new, mag_old;
-            lj_energy64<DIM, false>(g, A, P, t, nullptr, ft, k, true, lane, e_new, unused, mag_new);
-            lj_energy64<DIM, false>(g, A, P, si, nullptr, fi, k, true, lane, e_old, unused, mag_old);
+            lj_energy64<DIM>(g, A, P, t, ft, k, lane, e_new, mag_new);
+            lj_energy64<DIM>(g, A, P, si, fi, k, lane, e_old, mag_old);
             du = dsub(e_new, e_old);
             const double u = uu[i];
             bool dec64 = du <= 0.0 || u < exp(ddiv(-du, kt));
@@ -780,9 +736,8 @@ __global__ void __launch_bounds__(128) k_eval_lj(Geometry g, Arrays A, Pair P, c
                 // space, they are evaluated in FP64 as the sweep never sees such a trial.
                 const bool same = mt[0] == mi[0] && mt[1] == mi[1] && (DIM == 2 || mt[2] == mi[2]);
                 if (same) {
-                    const float4 t32 = cell_offsets<DIM>(g, t, mt);
-                    const float4 c32 = __ldg(A.sorted_off + k);
-                    const Sums32 s = lj_energy32<DIM>(g, A, P, t32, c32, (int)mt[DIM - 1], ft, k, lane);
+                    const int4 c32 = __ldg(reinterpret_cast<const int4*>(A.sorted_off) + k);
+                    const Sums32 s = lj_energy32<DIM>(A, P, fixed_site<DIM>(g, t), c32, ft, k, lane);
                     const float d32 = s.e_new - s.e_old;
                     const float b = s.err + (float)(s.terms + 7) * kU32 * s.mag * 1.01f + kU32 * fabsf(d32) +
                                     1e-9f * (s.mag + 1.f);
@@ -847,10 +802,10 @@ __global__ void __launch_bounds__(32) k_tune_stream_lj(TuneJob* jobs, uint32_t n
             }
             const FlatStencil ft = flat_stencil<DIM>(g, A.cell_start, mt, lane);
             const FlatStencil fi = flat_stencil<DIM>(g, A.cell_start, mi, lane);
-            double e_new, e_old, unused, mag_new, mag_old;
-            lj_energy64<DIM, false>(g, A, P, t, nullptr, ft, k, true, lane, e_new, unused, mag_new);
+            double e_new, e_old, mag_new, mag_old;
+            lj_energy64<DIM>(g, A, P, t, ft, k, lane, e_new, mag_new);
             if (e_new == __longlong_as_double(0x7ff0000000000000ll)) return false;  // the reference stops here
-            lj_energy64<DIM, false>(g, A, P, si, nullptr, fi, k, true, lane, e_old, unused, mag_old);
+            lj_energy64<DIM>(g, A, P, si, fi, k, lane, e_old, mag_old);
             const double du = dsub(e_new, e_old);
             if (!(du != __longlong_as_double(0x7ff0000000000000ll))) return false;
             const uint32_t n = ft.total + fi.total;
@@ -897,60 +852,86 @@ __global__ void k_energy_lj(Geometry g, Arrays A, Pair P, uint32_t n, double* ou
 
 }  // namespace
 
-cudaError_t launch_sweep_lj(int dim, bool fp32, bool generic, const Geometry& g, const Arrays& a, const Pair& p,
-                            const Launch& l, cudaStream_t s, uint32_t variant) {
-    if (l.n_active == 0) return cudaSuccess;
-    static int max_blocks = 0;
-    if (max_blocks == 0) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        max_blocks = sms * 16;
+namespace {
+using LjKernel = void (*)(Geometry, Arrays, Pair, Launch, Batch, Injected);
+
+// The compiled launch variants 1 .. 4 of kLjShapes and kBatchLjShapes: teams of 1, 2, 4 and 8 warps.
+struct LjVariant {
+    LjKernel kernel;
+    uint32_t warps, team;  // per block, per trial
+};
+// Variant 0: the largest team of which the chip holds about as many as one colour has trials (`list`):
+// a larger team decides a trial in less time, but fewer fit (148 SMs hold about 440 of 8 warps, 890 of
+// 4, 1,780 of 2). And no warp without two steps of candidates (a stencil's mean number).
+// Four sweeps of n sites at density 0.8, teams of 1 / 2 / 4 / 8 warps, us, FP32: n = 16,384 (216
+// trials a colour) 5971 / 4565 / 3712 / 3469; 65,536 (512) 6404 / 4617 / 3713 / 3835; 131,072 (1,000)
+// 6895 / 5102 / 4331 / 6467; 262,144 (2,197) 6239 / 5284 / 6670 / 12043; 2-D (40 candidates), 65,536 sites
+// (3,844): 654 / 990 / 1575 / 2802.
+uint32_t lj_team_variant(uint32_t list, double candidates) {
+    const uint32_t by_trials = list > 2300 ? 1u : (list > 1060 ? 2u : (list > 480 ? 3u : 4u));
+    const uint32_t by_steps = candidates < 128 ? 1u : (candidates < 192 ? 2u : (candidates < 256 ? 3u : 4u));
+    return by_trials < by_steps ? by_trials : by_steps;
+}
+template <int DIM, bool FP32, bool GENERIC, bool BATCH>
+LjVariant lj_kernel(uint32_t v) {
+    // single-warp teams share a block: FP32 staging buffers of four, FP64 of two fit 48 KB
+    constexpr int N = FP32 ? 4 : 2;
+    switch (v) {
+        case 2: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 2, FP32 ? 12 : 8, 2>, 2, 2};
+        case 3: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 4, 6, 4>, 4, 4};
+        case 4: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 8, 3, 8>, 8, 8};
+        default: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, N, FP32 ? 6 : 8, 1>, N, 1};
     }
-    uint32_t blocks = (l.n_active + 3) / 4;  // four warps (trials) per block
-    if (blocks > (uint32_t)max_blocks) blocks = (uint32_t)max_blocks;
-    PassLaunch pl(blocks, l.overlap_previous != 0 || l.early_wait != 0, s);
-    using LjKernel = void (*)(Geometry, Arrays, Pair, Launch, Injected);
-    // the compiled launch variants, in the order of kLjShapes ([dim == 3][fp32][variant])
-    // (variants 3 and 4 take two candidates per lane and step)
-    static const LjKernel kernels[2][2][5] = {
-        {{k_sweep_lj<2, false, 9, false>, k_sweep_lj<2, false, 7, false>, k_sweep_lj<2, false, 11, false>,
-          k_sweep_lj<2, false, 7, false, 2>, k_sweep_lj<2, false, 9, false, 2>},
-         {k_sweep_lj32<2, false, 9>, k_sweep_lj32<2, false, 7>, k_sweep_lj32<2, false, 11>,
-          k_sweep_lj32<2, false, 7, 2>, k_sweep_lj32<2, false, 9, 2>}},
-        {{k_sweep_lj<3, false, 9, false>, k_sweep_lj<3, false, 7, false>, k_sweep_lj<3, false, 11, false>,
-          k_sweep_lj<3, false, 7, false, 2>, k_sweep_lj<3, false, 9, false, 2>},
-         {k_sweep_lj32<3, false, 9>, k_sweep_lj32<3, false, 7>, k_sweep_lj32<3, false, 11>,
-          k_sweep_lj32<3, false, 7, 2>, k_sweep_lj32<3, false, 9, 2>}}};
-    // the overlap penalty and Isotropic: the FP64 pass with the dispatching pair energy
-    static const LjKernel generic_kernels[2][5] = {
-        {k_sweep_lj<2, false, 9, true>, k_sweep_lj<2, false, 7, true>, k_sweep_lj<2, false, 11, true>,
-         k_sweep_lj<2, false, 7, true, 2>, k_sweep_lj<2, false, 9, true, 2>},
-        {k_sweep_lj<3, false, 9, true>, k_sweep_lj<3, false, 7, true>, k_sweep_lj<3, false, 11, true>,
-         k_sweep_lj<3, false, 7, true, 2>, k_sweep_lj<3, false, 9, true, 2>}};
-    static_assert(n_shapes(kLjShapes) == 5, "one compiled kernel per Lennard-Jones variant");
-    const LjKernel k = generic ? generic_kernels[dim == 3][variant < 5 ? variant : 0]
-                               : kernels[dim == 3][fp32][variant < 5 ? variant : 0];
-    return cudaLaunchKernelEx(&pl.cfg, k, g, a, p, l, Injected{});
+}
+LjVariant lj_kernel(int dim, bool fp32, bool generic, bool batch, uint32_t variant, uint32_t list, double per_space) {
+    static_assert(n_shapes(kLjShapes) == 5 && n_shapes(kBatchLjShapes) == 5, "the rule and four kernels");
+    const uint32_t v = variant == 0 || variant > 4 ? lj_team_variant(list, per_space * (dim == 3 ? 27 : 9)) : variant;
+    if (batch) {
+        if (dim == 2) return fp32 ? lj_kernel<2, true, false, true>(v) : lj_kernel<2, false, false, true>(v);
+        return fp32 ? lj_kernel<3, true, false, true>(v) : lj_kernel<3, false, false, true>(v);
+    }
+    if (generic) return dim == 2 ? lj_kernel<2, false, true, false>(v) : lj_kernel<3, false, true, false>(v);
+    if (dim == 2) return fp32 ? lj_kernel<2, true, false, false>(v) : lj_kernel<2, false, false, false>(v);
+    return fp32 ? lj_kernel<3, true, false, false>(v) : lj_kernel<3, false, false, false>(v);
 }
 
-cudaError_t launch_propose_lj(int dim, bool fp32, const Geometry& g, const Arrays& a, const Launch& l, cudaStream_t s) {
-    const uint64_t n = (uint64_t)g.color_stride << dim;
-    if (n == 0) return cudaSuccess;
-    static int max_blocks = 0;
-    if (max_blocks == 0) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        max_blocks = sms * 16;
-    }
-    uint32_t blocks = (uint32_t)((n + 127) / 128);
-    if (blocks > (uint32_t)max_blocks) blocks = (uint32_t)max_blocks;
-    if (dim == 2)
-        fp32 ? k_propose_lj<2, true><<<blocks, 128, 0, s>>>(g, a, l) : k_propose_lj<2, false><<<blocks, 128, 0, s>>>(g, a, l);
-    else
-        fp32 ? k_propose_lj<3, true><<<blocks, 128, 0, s>>>(g, a, l) : k_propose_lj<3, false><<<blocks, 128, 0, s>>>(g, a, l);
-    return cudaGetLastError();
+// The two kernels of a range of colour sets whose longest colour list has at most `list` entries.
+// The flow kernel gets a team for each trial of two colour lists (the trials behind the running
+// colour wait at most for it), at most one resident wave.
+cudaError_t launch_flow(int dim, bool batch, const LjVariant& v, const Geometry& g, const Arrays& a, const Pair& p,
+                        const Launch& l, const Batch& b, uint32_t list, cudaStream_t s) {
+    if (list == 0) return cudaSuccess;
+    using DrawKernel = void (*)(Geometry, Arrays, Launch, Batch);
+    const DrawKernel d = dim == 2 ? (batch ? k_draw_lj<2, true> : k_draw_lj<2, false>)
+                                  : (batch ? k_draw_lj<3, true> : k_draw_lj<3, false>);
+    const uint64_t entries = ((uint64_t)list << dim) * 16u;
+    uint64_t blocks = (entries + 127) / 128;
+    const uint64_t wave_d = (uint64_t)resident_wave((const void*)d);
+    PassLaunch pd((uint32_t)(blocks < wave_d ? blocks : wave_d), true, s);
+    cudaError_t e = cudaLaunchKernelEx(&pd.cfg, d, g, a, l, b);
+    if (e != cudaSuccess) return e;
+    blocks = ((uint64_t)list * 2 * v.team + v.warps - 1) / v.warps;
+    const uint64_t wave = (uint64_t)resident_wave((const void*)v.kernel, (int)(32 * v.warps));
+    PassLaunch pl((uint32_t)(blocks < wave ? blocks : wave), true, s, 32 * v.warps);
+    return cudaLaunchKernelEx(&pl.cfg, v.kernel, g, a, p, l, b, Injected{});
+}
+}  // namespace
+
+cudaError_t launch_flow_lj(int dim, bool fp32, bool generic, const Geometry& g, const Arrays& a, const Pair& p,
+                           const Launch& l, cudaStream_t s, uint32_t variant) {
+    return launch_flow(dim, false, lj_kernel(dim, fp32, generic, false, variant, g.color_stride, (double)l.n_bodies / g.n_cells),
+                       g, a, p, l, Batch{},
+                       g.color_stride, s);
+}
+
+cudaError_t launch_flow_batch_lj(int dim, bool fp32, const Batch& b, const Arrays& a, uint32_t round,
+                                 uint32_t round_end, cudaStream_t s, uint32_t variant) {
+    Launch l{};
+    l.round = round;
+    l.round_end = round_end;
+    return launch_flow(dim, true, lj_kernel(dim, fp32, false, true, variant, b.color_stride, (double)b.n_bodies / b.n_cells),
+                       Geometry{}, a, Pair{}, l, b,
+                       b.color_stride, s);
 }
 
 cudaError_t launch_tune_stream_lj(int dim, TuneJob* jobs, uint32_t n_jobs, cudaStream_t s) {
@@ -967,50 +948,15 @@ cudaError_t launch_trials_lj(int dim, bool fp32, const Geometry& g, const Arrays
     if (j.n == 0) return cudaSuccess;
     Launch l{};
     l.kt = kt;
-    const uint32_t blocks = (j.n + 3) / 4;  // four warps (trials) per block
-    if (dim == 2) {
-        if (fp32)
-            k_sweep_lj32<2, true><<<blocks, 128, 0, s>>>(g, a, p, l, j);
-        else
-            k_sweep_lj<2, true><<<blocks, 128, 0, s>>>(g, a, p, l, j);
-    } else {
-        if (fp32)
-            k_sweep_lj32<3, true><<<blocks, 128, 0, s>>>(g, a, p, l, j);
-        else
-            k_sweep_lj<3, true><<<blocks, 128, 0, s>>>(g, a, p, l, j);
-    }
+    // single-warp teams, as the sweep's variant 1
+    const LjKernel k = dim == 2 ? (fp32 ? k_flow_lj<2, true, false, false, true, 4, 6, 1>
+                                        : k_flow_lj<2, false, true, false, true, 2, 8, 1>)
+                                : (fp32 ? k_flow_lj<3, true, false, false, true, 4, 6, 1>
+                                        : k_flow_lj<3, false, true, false, true, 2, 8, 1>);
+    const uint32_t warps = fp32 ? 4u : 2u, n = (j.n + warps - 1) / warps;
+    const uint32_t wave = (uint32_t)resident_wave((const void*)k, (int)(32 * warps));
+    k<<<n < wave ? n : wave, 32 * warps, 0, s>>>(g, a, p, l, Batch{}, j);
     return cudaGetLastError();
-}
-
-cudaError_t launch_sweep_batch_lj(int dim, bool fp32, const Batch& b, const Arrays& a, uint32_t color, uint32_t round,
-                                  uint32_t max_active, bool overlap_previous, bool early_wait, cudaStream_t s,
-                                  uint32_t variant) {
-    if (max_active == 0) return cudaSuccess;
-    static int max_blocks = 0;
-    if (max_blocks == 0) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        max_blocks = sms * 16;
-    }
-    uint32_t blocks = (max_active + 3) / 4;  // four warps (trials) per block
-    if (blocks > (uint32_t)max_blocks) blocks = (uint32_t)max_blocks;
-    PassLaunch pl(blocks, overlap_previous || early_wait, s);
-    const uint32_t ew = early_wait ? 1u : 0u;
-    using BatchLjKernel = void (*)(Batch, Arrays, uint32_t, uint32_t, uint32_t);
-    // the compiled launch variants, in the order of kBatchLjShapes ([dim == 3][fp32][variant])
-    // (variants 3 and 4 take two candidates per lane and step)
-    static const BatchLjKernel kernels[2][2][5] = {
-        {{k_sweep_batch_lj<2, 7>, k_sweep_batch_lj<2, 9>, k_sweep_batch_lj<2, 5>, k_sweep_batch_lj<2, 7, 2>,
-          k_sweep_batch_lj<2, 9, 2>},
-         {k_sweep_batch_lj32<2, 7>, k_sweep_batch_lj32<2, 9>, k_sweep_batch_lj32<2, 5>, k_sweep_batch_lj32<2, 7, 2>,
-          k_sweep_batch_lj32<2, 9, 2>}},
-        {{k_sweep_batch_lj<3, 7>, k_sweep_batch_lj<3, 9>, k_sweep_batch_lj<3, 5>, k_sweep_batch_lj<3, 7, 2>,
-          k_sweep_batch_lj<3, 9, 2>},
-         {k_sweep_batch_lj32<3, 7>, k_sweep_batch_lj32<3, 9>, k_sweep_batch_lj32<3, 5>, k_sweep_batch_lj32<3, 7, 2>,
-          k_sweep_batch_lj32<3, 9, 2>}}};
-    static_assert(n_shapes(kBatchLjShapes) == 5, "one compiled kernel per Lennard-Jones batch variant");
-    return cudaLaunchKernelEx(&pl.cfg, kernels[dim == 3][fp32][variant < 5 ? variant : 0], b, a, color, round, ew);
 }
 
 cudaError_t launch_eval_lj(int dim, bool fp32, const Geometry& g, const Arrays& a, const Pair& p,
