@@ -239,7 +239,6 @@ void lj_setup_for(int dim, const Geometry& geom, Pair& P, double eps, double sig
     const double scale = fp32_band_scale();
     const double E = (std::ldexp(1.1 * Lmax, -32) + 16.0 * u64 * (Lmax + wmax)) * scale;
     const double rel = 10.4 * u32 * scale;
-    for (int a = 0; a < 3; ++a) P.lj_fix[a] = a < dim ? (float)std::ldexp(geom.L[a], -32) : 0.f;
     P.lj_disp_err = (float)(E * 1.01);
     P.lj_rel_err = (float)(rel * 1.01);
     const double band = 2.0 * (3.5 * E * (rcut + E) + rel * rcut * rcut);
@@ -294,6 +293,18 @@ void pair_setup(hmc_system* s) {
         s->pair.sigma2 = s->poly_rcut2;  // the FP32 prefilter threshold reuses the sphere bound
         sphere_bound(s);
         s->poly_rcut2_hi32 = s->pair.sig2_hi32;
+        if (s->arr.fixed_sites) {
+            // fixed-point sites: the r^2 bound of lj_setup_for at the circumsphere distance, twice
+            const double u32 = std::ldexp(1.0, -24), u64 = std::ldexp(1.0, -53), r = std::sqrt(s->poly_rcut2);
+            double wmax = 0, Lmax = 0;
+            for (int a = 0; a < s->dim; ++a) {
+                wmax = std::max(wmax, s->geom.width[a]);
+                Lmax = std::max(Lmax, s->geom.L[a]);
+            }
+            const double E = std::ldexp(1.1 * Lmax, -32) + 16.0 * u64 * (Lmax + wmax);
+            const double band = 2.0 * (3.5 * E * (r + E) + 10.4 * u32 * s->poly_rcut2) * fp32_band_scale();
+            s->poly_rcut2_hi32 = std::nextafter((float)(s->poly_rcut2 + band), INFINITY);
+        }
     } else if (s->interaction == HMC_LENNARD_JONES) {
         lj_setup(s, s->lj_params[0], s->lj_params[1], s->lj_params[2], s->lj_params[3]);
     }
@@ -303,7 +314,7 @@ void pair_setup(hmc_system* s) {
 // 97-107) and HypercuboidCheckerboard::compute_dimensions (hypercuboid.rs:188-228). The
 // checkerboard arrays grow when the box needs more spaces than they hold.
 hmc_status setup_geometry(hmc_system* s, const double* L) {
-    s->arr.fixed_sites = s->soft_fp32() ? 1u : 0u;
+    s->arr.fixed_sites = s->soft_fp32() || s->interaction == HMC_HARD_CONVEX_POLYHEDRON ? 1u : 0u;
     Geometry g = s->geom;
     for (int a = 0; a < 3; ++a) g.L[a] = a < s->dim ? L[a] : 1.0;
     double min_l = g.L[0];
@@ -322,6 +333,7 @@ hmc_status setup_geometry(hmc_system* s, const double* L) {
         g.ghost_hi[a] = g.half[a] - s->boundary_range;
         g.ghost_lo[a] = -g.half[a] + s->boundary_range;
         g.w32[a] = (float)g.width[a];
+        g.fix[a] = (float)std::ldexp(g.L[a], -32);
         g.invL[a] = 1.0 / g.L[a];
         g.invW[a] = 1.0 / g.width[a];
         g.half_shape[a] = g.shape[a] / 2;
@@ -416,7 +428,9 @@ hmc_status flow_buffers(hmc_system* s) {
 }
 
 // Whether the system's sweeps run in dataflow order, and the colour sets one launch then holds.
-bool flow_of(const hmc_system* s) { return s->soft(); }
+bool flow_of(const hmc_system* s) {
+    return s->soft() || (s->interaction == HMC_HARD_CONVEX_POLYHEDRON && !s->shape_soft);
+}
 uint32_t flow_sets(const hmc_system* s) {
     const uint64_t cells = s->geom.n_cells;
     if (s->flow_entries >= s->n + cells) return UINT32_MAX;
@@ -1056,7 +1070,11 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
             L.round = r;
             L.round_end = r + std::min(sets, r1 - r);
             // the overlap penalty and Isotropic have no FP32 path: FP64 in both modes
-            HMC_CUDA(launch_flow_lj(s->dim, fp32 && s->soft_fp32(), !s->soft_fp32(), s->geom, s->arr, s->pair, L,
+            if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON)
+                HMC_CUDA(launch_flow_poly(fp32, s->geom, s->arr, s->verts, s->n_vertices, s->poly_rcut2,
+                                          s->poly_rcut2_hi32, L, p->move == HMC_ROTATE, s->stream, sp.variant));
+            else
+                HMC_CUDA(launch_flow_lj(s->dim, fp32 && s->soft_fp32(), !s->soft_fp32(), s->geom, s->arr, s->pair, L,
                                     s->stream, sp.variant));
             s->prof.kernel_launches += 2;
         }
@@ -1066,8 +1084,7 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
         L.substep = s->substep + r;  // increment_substep after every full colour set
         L.round = r;
         if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON) {
-            HMC_CUDA(launch_propose_poly(fp32 && !s->shape_soft, s->geom, s->arr, L, p->move == HMC_ROTATE,
-                                         s->shape_soft, s->stream));
+            HMC_CUDA(launch_propose_poly(s->geom, s->arr, L, p->move == HMC_ROTATE, s->stream));
             s->prof.kernel_launches += 1;
         } else if (s->polygon()) {
             HMC_CUDA(launch_propose_poly2(sp.poly2_fp32 && !s->shape_soft, s->geom, s->arr, L, p->move == HMC_ROTATE,
@@ -1085,9 +1102,6 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
             else if (s->shape_soft)
                 HMC_CUDA(launch_sweep_poly2_soft(s->sat(), s->geom, s->arr, s->verts, s->n_vertices, s->so, L,
                                                  s->stream));
-            else if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON)
-                HMC_CUDA(launch_sweep_poly(fp32, s->geom, s->arr, s->verts, s->n_vertices, s->poly_rcut2,
-                                           s->poly_rcut2_hi32, L, p->move == HMC_ROTATE, s->stream, sp.variant));
             else if (s->polygon())
                 HMC_CUDA(launch_sweep_poly2(sp.poly2_fp32, s->sat(), s->geom, s->arr, s->verts, s->n_vertices,
                                             s->poly_rcut2, s->poly_rcut2_hi32, L, p->move == HMC_ROTATE, s->stream));
@@ -1752,6 +1766,7 @@ static hmc_status pair_histogram(hmc_system* s, bool sdf, double sigma, double l
     g.any_two = 0;
     for (int a = 0; a < s->dim; ++a) {
         g.w32[a] = (float)g.width[a];
+        g.fix[a] = (float)std::ldexp(g.L[a], -32);
         g.invW[a] = 1.0 / g.width[a];
         g.half_shape[a] = g.shape[a] / 2;
         if (g.shape[a] == 2) g.any_two = 1;
@@ -2646,6 +2661,7 @@ hmc_status hmc_batch_create(hmc_context* ctx, uint32_t n_replicas, const hmc_sys
             r.g.ghost_hi[a] = r.g.half[a] - boundary_range;
             r.g.ghost_lo[a] = -r.g.half[a] + boundary_range;
             r.g.w32[a] = (float)r.g.width[a];
+            r.g.fix[a] = (float)std::ldexp(r.g.L[a], -32);
             r.g.invL[a] = 1.0 / r.g.L[a];
             r.g.invW[a] = 1.0 / r.g.width[a];
             r.g.half_shape[a] = r.g.shape[a] / 2;
@@ -3208,6 +3224,7 @@ hmc_status hmc_batch_sdf(hmc_batch* bt, double x_max, uint32_t n_bins, uint64_t*
         g.any_two = 0;
         for (int a = 0; a < bt->dim; ++a) {
             g.w32[a] = (float)g.width[a];
+            g.fix[a] = (float)std::ldexp(g.L[a], -32);
             g.invW[a] = 1.0 / g.width[a];
             g.half_shape[a] = g.shape[a] / 2;
             if (g.shape[a] == 2) g.any_two = 1;

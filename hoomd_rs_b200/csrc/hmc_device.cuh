@@ -54,10 +54,10 @@ __device__ __forceinline__ float4 cell_offsets(const Geometry& g, const double* 
     return make_float4(o[0], o[1], o[2], __int_as_float((int)m[DIM - 1]));
 }
 
-// Lennard-Jones FP32 sites: per axis the site's place in the box in units of L / 2^32, as 32-bit
+// Fixed-point sites (Lennard-Jones, polyhedra): per axis the site's place in the box in units of L / 2^32, as 32-bit
 // integers whose differences wrap to the minimum image. The difference of two such sites is exact up
 // to their own roundings (half a unit each), needs no cell shift, and rounds once more on its
-// way to FP32 (lj_fix: L / 2^32 per axis).
+// way to FP32 (Geometry::fix: L / 2^32 per axis).
 __device__ __forceinline__ int fixed_axis(double invL, double s) {
     return (int)(uint32_t)__double2ll_rn(dmul(dmul(s, invL), 4294967296.0));
 }
@@ -67,12 +67,12 @@ __device__ __forceinline__ int4 fixed_site(const Geometry& g, const double* s) {
                      DIM == 3 ? fixed_axis(g.invL[2], s[2]) : 0, 0);
 }
 template <int DIM>
-__device__ __forceinline__ float fixed_dist2(const Pair& P, const int4& a, const int4& b) {
-    const float x = (float)(int)((uint32_t)a.x - (uint32_t)b.x) * P.lj_fix[0];
-    const float y = (float)(int)((uint32_t)a.y - (uint32_t)b.y) * P.lj_fix[1];
+__device__ __forceinline__ float fixed_dist2(const Geometry& g, const int4& a, const int4& b) {
+    const float x = (float)(int)((uint32_t)a.x - (uint32_t)b.x) * g.fix[0];
+    const float y = (float)(int)((uint32_t)a.y - (uint32_t)b.y) * g.fix[1];
     float r2 = x * x + y * y;
     if (DIM == 3) {
-        const float z = (float)(int)((uint32_t)a.z - (uint32_t)b.z) * P.lj_fix[2];
+        const float z = (float)(int)((uint32_t)a.z - (uint32_t)b.z) * g.fix[2];
         r2 += z * z;
     }
     return r2;

@@ -25,43 +25,60 @@
 
 namespace hmc {
 
-// The colour sets [r0, r1) one launch runs, and where its trials stand. `draws` entry e of the
-// trial with number e (k_draw_*): what the trial's random stream gives, which depends on no site.
+// The colour sets [r0, r1) one launch runs, and where its trials stand: trial number e is entry e of
+// the draws (k_draw_*: what the trial's random stream gives, which depends on no site). A kernel
+// whose warps take several trials at a time takes units of `group` trials of one colour, numbered
+// in the same order (trials of two colours may touch and cannot wait for one another in one warp).
 struct FlowRange {
     uint32_t r0, r1;
-    uint32_t prefix[8];  // trials of the colours before colour c in one colour set
-    uint32_t per_set;    // trials of one colour set
-    uint32_t n;          // trials of the range
+    uint32_t count[8];   // trials of colour c in one colour set
+    uint32_t prefix[8];  // of the colours before c
+    uint32_t per_set;    // of one colour set
+    uint32_t n;          // of the range
+    uint32_t unit_prefix[8], units_per_set, n_units;
 };
 
 __device__ __forceinline__ FlowRange flow_range(const DeviceStats* st, uint32_t round, uint32_t round_end,
-                                                uint32_t colors) {
+                                                uint32_t colors, uint32_t group = 1) {
     FlowRange f;
     f.r0 = round;
     f.r1 = min(round_end, st->rounds);
-    f.per_set = 0;
+    f.per_set = f.units_per_set = 0;
 #pragma unroll
     for (uint32_t c = 0; c < 8; ++c) {
         f.prefix[c] = f.per_set;
-        if (c < colors) f.per_set += st->color_count[c];
+        f.unit_prefix[c] = f.units_per_set;
+        f.count[c] = c < colors ? st->color_count[c] : 0u;
+        f.per_set += f.count[c];
+        f.units_per_set += (f.count[c] + group - 1u) / group;
     }
-    f.n = st->error_flags != 0u || f.r1 <= f.r0 ? 0u : (f.r1 - f.r0) * f.per_set;
+    const uint32_t sets = st->error_flags != 0u || f.r1 <= f.r0 ? 0u : f.r1 - f.r0;
+    f.n = sets * f.per_set;
+    f.n_units = sets * f.units_per_set;
     return f;
 }
 
-// Trial number e: its colour set (absolute), colour and place in the colour's list.
-__device__ __forceinline__ void flow_item(const FlowRange& f, uint32_t e, uint32_t& round, uint32_t& color,
-                                          uint32_t& entry) {
-    const uint32_t s = e / f.per_set, rem = e - s * f.per_set;
-    round = f.r0 + s;
+// Number e in a range with these prefixes: its colour set (absolute), colour and place in the colour.
+__device__ __forceinline__ void flow_place(uint32_t r0, const uint32_t* prefix, uint32_t per_set, uint32_t e,
+                                           uint32_t& round, uint32_t& color, uint32_t& entry) {
+    const uint32_t s = e / per_set, rem = e - s * per_set;
+    round = r0 + s;
     color = 0;
     entry = rem;
 #pragma unroll
     for (uint32_t c = 1; c < 8; ++c)
-        if (rem >= f.prefix[c] && f.prefix[c] < f.per_set) {
+        if (rem >= prefix[c] && prefix[c] < per_set) {
             color = c;
-            entry = rem - f.prefix[c];
+            entry = rem - prefix[c];
         }
+}
+__device__ __forceinline__ void flow_item(const FlowRange& f, uint32_t e, uint32_t& round, uint32_t& color,
+                                          uint32_t& entry) {
+    flow_place(f.r0, f.prefix, f.per_set, e, round, color, entry);
+}
+__device__ __forceinline__ void flow_unit(const FlowRange& f, uint32_t u, uint32_t& round, uint32_t& color,
+                                          uint32_t& entry) {
+    flow_place(f.r0, f.unit_prefix, f.units_per_set, u, round, color, entry);
 }
 
 __device__ __forceinline__ uint32_t load_acquire(const uint32_t* p) {
@@ -116,7 +133,7 @@ __device__ __forceinline__ void flow_need(const Geometry& g, const uint32_t* m, 
 // left, except at the list's two ends, which touch across the periodic boundary: the first trials
 // of a colour would wait for the last of the colour before. Every colour therefore starts two
 // spaces of the slow axis (one of its own planes) further on than the colour before.
-__device__ __forceinline__ uint32_t flow_rotated(const FlowRange& f, uint32_t count, uint32_t round, uint32_t color,
+__device__ __forceinline__ uint32_t flow_rotated(uint32_t count, uint32_t round, uint32_t color,
                                                  uint32_t colors, uint32_t planes, uint32_t entry) {
     const uint32_t level = (round * colors + color) % (planes / 2u);  // planes is even
     const uint32_t shift = (uint32_t)((uint64_t)count * level / (planes / 2u));
@@ -133,6 +150,42 @@ __device__ __forceinline__ bool flow_wait(const uint32_t* word, uint32_t need, u
     for (uint32_t spins = 0;; ++spins) {
         if (!ok) ok = load_acquire(word) >= need;
         if ((__ballot_sync(full, ok) & lanes) == lanes) return true;
+        __nanosleep(20);
+        if ((spins & 1023u) == 1023u) {
+            const unsigned long long now = global_ns();
+            if (t0 == 0) t0 = now;
+            bool stop = *(volatile unsigned int*)&stats->error_flags != 0u;
+            if (now - t0 > kFlowWaitNs) {
+                atomicOr(&stats->error_flags, kErrFlowTimeout);
+                stop = true;
+            }
+            if (__any_sync(full, stop)) return false;
+        }
+    }
+}
+
+// The same for lanes with up to N words each (bit i of pending: word words[first + i * stride] is
+// still short): returns once no lane has a pending word among those of `mask`.
+template <uint32_t N>
+__device__ __forceinline__ bool flow_wait_words(const uint32_t* progress, const uint2* words, uint32_t first,
+                                           uint32_t stride, unsigned& pending, unsigned mask, DeviceStats* stats) {
+    const unsigned full = 0xffffffffu;
+    unsigned long long t0 = 0;
+    for (uint32_t spins = 0;; ++spins) {
+        uint32_t v[N], need[N];
+#pragma unroll
+        for (uint32_t i = 0; i < N; ++i) {
+            v[i] = need[i] = 0;
+            if ((pending >> i) & 1u) {
+                const uint2 w = words[first + i * stride];
+                need[i] = w.y;
+                v[i] = load_acquire(progress + w.x);
+            }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < N; ++i)
+            if (v[i] >= need[i]) pending &= ~(1u << i);
+        if (!__any_sync(full, (pending & mask) != 0u)) return true;
         __nanosleep(20);
         if ((spins & 1023u) == 1023u) {
             const unsigned long long now = global_ns();

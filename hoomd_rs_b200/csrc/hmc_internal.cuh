@@ -47,6 +47,7 @@ struct Geometry {
     double invL[3];     // RN(1 / L), for div_fixed
     double invW[3];     // RN(1 / width), for div_fixed
     float w32[3];       // width rounded to FP32
+    float fix[3];       // L / 2^32 (fixed_site)
     uint32_t shape[3];  // spaces per axis (even)
     uint32_t half_shape[3];
     uint32_t n_cells;
@@ -90,7 +91,7 @@ struct Arrays {
     double4* draw_d;
     uint4* draw_i;
     uint32_t* progress;      // [cells]
-    uint32_t fixed_sites;    // Lennard-Jones: sorted_off holds fixed-point sites
+    uint32_t fixed_sites;    // Lennard-Jones and polyhedra: sorted_off holds fixed-point sites
 };
 constexpr uint32_t kNoTrial = 0xffffffffu;
 
@@ -112,7 +113,6 @@ struct Pair {
     float lj_rcut2_hi32;  // r_cut^2 plus the bound: at or above, outside for certain
     float lj_disp_err;    // per-axis FP32 displacement error bound E
     float lj_rel_err;     // the part of the FP32 r^2 error that grows with r^2, as a fraction of it
-    float lj_fix[3];      // L / 2^32 per axis (fixed_site)
     float lj_band_energy; // bound on |pair energy| for a pair inside the cut-off band
     // Isotropic<Expanded<OverlapPenalty>> (overlap_penalty.rs:109-115, expanded.rs:64-66):
     // r^2 >= r_cut^2 -> 0; x = sqrt(r^2) - delta; x < -d_max -> inf; x < 0 -> (0.5 k) x^2 + eps
@@ -313,7 +313,7 @@ constexpr LaunchShape kSphereCoopShapes[] = {{6, 1, 2}, {6, 1, 1}, {6, 1, 3}, {5
 // Lennard-Jones and Isotropic trials; own_steps: warps per trial (variant 0: by the trials of a
 // colour)
 constexpr LaunchShape kLjShapes[] = {{0, 1, 0}, {6, 1, 1}, {12, 1, 2}, {6, 1, 4}, {3, 1, 8}};
-constexpr LaunchShape kPolyShapes[] = {{5, 4, 0}, {5, 2, 0}, {5, 8, 0}};
+constexpr LaunchShape kPolyShapes[] = {{4, 4, 0}, {3, 4, 0}};
 constexpr LaunchShape kBatchShapes[] = {{4, 1, 0}, {3, 1, 0}, {5, 1, 0}, {6, 1, 0}, {7, 1, 0}, {8, 1, 0}};
 // The polygon pass: one compiled shape; in the FP32 mode, variant 1 runs the FP64 pass instead
 // of the FP32 prefilter (the same decisions; the prefilter saves little where the FP64
@@ -328,7 +328,7 @@ constexpr uint32_t n_shapes(const LaunchShape (&)[N]) {
 
 // Blocks in one resident wave of a kernel with `threads` per block on the current device (SMs x
 // resident blocks per SM), cached per kernel.
-int resident_wave(const void* kernel, int threads = 128);
+int resident_wave(const void* kernel, int threads = 128, size_t dynamic_bytes = 0);
 
 // Launch configuration of a colour pass: 128 threads per block; overlap = programmatic
 // dependent launch after the previous colour pass of the same sweep (the kernel waits with
@@ -451,8 +451,7 @@ cudaError_t launch_flow_lj(int dim, bool fp32, bool generic, const Geometry& g, 
 // per trial; launched in stream order before the round's colour passes of the passes that give a
 // trial several lanes (convex polyhedra, convex polygons).
 // soft: the trial also draws the Metropolis uniform after the move (trial_t.w in 3-D, .z in 2-D).
-cudaError_t launch_propose_poly(bool fp32, const Geometry& g, const Arrays& a, const Launch& l, bool rotate,
-                                bool soft, cudaStream_t s);
+cudaError_t launch_propose_poly(const Geometry& g, const Arrays& a, const Launch& l, bool rotate, cudaStream_t s);
 cudaError_t launch_propose_poly2(bool fp32, const Geometry& g, const Arrays& a, const Launch& l, bool rotate,
                                  bool soft, cudaStream_t s);
 
@@ -491,9 +490,10 @@ cudaError_t launch_eval_lj(int dim, bool fp32, const Geometry& g, const Arrays& 
                            uint8_t* decisions, uint8_t* rechecked, double* delta_h, cudaStream_t s);
 cudaError_t launch_energy_lj(int dim, const Geometry& g, const Arrays& a, const Pair& p, uint32_t n, double* out,
                              cudaStream_t s);
-cudaError_t launch_sweep_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
-                              double rcut2, float rcut2_hi32, const Launch& l, bool rotate, cudaStream_t s,
-                              uint32_t variant = 0);
+// Hard convex polyhedra: the colour sets [l.round, l.round_end), two kernels as in launch_flow_lj.
+cudaError_t launch_flow_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
+                             double rcut2, float rcut2_hi32, const Launch& l, bool rotate, cudaStream_t s,
+                             uint32_t variant = 0);
 cudaError_t launch_eval_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
                              double rcut2, float rcut2_hi32, const uint64_t* bodies, const double4* trial,
                              const double4* trial_q, uint32_t n, uint8_t* decisions, cudaStream_t s);

@@ -1948,7 +1948,7 @@ SphereKernel coop_kernel(int dim, bool fp32, uint32_t v) {
 
 }  // namespace
 
-int resident_wave(const void* kernel, int threads) {
+int resident_wave(const void* kernel, int threads, size_t dynamic_bytes) {
     static std::mutex mu;
     static std::unordered_map<const void*, int> cache;
     int dev = 0;
@@ -1959,7 +1959,7 @@ int resident_wave(const void* kernel, int threads) {
     if (it != cache.end()) return it->second;
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, dynamic_bytes) != cudaSuccess) {
         cudaGetLastError();
         per_sm = 1;
     }

@@ -104,7 +104,7 @@ struct Sums32 {
 // FP32 energies of the trial site t32 and the current site c32 (fixed_site) against the stencil fs
 // of their common space, with error bounds (hmc_eval_moves).
 template <int DIM>
-__device__ __forceinline__ Sums32 lj_energy32(const Arrays& A, const Pair& P, const int4& t32, const int4& c32,
+__device__ __forceinline__ Sums32 lj_energy32(const Geometry& g, const Arrays& A, const Pair& P, const int4& t32, const int4& c32,
                                                const FlatStencil& fs, uint32_t self, uint32_t lane) {
     Sums32 s{0.f, 0.f, 0.f, 0.f, 0u};
 #pragma unroll 1
@@ -114,7 +114,7 @@ __device__ __forceinline__ Sums32 lj_energy32(const Arrays& A, const Pair& P, co
         const uint32_t q = flat_slot(fs, j, part);
         if (j >= fs.total || q == self) continue;
         const int4 o = __ldg(reinterpret_cast<const int4*>(A.sorted_off) + q);
-        const float r2[2] = {fixed_dist2<DIM>(P, t32, o), fixed_dist2<DIM>(P, c32, o)};
+        const float r2[2] = {fixed_dist2<DIM>(g, t32, o), fixed_dist2<DIM>(g, c32, o)};
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             if (!(r2[i] < P.lj_rcut2_hi32)) continue;
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(128) k_draw_lj(Geometry g, Arrays A, Launch L,
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += gridDim.x * blockDim.x) {
         uint32_t round, color, entry;
         flow_item(f, i, round, color, entry);
-        if (!BATCH) entry = flow_rotated(f, A.stats->color_count[color], round, color, 1u << DIM, g.shape[0], entry);
+        if (!BATCH) entry = flow_rotated(A.stats->color_count[color], round, color, 1u << DIM, g.shape[0], entry);
         const size_t e = (size_t)color * stride + entry;
         const uint32_t packed = __ldg(A.color_cells + e);
         uint32_t m[3] = {0, 0, 0};
@@ -289,7 +289,7 @@ __device__ __forceinline__ void team_stage(const Arrays& A, uint32_t c0, uint32_
 // lane busy (two evaluations per trial instead of one per 32 candidates with five lanes). `phase`:
 // the parity of the staging barrier, the first chunk already on its way.
 template <int DIM, int W, typename T>
-__device__ __forceinline__ void lj_delta32(const Arrays& A, const Pair& P, uint32_t lane, uint32_t warp, T& S,
+__device__ __forceinline__ void lj_delta32(const Geometry& g, const Arrays& A, const Pair& P, uint32_t lane, uint32_t warp, T& S,
                                            uint32_t& phase, float& d32, float& bound) {
     const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
     float2* list = S.list[warp].q32;
@@ -327,7 +327,7 @@ __device__ __forceinline__ void lj_delta32(const Arrays& A, const Pair& P, uint3
         for (uint32_t j0 = 32u * warp; j0 < n; j0 += 32u * W) {
             const uint32_t j = j0 + lane;
             const int4 o = S.site[j];  // (j < kStage; stale beyond n)
-            const float rn = fixed_dist2<DIM>(P, t32, o), ro = fixed_dist2<DIM>(P, s32, o);
+            const float rn = fixed_dist2<DIM>(g, t32, o), ro = fixed_dist2<DIM>(g, s32, o);
             const bool need = fminf(rn, ro) < cut2 && j < n && j != self;
             const unsigned b = __ballot_sync(full, need);
             if (need) list[listed + __popc(b & below)] = make_float2(rn, ro);
@@ -472,7 +472,7 @@ __device__ __forceinline__ bool lj_decide(const Geometry& g, const Arrays& A, co
     float d32 = 0.f;
     if constexpr (FP32) {
         float b;
-        lj_delta32<DIM, W>(A, P, lane, warp, S, phase, d32, b);
+        lj_delta32<DIM, W>(g, A, P, lane, warp, S, phase, d32, b);
         if (lane == 0 && warp == 0) pst.checks += 2u * (S.total - 1u);
         const float lo = __fsub_rd(d32, b), hi = __fadd_ru(d32, b);
         if (hi <= 0.f) return true;  // dU64 <= 0 for certain: accepted without a uniform
@@ -737,7 +737,7 @@ __global__ void __launch_bounds__(128) k_eval_lj(Geometry g, Arrays A, Pair P, c
                 const bool same = mt[0] == mi[0] && mt[1] == mi[1] && (DIM == 2 || mt[2] == mi[2]);
                 if (same) {
                     const int4 c32 = __ldg(reinterpret_cast<const int4*>(A.sorted_off) + k);
-                    const Sums32 s = lj_energy32<DIM>(A, P, fixed_site<DIM>(g, t), c32, ft, k, lane);
+                    const Sums32 s = lj_energy32<DIM>(g, A, P, fixed_site<DIM>(g, t), c32, ft, k, lane);
                     const float d32 = s.e_new - s.e_old;
                     const float b = s.err + (float)(s.terms + 7) * kU32 * s.mag * 1.01f + kU32 * fabsf(d32) +
                                     1e-9f * (s.mag + 1.f);

@@ -17,20 +17,13 @@
 // decisions equal the FP64 pass.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
+#include "hmc_flow.cuh"
 #include "hmc_serial.cuh"
 
 namespace hmc {
 namespace {
-
-// The colour pass takes kPolyTrialsPerWarp trials per warp and is compiled for
-// HMC_POLY_MIN_BLOCKS resident blocks per SM (96 registers). On 2^18 hard cubes at packing
-// fraction 0.55 (10,648 trials per colour pass) this measured 1.69e8 (FP32 prefilter) and
-// 1.58e8 (FP64) trial moves/s, against 7.9e7 and 8.3e7 with one warp per trial, 1.38e8 and
-// 1.26e8 with 8 trials per warp, 1.48e8 and 1.43e8 with 4 trials at 80 registers.
-#ifndef HMC_POLY_MIN_BLOCKS
-#define HMC_POLY_MIN_BLOCKS 5
-#endif
-constexpr int kPolyTrialsPerWarp = 4;
 
 struct Q {
     double s, x, y, z;
@@ -212,9 +205,9 @@ __device__ __forceinline__ bool poly_overlap64(const Geometry& g, const Arrays& 
 }
 
 // Rotate<Versor>::propose (rotate/versor.rs:40-71, 112-123): Gaussian rotation vector with
-// standard deviation sigma, rejected beyond pi, lifted by the exponential map, composed in
-// front of the current orientation.
-__device__ __forceinline__ Q versor_move(Sfc64& rng, double sigma, const double* zx, const double* zf, const Q& q) {
+// standard deviation sigma, rejected beyond pi, lifted by the exponential map (versor_draw), composed
+// in front of the current orientation.
+__device__ __forceinline__ Q versor_draw(Sfc64& rng, double sigma, const double* zx, const double* zf) {
     for (;;) {
         double s0 = dadd(0.0, dmul(sigma, standard_normal(rng, zx, zf)));
         double s1 = dadd(0.0, dmul(sigma, standard_normal(rng, zx, zf)));
@@ -226,9 +219,11 @@ __device__ __forceinline__ Q versor_move(Sfc64& rng, double sigma, const double*
         portable_sincos(dmul(0.5, theta), &sh, &ch);
         double vf = ddiv(sh, theta);
         if (!isfinite(vf)) vf = 0.5;
-        const Q dq{ch, dmul(s0, vf), dmul(s1, vf), dmul(s2, vf)};
-        return qmul(dq, q);
+        return Q{ch, dmul(s0, vf), dmul(s1, vf), dmul(s2, vf)};
     }
+}
+__device__ __forceinline__ Q versor_move(Sfc64& rng, double sigma, const double* zx, const double* zf, const Q& q) {
+    return qmul(versor_draw(rng, sigma, zx, zf), q);
 }
 
 struct PolyShape {
@@ -236,48 +231,36 @@ struct PolyShape {
     uint32_t nv;
     double rcut2;     // (R_a + R_b)^2
     float rcut2_hi32; // FP32 threshold: at or above this, outside the circumsphere for certain
+    float site_err;   // per-axis error of a displacement of fixed-point sites beyond its FP32 roundings
 };
 
 __device__ __forceinline__ bool warp_any(bool v) { return __any_sync(0xffffffffu, v); }
 
-// Overlap of the trial (t, qi; FP32 offsets t32) with any candidate of the stencil fs,
-// skipping slot self. The warp takes the stencil's candidates 32 at a time across its rows
-// (at the bench's density one step holds the whole stencil, so the lanes that need the full
-// test run it together), and a vote after each step stops the warp at the first overlap.
-// FP32: the circumsphere prefilter in FP32 under the bound.
+// Overlap of the trial (t, qi; fixed-point site t32) with any candidate of the stencil fs,
+// skipping slot self (injected moves, the tuner). The warp takes the stencil's candidates 32 at a
+// time across its rows, and a vote after each step stops the warp at the first overlap. FP32: the
+// circumsphere prefilter in FP32 under the bound.
 template <bool FP32>
 __device__ __forceinline__ bool poly_overlaps(const Geometry& g, const Arrays& A, const PolyShape& sh, const double* t,
-                                              const Q& qi, float4 t32, int mf, const FlatStencil& fs, uint32_t self,
+                                              const Q& qi, const int4& t32, const FlatStencil& fs, uint32_t self,
                                               uint32_t lane, PairStats& st) {
-    const uint32_t sf = g.shape[2];
 #pragma unroll 1
     for (uint32_t j0 = 0; j0 < fs.total; j0 += 32) {
         const uint32_t j = j0 + lane;
         uint32_t part;
         const uint32_t q = flat_slot(fs, j, part);
-        const float s0 = __shfl_sync(0xffffffffu, fs.s0, part);
-        const float s1 = __shfl_sync(0xffffffffu, fs.s1, part);
         bool hit = false;
         if (j < fs.total && q != self) {
             bool test = true;
+            st.checks++;
             if (FP32) {
-                const float4 o = __ldg(A.sorted_off + q);
-                int dm = __float_as_int(o.w) - mf;
-                if (sf >= 4) {
-                    if (dm > 1)
-                        dm -= (int)sf;
-                    else if (dm < -1)
-                        dm += (int)sf;
-                }
-                st.checks++;
-                test = fp32_dist2<3>(g, t32, o, s0, s1, dm) < sh.rcut2_hi32;
+                test = fixed_dist2<3>(g, t32, __ldg(reinterpret_cast<const int4*>(A.sorted_off) + q)) < sh.rcut2_hi32;
                 if (test) st.rechecks++;
             }
             if (test) {
                 // shapes keep S in both precision modes (the FP32 pass only prefilters)
                 const double4 s4 = ldg4(A.sorted_s + q);
                 const double sj[3] = {s4.x, s4.y, s4.z};
-                if (!FP32) st.checks++;
                 hit = poly_overlap64(g, A, sh.verts, sh.nv, sh.rcut2, t, qi, sj, q);
             }
         }
@@ -286,55 +269,12 @@ __device__ __forceinline__ bool poly_overlaps(const Geometry& g, const Arrays& A
     return false;
 }
 
-// ---- the colour pass, G trials per warp -----------------------------------------------------
-// A trial's candidates mostly clear the circumsphere; the few that do not need the full FP64
-// test (XenoCollide, thousands of instructions). With one warp per trial that test runs with a
-// handful of lanes active. Here a warp takes G trials (32/G lanes each): every group computes
-// its trial, walks its stencil with the circumsphere test, and the candidates that need the
-// full test are compacted over the whole warp into a shared-memory list; the warp then runs
-// the full tests 32 pairs at a time and ORs the overlaps into a per-trial mask. Candidates of a
-// trial already known to overlap are skipped. The decision of each trial is the OR of the same
-// pair tests as in the warp-per-trial pass, so the trajectory is the same.
-struct PolyTrial {
-    double t[3];
-    double q[4];  // s, x, y, z
-};
-
-constexpr uint32_t kPairCap = 128;  // listed pairs per warp before the warp drains the list
-
-template <int G>
-__device__ __forceinline__ void drain_pairs(const Geometry& g, const Arrays& A, const PolyShape& sh,
-                                            const PolyTrial* trials, const uint32_t* pair_q, const uint8_t* pair_g,
-                                            uint32_t n_pairs, uint32_t lane, uint32_t& mask) {
-    __syncwarp();
-    for (uint32_t p0 = 0; p0 < n_pairs; p0 += 32) {
-        const uint32_t p = p0 + lane;
-        uint32_t bit = 0;
-        if (p < n_pairs) {
-            const uint32_t gg = pair_g[p];
-            if (!((mask >> gg) & 1u)) {
-                const uint32_t q = pair_q[p];
-                const PolyTrial& tr = trials[gg];
-                const double t[3] = {tr.t[0], tr.t[1], tr.t[2]};
-                const Q qi{tr.q[0], tr.q[1], tr.q[2], tr.q[3]};
-                const double4 s4 = ldg4(A.sorted_s + q);
-                const double sj[3] = {s4.x, s4.y, s4.z};
-                if (poly_overlap64(g, A, sh.verts, sh.nv, sh.rcut2, t, qi, sj, q)) bit = 1u << gg;
-            }
-        }
-        mask |= __reduce_or_sync(0xffffffffu, bit);
-    }
-    __syncwarp();
-}
-
 // A round's trial moves of convex polyhedra for every colour list (generate_trial_moves,
 // parallel_sweep.rs:231-278, up to delta_energy_one), one thread per trial: the chosen body,
 // Translate (Ball::sample) or Rotate<Versor>, W1 = wrap(propose(..)), the space check, the trial
 // site T = wrap(W1) and its FP32 offsets; the packed pass reads them instead of computing each
 // move on the 8 lanes of its group.
-template <bool FP32>
-__global__ void __launch_bounds__(128) k_propose_poly3(Geometry g, Arrays A, Launch L, uint32_t rotate,
-                                                       uint32_t soft) {
+__global__ void __launch_bounds__(128) k_propose_poly3(Geometry g, Arrays A, Launch L, uint32_t rotate) {
     const DeviceStats* st = A.stats;
     if (st->error_flags != 0u || L.round >= st->rounds) return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 8u * g.color_stride; i += gridDim.x * blockDim.x) {
@@ -358,8 +298,7 @@ __global__ void __launch_bounds__(128) k_propose_poly3(Geometry g, Arrays A, Lau
             ball_sample<3>(rng, L.max_move, A.zig_x, A.zig_f, dv);
             for (int a = 0; a < 3; ++a) x[a] = dadd(x[a], dv[a]);
         }
-        // soft: the Metropolis uniform, the stream's next draw after the move
-        const double u = soft ? uniform01(rng) : 0.0;
+        const double u = uniform01(rng);  // the Metropolis uniform, the stream's next draw after the move
         wrap_inv<3>(g.L, g.invL, x);  // W1 = wrap(propose(..))
         uint32_t mt[3];
         if (!(point_to_space<3>(g, x, mt) && cell_index<3>(g, mt) == cell)) {
@@ -370,150 +309,646 @@ __global__ void __launch_bounds__(128) k_propose_poly3(Geometry g, Arrays A, Lau
         wrap_inv<3>(g.L, g.invL, t);
         A.trial_t[i] = make_double4(t[0], t[1], t[2], u);
         A.trial_q[i] = make_double4(qi.s, qi.x, qi.y, qi.z);
-        if (FP32) A.trial_o[i] = cell_offsets<3>(g, t, m);
         A.trial_k[i] = k;
     }
 }
 
-// INJ: the probe mode (Injected): group trial w is injected trial w, walked around the space of
-// its W1, and its decision is written instead of committed.
-template <bool FP32, int G, bool INJ = false>
-__global__ void __launch_bounds__(128, HMC_POLY_MIN_BLOCKS)
-    k_sweep_poly3_packed(Geometry g, Arrays A, PolyShape sh, Launch L, uint32_t rotate, Injected J) {
-    static_assert(G == 2 || G == 4 || G == 8, "G trials per warp");
-    constexpr uint32_t S = 32 / G;  // lanes per trial
-    if (L.early_wait) grid_dependency_wait();  // first pass: the rebuild's arrays are read at once
-    __shared__ PolyTrial s_trial[4][G];
-    __shared__ uint32_t s_pair_q[4][kPairCap];
-    __shared__ uint8_t s_pair_g[4][kPairCap];
-    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    const uint32_t grp = lane / S, sub = lane % S;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+// ---- the sweep --------------------------------------------------------------------------------
+// What the random streams of the trials of colour sets [L.round, L.round_end) give, one thread per
+// trial (generate_trial_moves, parallel_sweep.rs:231-278): the chosen body's slot and space in
+// draw_i, and in draw_d the displacement (Ball::sample) or the rotation's versor (Rotate<Versor>), which
+// depend on no site. Each space's progress is set to the first colour set; the ticket starts at 0.
+__global__ void __launch_bounds__(128) k_draw_poly3(Geometry g, Arrays A, Launch L, uint32_t rotate) {
+    grid_dependency_wait();
+    allow_dependent_launch();
+    const FlowRange f = flow_range(A.stats, L.round, L.round_end, 8);
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.stats->ticket = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += gridDim.x * blockDim.x) {
+        uint32_t round, color, entry;
+        flow_item(f, i, round, color, entry);
+        entry = flow_rotated(A.stats->color_count[color], round, color, 8, g.shape[0], entry);
+        const uint32_t packed = __ldg(A.color_cells + (size_t)color * g.color_stride + entry);
+        uint32_t m[3];
+        unpack_m<3>(packed, m);
+        const uint32_t cell = cell_index<3>(g, m);
+        if (round == f.r0) A.progress[cell] = f.r0;
+        const uint32_t start = __ldg(A.cell_start + cell);
+        const uint32_t count = __ldg(A.cell_start + cell + 1) - start;
+        Sfc64 rng = make_rng(L.step, L.substep + round, L.seed, (uint64_t)cell);
+        const uint32_t k = start + canon_range_u32(rng, count);
+        double4 d;
+        if (rotate) {
+            const Q dq = versor_draw(rng, L.max_move, A.zig_x, A.zig_f);
+            d = make_double4(dq.s, dq.x, dq.y, dq.z);
+        } else {
+            double dv[3];
+            ball_sample<3>(rng, L.max_move, A.zig_x, A.zig_f, dv);
+            d = make_double4(dv[0], dv[1], dv[2], 0.0);
+        }
+        A.draw_d[i] = d;
+        A.draw_i[i] = make_uint4(k, packed, 0u, 0u);
+    }
+}
+
+// The shape's vertices in a block's shared memory: FP64 for the support mapping's values, FP32 to
+// find which vertex it is, with the largest coordinate.
+struct ShapeTable {
+    float4 v32[32];
+    double v[32][3];
+    uint32_t nv;
+    float vmax;
+};
+
+// ConvexPolytope::support_mapping (support above): which vertex has the first maximum of ((v0 n0) + v1
+// n1) + v2 n2.
+__device__ __noinline__ uint32_t support64(const ShapeTable& T, V3 n) {
+    uint32_t arg = 0;
+    double best = -INFINITY;
+    for (uint32_t i = 0; i < T.nv; ++i) {
+        const double x = dadd(dadd(dmul(T.v[i][0], n.x), dmul(T.v[i][1], n.y)), dmul(T.v[i][2], n.z));
+        if (x > best) {
+            best = x;
+            arg = i;
+        }
+    }
+    return arg;
+}
+
+// One pair test in steps: XenoCollide (collide3d) written so that every step is one composite support
+// mapping followed by the little that depends on the phase; the lanes of a warp then share the
+// support mappings, which are nearly all of the work, whatever phase each is in.
+struct PairLane {
+    V3 v0, p0, p1, p2, n;  // v0; the portal; the direction of the next support mapping
+    M3 q;                  // orientation of the other shape in the trial's frame
+    uint32_t phase, count;
+};
+
+// composite_support_mapping (xenocollide.rs:318-328) in direction n by the two lanes of a pair test:
+// role 0 finds the trial shape's vertex in direction -n, role 1 the other's in direction q^T n.
+// FP32: the vertex is looked for in FP32 first: with |v_a| <= vmax, vertices and direction components
+// rounded once and three roundings per sum, a product is off by at most 6 u32 vmax |n|_1 (role 1:
+// |q^T n|_1 <= sqrt(3) |n|_1: by 11), so a maximum ahead of the runner-up by more than
+// 64 u32 vmax |n|_1 is the FP64 maximum too; else (ties, as along the edges of a portal) the FP64
+// products decide. FP32 takes 8 instructions per vertex against 17 (FP64 issues at half rate).
+template <bool FP32>
+__device__ __forceinline__ V3 pair_support(const ShapeTable& T, const M3& q, const V3& vij, const V3& n, uint32_t role,
+                                           unsigned active) {
+    const V3 dir = role ? mat_rotate(transpose(q), n) : neg3(n);
+    uint32_t mine = 0;
+    if constexpr (FP32) {
+        const float x = (float)dir.x, y = (float)dir.y, z = (float)dir.z;
+        float first = -INFINITY, second = -INFINITY;
+#pragma unroll 4
+        for (uint32_t i = 0; i < T.nv; ++i) {
+            const float4 v = T.v32[i];
+            const float p = v.x * x + v.y * y + v.z * z;
+            second = fmaxf(second, fminf(first, p));
+            mine = p > first ? i : mine;
+            first = fmaxf(first, p);
+        }
+        const float gap = 64.f * 5.9604645e-8f * 1.01f * T.vmax * (fabsf((float)n.x) + fabsf((float)n.y) + fabsf((float)n.z)) + 1e-35f;
+        if (!(first - second > gap)) mine = support64(T, dir);
+    } else {
+        mine = support64(T, dir);
+    }
+    const uint32_t other = __shfl_xor_sync(active, mine, 1);
+    const uint32_t ia = role ? other : mine, ib = role ? mine : other;
+    V3 r = mat_rotate(q, V3{T.v[ib][0], T.v[ib][1], T.v[ib][2]});
+    r = {dadd(r.x, vij.x), dadd(r.y, vij.y), dadd(r.z, vij.z)};
+    return sub3(r, V3{T.v[ia][0], T.v[ia][1], T.v[ia][2]});
+}
+
+// The step after a support mapping v: -1 undecided (s.n: the next direction), else the result. The
+// phases are collide3d's: 0 the first support, 1 the second, 2 portal discovery (p0, p1, p2 = v1, v2,
+// v3), 3 portal refinement. Each expression is collide3d's own; lanes in different phases share the
+// first test (in phase 0 n = -v0, and v . v0 > 0 is v . n < 0, the products being exactly negated)
+// and the portal's normal.
+__device__ __forceinline__ int pair_step(PairLane& s, const V3& v) {
+    const double TOL = 2e-12;
+    const double along = dot3(v, s.n);
+    if (s.phase == 2 ? along <= 0.0 : along < 0.0) return 0;
+    if (s.phase < 2) {
+        if (s.phase == 0) {
+            s.p0 = v;
+            s.n = cross3(v, s.v0);
+            s.phase = 1;
+            return fabs(s.n.x) < TOL && fabs(s.n.y) < TOL && fabs(s.n.z) < TOL ? 1 : -1;
+        }
+        s.p1 = v;
+        s.n = cross3(sub3(s.p0, s.v0), sub3(s.p1, s.v0));
+        if (dot3(s.n, s.v0) > 0.0) {
+            const V3 t = s.p0;
+            s.p0 = s.p1;
+            s.p1 = t;
+            s.n = neg3(s.n);
+        }
+        s.phase = 2;
+        s.count = 1;
+        return -1;
+    }
+    if (s.phase == 2) {
+        bool again = true;
+        if (dot3(cross3(s.p0, v), s.v0) < 0.0)
+            s.p1 = v;
+        else if (dot3(cross3(v, s.p1), s.v0) < 0.0)
+            s.p0 = v;
+        else
+            again = false;
+        if (again) {
+            s.n = cross3(sub3(s.p0, s.v0), sub3(s.p1, s.v0));
+            s.count += 1;
+            return s.count >= kXenoMaxIter ? 1 : -1;
+        }
+        s.p2 = v;
+        s.count = 1;
+        s.phase = 3;
+    } else {
+        // |x| < TOL sqrt(n . n), the root only where x^2 does not rule it out by far
+        const double nn2 = dot3(s.n, s.n), far2 = 1.5 * TOL * TOL * nn2;
+        const double x0 = dot3(sub3(v, s.p0), s.n), x1 = dot3(s.p0, s.n);
+        if (!(x0 * x0 > far2 && x1 * x1 > far2)) {
+            const double tol = dmul(TOL, dsqrt(nn2));
+            if (fabs(x0) < tol) return 0;
+            if (fabs(x1) < tol) return 1;
+        }
+        const V3 vp = cross3(v, s.v0);
+        const bool t1 = dot3(vp, s.p0) > 0.0, t2 = dot3(vp, s.p1) > 0.0, t3 = dot3(vp, s.p2) > 0.0;
+        if (t1 && !t2)
+            s.p2 = v;
+        else if (!t1 && t3)
+            s.p1 = v;
+        else
+            s.p0 = v;
+        if (s.count >= kXenoMaxIter) return 1;
+        s.count += 1;
+    }
+    // the refinement loop's head: the portal's normal away from v0; the origin inside: overlap
+    V3 nn = cross3(sub3(s.p1, s.p0), sub3(s.p2, s.p0));
+    if (dot3(sub3(s.p0, s.v0), nn) < 0.0) nn = neg3(nn);
+    s.n = nn;
+    return dot3(s.p0, nn) >= 0.0 ? 1 : -1;
+}
+
+// FP32 form of the first test of XenoCollide (phase 0: v1 . v0 > 0, the shapes are separated along the
+// line of centres), which ends 7 in 10 of the pairs inside the circumsphere. With v0 and the relative
+// orientation M by the FP64 path's formulas in FP32 from d (the other site minus the trial's),
+// v1 . v0 = |v0|^2 - max_a a . v0 - max_b b . (-M^T v0). An FP32 value above its error bound decides:
+// the FP64 test is then positive too, whichever of tied vertices it takes (its own roundings
+// are of order 1e-15). Bound, with si, sj = |q|^2 (1 for versors) and D = |d|_1: v0 is off by at most 16 u32
+// si D per component, M by 28 u32 si sj per entry (Cauchy's inequality over the quaternion products),
+// M^T v0 by 106 u32 si^2 sj D, so the value by 110 u32 T, T = si D (si D + 3 vmax (1 + si sj)); the
+// sites' own error moves it by 2 T / D times its 1-norm. 128 u32 leaves room for the bound's roundings.
+__device__ __forceinline__ bool separated32(const ShapeTable& T, float dx, float dy, float dz, float4 qi, float4 qj,
+                                            float site_err) {
+    // ia = conj(qi) = (s, -x, -y, -z); v0 = vrotate(ia, d); o = ia qj; M = mat_from(o)
+    const float s = qi.x, x = -qi.y, y = -qi.z, z = -qi.w;
+    const float si = s * s + x * x + y * y + z * z, sj = qj.x * qj.x + qj.y * qj.y + qj.z * qj.z + qj.w * qj.w;
+    const float k1 = s * s - (x * x + y * y + z * z), k2 = 2.f * s, k3 = 2.f * (x * dx + y * dy + z * dz);
+    const float vx = dx * k1 + (y * dz - z * dy) * k2 + x * k3;
+    const float vy = dy * k1 + (z * dx - x * dz) * k2 + y * k3;
+    const float vz = dz * k1 + (x * dy - y * dx) * k2 + z * k3;
+    const float a = s * qj.x - (x * qj.y + y * qj.z + z * qj.w);
+    const float b = qj.y * s + x * qj.x + (y * qj.w - z * qj.z);
+    const float c = qj.z * s + y * qj.x + (z * qj.y - x * qj.w);
+    const float d = qj.w * s + z * qj.x + (x * qj.z - y * qj.y);
+    // -M^T v0
+    const float bx = -((a * a + b * b - c * c - d * d) * vx + 2.f * (b * c + a * d) * vy + 2.f * (b * d - a * c) * vz);
+    const float by = -(2.f * (b * c - a * d) * vx + (a * a - b * b + c * c - d * d) * vy + 2.f * (c * d + a * b) * vz);
+    const float bz = -(2.f * (b * d + a * c) * vx + 2.f * (c * d - a * b) * vy + (a * a - b * b - c * c + d * d) * vz);
+    float ha = -INFINITY, hb = -INFINITY;
+#pragma unroll 4
+    for (uint32_t i = 0; i < T.nv; ++i) {
+        const float4 v = T.v32[i];
+        ha = fmaxf(ha, v.x * vx + v.y * vy + v.z * vz);
+        hb = fmaxf(hb, v.x * bx + v.y * by + v.z * bz);
+    }
+    const float D = fabsf(dx) + fabsf(dy) + fabsf(dz);
+    const float scale = si * (si * D + 3.f * T.vmax * (1.f + si * sj));
+    return vx * vx + vy * vy + vz * vz - ha - hb > scale * (128.f * 5.9604645e-8f * D + 6.f * site_err);
+}
+
+// A warp decides kGroup trials at a time, kGroupLanes lanes for each where a trial's own work is done;
+// the kWarps warps of a block go through the steps together (k_flow_poly3).
+constexpr uint32_t kGroup = 4, kGroupLanes = 32 / kGroup, kWarps = 4;
+constexpr uint32_t kPairs = 128;  // pairs a warp lists before it tests them
+struct alignas(16) PolyTeam {
+    uint2 step[kGroup][32];  // a trial's stencil in steps of kGroupLanes candidates: first slot, length
+    uint2 near[kGroup][28];  // the progress words around each trial's space and the values it needs
+    uint32_t pair_q[kPairs];
+    uint8_t pair_g[kPairs];
+    double t[kGroup][3], q[kGroup][4];  // the trials: site T and versor
+    float4 q32[kGroup];                 // the versor in FP32
+    int4 t32[kGroup];                   // T in fixed point
+};
+
+// The pair of the trial (t, q of the warp's trial `mine`) and slot q: pair_system_to_local as
+// poly_overlap64 does it. 0: outside the circumsphere, 1: overlap (coincident centres), -1: to be tested.
+__device__ __forceinline__ int pair_begin(const Geometry& g, const Arrays& A, double rcut2, const PolyTeam& S,
+                                          uint32_t mine, uint32_t q, PairLane& s) {
+    const double4 s4 = ldcg4(A.sorted_s + q), o4 = ldcg4(A.sorted_q + q);
+    const double t[3] = {S.t[mine][0], S.t[mine][1], S.t[mine][2]}, sj[3] = {s4.x, s4.y, s4.z};
+    double d[3];
+    if (!(ref_disp<3>(g, t, sj, d) < rcut2)) return 0;
+    const Q ia{S.q[mine][0], -S.q[mine][1], -S.q[mine][2], -S.q[mine][3]};
+    s.v0 = vrotate(ia, V3{-d[0], -d[1], -d[2]});
+    s.q = mat_from(qmul(ia, Q{o4.x, o4.y, o4.z, o4.w}));
+    s.n = neg3(s.v0);
+    s.phase = 0;
+    return fabs(s.v0.x) < 2e-12 && fabs(s.v0.y) < 2e-12 && fabs(s.v0.z) < 2e-12 ? 1 : -1;
+}
+
+// The pair tests of a warp's n listed pairs, two lanes each: bit g of the result is set when trial g
+// overlaps. Two lanes that have their result take the next pair, so that the tests' different
+// lengths leave few lanes idle; pairs of a trial that is known to overlap are dropped.
+template <bool FP32>
+__device__ __forceinline__ uint32_t test_pairs(const Geometry& g, const Arrays& A, const ShapeTable& T, double rcut2,
+                                               const PolyTeam& S, uint32_t n, uint32_t lane, uint32_t mask) {
+    const unsigned full = 0xffffffffu;
+    const uint32_t role = lane & 1u;
+    uint32_t head = 0, mine = 0;
+    bool busy = false;
+    PairLane s;
+    for (;;) {
+        const unsigned idle = __ballot_sync(full, !busy && role == 0u);
+        const uint32_t n_idle = __popc(idle);
+        uint32_t hit = 0;
+        if (head < n && n_idle >= 4u) {
+            const uint32_t at = head + __popc(idle & ((1u << (lane & ~1u)) - 1u));
+            head += min(n_idle, n - head);
+            if (!busy && at < n) {
+                mine = S.pair_g[at];
+                if (!((mask >> mine) & 1u)) {
+                    const int b = pair_begin(g, A, rcut2, S, mine, S.pair_q[at], s);
+                    busy = b < 0;
+                    if (b == 1) hit = 1u << mine;
+                }
+            }
+        } else if (n_idle == 16u) {
+            return mask;
+        }
+        const unsigned active = __ballot_sync(full, busy);
+        if (busy) {
+            const V3 v = pair_support<FP32>(T, s.q, s.v0, s.n, role, active);
+            const int res = pair_step(s, v);
+            busy = res < 0;
+            if (res == 1) hit = 1u << mine;
+        }
+        mask |= __reduce_or_sync(full, hit);
+        busy = busy && !((mask >> mine) & 1u);
+    }
+}
+
+// The listed pairs through XenoCollide's first test, which ends 7 in 10 of them; returns how many
+// are left (at the list's front, in order). FP32: separated32, a lane per pair. FP64: the test itself,
+// two lanes per pair.
+template <bool FP32>
+__device__ __forceinline__ uint32_t poly_screen(const Geometry& g, const Arrays& A, const PolyShape& sh,
+                                                const ShapeTable& T, PolyTeam& S, uint32_t n, uint32_t lane) {
+    const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+    constexpr uint32_t per = FP32 ? 32 : 16;
+    uint32_t kept = 0;
+#pragma unroll 1
+    for (uint32_t p0 = 0; p0 < n; p0 += per) {
+        const uint32_t p = p0 + (FP32 ? lane : lane >> 1);
+        uint32_t q = 0, mine = 0;
+        bool keep = p < n;
+        if (keep) {
+            q = S.pair_q[p];
+            mine = S.pair_g[p];
+        }
+        if constexpr (FP32) {
+            if (keep) {
+                const int4 o = __ldcg(reinterpret_cast<const int4*>(A.sorted_off) + q), t = S.t32[mine];
+                const double4 o4 = ldcg4(A.sorted_q + q);
+                keep = !separated32(T, (float)(int)((uint32_t)o.x - (uint32_t)t.x) * g.fix[0],
+                                    (float)(int)((uint32_t)o.y - (uint32_t)t.y) * g.fix[1],
+                                    (float)(int)((uint32_t)o.z - (uint32_t)t.z) * g.fix[2], S.q32[mine],
+                                    make_float4((float)o4.x, (float)o4.y, (float)o4.z, (float)o4.w), sh.site_err);
+            }
+        } else {
+            PairLane s;
+            if (keep) keep = pair_begin(g, A, sh.rcut2, S, mine, q, s) != 0;  // (an overlap is found again)
+            const unsigned active = __ballot_sync(full, keep);
+            if (keep) keep = !(dot3(pair_support<false>(T, s.q, s.v0, s.n, lane & 1u, active), s.v0) > 0.0);
+            if (lane & 1u) keep = false;  // one entry per pair
+        }
+        const unsigned b = __ballot_sync(full, keep);
+        if (keep) {  // (in place: no entry is written beyond those already read)
+            S.pair_q[kept + __popc(b & below)] = q;
+            S.pair_g[kept + __popc(b & below)] = (uint8_t)mine;
+        }
+        kept += __popc(b);
+        __syncwarp();
+    }
+    return kept;
+}
+
+// The warp's trials (slot k, space m; valid the same in a trial's lanes) against their stencils: the
+// circumsphere test (FP32: under the error bound), 8 lanes per trial and a row of the stencil in
+// steps of 8 candidates; then the pairs that need the full test are listed, those with the closest centres
+// first (they overlap most often), and tested. Returns the trials that overlap. The circumsphere loop
+// only collects bits, so the loads of its steps are in flight together (bulk copies into shared
+// memory, as for Lennard-Jones, took longer: the rows are 9 candidates long); the list is written
+// once per 32 steps by a scan over the lanes.
+template <bool FP32, bool SYNC>
+__device__ __forceinline__ uint32_t poly_decide(const Geometry& g, const Arrays& A, const PolyShape& sh,
+                                                const ShapeTable& T, const uint32_t* m, uint32_t k, bool valid,
+                                                uint32_t lane, PolyTeam& S, const uint3& lo, const uint3& len,
+                                                PairStats& st) {
+    const unsigned full = 0xffffffffu;
+    const uint32_t grp = lane / kGroupLanes, sub = lane % kGroupLanes;
+    // this lane's parts as steps [a, a + sum) of the trial's
+    const uint32_t ls[3] = {lo.x, lo.y, lo.z}, ns[3] = {len.x, len.y, len.z};
+    uint32_t sum = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) sum += valid ? (ns[i] + kGroupLanes - 1) / kGroupLanes : 0u;
+    uint32_t end = sum;
+#pragma unroll
+    for (uint32_t o = 1; o < kGroupLanes; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(full, end, o, kGroupLanes);
+        if (sub >= o) end += y;
+    }
+    const uint32_t steps = __shfl_sync(full, end, kGroupLanes - 1, kGroupLanes);
+    const uint32_t longest = __reduce_max_sync(full, steps);
+    const int4 t32 = S.t32[grp];
+    const double t[3] = {S.t[grp][0], S.t[grp][1], S.t[grp][2]};
+    const float near32 = 0.45f * sh.rcut2_hi32;
+    const double near64 = 0.45 * sh.rcut2;
+    const unsigned bv = __ballot_sync(full, valid && sub == 0u);
+    uint32_t which = 0, mask = 0;  // bit i: trial i
+#pragma unroll
+    for (uint32_t i = 0; i < kGroup; ++i) which |= ((bv >> (i * kGroupLanes)) & 1u) << i;
+    bool first_pass = true;
+#pragma unroll 1
+    for (uint32_t s0 = 0; s0 < longest || (SYNC && first_pass); s0 += 32u) {
+        __syncwarp();  // the steps before have been read
+        if (valid) {
+            uint32_t at = end - sum;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                for (uint32_t c = 0; c < ns[i]; c += kGroupLanes, ++at)
+                    if (at - s0 < 32u) S.step[grp][at - s0] = make_uint2(ls[i] + c, min(ns[i] - c, kGroupLanes));
+        }
+        __syncwarp();
+        const uint32_t n = steps > s0 ? min(32u, steps - s0) : 0u, n_max = min(32u, longest - s0);
+        uint32_t need = 0, close = 0;  // bit i: candidate `sub` of step i
+#pragma unroll 2
+        for (uint32_t i = 0; i < n_max; ++i) {
+            const uint2 p = S.step[grp][i];  // (stale beyond n)
+            const uint32_t q = p.x + sub;
+            const bool ok = i < n && sub < p.y && q != k;
+            bool in, cl;
+            if constexpr (FP32) {
+                const int4 o = ok ? __ldcg(reinterpret_cast<const int4*>(A.sorted_off) + q) : make_int4(0, 0, 0, 0);
+                const float d2 = fixed_dist2<3>(g, t32, o);
+                in = d2 < sh.rcut2_hi32;
+                cl = d2 < near32;
+            } else {
+                // the circumsphere test that opens poly_overlap64
+                const double4 s4 = ok ? ldcg4(A.sorted_s + q) : make_double4(0.0, 0.0, 0.0, 0.0);
+                const double sj[3] = {s4.x, s4.y, s4.z};
+                double d[3];
+                const double d2 = ref_disp<3>(g, t, sj, d);
+                in = d2 < sh.rcut2;
+                cl = d2 < near64;
+            }
+            need |= (ok && in ? 1u : 0u) << i;
+            close |= (ok && cl ? 1u : 0u) << i;
+            st.checks += ok ? 1u : 0u;
+        }
+        if (FP32) st.rechecks += __popc(need);
+        if ((mask >> grp) & 1u) need = 0;
+        while (__any_sync(full, need != 0u) || (SYNC && first_pass)) {
+            // this lane's places: the close pairs of all lanes first, then the others
+            uint32_t x = __popc(need & close) | (__popc(need & ~close) << 16);
+            const uint32_t own = x;
+#pragma unroll
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(full, x, o);
+                if (lane >= o) x += y;
+            }
+            const uint32_t all = __shfl_sync(full, x, 31), n_close = all & 0xffffu, n_pairs = n_close + (all >> 16);
+            uint32_t at_close = (x - own) & 0xffffu, at_far = n_close + ((x - own) >> 16);
+            uint32_t left = need;
+            while (left) {
+                const uint32_t i = (uint32_t)__ffs(left) - 1u, bit = 1u << i;
+                left &= left - 1u;
+                const uint32_t at = close & bit ? at_close++ : at_far++;
+                if (at < kPairs) {
+                    S.pair_q[at] = S.step[grp][i].x + sub;
+                    S.pair_g[at] = (uint8_t)grp;
+                    need &= ~bit;
+                }
+            }
+            __syncwarp();
+            if (SYNC && first_pass) __syncthreads();
+            const uint32_t listed = poly_screen<FP32>(g, A, sh, T, S, min(n_pairs, kPairs), lane);
+            if (SYNC && first_pass) __syncthreads();
+            first_pass = false;
+            mask = test_pairs<FP32>(g, A, T, sh.rcut2, S, listed, lane, mask);
+            if ((mask >> grp) & 1u) need = 0;
+            __syncwarp();
+        }
+        if ((mask & which) == which && !(SYNC && first_pass)) break;  // every trial is decided
+    }
+    return mask;
+}
+
+// The stencils around the spaces m of the warp's trials (valid the same in a trial's lanes): lane `sub`
+// < 6 of a trial has the slots of parts 3 sub .. 3 sub + 2, so the loads of all trials are in flight
+// together.
+__device__ __forceinline__ void poly_parts(const Geometry& g, const Arrays& A, const uint32_t* m, bool valid, uint32_t sub,
+                                           uint3& lo, uint3& len) {
+    uint32_t l[3], n[3];
+#pragma unroll
+    for (uint32_t i = 0; i < 3; ++i) {
+        const uint32_t p = 3u * sub + i;
+        float s0, s1;
+        l[i] = n[i] = 0;
+        if (valid && p < 2u * kRows<3>)
+            stencil_part<3>(g, A.cell_start, m, (int)(p >> 1), (p & 1u) != 0, l[i], n[i], s0, s1);
+    }
+    lo = make_uint3(l[0], l[1], l[2]);
+    len = make_uint3(n[0], n[1], n[2]);
+}
+
+// The sweep of hard convex polyhedra: a block takes kWarps x kGroup trials of one colour (one unit) in
+// dataflow order (hmc_flow.cuh), all colour passes of colour sets [L.round, L.round_end) in one
+// launch. The trials of a unit are neighbours in their colour's list, so they wait for the same
+// slab of the box. INJ: the probe mode, warp w decides injected trials kGroup w .. against the
+// unchanged state.
+// Bound: instruction fetch. The four steps of a unit (set-up, circumspheres, screen, XenoCollide) are
+// some 2,000 instructions; with every warp at its own place among them the schedulers found no
+// instruction in a third of the cycles, so the block's warps take the steps together (a barrier before
+// each): 24.6 -> 20.9 ms on 2^18 cubes at packing fraction 0.55, ten sweeps of each move (FP32;
+// FP64 44.7 -> 30.6). One launch per colour pass with four trials per warp and a lane per pair test:
+// 42.0 ms (FP64 44.3).
+template <bool FP32, bool INJ, int MINB>
+__global__ void __launch_bounds__(32 * kWarps, MINB)
+    k_flow_poly3(Geometry g, Arrays A, PolyShape sh, Launch L, uint32_t rotate, Injected J) {
+    constexpr unsigned full = 0xffffffffu;
+    // each lane polls up to kWarpsords of its trial's 27 progress words: word sub + i lanes, i < kWarpsords;
+    // the own space's is word 13
+    constexpr uint32_t kWarpsords = (27 + kGroupLanes - 1) / kGroupLanes;
+    constexpr uint32_t kOwnLane = 13 % kGroupLanes, kOwnBit = 1u << (13 / kGroupLanes);
+    __shared__ PolyTeam s_team[kWarps];
+    __shared__ uint32_t s_unit;
+    __shared__ FlowRange s_range;
+    __shared__ ShapeTable T;
+    const uint32_t lane = threadIdx.x & 31u, grp = lane / kGroupLanes, sub = lane % kGroupLanes;
+    PolyTeam& S = s_team[threadIdx.x >> 5];
+    if (threadIdx.x < 32u) {
+        float vmax = 0.f;
+        if (threadIdx.x < sh.nv) {
+            const double4 v = ldg4(sh.verts + threadIdx.x);
+            T.v[threadIdx.x][0] = v.x, T.v[threadIdx.x][1] = v.y, T.v[threadIdx.x][2] = v.z;
+            T.v32[threadIdx.x] = make_float4((float)v.x, (float)v.y, (float)v.z, 0.f);
+            vmax = __double2float_ru(fmax(fabs(v.x), fmax(fabs(v.y), fabs(v.z))));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(full, vmax, o));
+        if (threadIdx.x == 0) T.vmax = vmax, T.nv = sh.nv;
+    }
+    if (!INJ) {
+        grid_dependency_wait();
+        if (threadIdx.x == 0) s_range = flow_range(A.stats, L.round, L.round_end, 8, kGroup * kWarps);
+    }
+    __syncthreads();
+    const FlowRange& f = s_range;
+    const uint32_t n = INJ ? (J.n + kGroup - 1) / kGroup : f.n_units;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, n_warps = (gridDim.x * blockDim.x) >> 5;
     uint32_t n_accepted = 0;
     PairStats st;
-    const uint32_t sf = g.shape[2];
-    const uint32_t n_active = INJ ? J.n : active_count(A, L.color, L.round);
-    for (uint32_t w0 = warp * G; w0 < n_active; w0 += n_warps * G) {  // warp-uniform
-        const uint32_t w = w0 + grp;
-        uint32_t m[3] = {0, 0, 0};
-        uint32_t k = 0;
+    uint32_t next = INJ ? warp : (threadIdx.x == 0 ? atomicAdd(&A.stats->ticket, 1u) : 0u);
+    for (;;) {
+        uint32_t unit = next;
+        if (!INJ) {
+            if (threadIdx.x == 0) s_unit = next;
+            __syncthreads();
+            unit = s_unit;
+        }
+        if (unit >= n) break;
+        if (INJ) next = unit + n_warps;
+        else if (threadIdx.x == 0) next = atomicAdd(&A.stats->ticket, 1u);
+        uint32_t m[3] = {0, 0, 0}, k = 0, round = 0, e = 0;
         bool valid = false;
-        double t[3] = {0.0, 0.0, 0.0};
+        double ta = 0.0;
         Q qi{1.0, 0.0, 0.0, 0.0};
         uint8_t flag = 0;
-        float4 t32p = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (INJ && w < n_active) {  // the injected trial (W1, versor), by the group's S lanes alike
-            const uint64_t body = J.bodies[w];
-            k = A.slot_of_body[body];
-            const double4 w4 = J.trial[w];
-            const double x[3] = {w4.x, w4.y, w4.z};
-            const double4 q4 = J.trial_q[w];
-            qi = Q{q4.x, q4.y, q4.z, q4.w};
-            valid = point_to_space<3>(g, x, m);
-            if (!valid)
-                atomicOr(&A.stats->error_flags, kErrOutsideCheckerboard);
-            else if (cell_index<3>(g, m) != A.body_cell[body])
-                flag |= kTrialOutsideSpace;
-            t[0] = x[0];
-            t[1] = x[1];
-            t[2] = x[2];
-            wrap_inv<3>(g.L, g.invL, t);
-        } else if (w < n_active) {  // the group's trial from k_propose_poly3
-            const size_t e = (size_t)L.color * g.color_stride + w;
-            k = __ldg(A.trial_k + e);
-            valid = k != kNoTrial;
-            if (valid) {
-                unpack_m<3>(__ldg(A.color_cells + e), m);
-                const double4 t4 = ldg4(A.trial_t + e);
-                t[0] = t4.x;
-                t[1] = t4.y;
-                t[2] = t4.z;
-                const double4 q4 = ldg4(A.trial_q + e);
-                qi = Q{q4.x, q4.y, q4.z, q4.w};
-                if (FP32) t32p = __ldg(A.trial_o + e);
-            }
-        }
-        const float4 t32 = FP32 && valid ? (INJ ? cell_offsets<3>(g, t, m) : t32p) : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (sub == 0) {
-            PolyTrial& tr = s_trial[wib][grp];
-            tr.t[0] = t[0];
-            tr.t[1] = t[1];
-            tr.t[2] = t[2];
-            tr.q[0] = qi.s;
-            tr.q[1] = qi.x;
-            tr.q[2] = qi.y;
-            tr.q[3] = qi.z;
-        }
-        grid_dependency_wait();  // the previous colour's moves are visible from here on
-        allow_dependent_launch();
-        uint32_t mask = 0, n_pairs = 0;  // warp-uniform
-#pragma unroll 1
-        for (int part = 0; part < 2 * kRows<3>; ++part) {
-            uint32_t lo = 0, len = 0;
-            float s0 = 0.f, s1 = 0.f;
-            if (valid) stencil_part<3>(g, A.cell_start, m, part >> 1, (part & 1) != 0, lo, len, s0, s1);
-            const uint32_t iters = __reduce_max_sync(0xffffffffu, (len + S - 1) / S);
-            for (uint32_t it = 0; it < iters; ++it) {
-                const uint32_t j = it * S + sub;
-                const uint32_t q = lo + j;
-                bool need = false;
-                if (j < len && q != k && !((mask >> grp) & 1u)) {
-                    st.checks++;
-                    if (FP32) {
-                        const float4 o = __ldg(A.sorted_off + q);
-                        int dm = __float_as_int(o.w) - (int)m[2];
-                        if (sf >= 4) {
-                            if (dm > 1)
-                                dm -= (int)sf;
-                            else if (dm < -1)
-                                dm += (int)sf;
-                        }
-                        need = fp32_dist2<3>(g, t32, o, s0, s1, dm) < sh.rcut2_hi32;
-                        if (need) st.rechecks++;
-                    } else {
-                        // the circumsphere test that opens poly_overlap64
-                        const double4 s4 = ldg4(A.sorted_s + q);
-                        const double sj[3] = {s4.x, s4.y, s4.z};
-                        double d[3];
-                        need = ref_disp<3>(g, t, sj, d) < sh.rcut2;
-                    }
-                }
-                const unsigned b = __ballot_sync(0xffffffffu, need);
-                if (need) {
-                    const uint32_t pos = n_pairs + __popc(b & ((1u << lane) - 1u));
-                    s_pair_q[wib][pos] = q;
-                    s_pair_g[wib][pos] = (uint8_t)grp;
-                }
-                n_pairs += __popc(b);
-                if (n_pairs > kPairCap - 32) {
-                    drain_pairs<G>(g, A, sh, s_trial[wib], s_pair_q[wib], s_pair_g[wib], n_pairs, lane, mask);
-                    n_pairs = 0;
-                }
-            }
-        }
-        drain_pairs<G>(g, A, sh, s_trial[wib], s_pair_q[wib], s_pair_g[wib], n_pairs, lane, mask);
+        const uint32_t axis = sub < 3 ? sub : 0u;
         if constexpr (INJ) {
-            if (sub == 0 && w < n_active) {
-                J.decisions[w] = valid && !((mask >> grp) & 1u);
+            const uint32_t w = unit * kGroup + grp;
+            if (w < J.n) {
+                const uint64_t body = J.bodies[w];
+                k = A.slot_of_body[body];
+                const double4 w4 = J.trial[w], q4 = J.trial_q[w];
+                double x[3] = {w4.x, w4.y, w4.z};
+                qi = Q{q4.x, q4.y, q4.z, q4.w};
+                valid = point_to_space<3>(g, x, m);
+                if (!valid)
+                    atomicOr(&A.stats->error_flags, kErrOutsideCheckerboard);
+                else if (cell_index<3>(g, m) != A.body_cell[body])
+                    flag |= kTrialOutsideSpace;
+                wrap_inv<3>(g.L, g.invL, x);
+                ta = axis == 0 ? x[0] : (axis == 1 ? x[1] : x[2]);
+            }
+        } else {
+            uint32_t color, entry;
+            flow_unit(f, unit, round, color, entry);
+            entry = (entry * kWarps + (threadIdx.x >> 5)) * kGroup + grp;
+            valid = entry < f.count[color];
+            uint4 di = make_uint4(0u, 0u, 0u, 0u);
+            e = (round - f.r0) * f.per_set + f.prefix[color] + entry;
+            if (valid) di = __ldg(A.draw_i + e);
+            k = di.x;
+            unpack_m<3>(di.y, m);
+        }
+        const bool listed = valid;  // the group has a trial (its space is finished below)
+        uint3 lo, len;
+        poly_parts(g, A, m, valid, sub, lo, len);
+        if (!INJ && valid) {
+            const uint32_t color = ((m[0] & 1u) << 2) | ((m[1] & 1u) << 1) | (m[2] & 1u);
+#pragma unroll 1
+            for (uint32_t i = sub; i < 27u; i += kGroupLanes) {
+                uint2 w;
+                flow_need<3>(g, m, color, round, i, w.x, w.y);
+                S.near[grp][i] = w;
+            }
+        }
+        __syncwarp();
+        if constexpr (!INJ) {
+            unsigned pending = 0;
+            if (valid) pending = (1u << kWarpsords) - 1u;
+            if (sub + (kWarpsords - 1u) * kGroupLanes >= 27u) pending &= ~(1u << (kWarpsords - 1u));
+            // the own space first: the proposal needs no other
+            bool going = flow_wait_words<kWarpsords>(A.progress, S.near[grp], sub, kGroupLanes, pending,
+                                                 sub == kOwnLane ? kOwnBit : 0u, A.stats);
+            __syncwarp();
+            const AxisGeometry ax = axis_geometry<3>(g, axis);
+            const uint32_t ma = axis == 0 ? m[0] : (axis == 1 ? m[1] : m[2]);
+            double x = 0.0, w1 = 0.0;
+            if (valid) {
+                const double* draw = reinterpret_cast<const double*>(A.draw_d + e);
+                x = __ldcg(reinterpret_cast<const double*>(A.sorted_b + k) + axis);
+                const double4 q4 = ldcg4(A.sorted_q + k);
+                qi = Q{q4.x, q4.y, q4.z, q4.w};
+                if (rotate)
+                    qi = qmul(Q{__ldg(draw), __ldg(draw + 1), __ldg(draw + 2), __ldg(draw + 3)}, qi);
+                else
+                    x = dadd(x, __ldg(draw + axis));
+                w1 = wrap_axis(ax.L, ax.invL, x);  // W1 = wrap(propose(..))
+            }
+            const bool in_axis = !valid || axis_in_space(ax.origin, ax.width, ax.invW, ax.shape, ma, w1);
+            const unsigned in = __ballot_sync(full, in_axis);
+            constexpr unsigned all = (1u << kGroupLanes) - 1u;
+            valid = valid && ((in >> (grp * kGroupLanes)) & all) == all;
+            if (valid) ta = wrap_axis(ax.L, ax.invL, w1);  // the trial site T = wrap(W1)
+            if (!valid) pending = 0;
+            if (going)
+                going = flow_wait_words<kWarpsords>(A.progress, S.near[grp], sub, kGroupLanes, pending, ~0u, A.stats);
+            if (!going) valid = false;
+            if (__syncthreads_or(!going)) break;
+            __syncwarp();
+        }
+        if (valid) {
+            if (sub < 3u) {
+                S.t[grp][sub] = ta;
+                reinterpret_cast<int*>(&S.t32[grp])[sub] = fixed_axis(g.invL[axis], ta);
+            }
+            if (sub == 3u) {
+                S.q[grp][0] = qi.s, S.q[grp][1] = qi.x, S.q[grp][2] = qi.y, S.q[grp][3] = qi.z;
+                S.q32[grp] = make_float4((float)qi.s, (float)qi.x, (float)qi.y, (float)qi.z);
+            }
+        }
+        __syncwarp();
+        const uint32_t mask = poly_decide<FP32, !INJ>(g, A, sh, T, m, k, valid, lane, S, lo, len, st);
+        const bool accept = valid && !((mask >> grp) & 1u);
+        if constexpr (INJ) {
+            const uint32_t w = unit * kGroup + grp;
+            if (sub == 0 && w < J.n) {
+                J.decisions[w] = accept;
                 J.flags[w] = flag;
             }
-        } else if (sub == 0 && valid && !((mask >> grp) & 1u)) {
-            n_accepted++;
-            double sv[3] = {t[0], t[1], t[2]};
-            wrap_inv<3>(g.L, g.invL, sv);
-            const uint32_t body = A.sorted_body[k];
-            A.sorted_b[k] = make_double4(t[0], t[1], t[2], 0.0);
-            A.sorted_s[k] = make_double4(sv[0], sv[1], sv[2], 0.0);
-            A.sorted_off[k] = cell_offsets<3>(g, sv, m);
-            A.sorted_q[k] = make_double4(qi.s, qi.x, qi.y, qi.z);
-            A.body_pos[body] = make_double4(t[0], t[1], t[2], 0.0);
-            A.body_ori[body] = make_double4(qi.s, qi.x, qi.y, qi.z);
+        } else {
+            if (accept) {
+                // update_body_properties: body = T, site = wrap(body)
+                const uint32_t body = A.sorted_body[k];
+                if (sub < 3u) {
+                    const double tc = S.t[grp][sub], sv = wrap_axis(g.L[axis], g.invL[axis], tc);
+                    reinterpret_cast<double*>(A.sorted_b + k)[sub] = tc;
+                    reinterpret_cast<double*>(A.sorted_s + k)[sub] = sv;
+                    if (FP32) reinterpret_cast<int*>(A.sorted_off + k)[sub] = fixed_axis(g.invL[axis], sv);
+                    reinterpret_cast<double*>(A.body_pos + body)[sub] = tc;
+                }
+                const double4 q4 = make_double4(S.q[grp][0], S.q[grp][1], S.q[grp][2], S.q[grp][3]);
+                if (sub == 3u) A.sorted_q[k] = A.body_ori[body] = q4;
+                n_accepted += sub == 0u;
+            }
+            __syncwarp();
+            if (listed && sub == 0u) store_release(A.progress + cell_index<3>(g, m), round + 1u);
         }
         __syncwarp();
     }
-    grid_dependency_wait();
-    allow_dependent_launch();
     flush_stats(A.stats, st, n_accepted);
 }
 
@@ -752,9 +1187,8 @@ __global__ void __launch_bounds__(128) k_eval_poly3(Geometry g, Arrays A, PolySh
         uint32_t m[3];
         uint8_t dec = 0;
         if (point_to_space<3>(g, t, m)) {
-            const float4 t32 = FP32 ? cell_offsets<3>(g, t, m) : make_float4(0.f, 0.f, 0.f, 0.f);
             const FlatStencil fs = flat_stencil<3>(g, A.cell_start, m, lane);
-            dec = poly_overlaps<FP32>(g, A, sh, t, qi, t32, (int)m[2], fs, k, lane, st) ? 0 : 1;
+            dec = poly_overlaps<FP32>(g, A, sh, t, qi, fixed_site<3>(g, t), fs, k, lane, st) ? 0 : 1;
         } else if (lane == 0) {
             atomicOr(&A.stats->error_flags, kErrOutsideCheckerboard);
         }
@@ -868,8 +1302,7 @@ __global__ void __launch_bounds__(32) k_tune_stream_poly3(TuneJob* jobs, uint32_
             }
             const FlatStencil fs = flat_stencil<3>(g, A.cell_start, m, lane);
             const Q qi{q[0], q[1], q[2], q[3]};
-            return !poly_overlaps<false>(g, A, sh, t, qi, make_float4(0.f, 0.f, 0.f, 0.f), (int)m[2], fs,
-                                         A.slot_of_body[b], lane, st);
+            return !poly_overlaps<false>(g, A, sh, t, qi, make_int4(0, 0, 0, 0), fs, A.slot_of_body[b], lane, st);
         });
 }
 
@@ -986,21 +1419,15 @@ cudaError_t launch_serial_poly(const Geometry& g, const Arrays& a, const double4
     const SerialGrid G = make_grid(3, nc, w, cap, size, items, cell_of, site);
     cudaError_t e = build_grid(3, g, a, G, l.n_bodies, s);
     if (e != cudaSuccess || l.n_bodies == 0) return e;
-    k_serial_poly3<<<1, 32, 0, s>>>(g, a, G, PolyShape{verts, nv, rcut2, 0.f}, l, rotate ? 1u : 0u, mask);
+    k_serial_poly3<<<1, 32, 0, s>>>(g, a, G, PolyShape{verts, nv, rcut2, 0.f, 0.f}, l, rotate ? 1u : 0u, mask);
     return cudaGetLastError();
 }
 
-cudaError_t launch_propose_poly(bool fp32, const Geometry& g, const Arrays& a, const Launch& l, bool rotate,
-                                bool soft, cudaStream_t s) {
-    const uint64_t n = (uint64_t)g.color_stride << 3;
+cudaError_t launch_propose_poly(const Geometry& g, const Arrays& a, const Launch& l, bool rotate, cudaStream_t s) {
+    const uint64_t n = (uint64_t)g.color_stride * 8u;
     if (n == 0) return cudaSuccess;
-    const int wave = resident_wave((const void*)(fp32 ? k_propose_poly3<true> : k_propose_poly3<false>));
-    uint32_t blocks = (uint32_t)((n + 127) / 128);
-    if (blocks > (uint32_t)wave) blocks = (uint32_t)wave;
-    if (fp32)
-        k_propose_poly3<true><<<blocks, 128, 0, s>>>(g, a, l, rotate ? 1u : 0u, soft ? 1u : 0u);
-    else
-        k_propose_poly3<false><<<blocks, 128, 0, s>>>(g, a, l, rotate ? 1u : 0u, soft ? 1u : 0u);
+    const uint64_t blocks = (n + 127) / 128, wave = (uint64_t)resident_wave((const void*)k_propose_poly3);
+    k_propose_poly3<<<(uint32_t)(blocks < wave ? blocks : wave), 128, 0, s>>>(g, a, l, rotate ? 1u : 0u);
     return cudaGetLastError();
 }
 
@@ -1039,48 +1466,48 @@ cudaError_t launch_quick_insert_poly3(const Geometry& g, const Arrays& a, const 
 cudaError_t launch_tune_stream_poly(TuneJob* jobs, uint32_t n_jobs, const double4* verts, uint32_t nv, double rcut2,
                                     cudaStream_t s) {
     if (n_jobs == 0) return cudaSuccess;
-    k_tune_stream_poly3<<<n_jobs, 32, 0, s>>>(jobs, n_jobs, PolyShape{verts, nv, rcut2, 0.f});
+    k_tune_stream_poly3<<<n_jobs, 32, 0, s>>>(jobs, n_jobs, PolyShape{verts, nv, rcut2, 0.f, 0.f});
     return cudaGetLastError();
 }
 
-cudaError_t launch_sweep_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
-                              double rcut2, float rcut2_hi32, const Launch& l, bool rotate, cudaStream_t s,
-                              uint32_t variant) {
+namespace {
+// Fixed-point sites (fixed_site): half a unit of L / 2^32 each, and FP64's own (a relative 2^-49 of L).
+float site_error(const Geometry& g) {
+    const double L = fmax(g.L[0], fmax(g.L[1], g.L[2]));
+    return (float)(1.2 * L / 4294967296.0);
+}
+using PolyKernel = void (*)(Geometry, Arrays, PolyShape, Launch, uint32_t, Injected);
+}  // namespace
+
+cudaError_t launch_flow_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
+                             double rcut2, float rcut2_hi32, const Launch& l, bool rotate, cudaStream_t s,
+                             uint32_t variant) {
     if (l.n_active == 0) return cudaSuccess;
-    static int max_blocks = 0;
-    if (max_blocks == 0) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        max_blocks = sms * 16;
-    }
-    PolyShape sh{verts, nv, rcut2, rcut2_hi32};
-    const uint32_t per_block = 4u * kPolyShapes[variant < 3 ? variant : 0].trials_per_warp;  // four warps per block
-    uint32_t blocks = (l.n_active + per_block - 1) / per_block;
-    if (blocks > (uint32_t)max_blocks) blocks = (uint32_t)max_blocks;
-    PassLaunch pl(blocks, l.overlap_previous != 0 || l.early_wait != 0, s);
     const uint32_t rot = rotate ? 1u : 0u;
-    using PolyKernel = void (*)(Geometry, Arrays, PolyShape, Launch, uint32_t, Injected);
-    // the compiled launch variants, in the order of kPolyShapes (trials per warp 4, 2, 8)
-    static const PolyKernel kernels[2][3] = {
-        {k_sweep_poly3_packed<false, 4>, k_sweep_poly3_packed<false, 2>, k_sweep_poly3_packed<false, 8>},
-        {k_sweep_poly3_packed<true, 4>, k_sweep_poly3_packed<true, 2>, k_sweep_poly3_packed<true, 8>}};
-    static_assert(n_shapes(kPolyShapes) == 3, "one compiled kernel per polyhedron variant");
-    const uint32_t v = variant < 3 ? variant : 0;
-    return cudaLaunchKernelEx(&pl.cfg, kernels[fp32][v], g, a, sh, l, rot, Injected{});
+    const uint64_t entries = (uint64_t)g.color_stride * 8u * 4u;
+    uint64_t blocks = (entries + 127) / 128;
+    const uint64_t wave_d = (uint64_t)resident_wave((const void*)k_draw_poly3);
+    PassLaunch pd((uint32_t)(blocks < wave_d ? blocks : wave_d), true, s);
+    cudaError_t e = cudaLaunchKernelEx(&pd.cfg, k_draw_poly3, g, a, l, rot);
+    if (e != cudaSuccess) return e;
+    // the compiled launch variants, in the order of kPolyShapes
+    static const PolyKernel kernels[2][2] = {{k_flow_poly3<false, false, 4>, k_flow_poly3<false, false, 3>},
+                                             {k_flow_poly3<true, false, 4>, k_flow_poly3<true, false, 3>}};
+    static_assert(n_shapes(kPolyShapes) == 2, "one compiled kernel per polyhedron variant");
+    const PolyKernel k = kernels[fp32][variant < 2 ? variant : 0];
+    const uint64_t wave = (uint64_t)resident_wave((const void*)k, 32 * kWarps);
+    blocks = ((uint64_t)g.color_stride * 2 + kWarps * kGroup - 1) / (kWarps * kGroup);  // warps for two colours' units
+    PassLaunch pl((uint32_t)(blocks < wave ? blocks : wave), true, s, 32 * kWarps);
+    return cudaLaunchKernelEx(&pl.cfg, k, g, a, PolyShape{verts, nv, rcut2, rcut2_hi32, site_error(g)}, l, rot,
+                              Injected{});
 }
 
 cudaError_t launch_trials_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
                                double rcut2, float rcut2_hi32, const Injected& j, cudaStream_t s) {
     if (j.n == 0) return cudaSuccess;
-    PolyShape sh{verts, nv, rcut2, rcut2_hi32};
-    const Launch l{};
-    const uint32_t per_block = 4u * kPolyTrialsPerWarp;  // four warps per block
-    const uint32_t blocks = (j.n + per_block - 1) / per_block;
-    if (fp32)
-        k_sweep_poly3_packed<true, kPolyTrialsPerWarp, true><<<blocks, 128, 0, s>>>(g, a, sh, l, 0u, j);
-    else
-        k_sweep_poly3_packed<false, kPolyTrialsPerWarp, true><<<blocks, 128, 0, s>>>(g, a, sh, l, 0u, j);
+    const PolyKernel k = fp32 ? k_flow_poly3<true, true, 1> : k_flow_poly3<false, true, 1>;
+    const uint32_t wave = (uint32_t)resident_wave((const void*)k), n = (j.n + 4 * kGroup - 1) / (4 * kGroup);
+    k<<<n < wave ? n : wave, 128, 0, s>>>(g, a, PolyShape{verts, nv, rcut2, rcut2_hi32, site_error(g)}, Launch{}, 0u, j);
     return cudaGetLastError();
 }
 
@@ -1088,7 +1515,7 @@ cudaError_t launch_eval_poly(bool fp32, const Geometry& g, const Arrays& a, cons
                              double rcut2, float rcut2_hi32, const uint64_t* bodies, const double4* trial,
                              const double4* trial_q, uint32_t n, uint8_t* decisions, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    PolyShape sh{verts, nv, rcut2, rcut2_hi32};
+    PolyShape sh{verts, nv, rcut2, rcut2_hi32, 0.f};
     const uint32_t blocks = (n + 3) / 4;
     if (fp32)
         k_eval_poly3<true><<<blocks, 128, 0, s>>>(g, a, sh, bodies, trial, trial_q, n, decisions);

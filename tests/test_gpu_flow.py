@@ -10,8 +10,8 @@ import numpy as np
 import pytest
 
 import oracle
-from hoomd_rs_b200 import (FP32_RECHECK, FP64, TRANSLATE, Context, Isotropic, LennardJones, Microstate,
-                           PairwiseCutoff, Periodic, Shifted, lattice)
+from hoomd_rs_b200 import (FP32_RECHECK, FP64, ROTATE, TRANSLATE, Context, ConvexPolyhedron, HardShape, Isotropic,
+                           LennardJones, Microstate, PairwiseCutoff, Periodic, Shifted, lattice)
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +65,48 @@ def test_lj_one_colour_set_per_launch(ctx, precision, one_call, monkeypatch):
     monkeypatch.setenv("HMC_B200_FLOW_SETS", "1")
     g, o = lj(ctx, 3, 1500, 1.1, 2.7)
     check(g, o, precision, 2.7, sweeps=3, one_call=one_call)
+
+
+BOX = np.array([[x, y, z] for x in (-1.0, 1.0) for y in (-1.0, 1.0) for z in (-1.0, 1.0)])
+TETRAHEDRON = np.array([[1.0, 1.0, 1.0], [1.0, -1.0, -1.0], [-1.0, 1.0, -1.0], [-1.0, -1.0, 1.0]]) * 0.5
+ROUND = np.random.default_rng(11).normal(size=(32, 3))
+ROUND *= 0.55 / np.linalg.norm(ROUND, axis=1)[:, None]
+# shape, sites per axis, spacing per axis: units of one to sixteen trials with remainders, two spaces
+# per axis, 4 and 32 vertices, and thin rods, whose circumspheres hold more pairs than a warp's list
+# and whose rows hold more candidates than one pass over a stencil takes
+SHAPES = {"cubes_two_spaces": (BOX * 0.5, (3, 3, 3), (1.25, 1.25, 1.25)),
+          "cubes": (BOX * 0.5, (9, 8, 7), (1.2, 1.25, 1.3)),
+          "tetrahedra": (TETRAHEDRON, (7, 7, 7), (1.25, 1.25, 1.25)),
+          "round_32": (ROUND, (8, 7, 6), (1.2, 1.2, 1.2)),
+          "rods": (BOX * [0.1, 0.1, 1.0], (18, 18, 4), (0.5, 0.5, 2.2))}
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_RECHECK])
+@pytest.mark.parametrize("name", sorted(SHAPES))
+def test_polyhedra(ctx, name, precision):
+    verts, sites, spacing = SHAPES[name]
+    L = [n * a for n, a in zip(sites, spacing)]
+    rng = np.random.default_rng(5)
+    pos = (np.stack(np.meshgrid(*[np.arange(n) for n in sites], indexing="ij"), -1).reshape(-1, 3) + 0.5) * spacing
+    pos = pos - np.array(L) / 2 + rng.uniform(-0.01, 0.01, pos.shape)
+    reach = 2.0 * float(np.sqrt((verts ** 2).sum(axis=1).max()))
+    h = PairwiseCutoff(HardShape(ConvexPolyhedron.with_vertices(verts)))
+    o = oracle.System(3, L, pos, seed=77, interaction=oracle.HARD_CONVEX_POLYHEDRON, vertices=verts)
+    gs = [Microstate(ctx, Periodic(reach, L), pos, h, seed=77) for _ in range(2)]
+    for v, g in enumerate(gs):
+        g.set_launch_variant(precision, v)
+    for sweep in range(6):
+        move, maximum = ((TRANSLATE, 0.1), (ROTATE, 0.15))[sweep % 2]
+        want = o.parallel_sweep(oracle.TRANSLATE if move == TRANSLATE else oracle.ROTATE, maximum, 1.0, reach)
+        o.increment_step()
+        for g in gs:
+            c = g.sweep(move, maximum, 1.0, precision, n_sweeps=1, increment_step=True)
+            assert (c.accepted, c.rejected) == tuple(want), sweep
+    for g in gs:
+        assert np.array_equal(g.positions(), o.state()[0])
+        assert np.array_equal(g.orientations(), o.state()[1])
+
+
+def test_polyhedra_one_colour_set_per_launch(ctx, monkeypatch):
+    monkeypatch.setenv("HMC_B200_FLOW_SETS", "1")
+    test_polyhedra(ctx, "cubes", FP32_RECHECK)
