@@ -357,6 +357,8 @@ hmc_status setup_geometry(hmc_system* s, const double* L) {
         dfree(s, &A.cell_start);
         dfree(s, &A.block_sums);
         dfree(s, &A.color_cells);
+        dfree(s, &A.progress);  // the next sweep's flow_buffers allocates it for the new count
+        s->flow_cells = 0;
         const uint32_t scan_blocks = (uint32_t)((cells + 2047) / 2048);
         hmc_status st;
         if ((st = dalloc(s, &A.cell_count, cells)) || (st = dalloc(s, &A.cell_start, cells + 1)) ||
@@ -404,9 +406,12 @@ hmc_status flow_buffers(hmc_system* s) {
     const uint64_t cells = s->geom.n_cells;
     hmc_status st;
     if (s->flow_cells < cells) {
+        // every rebuild writes progress: as long as the other arrays by space, so that a box that grows
+        // between two sweeps finds room
         dfree(s, &A.progress);
-        if ((st = dalloc(s, &A.progress, cells))) return st;
-        s->flow_cells = (uint32_t)cells;
+        s->flow_cells = 0;
+        if ((st = dalloc(s, &A.progress, s->cells_alloc))) return st;
+        s->flow_cells = (uint32_t)s->cells_alloc;
     }
     const uint64_t want = s->capacity + cells;
     if (s->flow_entries >= want) return HMC_OK;

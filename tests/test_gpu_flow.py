@@ -110,3 +110,21 @@ def test_polyhedra(ctx, name, precision):
 def test_polyhedra_one_colour_set_per_launch(ctx, monkeypatch):
     monkeypatch.setenv("HMC_B200_FLOW_SETS", "1")
     test_polyhedra(ctx, "cubes", FP32_RECHECK)
+
+
+@pytest.mark.parametrize("scales", [(1.6,), (0.9, 1.4)])
+def test_box_grows_between_sweeps(ctx, scales):
+    """Estimators rebuild the cell list of the grown box before the next sweep does."""
+    g, o = lj(ctx, 3, 1500, 0.6, 2.5)
+    check(g, o, FP32_RECHECK, 2.5, sweeps=1)
+    L = g.edge_lengths[0]
+    for scale in scales:
+        L *= scale
+        g.set_box([L] * 3)
+        assert np.isfinite(g.total_energy())
+    fresh = Microstate(ctx, Periodic(2.5, [L] * 3), g.positions(),
+                       PairwiseCutoff(Isotropic(Shifted(LennardJones(1.0, 1.0), 2.5), 2.5)), seed=0x5EED0071, step=1)
+    assert fresh.total_energy() == pytest.approx(g.total_energy(), rel=1e-12)
+    for s in (g, fresh):
+        s.sweep(TRANSLATE, 0.12, 1.3, FP32_RECHECK, n_sweeps=2, increment_step=True)
+    assert np.array_equal(g.positions(), fresh.positions())
