@@ -432,9 +432,20 @@ hmc_status flow_buffers(hmc_system* s) {
     return HMC_OK;
 }
 
+// Hard spheres run in dataflow order (hmc_sphere.cu) while a colour holds few bodies, unless a colour pass
+// was chosen for the system. Both forms cost the same near (us per sweep, colour passes / dataflow; colour
+// passes by the faster of a lane and a warp per trial): 3-D FP32 100,003 bodies 233 / 187, 200,003
+// 254 / 302; 3-D FP64 200,003 495 / 345, 300,007 523 / 491, 500,009 572 / 793; 2-D FP32 16,384 77 / 71,
+// 50,021 80 / 99; 2-D FP64 16,384 87 / 71, 50,021 91 / 90, 100,003 95 / 128. The lines lie below
+// those points: at 114,688 and 262,144 bodies in 3-D, at 24,576 in 2-D.
+bool sphere_flow(const hmc_system* s, bool fp32) {
+    const uint64_t most = s->dim == 2 ? 6144 : (fp32 ? 14336 : 32768);  // bodies per colour
+    return s->interaction == HMC_HARD_SPHERE && !s->coop_set[fp32] && (s->n >> s->dim) <= most;
+}
+
 // Whether the system's sweeps run in dataflow order, and the colour sets one launch then holds.
-bool flow_of(const hmc_system* s) {
-    return s->soft() || (s->interaction == HMC_HARD_CONVEX_POLYHEDRON && !s->shape_soft);
+bool flow_of(const hmc_system* s, bool fp32) {
+    return s->soft() || (s->interaction == HMC_HARD_CONVEX_POLYHEDRON && !s->shape_soft) || sphere_flow(s, fp32);
 }
 uint32_t flow_sets(const hmc_system* s) {
     const uint64_t cells = s->geom.n_cells;
@@ -444,7 +455,7 @@ uint32_t flow_sets(const hmc_system* s) {
 
 // ---- launch variants -------------------------------------------------------------------------
 // The colour-pass kernel family a system's sweep runs in a precision, and its variant table.
-enum VariantFamily : uint32_t { kFamSphereDirect, kFamSphereCoop, kFamLj, kFamPoly3, kFamPoly2, kFamBatch, kFamBatchLj };
+enum VariantFamily : uint32_t { kFamSphereDirect, kFamSphereCoop, kFamSphereFlow, kFamLj, kFamPoly3, kFamPoly2, kFamBatch, kFamBatchLj };
 
 bool coop_of(const hmc_system* s, bool fp32);
 
@@ -452,6 +463,7 @@ uint32_t family_of(const hmc_system* s, bool fp32) {
     if (s->soft()) return kFamLj;
     if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON) return kFamPoly3;
     if (s->polygon()) return kFamPoly2;
+    if (sphere_flow(s, fp32)) return kFamSphereFlow;
     return coop_of(s, fp32) ? kFamSphereCoop : kFamSphereDirect;
 }
 
@@ -459,6 +471,7 @@ const LaunchShape* family_shapes(uint32_t fam, uint32_t* n) {
     switch (fam) {
         case kFamSphereDirect: *n = n_shapes(kSphereDirectShapes); return kSphereDirectShapes;
         case kFamSphereCoop: *n = n_shapes(kSphereCoopShapes); return kSphereCoopShapes;
+        case kFamSphereFlow: *n = n_shapes(kSphereFlowShapes); return kSphereFlowShapes;
         case kFamLj: *n = n_shapes(kLjShapes); return kLjShapes;
         case kFamPoly3: *n = n_shapes(kPolyShapes); return kPolyShapes;
         case kFamPoly2: *n = n_shapes(kPoly2Shapes); return kPoly2Shapes;
@@ -841,10 +854,12 @@ hmc_status hmc_system_create(hmc_context* ctx, const hmc_system_desc* d, const d
         hmc_status st = setup_geometry(s, d->edge_lengths);
         if (st) return destroy_fail(st);
     }
-    // The hard-sphere colour pass: per lane for FP32 (cheap pair tests), warp-cooperative for
-    // FP64 (each pair test costs more than the coordination), as measured on B200;
+    // The hard-sphere colour pass: per lane for FP32 (cheap pair tests) and for disks (nine spaces;
+    // FP64, 100,003 disks: 95 us per sweep against 192), warp-cooperative for FP64 in 3-D (each
+    // pair test costs more than the coordination), as measured on B200;
     // HMC_B200_SWEEP_KERNEL=direct or =coop forces one of them for both precisions.
     // HMC_B200_PDL=0 launches every colour pass after the previous one has ended.
+    if (s->dim == 2) s->coop[0] = false;
     if (const char* pdl = std::getenv("HMC_B200_PDL")) s->pdl = std::strcmp(pdl, "0") != 0;
     if (const char* kern = std::getenv("HMC_B200_SWEEP_KERNEL")) {
         const bool direct = std::strcmp(kern, "direct") == 0, coop = std::strcmp(kern, "coop") == 0;
@@ -1044,7 +1059,7 @@ static SweepPlan sweep_plan(const hmc_system* s, const hmc_sweep_params* p) {
 // The cell-list rebuild of the current sweep; shapes read S in both modes, and the colour passes
 // do not read slot_of_body.
 static hmc_status sweep_rebuild(hmc_system* s, const SweepPlan& sp) {
-    if (flow_of(s)) {
+    if (flow_of(s, sp.fp32)) {
         hmc_status st = flow_buffers(s);
         if (st) return st;
     }
@@ -1068,14 +1083,16 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
                                uint32_t r1) {
     const bool fp32 = sp.fp32;
     const uint32_t colors = 1u << s->dim;
-    if (flow_of(s)) {
+    if (flow_of(s, fp32)) {
         const uint32_t sets = flow_sets(s);
         L.substep = s->substep;  // the kernels add the colour set
         for (uint32_t r = r0; r < r1; r += std::min(sets, r1 - r)) {
             L.round = r;
             L.round_end = r + std::min(sets, r1 - r);
             // the overlap penalty and Isotropic have no FP32 path: FP64 in both modes
-            if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON)
+            if (s->interaction == HMC_HARD_SPHERE)
+                HMC_CUDA(launch_flow_sphere(s->dim, fp32, s->geom, s->arr, s->pair, L, s->stream, sp.variant));
+            else if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON)
                 HMC_CUDA(launch_flow_poly(fp32, s->geom, s->arr, s->verts, s->n_vertices, s->poly_rcut2,
                                           s->poly_rcut2_hi32, L, p->move == HMC_ROTATE, s->stream, sp.variant));
             else
@@ -1121,8 +1138,8 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
 
 // The colour sets the host enqueues before it knows a sweep's count: the last sweep's, or all of
 // them where one dataflow launch runs however many there are.
-static uint32_t guessed_sets(const hmc_system* s) {
-    return flow_of(s) && flow_sets(s) == UINT32_MAX ? UINT32_MAX : std::max(1u, s->rounds_guess);
+static uint32_t guessed_sets(const hmc_system* s, bool fp32) {
+    return flow_of(s, fp32) && flow_sets(s) == UINT32_MAX ? UINT32_MAX : std::max(1u, s->rounds_guess);
 }
 
 // A finished sweep into the call's Count and the system's Counter.
@@ -1174,7 +1191,7 @@ static hmc_status sweep_pipelined(hmc_system* s, const hmc_sweep_params* p, hmc_
             s->step = step0 + j;
             s->substep = j == 0 ? substep0 : 0u;
             if ((st = sweep_rebuild(s, sp))) break;
-            if (j == 0) guess = guessed_sets(s);
+            if (j == 0) guess = guessed_sets(s, sp.fp32);
             Launch L = sweep_launch(s, p);
             if ((st = enqueue_sets(s, p, sp, L, 0, guess))) break;
             cudaError_t e = launch_sweep_guard(s->arr.stats, guess, s->arr.abort_word, s->stream);
@@ -1255,7 +1272,7 @@ hmc_status hmc_sweep(hmc_system* s, const hmc_sweep_params* p, hmc_count* out) {
         // The rounds (while count.total() < N, :402-418) are known on the device after the
         // rebuild; the host enqueues the previous sweep's number of colour sets without
         // waiting, the kernels skip sets beyond the true count, and any missing sets follow.
-        const uint32_t guess = s->n == 0 ? 0u : guessed_sets(s);
+        const uint32_t guess = s->n == 0 ? 0u : guessed_sets(s, sp.fp32);
         if ((st = enqueue_sets(s, p, sp, L, 0, guess))) return st;
         // the passes' end is recorded before the host waits for the counts, so that profiling adds
         // no host round trip to the sweep
@@ -1277,7 +1294,7 @@ hmc_status hmc_sweep(hmc_system* s, const hmc_sweep_params* p, hmc_count* out) {
             s->prof.rebuild_launches += rebuild_kernels(s);
             s->prof.sweep_ms += t_sweep;
             // a dataflow launch holds several colour passes
-            s->prof.sweep_launches += flow_of(s) ? (guess == UINT32_MAX ? 1u : std::max(rounds, guess))
+            s->prof.sweep_launches += flow_of(s, sp.fp32) ? (guess == UINT32_MAX ? 1u : std::max(rounds, guess))
                                                  : (uint64_t)std::max(rounds, guess) * colors;
             s->prof.sweeps += 1;
         }
@@ -1387,7 +1404,7 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
     // hard spheres without a pass chosen for the system: both passes (a lane or a warp per
     // trial) and each one's variants, the current pass first
     const bool coop0 = coop_of(s, fp32), coop_set0 = s->coop_set[fp32], coop_own0 = s->coop[fp32];
-    const bool both = s->interaction == HMC_HARD_SPHERE && !coop_set0;
+    const bool both = s->interaction == HMC_HARD_SPHERE && !coop_set0 && !sphere_flow(s, fp32);
     // the state to start every variant from
     const uint64_t n = s->n;
     const uint64_t step0 = s->step;
@@ -2309,6 +2326,8 @@ hmc_status hmc_eval_trials(hmc_system* s, const hmc_injected_move* moves, uint64
         else if (s->oriented())
             e = launch_trials_poly(fp32, s->geom, s->arr, s->verts, s->n_vertices, s->poly_rcut2, s->poly_rcut2_hi32, j,
                                    s->stream);
+        else if (sphere_flow(s, fp32))
+            e = launch_flow_trials_sphere(s->dim, fp32, s->geom, s->arr, s->pair, j, s->stream);
         else
             e = launch_trials_sphere(s->dim, fp32, coop_of(s, fp32), s->geom, s->arr, s->pair, j, s->stream);
         s->prof.kernel_launches++;

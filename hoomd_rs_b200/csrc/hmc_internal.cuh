@@ -309,6 +309,7 @@ struct LaunchShape {
     uint32_t blocks_per_sm, trials_per_warp, own_steps;
 };
 constexpr LaunchShape kSphereDirectShapes[] = {{6, 1, 0}, {5, 1, 0}, {7, 1, 0}};
+constexpr LaunchShape kSphereFlowShapes[] = {{4, 3, 0}, {6, 3, 0}};
 constexpr LaunchShape kSphereCoopShapes[] = {{6, 1, 2}, {6, 1, 1}, {6, 1, 3}, {5, 1, 2}, {7, 1, 2}};
 // Lennard-Jones and Isotropic trials; own_steps: warps per trial (variant 0: by the trials of a
 // colour)
@@ -441,6 +442,12 @@ cudaError_t launch_flow_batch_lj(int dim, bool fp32, const Batch& b, const Array
 // coop selects the warp-cooperative pass (the per-lane pass otherwise).
 cudaError_t launch_sweep_sphere(int dim, bool fp32, const Geometry& g, const Arrays& a, const Pair& p,
                                 const Launch& l, bool coop, cudaStream_t s, uint32_t variant = 0);
+// Hard spheres in dataflow order (hmc_sphere.cu): the colour sets [l.round, l.round_end), two kernels as in
+// launch_flow_lj.
+cudaError_t launch_flow_sphere(int dim, bool fp32, const Geometry& g, const Arrays& a, const Pair& p, const Launch& l,
+                               cudaStream_t s, uint32_t variant = 0);
+cudaError_t launch_flow_trials_sphere(int dim, bool fp32, const Geometry& g, const Arrays& a, const Pair& p,
+                                      const Injected& j, cudaStream_t s);
 cudaError_t launch_overlap_sphere(int dim, const Geometry& g, const Arrays& a, const Pair& p, uint32_t n,
                                   cudaStream_t s);
 // generic: the system's energy is not Shifted Lennard-Jones (the overlap penalty, Isotropic).

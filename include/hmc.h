@@ -252,9 +252,9 @@ hmc_status hmc_overlap_check(hmc_system* sys, uint64_t* n_overlaps);
 hmc_status hmc_eval_moves(hmc_system* sys, const hmc_injected_move* moves, uint64_t n, double temperature,
                           uint32_t precision, uint8_t* decisions, uint8_t* rechecked, double* delta_h);
 /* The colour pass's own decision for injected trial moves: the kernel that hmc_sweep runs for
- * the system's interaction and `precision` (hard spheres: the per-lane FP32 pass or the
- * warp-cooperative FP64 pass; Lennard-Jones and the overlap penalty: the warp-per-trial passes;
- * convex polyhedra: the packed pass) takes each move in place of a drawn trial
+ * the system's interaction and `precision` (hard spheres: the dataflow sweep of a small box, the
+ * per-lane or the warp-cooperative pass; Lennard-Jones and the overlap penalty: teams of warps per
+ * trial; convex polyhedra: the packed pass) takes each move in place of a drawn trial
  * (generate_trial_moves, parallel_sweep.rs:231-278) and writes its decision instead of
  * committing it; the state does not change. The checkerboard is the one the next hmc_sweep lays
  * out (update_checkerboard, parallel_sweep.rs:176-201: origin from the system's counter).
@@ -273,8 +273,8 @@ hmc_status hmc_total_energy(hmc_system* sys, double* energy);
 
 /* ---- launch variants and the autotuner (no counterpart in the reference) ----
  * Every colour-pass kernel is compiled in a few launch shapes: the resident blocks per SM it
- * is built for (its register cap), the trials a warp takes (convex polyhedra: 4, 2 or 8) and,
- * for the warp-cooperative FP64 sphere pass, the candidates per stencil row a lane tests before
+ * is built for (its register cap), the trials a warp takes (convex polyhedra: 4; hard spheres in
+ * dataflow order: 3) and, for the warp-cooperative FP64 sphere pass, the candidates per stencil row a lane tests before
  * handing the rest to its warp; for convex polygons in HMC_FP32_RECHECK, variant 1 runs the FP64
  * pass instead of the FP32 prefilter. All take the same decisions, so the trajectory is the same
  * in every variant; only the speed differs, by shape and density. hmc_autotune times `sweeps`
@@ -297,10 +297,12 @@ hmc_status hmc_get_launch_variant(hmc_system* sys, uint32_t precision, uint32_t 
 /* index UINT32_MAX: drop the system's own choice (the recorded one for its band, else 0). */
 hmc_status hmc_set_launch_variant(hmc_system* sys, uint32_t precision, uint32_t index);
 /* Hard spheres and disks: which colour pass a precision runs, one lane per trial (cooperative = 0,
- * the FP32 default) or the warp-cooperative pass (1, the FP64 default). Both make the same pair
- * tests, so the trajectory does not depend on the choice; the launch variants are those of the
- * chosen pass. A system without its own choice runs the one hmc_autotune recorded for its
- * dimension, precision and density band, else the default. HMC_NOT_SUPPORTED for other
+ * the FP32 default and the default of disks) or the warp-cooperative pass (1, the FP64 default in
+ * 3-D). Both make the same pair tests, so the trajectory does not depend on the choice; the launch
+ * variants are those of the chosen pass. A system without its own choice runs the one hmc_autotune
+ * recorded for its dimension, precision and density band, else the default; with few bodies (up to
+ * 114,688 spheres in FP32, 262,144 in FP64, 24,576 disks) it runs its sweeps in dataflow order, one
+ * launch for all colour passes, with launch variants of its own. HMC_NOT_SUPPORTED for other
  * interactions. */
 hmc_status hmc_set_cooperative_pass(hmc_system* sys, uint32_t precision, uint32_t cooperative);
 hmc_status hmc_get_cooperative_pass(hmc_system* sys, uint32_t precision, uint32_t* cooperative);

@@ -10,8 +10,8 @@ import numpy as np
 import pytest
 
 import oracle
-from hoomd_rs_b200 import (FP32_RECHECK, FP64, ROTATE, TRANSLATE, Context, ConvexPolyhedron, HardShape, Isotropic,
-                           LennardJones, Microstate, PairwiseCutoff, Periodic, Shifted, lattice)
+from hoomd_rs_b200 import (FP32_RECHECK, FP64, ROTATE, TRANSLATE, Context, ConvexPolyhedron, HardShape, HardSphere,
+                           Isotropic, LennardJones, Microstate, PairwiseCutoff, Periodic, Shifted, lattice)
 
 pytestmark = pytest.mark.gpu
 
@@ -128,3 +128,70 @@ def test_box_grows_between_sweeps(ctx, scales):
     for s in (g, fresh):
         s.sweep(TRANSLATE, 0.12, 1.3, FP32_RECHECK, n_sweeps=2, increment_step=True)
     assert np.array_equal(g.positions(), fresh.positions())
+
+# spaces per axis (of width 1.02 .. 1.3), sites per axis: two spaces on an axis (images of one space),
+# units of one to three trials, spaces with one and several bodies, empty spaces
+SPHERES = [(3, (2, 2, 2), (2, 2, 2)), (3, (2, 4, 6), (2, 4, 6)), (3, (4, 4, 4), (2, 2, 2)), (3, (6, 6, 6), (6, 6, 6)),
+           (3, (8, 10, 12), (7, 9, 10)), (2, (2, 2), (2, 2)), (2, (2, 6), (2, 6)), (2, (12, 14), (12, 13))]
+
+
+def spheres(ctx, dim, spaces, sites, seed=0x5EED0081):
+    L = [1.02 * n + 0.05 for n in spaces]
+    rng = np.random.default_rng(3)
+    grid = np.stack(np.meshgrid(*[np.arange(n) for n in sites], indexing="ij"), -1).reshape(-1, dim)
+    pos = (grid + 0.5) * np.array(L) / np.array(sites) - np.array(L) / 2 + rng.uniform(-0.005, 0.005, grid.shape)
+    g = Microstate(ctx, Periodic(1.0, L), pos, PairwiseCutoff(HardSphere(1.0)), seed=seed)
+    return g, oracle.System(dim, L, pos, diameter=1.0, seed=seed)
+
+
+def check_spheres(g, o, precision, one_call=False, sweeps=4):
+    want = np.zeros(2, dtype=np.int64)
+    for _ in range(sweeps):
+        want += o.parallel_sweep(oracle.TRANSLATE, 0.2, 1.0, 1.0)
+        o.increment_step()
+    if one_call:
+        c = g.sweep(TRANSLATE, 0.2, 1.0, precision, n_sweeps=sweeps, increment_step=True)
+        got = (c.accepted, c.rejected)
+    else:
+        cs = [g.sweep(TRANSLATE, 0.2, 1.0, precision, n_sweeps=1, increment_step=True) for _ in range(sweeps)]
+        got = (sum(c.accepted for c in cs), sum(c.rejected for c in cs))
+    assert got == tuple(want)
+    assert np.array_equal(g.positions(), o.state()[0])
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_RECHECK])
+@pytest.mark.parametrize("dim,spaces,sites", SPHERES)
+def test_spheres(ctx, dim, spaces, sites, precision):
+    for variant in range(2):
+        g, o = spheres(ctx, dim, spaces, sites)
+        assert g.launch_variant(precision)["trials_per_warp"] == 3  # the dataflow family
+        g.set_launch_variant(precision, variant)
+        check_spheres(g, o, precision)
+        g.close()
+
+
+@pytest.mark.parametrize("one_call", [False, True])
+@pytest.mark.parametrize("precision", [FP64, FP32_RECHECK])
+def test_spheres_one_colour_set_per_launch(ctx, precision, one_call, monkeypatch):
+    monkeypatch.setenv("HMC_B200_FLOW_SETS", "1")
+    g, o = spheres(ctx, 3, (8, 10, 12), (7, 9, 10))
+    check_spheres(g, o, precision, one_call)
+
+
+@pytest.mark.parametrize("precision,n", [(FP64, 262144), (FP32_RECHECK, 114688)])
+def test_spheres_beside_the_line(ctx, precision, n):
+    """The largest box in dataflow order and the smallest in colour passes, each against the other form."""
+    for bodies in (n + 7, n + 8):
+        pos, L = lattice.hard_sphere_box(bodies, 0.45, 3, 5)
+        runs = []
+        for forced in (False, True):
+            g = Microstate(ctx, Periodic(1.0, [L] * 3), pos, PairwiseCutoff(HardSphere(1.0)), seed=9)
+            if forced:
+                g.set_cooperative_pass(precision, False)
+            flow = g.launch_variant(precision)["trials_per_warp"] == 3
+            assert flow == (not forced and bodies == n + 7)
+            c = g.sweep(TRANSLATE, 0.15, 1.0, precision, n_sweeps=2, increment_step=True)
+            runs.append((c.accepted, c.rejected, g.positions()))
+            g.close()
+        assert runs[0][:2] == runs[1][:2]
+        assert np.array_equal(runs[0][2], runs[1][2])
