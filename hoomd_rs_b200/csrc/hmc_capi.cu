@@ -1126,7 +1126,7 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
                                                  s->stream));
             else if (s->polygon())
                 HMC_CUDA(launch_sweep_poly2(sp.poly2_fp32, s->sat(), s->geom, s->arr, s->verts, s->n_vertices,
-                                            s->poly_rcut2, s->poly_rcut2_hi32, L, p->move == HMC_ROTATE, s->stream));
+                                            s->poly_rcut2, s->poly_rcut2_hi32, L, s->stream));
             else
                 HMC_CUDA(launch_sweep_sphere(s->dim, fp32, s->geom, s->arr, s->pair, L, sp.coop, s->stream,
                                              sp.variant));

@@ -319,7 +319,7 @@ constexpr LaunchShape kBatchShapes[] = {{4, 1, 0}, {3, 1, 0}, {5, 1, 0}, {6, 1, 
 // The polygon pass: one compiled shape; in the FP32 mode, variant 1 runs the FP64 pass instead
 // of the FP32 prefilter (the same decisions; the prefilter saves little where the FP64
 // circumsphere test is cheap against the separating-axis or XenoCollide test behind it).
-constexpr LaunchShape kPoly2Shapes[] = {{8, 4, 0}, {8, 4, 0}};
+constexpr LaunchShape kPoly2Shapes[] = {{6, 8, 0}, {6, 8, 0}};
 // the Lennard-Jones replicas, as kLjShapes
 constexpr LaunchShape kBatchLjShapes[] = {{0, 1, 0}, {6, 1, 1}, {12, 1, 2}, {6, 1, 4}, {3, 1, 8}};
 template <size_t N>
@@ -512,8 +512,7 @@ cudaError_t launch_tune_moves(int dim, const Geometry& g, const Arrays& a, const
 // Hard convex polygons (hmc_poly2.cu): XenoCollide (sat = false) or separating axes (sat =
 // true); orientations are angles in .x of body_ori / sorted_q / trial_q.
 cudaError_t launch_sweep_poly2(bool fp32, bool sat, const Geometry& g, const Arrays& a, const double4* verts,
-                               uint32_t nv, double rcut2, float rcut2_hi32, const Launch& l, bool rotate,
-                               cudaStream_t s);
+                               uint32_t nv, double rcut2, float rcut2_hi32, const Launch& l, cudaStream_t s);
 cudaError_t launch_eval_poly2(bool fp32, bool sat, const Geometry& g, const Arrays& a, const double4* verts,
                               uint32_t nv, double rcut2, float rcut2_hi32, const uint64_t* bodies,
                               const double4* trial, const double4* trial_q, uint32_t n, uint8_t* decisions,

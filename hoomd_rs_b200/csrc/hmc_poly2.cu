@@ -10,7 +10,7 @@
 // multiply-add follows the reference's expression order; sin and cos are correctly rounded
 // (cr_sincos), so the FP64 decision is the reference's on a correctly rounded libm.
 //
-// The colour pass gives a warp four trials, as for polyhedra (k_sweep_poly2); injected moves
+// The colour pass gives a warp eight trials (k_sweep_poly2); injected moves
 // take one warp per move and the stencil's candidates 32 at a time, with an early exit by
 // vote. FP32 + recheck: candidates whose FP32 centre distance clears the circumcircles by more
 // than the FP32 error bound are skipped; every other candidate runs the FP64 test.
@@ -21,13 +21,16 @@
 namespace hmc {
 namespace {
 
-// Resident blocks per SM the colour pass is compiled for: 8 caps it at 64 registers. On 2^18
-// hard squares at area fraction 0.60 this measured 6.4e8 (FP32 prefilter) and 6.7e8 (FP64)
-// trial moves/s, against 6.1e8 and 6.5e8 at 80 registers, 4.3e8 and 4.2e8 uncapped (180
-// registers) and 1.5e8 and 1.6e8 with one warp per trial.
-#ifndef HMC_POLY2_MIN_BLOCKS
-#define HMC_POLY2_MIN_BLOCKS 8
-#endif
+// The colour pass: trials a warp takes, and resident blocks per SM it is compiled for. 2^18 hard squares at
+// area fraction 0.60 have 2.7 candidates a trial inside the circumcircles, and the test of such a
+// pair is most of the work (FP64: two sines and cosines, XenoCollide's supports), so a warp tests
+// the pairs of its trials together: 8 trials list about 22, near a full warp's 32. Ten translation and
+// rotation sweeps of that box (ms; FP32 prefilter / FP64): 12.4 / 11.5 with 4 trials, the sine and
+// cosine of the trial's own angle per pair and the vertices in global memory; 11.5 / 11.3 with 4
+// trials, that sine per trial and the vertices in shared memory; 8.1 / 7.8 with 8 trials; 8.4 / 8.3 with
+// 16. At 8 trials: 6 blocks per SM (80 registers) 8.1 / 7.8, 4: 8.2 / 8.2, 8: 8.5 / 8.1.
+constexpr uint32_t kPoly2Trials = 8;
+constexpr int kPoly2Blocks = 6;
 
 struct V2 {
     double x, y;
@@ -51,27 +54,37 @@ __device__ __forceinline__ bool mat2_from_angle(double theta, M2* m) {
     return true;
 }
 
+__device__ __forceinline__ V2 vertex(const double4* __restrict__ verts, uint32_t i) {
+    const double4 v = ldg4(verts + i);
+    return {v.x, v.y};
+}
+__device__ __forceinline__ V2 vertex(const double2* verts, uint32_t i) {  // (a block's copy in shared memory)
+    const double2 v = verts[i];
+    return {v.x, v.y};
+}
+
 // ConvexPolytope::support_mapping in 2-D: argmax of v0 n0 + v1 n1, first maximum wins.
-__device__ __forceinline__ V2 support2(const double4* __restrict__ verts, uint32_t nv, const V2& n) {
+template <typename Vertex>
+__device__ __forceinline__ V2 support2(const Vertex* verts, uint32_t nv, const V2& n) {
     uint32_t arg = 0;
     double best = -INFINITY;
 #pragma unroll 4  // vertex loads of several iterations in flight; comparisons stay in order
     for (uint32_t i = 0; i < nv; ++i) {
-        const double4 v = ldg4(verts + i);
+        const V2 v = vertex(verts, i);
         const double x = dadd(dmul(v.x, n.x), dmul(v.y, n.y));
         if (x > best) {
             best = x;
             arg = i;
         }
     }
-    const double4 v = ldg4(verts + arg);
-    return {v.x, v.y};
+    return vertex(verts, arg);
 }
 
 constexpr int kXenoMaxIter2 = 1024;  // xenocollide.rs:38
 
 // collide for N = 2 (xenocollide.rs:92-154, :361-414); the iteration cap returns overlap.
-__device__ __noinline__ bool collide2d(const double4* verts, uint32_t nv, const V2& vij, const M2& q) {
+template <typename Vertex>
+__device__ __noinline__ bool collide2d(const Vertex* verts, uint32_t nv, const V2& vij, const M2& q) {
     const M2 qinv = transpose2(q);
     // composite_support_mapping (xenocollide.rs:318-328)
     auto s = [&](const V2& n) -> V2 {
@@ -114,21 +127,21 @@ __device__ __noinline__ bool collide2d(const double4* verts, uint32_t nv, const 
 }
 
 // is_separating (convex_surface_mesh_2d.rs:625-640): every vertex of a strictly outside.
-__device__ __forceinline__ bool is_separating(const double4* verts, uint32_t nv, const V2& p, const V2& n) {
+template <typename Vertex>
+__device__ __forceinline__ bool is_separating(const Vertex* verts, uint32_t nv, const V2& p, const V2& n) {
     const double n_dot_p = dot2(n, p);
     for (uint32_t i = 0; i < nv; ++i) {
-        const double4 v = ldg4(verts + i);
-        if (dsub(dot2(n, V2{v.x, v.y}), n_dot_p) <= 0.0) return false;
+        if (dsub(dot2(n, vertex(verts, i)), n_dot_p) <= 0.0) return false;
     }
     return true;
 }
 // b_edge_separates (:597-623) with a = b = the shape.
-__device__ __forceinline__ bool b_edge_separates(const double4* verts, uint32_t nv, const V2& v_ab, const M2& o_b) {
+template <typename Vertex>
+__device__ __forceinline__ bool b_edge_separates(const Vertex* verts, uint32_t nv, const V2& v_ab, const M2& o_b) {
     uint32_t previous = nv - 1;
     for (uint32_t current = 0; current < nv; ++current) {
-        const double4 pc = ldg4(verts + current), pp = ldg4(verts + previous);
-        const V2 p{pc.x, pc.y};
-        const V2 edge = sub2(p, V2{pp.x, pp.y});
+        const V2 p = vertex(verts, current);
+        const V2 edge = sub2(p, vertex(verts, previous));
         const V2 n{edge.y, -edge.x};  // -edge.perpendicular()
         V2 pa = mat2_rotate(o_b, p);
         pa = {dadd(pa.x, v_ab.x), dadd(pa.y, v_ab.y)};
@@ -139,7 +152,8 @@ __device__ __forceinline__ bool b_edge_separates(const double4* verts, uint32_t 
     return false;
 }
 // ConvexSurfaceMesh2d::intersects_at (:578-593).
-__device__ __noinline__ bool sat_intersects(const double4* verts, uint32_t nv, const V2& v_ij, const M2& o_j) {
+template <typename Vertex>
+__device__ __noinline__ bool sat_intersects(const Vertex* verts, uint32_t nv, const V2& v_ij, const M2& o_j) {
     if (b_edge_separates(verts, nv, v_ij, o_j)) return false;
     const M2 inv = transpose2(o_j);
     const V2 v_ji = mat2_rotate(inv, V2{-v_ij.x, -v_ij.y});
@@ -221,38 +235,56 @@ __device__ __forceinline__ bool poly2_overlaps(const Geometry& g, const Arrays& 
     return false;
 }
 
-// ---- the colour pass, four trials per warp ---------------------------------------------------
-// As for polyhedra (hmc_poly.cu): each group of 8 lanes computes its trial and prefilters its
+// ---- the colour pass, eight trials per warp --------------------------------------------------
+// Each group of 4 lanes (a row of the stencil holds about 4 candidates) takes a trial and prefilters its
 // candidates by circumcircle, the candidates that need the full FP64 test are compacted over
 // the warp into a shared-memory list, and the warp runs those tests 32 pairs at a time, ORing
 // overlaps into a per-trial mask (a trial known to overlap lists no further candidates). The
 // decision of each trial is the OR of the same pair tests as with one warp per trial.
-constexpr int kPoly2TrialsPerWarp = 4;
 constexpr uint32_t kPair2Cap = 128;  // listed pairs per warp before the warp drains the list
+constexpr uint32_t kVerts2 = 32;     // a polygon's vertices at most
 
 struct Poly2Trial {
     double t[2];
-    double angle;
+    double inv;     // Angle::inverted
+    double sn, cs;  // of inv
+    bool bad;       // inv is beyond the range of cr_sincos
 };
+
+// poly2_overlap64 of a trial whose sine and cosine are known.
+template <bool SAT, typename Vertex>
+__device__ __forceinline__ bool trial_overlap64(const Geometry& g, const Arrays& A, const PolyShape2& sh,
+                                                const Vertex* verts, const Poly2Trial& tr, uint32_t q,
+                                                bool* range_error) {
+    const double4 s4 = ldg4(A.sorted_s + q);
+    const double t[3] = {tr.t[0], tr.t[1], 0.0}, sj[3] = {s4.x, s4.y, 0.0};
+    double d[3];
+    if (ref_disp<2>(g, t, sj, d) >= sh.rcut2) return false;
+    const V2 rab{-d[0], -d[1]};  // image - t
+    M2 m;
+    if (tr.bad || !mat2_from_angle(dadd(tr.inv, __ldg(&A.sorted_q[q].x)), &m)) {
+        *range_error = true;
+        return true;
+    }
+    const V2 vij{dsub(dmul(rab.x, tr.cs), dmul(rab.y, tr.sn)), dadd(dmul(rab.x, tr.sn), dmul(rab.y, tr.cs))};
+    return SAT ? sat_intersects(verts, sh.nv, vij, m) : collide2d(verts, sh.nv, vij, m);
+}
 
 template <bool SAT>
 __device__ __forceinline__ void drain_pairs2(const Geometry& g, const Arrays& A, const PolyShape2& sh,
-                                             const Poly2Trial* trials, const uint32_t* pair_q, const uint8_t* pair_g,
-                                             uint32_t n_pairs, uint32_t lane, uint32_t& mask, bool* range_error) {
+                                             const double2* verts, const Poly2Trial* trials, const uint32_t* pair_q,
+                                             const uint8_t* pair_g, uint32_t n_pairs, uint32_t lane, uint32_t& mask,
+                                             bool* range_error) {
     __syncwarp();
+#pragma unroll 1
     for (uint32_t p0 = 0; p0 < n_pairs; p0 += 32) {
         const uint32_t p = p0 + lane;
         uint32_t bit = 0;
         if (p < n_pairs) {
             const uint32_t gg = pair_g[p];
-            if (!((mask >> gg) & 1u)) {
-                const uint32_t q = pair_q[p];
-                const Poly2Trial& tr = trials[gg];
-                const double t[3] = {tr.t[0], tr.t[1], 0.0};
-                const double4 s4 = ldg4(A.sorted_s + q);
-                const double sj[3] = {s4.x, s4.y, 0.0};
-                if (poly2_overlap64<SAT>(g, A, sh, t, tr.angle, sj, q, range_error)) bit = 1u << gg;
-            }
+            if (!((mask >> gg) & 1u) &&
+                trial_overlap64<SAT>(g, A, sh, verts, trials[gg], pair_q[p], range_error))
+                bit = 1u << gg;
         }
         mask |= __reduce_or_sync(0xffffffffu, bit);
     }
@@ -260,9 +292,15 @@ __device__ __forceinline__ void drain_pairs2(const Geometry& g, const Arrays& A,
 }
 
 template <bool FP32, bool SAT>
-__global__ void __launch_bounds__(128, HMC_POLY2_MIN_BLOCKS)
-    k_sweep_poly2(Geometry g, Arrays A, PolyShape2 sh, Launch L, uint32_t rotate) {
-    constexpr uint32_t G = kPoly2TrialsPerWarp, S = 32 / G;  // trials per warp, lanes per trial
+__global__ void __launch_bounds__(128, kPoly2Blocks)
+    k_sweep_poly2(Geometry g, Arrays A, PolyShape2 sh, Launch L) {
+    constexpr uint32_t G = kPoly2Trials, S = 32 / G;  // trials per warp, lanes per trial
+    __shared__ double2 s_verts[kVerts2];
+    for (uint32_t i = threadIdx.x; i < sh.nv; i += blockDim.x) {
+        const V2 v = vertex(sh.verts, i);
+        s_verts[i] = make_double2(v.x, v.y);
+    }
+    __syncthreads();
     if (L.early_wait) grid_dependency_wait();  // first pass: the rebuild's arrays are read at once
     __shared__ Poly2Trial s_trial[4][G];
     __shared__ uint32_t s_pair_q[4][kPair2Cap];
@@ -301,13 +339,16 @@ __global__ void __launch_bounds__(128, HMC_POLY2_MIN_BLOCKS)
             Poly2Trial& tr = s_trial[wib][grp];
             tr.t[0] = t[0];
             tr.t[1] = t[1];
-            tr.angle = ti;
+            tr.inv = -ti;
+            tr.bad = !cr_sincos(tr.inv, &tr.sn, &tr.cs);
         }
         grid_dependency_wait();  // the previous colour's moves are visible from here on
         allow_dependent_launch();
         uint32_t mask = 0, n_pairs = 0;  // warp-uniform
+        // (the odd parts are the rows' spaces across the fast-axis end)
+        const int step = __any_sync(0xffffffffu, valid && sf > 2 && (m[1] == 0 || m[1] + 1 == sf)) ? 1 : 2;
 #pragma unroll 1
-        for (int part = 0; part < 2 * kRows<2>; ++part) {
+        for (int part = 0; part < 2 * kRows<2>; part += step) {
             uint32_t lo = 0, len = 0;
             float s0 = 0.f, s1 = 0.f;
             if (valid) stencil_part<2>(g, A.cell_start, m, part >> 1, (part & 1) != 0, lo, len, s0, s1);
@@ -345,15 +386,19 @@ __global__ void __launch_bounds__(128, HMC_POLY2_MIN_BLOCKS)
                 }
                 n_pairs += __popc(b);
                 if (n_pairs > kPair2Cap - 32) {
-                    drain_pairs2<SAT>(g, A, sh, s_trial[wib], s_pair_q[wib], s_pair_g[wib], n_pairs, lane, mask,
+                    drain_pairs2<SAT>(g, A, sh, s_verts, s_trial[wib], s_pair_q[wib], s_pair_g[wib], n_pairs, lane, mask,
                                       &range_error);
                     n_pairs = 0;
                 }
             }
         }
-        drain_pairs2<SAT>(g, A, sh, s_trial[wib], s_pair_q[wib], s_pair_g[wib], n_pairs, lane, mask, &range_error);
+        drain_pairs2<SAT>(g, A, sh, s_verts, s_trial[wib], s_pair_q[wib], s_pair_g[wib], n_pairs, lane, mask, &range_error);
         if (sub == 0 && valid && !((mask >> grp) & 1u)) {
             n_accepted++;
+            const Poly2Trial& tr = s_trial[wib][grp];
+            t[0] = tr.t[0];
+            t[1] = tr.t[1];
+            const double ti = -tr.inv;
             double sv[3] = {t[0], t[1], 0.0};
             wrap_inv<2>(g.L, g.invL, sv);
             const uint32_t body = A.sorted_body[k];
@@ -818,27 +863,17 @@ __global__ void k_sincos(const double* x, uint64_t n, double* s, double* c, uint
 }  // namespace
 
 cudaError_t launch_sweep_poly2(bool fp32, bool sat, const Geometry& g, const Arrays& a, const double4* verts,
-                               uint32_t nv, double rcut2, float rcut2_hi32, const Launch& l, bool rotate,
-                               cudaStream_t s) {
+                               uint32_t nv, double rcut2, float rcut2_hi32, const Launch& l, cudaStream_t s) {
     if (l.n_active == 0) return cudaSuccess;
-    static int max_blocks = 0;
-    if (max_blocks == 0) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        max_blocks = sms * 16;
-    }
     PolyShape2 sh{verts, nv, rcut2, rcut2_hi32};
-    const uint32_t per_block = 4u * kPoly2TrialsPerWarp;  // four warps per block
+    using Kernel = void (*)(Geometry, Arrays, PolyShape2, Launch);
+    const Kernel k = fp32 ? (sat ? k_sweep_poly2<true, true> : k_sweep_poly2<true, false>)
+                          : (sat ? k_sweep_poly2<false, true> : k_sweep_poly2<false, false>);
+    const uint32_t per_block = 4u * kPoly2Trials, wave = (uint32_t)resident_wave((const void*)k);
     uint32_t blocks = (l.n_active + per_block - 1) / per_block;
-    if (blocks > (uint32_t)max_blocks) blocks = (uint32_t)max_blocks;
-    const uint32_t rot = rotate ? 1u : 0u;
+    if (blocks > wave * 2u) blocks = wave * 2u;
     PassLaunch pl(blocks, l.overlap_previous != 0 || l.early_wait != 0, s);
-    if (fp32)
-        return sat ? cudaLaunchKernelEx(&pl.cfg, k_sweep_poly2<true, true>, g, a, sh, l, rot)
-                   : cudaLaunchKernelEx(&pl.cfg, k_sweep_poly2<true, false>, g, a, sh, l, rot);
-    return sat ? cudaLaunchKernelEx(&pl.cfg, k_sweep_poly2<false, true>, g, a, sh, l, rot)
-               : cudaLaunchKernelEx(&pl.cfg, k_sweep_poly2<false, false>, g, a, sh, l, rot);
+    return cudaLaunchKernelEx(&pl.cfg, k, g, a, sh, l);
 }
 
 cudaError_t launch_propose_poly2(bool fp32, const Geometry& g, const Arrays& a, const Launch& l, bool rotate,

@@ -273,8 +273,8 @@ hmc_status hmc_total_energy(hmc_system* sys, double* energy);
 
 /* ---- launch variants and the autotuner (no counterpart in the reference) ----
  * Every colour-pass kernel is compiled in a few launch shapes: the resident blocks per SM it
- * is built for (its register cap), the trials a warp takes (convex polyhedra: 4; hard spheres in
- * dataflow order: 3) and, for the warp-cooperative FP64 sphere pass, the candidates per stencil row a lane tests before
+ * is built for (its register cap), the trials a warp takes (convex polyhedra: 4; convex polygons: 8;
+ * hard spheres in dataflow order: 3) and, for the warp-cooperative FP64 sphere pass, the candidates per stencil row a lane tests before
  * handing the rest to its warp; for convex polygons in HMC_FP32_RECHECK, variant 1 runs the FP64
  * pass instead of the FP32 prefilter. All take the same decisions, so the trajectory is the same
  * in every variant; only the speed differs, by shape and density. hmc_autotune times `sweeps`
