@@ -77,14 +77,6 @@ __device__ __forceinline__ float fixed_dist2(const Geometry& g, const int4& a, c
     }
     return r2;
 }
-// The FP32 form of site s in space m that the system's sorted_off holds.
-template <int DIM>
-__device__ __forceinline__ float4 site32(const Geometry& g, const Arrays& A, const double* s, const uint32_t* m) {
-    if (!A.fixed_sites) return cell_offsets<DIM>(g, s, m);
-    const int4 f = fixed_site<DIM>(g, s);
-    return make_float4(__int_as_float(f.x), __int_as_float(f.y), __int_as_float(f.z), 0.f);
-}
-
 // Squared distance between a trial site t and a site s exactly as the reference computes
 // it against s's primary and ghost images: the ghost rule of generate_ghosts_in_range
 // (boundary/periodic/cuboid.rs:109-161) gives the image translations that exist, and

@@ -1059,10 +1059,24 @@ __global__ void __launch_bounds__(kCellThreads) k_cells(Geometry g, Arrays A, ui
     if (threadIdx.x == 0 && s_nonempty) atomicAdd(&A.stats->nonempty, s_nonempty);
 }
 
+// The FP32 form of body i's site s that sorted_off holds.
+template <int DIM, bool FIXED>
+__device__ __forceinline__ float4 gathered_site(const Geometry& g, const Arrays& A, uint32_t i, const double* s) {
+    if (FIXED) {
+        const int4 f = fixed_site<DIM>(g, s);
+        return make_float4(__int_as_float(f.x), __int_as_float(f.y), __int_as_float(f.z), 0.f);
+    }
+    uint32_t m[3] = {0, 0, 0};
+    unpack_m<DIM>(A.body_m[i], m);
+    return cell_offsets<DIM>(g, s, m);
+}
+
 // Per cell-order slot: gather B, S = wrap(B) (when WRITE_S), the FP32 offsets of S from its
 // space corner and the orientation, and (when WRITE_SLOTS, for the injected-move and tuner
-// kernels) the slot of each body; slot 0 also sets the sweep's rounds.
-template <int DIM, bool WRITE_S, bool WRITE_SLOTS>
+// kernels) the slot of each body; slot 0 also sets the sweep's rounds. FIXED: fixed-point sites
+// (a branch on Arrays::fixed_sites instead: 93.5 against 84.5 us for 6.4 million bodies of 256 boxes;
+// computing the space's index from the position again instead of gathering it: 101.6 us).
+template <int DIM, bool WRITE_S, bool WRITE_SLOTS, bool FIXED>
 __global__ void k_gather(Geometry g, Arrays A, uint32_t n) {
     grid_dependency_wait();  // rebuild kernels run back to back: the previous one has ended here
     allow_dependent_launch();
@@ -1080,9 +1094,7 @@ __global__ void k_gather(Geometry g, Arrays A, uint32_t n) {
     double sv[3] = {b.x, b.y, b.z};
     wrap_inv<DIM>(g.L, g.invL, sv);
     if (WRITE_S) A.sorted_s[k] = make_double4(sv[0], sv[1], sv[2], 0.0);
-    uint32_t m[3] = {0, 0, 0};
-    unpack_m<DIM>(A.body_m[i], m);
-    A.sorted_off[k] = site32<DIM>(g, A, sv, m);
+    A.sorted_off[k] = gathered_site<DIM, FIXED>(g, A, i, sv);
     if (A.sorted_q) A.sorted_q[k] = A.body_ori[i];
 }
 
@@ -1308,11 +1320,16 @@ __global__ void __launch_bounds__(kCellThreads) k_cells_batch(Batch B, Arrays A)
     if (A.progress && !has && c < B.n_cells) A.progress[c] = 0xffffffffu;
     uint32_t packed = 0, col = 0, r = 0xffffffffu;
     if (has) {
-        const uint32_t first = A.sorted_body[s];
-        packed = A.body_m[first];
-        r = __ldg(B.body_rep + first);
-        uint32_t m[3] = {0, 0, 0};
-        unpack_m<DIM>(packed, m);
+        // the replica by the slot (k_gather_batch), the multi-index from the space's own index (k_cells)
+        r = __ldg(B.body_rep + s);
+        const Replica& R = B.rep[r];
+        uint32_t m[3] = {0, 0, 0}, rem = c - R.cell_base;
+#pragma unroll
+        for (int ax = DIM - 1; ax >= 0; --ax) {
+            m[ax] = rem % R.g.shape[ax];
+            rem /= R.g.shape[ax];
+        }
+        packed = pack_m<DIM>(m);
         col = color_of<DIM>(m);
     }
     if (threadIdx.x == 0) s_nonempty = 0;
@@ -1338,22 +1355,23 @@ __global__ void __launch_bounds__(kCellThreads) k_cells_batch(Batch B, Arrays A)
     }
 }
 
-template <int DIM, bool WRITE_S>
+// A replica's bodies fill the slots that carry their numbers (its spaces follow one another in replica
+// order), so body_rep of a slot is its body's replica: read in order, where the body's own entry is
+// a gather more.
+template <int DIM, bool WRITE_S, bool FIXED>
 __global__ void k_gather_batch(Batch B, Arrays A, uint32_t n) {
     grid_dependency_wait();  // rebuild kernels run back to back: the previous one has ended here
     allow_dependent_launch();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t i = A.sorted_body[k];
-    const Geometry& g = B.rep[__ldg(B.body_rep + i)].g;  // (no batch kernel reads slot_of_body)
+    const Geometry& g = B.rep[__ldg(B.body_rep + k)].g;  // (no batch kernel reads slot_of_body)
     const double4 b = A.body_pos[i];
     A.sorted_b[k] = b;
     double sv[3] = {b.x, b.y, b.z};
     wrap_inv<DIM>(g.L, g.invL, sv);
     if (WRITE_S) A.sorted_s[k] = make_double4(sv[0], sv[1], sv[2], 0.0);
-    uint32_t m[3] = {0, 0, 0};
-    unpack_m<DIM>(A.body_m[i], m);
-    A.sorted_off[k] = site32<DIM>(g, A, sv, m);
+    A.sorted_off[k] = gathered_site<DIM, FIXED>(g, A, i, sv);
 }
 
 // Accepted moves per replica from one warp: the lanes of each replica in the warp add up.
@@ -1784,6 +1802,20 @@ cudaError_t launch_count_scan(const Arrays& a, uint32_t n_cells, cudaStream_t s,
 #endif
 constexpr uint32_t kBodyThreads = HMC_BODY_THREADS;
 
+template <int DIM>
+auto gather_kernel(bool fixed, bool write_s, bool write_slots) {
+    if (fixed)
+        return write_slots ? (write_s ? k_gather<DIM, true, true, true> : k_gather<DIM, false, true, true>)
+                           : (write_s ? k_gather<DIM, true, false, true> : k_gather<DIM, false, false, true>);
+    return write_slots ? (write_s ? k_gather<DIM, true, true, false> : k_gather<DIM, false, true, false>)
+                       : (write_s ? k_gather<DIM, true, false, false> : k_gather<DIM, false, false, false>);
+}
+template <int DIM>
+auto gather_batch_kernel(bool fixed, bool write_s) {
+    if (fixed) return write_s ? k_gather_batch<DIM, true, true> : k_gather_batch<DIM, false, true>;
+    return write_s ? k_gather_batch<DIM, true, false> : k_gather_batch<DIM, false, false>;
+}
+
 cudaError_t launch_rebuild(int dim, const Geometry& g, const Arrays& a, uint32_t n, bool write_s, cudaStream_t s,
                            bool write_slots) {
     cudaError_t e = cudaMemsetAsync(a.cell_count, 0, sizeof(uint32_t) * g.n_cells, s);
@@ -1804,13 +1836,11 @@ cudaError_t launch_rebuild(int dim, const Geometry& g, const Arrays& a, uint32_t
     const uint32_t cb = blocks_for(g.n_cells, kCellThreads), gb = blocks_for(n, kBodyThreads);
     if (dim == 2) {
         if ((e = launch_chained(k_cells<2>, cb, kCellThreads, true, s, g, a, lists)) != cudaSuccess) return e;
-        return launch_chained(write_slots ? (write_s ? k_gather<2, true, true> : k_gather<2, false, true>)
-                                          : (write_s ? k_gather<2, true, false> : k_gather<2, false, false>),
+        return launch_chained(gather_kernel<2>(a.fixed_sites != 0, write_s, write_slots),
                               gb, kBodyThreads, true, s, g, a, n);
     }
     if ((e = launch_chained(k_cells<3>, cb, kCellThreads, true, s, g, a, lists)) != cudaSuccess) return e;
-    return launch_chained(write_slots ? (write_s ? k_gather<3, true, true> : k_gather<3, false, true>)
-                                      : (write_s ? k_gather<3, true, false> : k_gather<3, false, false>),
+    return launch_chained(gather_kernel<3>(a.fixed_sites != 0, write_s, write_slots),
                           gb, kBodyThreads, true, s, g, a, n);
 }
 
@@ -1830,10 +1860,10 @@ cudaError_t launch_rebuild_batch(int dim, const Batch& b, const Arrays& a, uint3
     const uint32_t cb = blocks_for(b.n_cells, kCellThreads), gb = blocks_for(n, 256);
     if (dim == 2) {
         if ((e = launch_chained(k_cells_batch<2>, cb, kCellThreads, true, s, b, a)) != cudaSuccess) return e;
-        return launch_chained(write_s ? k_gather_batch<2, true> : k_gather_batch<2, false>, gb, 256, true, s, b, a, n);
+        return launch_chained(gather_batch_kernel<2>(a.fixed_sites != 0, write_s), gb, 256, true, s, b, a, n);
     }
     if ((e = launch_chained(k_cells_batch<3>, cb, kCellThreads, true, s, b, a)) != cudaSuccess) return e;
-    return launch_chained(write_s ? k_gather_batch<3, true> : k_gather_batch<3, false>, gb, 256, true, s, b, a, n);
+    return launch_chained(gather_batch_kernel<3>(a.fixed_sites != 0, write_s), gb, 256, true, s, b, a, n);
 }
 
 cudaError_t launch_sweep_batch(int dim, bool fp32, const Batch& b, const Arrays& a, uint32_t color, uint32_t round,
