@@ -67,6 +67,8 @@ struct hmc_context {
     std::atomic<int> refs{1};
 };
 
+constexpr uint32_t kHistogramBins = 8192;  // bins of a pair distribution at most
+
 struct hmc_system {
     hmc_context* ctx = nullptr;
     int dim = 3;
@@ -95,6 +97,9 @@ struct hmc_system {
     int32_t variant[2] = {-1, -1};  // launch variant per precision; -1: the cached choice or the default
     bool pdl = true;                // colour passes launch while the previous one finishes
     uint32_t rounds_guess = 2;      // colour sets enqueued before the sweep's count is known
+    // bins of the pair distributions, allocated on first use: an allocation per call (and the pool's
+    // release of it at the next synchronisation) took longer than the histogram
+    unsigned long long* histogram = nullptr;
     uint64_t flow_entries = 0;      // trials the draw buffers of dataflow launches hold
     uint32_t flow_cells = 0;        // spaces that progress holds
     // serial sweep grid (allocated on first use)
@@ -1777,7 +1782,7 @@ hmc_status hmc_overlap_check(hmc_system* s, uint64_t* n_overlaps) {
 // binned); the next sweep rebuilds its own checkerboard.
 static hmc_status pair_histogram(hmc_system* s, bool sdf, double sigma, double limit, double reach, uint32_t n_bins,
                                  uint64_t* counts) {
-    if (!counts || n_bins == 0 || n_bins > 8192) return fail(HMC_INVALID_ARGUMENT, "1 to 8192 bins");
+    if (!counts || n_bins == 0 || n_bins > kHistogramBins) return fail(HMC_INVALID_ARGUMENT, "1 to 8192 bins");
     if (!(limit > 0.0) || !std::isfinite(limit)) return fail(HMC_INVALID_ARGUMENT, "the histogram range must be positive");
     HMC_CUDA(cudaSetDevice(s->ctx->device));
     Geometry g = s->geom;
@@ -1799,18 +1804,17 @@ static hmc_status pair_histogram(hmc_system* s, bool sdf, double sigma, double l
     g.color_stride = (uint32_t)(cells >> s->dim);
     HMC_CUDA(cudaMemsetAsync(s->arr.stats, 0, sizeof(DeviceStats), s->stream));
     HMC_CUDA(launch_rebuild(s->dim, g, s->arr, (uint32_t)s->n, true, s->stream));
-    unsigned long long* d = nullptr;
-    HMC_CUDA(cudaMallocAsync((void**)&d, sizeof(unsigned long long) * n_bins, s->stream));
+    hmc_status st;
+    if (!s->histogram && (st = dalloc(s, &s->histogram, kHistogramBins))) return st;
+    unsigned long long* const d = s->histogram;
     cudaError_t e = launch_pair_histogram(s->dim, sdf, g, s->arr, (uint32_t)s->n, sigma, limit, (double)n_bins / limit,
                                           n_bins, d, s->stream);
     std::vector<unsigned long long> h(n_bins);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), d, sizeof(unsigned long long) * n_bins, cudaMemcpyDeviceToHost, s->stream);
-    cudaFreeAsync(d, s->stream);
     cudaError_t e2 = cudaStreamSynchronize(s->stream);
     if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return fail(HMC_CUDA_ERROR, "pair histogram: %s", cudaGetErrorString(e));
     s->prof.kernel_launches += s->n > 0 ? 7 : 2;  // the rebuild and the histogram
-    hmc_status st;
     if ((st = read_stats(s))) return st;
     if ((st = check_flags(s))) return st;
     for (uint32_t b = 0; b < n_bins; ++b) counts[b] = h[b];

@@ -403,6 +403,61 @@ __device__ __forceinline__ double4 ldg4(const double4* p) {
     return make_double4(a.x, a.y, b.x, b.y);
 }
 
+// The pairs i < j of the body in slot k of each lane (k < n) with the bodies of its stencil whose squared
+// distance dist(t, s) lies below r2_most: use(r2) for each, 32 pairs of the warp at a time. A lane finds
+// one in 13 (a 2.5 cut-off in spaces as wide) of its candidates in range, so evaluating a pair where it
+// is found runs the root and the divisions with two or three lanes of 32. list: 64 doubles of the warp's
+// own. Call with every lane of the warp.
+template <int DIM, typename DIST, typename USE>
+__device__ __forceinline__ void pairs_in_range(const Geometry& g, const Arrays& A, uint32_t n, uint32_t k,
+                                               double r2_most, double* list, DIST&& dist, USE&& use) {
+    const unsigned full = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t bi = 0, m[3] = {0, 0, 0};
+    double t[3] = {0.0, 0.0, 0.0};
+    if (k < n) {
+        bi = A.sorted_body[k];
+        const double4 s4 = ldg4(A.sorted_s + k);
+        t[0] = s4.x;
+        t[1] = s4.y;
+        t[2] = s4.z;
+        unpack_m<DIM>(A.body_m[bi], m);
+    }
+    uint32_t held = 0;
+#pragma unroll 1
+    for (int part = 0; part < 2 * kRows<DIM>; ++part) {
+        uint32_t lo = 0, len = 0;
+        float s0, s1;
+        if (k < n) stencil_part<DIM>(g, A.cell_start, m, part >> 1, (part & 1) != 0, lo, len, s0, s1);
+        const uint32_t steps = __reduce_max_sync(full, len);
+#pragma unroll 1
+        for (uint32_t j = 0; j < steps; ++j) {
+            double r2 = 0.0;
+            bool in = false;
+            if (j < len) {
+                const uint32_t bj = __ldg(A.sorted_body + lo + j);
+                const double4 s4 = ldg4(A.sorted_s + lo + j);
+                const double s[3] = {s4.x, s4.y, s4.z};
+                if (bj > bi) {
+                    r2 = dist(t, s, m);
+                    in = r2 < r2_most;
+                }
+            }
+            const unsigned b = __ballot_sync(full, in);
+            if (in) list[held + __popc(b & ((1u << lane) - 1u))] = r2;
+            held += __popc(b);
+            if (held >= 32u) {
+                __syncwarp();
+                held -= 32u;
+                use(list[held + lane]);
+                __syncwarp();
+            }
+        }
+    }
+    __syncwarp();
+    if (lane < held) use(list[lane]);
+}
+
 // Per-thread statistics of the FP32 path.
 struct PairStats {
     uint32_t checks = 0;

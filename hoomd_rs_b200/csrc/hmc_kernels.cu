@@ -1148,47 +1148,36 @@ __device__ __forceinline__ double min_image_dist2(const Geometry& g, const doubl
 #pragma unroll
     for (int a = 0; a < DIM; ++a) {
         double d = dsub(t[a], s[a]);
-        const double k = rint(ddiv(d, g.L[a]));
-        d = dsub(d, dmul(k, g.L[a]));
+        // below half a box the rounded quotient is 0 and d stays as it is, without the division
+        if (fabs(d) > 0.49 * g.L[a]) d = dsub(d, dmul(rint(ddiv(d, g.L[a])), g.L[a]));
         p = dadd(p, dmul(d, d));
     }
     return p;
 }
 
+// r2_most: at or beyond it a pair is certainly not binned. g(r) of 2^17 sites, 583 candidates each: 535 us with
+// three divisions and a root per pair where it is found, 371 us without those of pairs out of
+// range, 347 us with the pairs in range collected (pairs_in_range).
 template <int DIM, bool SDF>
 __global__ void __launch_bounds__(256) k_pair_histogram(Geometry g, Arrays A, uint32_t n, double sigma, double limit,
-                                                       double inv_width, uint32_t n_bins,
+                                                       double r2_most, double inv_width, uint32_t n_bins,
                                                        unsigned long long* counts) {
     extern __shared__ unsigned int s_hist[];
     for (uint32_t b = threadIdx.x; b < n_bins; b += blockDim.x) s_hist[b] = 0;
     __syncthreads();
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) {
-        const uint32_t bi = A.sorted_body[k];
-        const double4 s4 = A.sorted_s[k];
-        const double t[3] = {s4.x, s4.y, s4.z};
-        uint32_t m[3] = {0, 0, 0};
-        unpack_m<DIM>(A.body_m[bi], m);
-        for_each_neighbor<DIM>(g, A.cell_start, m, [&](uint32_t q, const float*) -> bool {
-            if (A.sorted_body[q] <= bi) return false;
-            const double4 o4 = A.sorted_s[q];
-            const double sv[3] = {o4.x, o4.y, o4.z};
-            const double r = dsqrt(min_image_dist2<DIM>(g, t, sv));
-            double v;
-            if (SDF) {
-                if (!(r > sigma)) return false;  // overlapping or touching pairs have no positive scale
-                v = dsub(1.0, ddiv(sigma, r));
-            } else {
-                v = r;
-            }
-            if (v < limit) {
-                const double f = floor(dmul(v, inv_width));
-                const uint32_t bin = f < (double)n_bins ? (uint32_t)f : n_bins - 1u;
-                atomicAdd(&s_hist[bin], 1u);
-            }
-            return false;
-        });
-    }
+    __shared__ double s_list[8][64];
+    const auto dist = [&](const double* t, const double* sv, const uint32_t*) { return min_image_dist2<DIM>(g, t, sv); };
+    pairs_in_range<DIM>(g, A, n, blockIdx.x * blockDim.x + threadIdx.x, r2_most, s_list[threadIdx.x >> 5], dist,
+                        [&](double r2) {
+                            const double r = dsqrt(r2);
+                            if (SDF && !(r > sigma)) return;  // overlapping or touching pairs have no positive scale
+                            const double v = SDF ? dsub(1.0, ddiv(sigma, r)) : r;
+                            if (v < limit) {
+                                const double f = floor(dmul(v, inv_width));
+                                const uint32_t bin = f < (double)n_bins ? (uint32_t)f : n_bins - 1u;
+                                atomicAdd(&s_hist[bin], 1u);
+                            }
+                        });
     __syncthreads();
     for (uint32_t b = threadIdx.x; b < n_bins; b += blockDim.x)
         if (s_hist[b]) atomicAdd(counts + b, (unsigned long long)s_hist[b]);
@@ -2069,16 +2058,19 @@ cudaError_t launch_pair_histogram(int dim, bool sdf, const Geometry& g, const Ar
     if (e != cudaSuccess || n == 0) return e;
     const size_t smem = sizeof(unsigned int) * n_bins;
     const uint32_t grid = blocks_for(n, 256);
+    // the distance at which v reaches the limit, and a margin far above the roundings of v
+    const double r_most = sdf ? (limit < 1.0 ? sigma / (1.0 - limit) : INFINITY) : limit;
+    const double r2_most = r_most * r_most * (1.0 + 1e-9);
     if (dim == 2) {
         if (sdf)
-            k_pair_histogram<2, true><<<grid, 256, smem, s>>>(g, a, n, sigma, limit, inv_width, n_bins, counts);
+            k_pair_histogram<2, true><<<grid, 256, smem, s>>>(g, a, n, sigma, limit, r2_most, inv_width, n_bins, counts);
         else
-            k_pair_histogram<2, false><<<grid, 256, smem, s>>>(g, a, n, sigma, limit, inv_width, n_bins, counts);
+            k_pair_histogram<2, false><<<grid, 256, smem, s>>>(g, a, n, sigma, limit, r2_most, inv_width, n_bins, counts);
     } else {
         if (sdf)
-            k_pair_histogram<3, true><<<grid, 256, smem, s>>>(g, a, n, sigma, limit, inv_width, n_bins, counts);
+            k_pair_histogram<3, true><<<grid, 256, smem, s>>>(g, a, n, sigma, limit, r2_most, inv_width, n_bins, counts);
         else
-            k_pair_histogram<3, false><<<grid, 256, smem, s>>>(g, a, n, sigma, limit, inv_width, n_bins, counts);
+            k_pair_histogram<3, false><<<grid, 256, smem, s>>>(g, a, n, sigma, limit, r2_most, inv_width, n_bins, counts);
     }
     return cudaGetLastError();
 }

@@ -823,31 +823,33 @@ __global__ void __launch_bounds__(32) k_tune_stream_lj(TuneJob* jobs, uint32_t n
 }
 
 // Total pair energy, pairs (i < j) in FP64 (PairwiseCutoff::total_energy,
-// pairwise_cutoff.rs:720-745); one thread per body, atomically summed.
+// pairwise_cutoff.rs:720-745); one thread per body, a warp's sums added atomically (one atomic per
+// body, all on one word, took most of the kernel). Away from the box's ends no image of a site is nearer
+// than the site (see lj_energies64), so the distance needs no ghost rule there. 2^17 sites at 0.8 with a cut-off
+// of 2.5: 402 us with both and a pair's energy where it is found, 352 us without both, 303 us with the
+// pairs in range collected (pairs_in_range).
 template <int DIM>
 __global__ void k_energy_lj(Geometry g, Arrays A, Pair P, uint32_t n, double* out) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double s_list[4][64];
     double e = 0.0;
-    if (k < n) {
-        const uint32_t bi = A.sorted_body[k];
-        const double4 s4 = A.sorted_s[k];
-        const double t[3] = {s4.x, s4.y, s4.z};
-        uint32_t m[3];
-        uint32_t c = A.body_cell[bi];
+    const auto dist = [&](const double* t, const double* s, const uint32_t* m) {
+        bool interior = true;
 #pragma unroll
-        for (int a = DIM - 1; a >= 0; --a) {
-            m[a] = c % g.shape[a];
-            c /= g.shape[a];
+        for (int a = 0; a < DIM; ++a) interior = interior && g.shape[a] >= 6 && m[a] >= 2 && m[a] + 2 <= g.shape[a];
+        if (!interior) return ref_dist2<DIM>(g, t, s);
+        double r2 = 0.0;
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) {
+            const double d = dsub(t[a], s[a]);
+            r2 = dadd(r2, dmul(d, d));
         }
-        for_each_neighbor<DIM>(g, A.cell_start, m, [&](uint32_t q, const float*) -> bool {
-            if (A.sorted_body[q] <= bi) return false;
-            const double4 o4 = A.sorted_s[q];
-            const double sv[3] = {o4.x, o4.y, o4.z};
-            e += lj_pair64(P, ref_dist2<DIM>(g, t, sv));
-            return false;
-        });
-        atomicAdd(out, e);
-    }
+        return r2;
+    };
+    // (the other soft energies test the cut-off themselves)
+    pairs_in_range<DIM>(g, A, n, blockIdx.x * blockDim.x + threadIdx.x, P.penalty ? INFINITY : P.lj_rcut2,
+                        s_list[threadIdx.x >> 5], dist, [&](double r2) { e += lj_pair64(P, r2); });
+    e = warp_sum(e);
+    if ((threadIdx.x & 31u) == 0 && e != 0.0) atomicAdd(out, e);
 }
 
 }  // namespace
