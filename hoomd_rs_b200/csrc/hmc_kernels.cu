@@ -1009,6 +1009,38 @@ __device__ __forceinline__ uint32_t append_by_color(DeviceStats* stats, bool has
 
 constexpr int kCellThreads = 512;  // 1024: 71.7 us per 2^20-sphere rebuild, 512: 70.7 us
 
+// The same order by a warp per space, for spaces of several bodies (soft potentials: 10 to 20): a lane per
+// body, which counts the lower indices of its space. A thread per space (k_cells) sorts those by
+// insertion, a chain of loads and stores as long as the square of their number: 2^17 sites, 14 a space,
+// 58 -> 4.6 us; 2^19 10 us; ten sweeps of 2^19 sites 14.0 -> 13.7 ms, of 20,011 7.76 -> 7.47 ms. With one
+// or two bodies a space (hard shapes) a warp would have little to share.
+__global__ void __launch_bounds__(256) k_order_spaces(Arrays A, uint32_t n_cells) {
+    grid_dependency_wait();  // rebuild kernels run back to back: the previous one has ended here
+    allow_dependent_launch();
+    const unsigned full = 0xffffffffu;
+    const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (c >= n_cells) return;
+    const uint32_t s = A.cell_start[c], n = A.cell_start[c + 1] - s;
+    if (n < 2u) return;
+    if (n <= 32u) {
+        const uint32_t v = lane < n ? A.sorted_body[s + lane] : 0xffffffffu;
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < n; ++j) rank += __shfl_sync(full, v, (int)j) < v ? 1u : 0u;
+        if (lane < n) A.sorted_body[s + rank] = v;
+    } else if (lane == 0) {
+        for (uint32_t k = s + 1; k < s + n; ++k) {
+            const uint32_t v = A.sorted_body[k];
+            uint32_t j = k;
+            while (j > s && A.sorted_body[j - 1] > v) {
+                A.sorted_body[j] = A.sorted_body[j - 1];
+                --j;
+            }
+            A.sorted_body[j] = v;
+        }
+    }
+}
+constexpr uint32_t kWideSpaces = 4;  // bodies per space from which a warp orders a space
+
 // Per space: order its bodies by index (the order update_checkerboard pushes them,
 // parallel_sweep.rs:194-200, which IndexedRandom::choose indexes), and (lists) list it under its
 // colour when it is not empty.
@@ -1818,17 +1850,21 @@ cudaError_t launch_rebuild(int dim, const Geometry& g, const Arrays& a, uint32_t
     // sorted colour lists for sweeps in dataflow order; beyond kScanDirectBlocks blocks the lists'
     // order of arrival is close enough to sorted (few of their blocks run at a time)
     const bool sorted = a.progress && blocks_for(g.n_cells, kScanTile) <= kScanDirectBlocks;
-    const uint32_t lists = sorted ? 0u : 1u;
+    // (with slots: the estimators and probes, which read no colour list)
+    const uint32_t lists = sorted || write_slots ? 0u : 1u;
     if ((e = launch_count_scan(a, g.n_cells, s, n > 0, sorted ? dim : 0, g)) != cudaSuccess) return e;
     if (n == 0) return cudaSuccess;
     if ((e = launch_chained(k_scatter, blocks_for(n, kBodyThreads), kBodyThreads, true, s, a, n)) != cudaSuccess) return e;
     const uint32_t cb = blocks_for(g.n_cells, kCellThreads), gb = blocks_for(n, kBodyThreads);
+    const bool wide = !lists && n / kWideSpaces >= g.n_cells;
+    if (wide && (e = launch_chained(k_order_spaces, blocks_for(g.n_cells, 8), 256, true, s, a, g.n_cells)) != cudaSuccess)
+        return e;
     if (dim == 2) {
-        if ((e = launch_chained(k_cells<2>, cb, kCellThreads, true, s, g, a, lists)) != cudaSuccess) return e;
+        if (!wide && (e = launch_chained(k_cells<2>, cb, kCellThreads, true, s, g, a, lists)) != cudaSuccess) return e;
         return launch_chained(gather_kernel<2>(a.fixed_sites != 0, write_s, write_slots),
                               gb, kBodyThreads, true, s, g, a, n);
     }
-    if ((e = launch_chained(k_cells<3>, cb, kCellThreads, true, s, g, a, lists)) != cudaSuccess) return e;
+    if (!wide && (e = launch_chained(k_cells<3>, cb, kCellThreads, true, s, g, a, lists)) != cudaSuccess) return e;
     return launch_chained(gather_kernel<3>(a.fixed_sites != 0, write_s, write_slots),
                           gb, kBodyThreads, true, s, g, a, n);
 }
@@ -1847,6 +1883,10 @@ cudaError_t launch_rebuild_batch(int dim, const Batch& b, const Arrays& a, uint3
     if (n == 0) return cudaSuccess;
     if ((e = launch_chained(k_scatter, blocks_for(n, 256), 256, true, s, a, n)) != cudaSuccess) return e;
     const uint32_t cb = blocks_for(b.n_cells, kCellThreads), gb = blocks_for(n, 256);
+    // (k_cells_batch then finds the spaces in order and lists them)
+    if (n / kWideSpaces >= b.n_cells &&
+        (e = launch_chained(k_order_spaces, blocks_for(b.n_cells, 8), 256, true, s, a, b.n_cells)) != cudaSuccess)
+        return e;
     if (dim == 2) {
         if ((e = launch_chained(k_cells_batch<2>, cb, kCellThreads, true, s, b, a)) != cudaSuccess) return e;
         return launch_chained(gather_batch_kernel<2>(a.fixed_sites != 0, write_s), gb, 256, true, s, b, a, n);

@@ -8,9 +8,9 @@
 // product, sum and fused multiply-add below follows the reference's expression order, so
 // the FP64 decision is the reference's.
 //
-// The colour pass gives a warp four trials (k_sweep_poly3_packed): each group of 8 lanes
-// computes its trial and prefilters its candidates by circumsphere, and the warp runs the full
-// tests of all four trials' remaining candidates together. Injected moves (k_eval_poly3) take
+// The sweep gives a warp four trials (k_flow_poly3): each group of 8 lanes computes its trial and
+// prefilters its candidates by circumsphere, and the warp runs the full tests of all four trials'
+// remaining candidates together. Injected moves (k_eval_poly3) take
 // one warp per move and the stencil's candidates 32 at a time, with an early exit by vote.
 // FP32 + recheck: a candidate whose FP32 centre distance clears the circumsphere by more
 // than the FP32 error bound is skipped; every other candidate runs the FP64 test, so the
