@@ -96,6 +96,8 @@ struct hmc_system {
     uint32_t slots_cap = 0;
     int32_t variant[2] = {-1, -1};  // launch variant per precision; -1: the cached choice or the default
     bool pdl = true;                // colour passes launch while the previous one finishes
+    FlowLimit flow_limit;           // of the dataflow launches (flow_limit_from_env)
+    uint32_t stall_set = 0;         // the colour set whose launch flow_limit.stall holds back
     uint32_t rounds_guess = 2;      // colour sets enqueued before the sweep's count is known
     // bins of the pair distributions, allocated on first use: an allocation per call (and the pool's
     // release of it at the next synchronisation) took longer than the histogram
@@ -401,6 +403,27 @@ hmc_status check_flags(hmc_system* s) {
     if (f & kErrIterationCap) return fail(HMC_ITERATION_CAP, "an approximate separation ran past its step bound");
     if (f & kErrFlowTimeout) return fail(HMC_TIMEOUT, "a trial waited for its neighbours past the time limit");
     return HMC_OK;
+}
+
+// The waits' time limit and what tests of it hold back. HMC_B200_FLOW_WAIT_MS=<ms>: the limit.
+// HMC_B200_FLOW_STALL=trial|copy[:<set>] (tests): FlowLimit::stall in the launch that holds colour set
+// <set> (0 where it is not given; captured batch sweeps: in every launch).
+void flow_limit_from_env(FlowLimit* limit, uint32_t* set) {
+    if (const char* ms = std::getenv("HMC_B200_FLOW_WAIT_MS")) {
+        const double v = std::atof(ms);
+        if (v > 0.0 && v < 1e6) limit->wait_ns = (unsigned long long)(v * 1e6);
+    }
+    if (const char* what = std::getenv("HMC_B200_FLOW_STALL")) {
+        if (std::strncmp(what, "trial", 5) == 0) limit->stall = kStallTrial;
+        if (std::strncmp(what, "copy", 4) == 0) limit->stall = kStallCopy;
+        const char* colon = std::strchr(what, ':');
+        *set = colon ? (uint32_t)std::atoi(colon + 1) : 0u;
+    }
+}
+FlowLimit flow_limit_of(const FlowLimit& limit, uint32_t set, uint32_t round, uint32_t round_end) {
+    FlowLimit f = limit;
+    if (round != kRoundFromDevice && (set < round || set >= round_end)) f.stall = kStallNone;
+    return f;
 }
 
 // The draw buffers of a system's dataflow launches (hmc_flow.cuh): one launch per sweep needs one
@@ -865,6 +888,7 @@ hmc_status hmc_system_create(hmc_context* ctx, const hmc_system_desc* d, const d
     // HMC_B200_SWEEP_KERNEL=direct or =coop forces one of them for both precisions.
     // HMC_B200_PDL=0 launches every colour pass after the previous one has ended.
     if (s->dim == 2) s->coop[0] = false;
+    flow_limit_from_env(&s->flow_limit, &s->stall_set);
     if (const char* pdl = std::getenv("HMC_B200_PDL")) s->pdl = std::strcmp(pdl, "0") != 0;
     if (const char* kern = std::getenv("HMC_B200_SWEEP_KERNEL")) {
         const bool direct = std::strcmp(kern, "direct") == 0, coop = std::strcmp(kern, "coop") == 0;
@@ -1094,6 +1118,7 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
         for (uint32_t r = r0; r < r1; r += std::min(sets, r1 - r)) {
             L.round = r;
             L.round_end = r + std::min(sets, r1 - r);
+            L.flow = flow_limit_of(s->flow_limit, s->stall_set, L.round, L.round_end);
             // the overlap penalty and Isotropic have no FP32 path: FP64 in both modes
             if (s->interaction == HMC_HARD_SPHERE)
                 HMC_CUDA(launch_flow_sphere(s->dim, fp32, s->geom, s->arr, s->pair, L, s->stream, sp.variant));
@@ -1221,7 +1246,8 @@ static hmc_status sweep_pipelined(hmc_system* s, const hmc_sweep_params* p, hmc_
             if (d.error_flags) {
                 *s->host_stats = d;
                 HMC_CUDA(cudaStreamSynchronize(s->stream));
-                return check_flags(s);  // the colour passes left the state untouched
+                // the passes left the state untouched, or (HMC_TIMEOUT) with part of the sweep done
+                return check_flags(s);
             }
             if (short_sets) {  // this sweep's missing colour sets, then the sweeps after it again
                 if ((st = sweep_rebuild(s, sp))) return st;
@@ -1283,7 +1309,8 @@ hmc_status hmc_sweep(hmc_system* s, const hmc_sweep_params* p, hmc_count* out) {
         // no host round trip to the sweep
         if (s->profiling) HMC_CUDA(cudaEventRecord(s->ev[3], s->stream));
         if ((st = read_stats(s))) return st;
-        if ((st = check_flags(s))) return st;  // the kernels left the state untouched
+        // the kernels left the state untouched, or (HMC_TIMEOUT) with part of the sweep done
+        if ((st = check_flags(s))) return st;
         const uint32_t rounds = s->host_stats->rounds;
         if (rounds > guess) {
             if ((st = enqueue_sets(s, p, sp, L, guess, rounds))) return st;
@@ -2380,6 +2407,8 @@ struct hmc_batch {
     int32_t variant[2] = {-1, -1};  // launch variant of the hard-sphere replica pass per precision
     uint32_t rounds_guess = 2;
     uint64_t flow_entries = 0;               // trials the draw buffers of dataflow launches hold
+    FlowLimit flow_limit;                    // as hmc_system's
+    uint32_t stall_set = 0;
     uint32_t interaction = HMC_HARD_SPHERE;  // the same for every replica
     std::vector<double> body_range;          // [R] ParallelSweep range of each replica
     // captured sweeps (hmc_batch_set_captured_sweeps): one sweep as a CUDA graph, built for a
@@ -2460,8 +2489,9 @@ uint32_t batch_sets(const hmc_batch* bt) {
 hmc_status batch_enqueue_sets(hmc_batch* bt, bool fp32, uint32_t round, bool first, uint32_t variant, cudaStream_t s) {
     if (bt->interaction == HMC_LENNARD_JONES) {
         const uint32_t sets = batch_sets(bt);
-        HMC_CUDA(launch_flow_batch_lj(bt->dim, fp32, bt->b, bt->arr, round, round == kRoundFromDevice ? sets : round + sets,
-                                      s, variant));
+        const uint32_t end = round == kRoundFromDevice ? sets : round + sets;
+        HMC_CUDA(launch_flow_batch_lj(bt->dim, fp32, bt->b, bt->arr, round, end,
+                                      flow_limit_of(bt->flow_limit, bt->stall_set, round, end), s, variant));
         return HMC_OK;
     }
     const uint32_t colors = 1u << bt->dim;
@@ -2780,6 +2810,7 @@ hmc_status hmc_batch_create(hmc_context* ctx, uint32_t n_replicas, const hmc_sys
         (st = balloc(bt, &bt->rep_counts, 2 * (size_t)n_replicas)) || (st = balloc(bt, &bt->totals, 1)))
         return destroy_fail(st);
     A.fixed_sites = lj ? 1u : 0u;
+    flow_limit_from_env(&bt->flow_limit, &bt->stall_set);
     if (lj) {  // the draws of all colour sets of equal replicas, or of one set where memory is short
         size_t free_bytes = 0, total_bytes = 0;
         cudaMemGetInfo(&free_bytes, &total_bytes);

@@ -13,7 +13,8 @@
 // Every wait ends: a trial waits only for trials with smaller numbers, each of which a running
 // warp holds or has finished (a warp takes the next number while it works on its present one, but
 // works in number order), so the smallest unfinished trial never waits. The waits carry a time
-// limit all the same (kErrFlowTimeout).
+// limit all the same (FlowLimit): a warp whose wait runs out raises kErrFlowTimeout and gives its trial
+// up undecided, the others stop at their next wait, and the state is left with part of the sweep done.
 //
 // Memory order: sites that the launch changes are read through L2 (ld.global.cg; an L1 line could
 // be stale) after an acquire of the neighbours' progress, and written before a release of the own.
@@ -97,8 +98,6 @@ __device__ __forceinline__ double4 ldcg4(const double4* p) {
     return make_double4(a.x, a.y, b.x, b.y);
 }
 
-constexpr unsigned long long kFlowWaitNs = 20ull * 1000 * 1000 * 1000;  // far beyond any trial
-
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -144,7 +143,7 @@ __device__ __forceinline__ uint32_t flow_rotated(uint32_t count, uint32_t round,
 // Poll a lane's progress word until it reaches `need` (ok: it has) in every lane of `lanes`. False:
 // the launch is given up (another warp's or this one's time limit).
 __device__ __forceinline__ bool flow_wait(const uint32_t* word, uint32_t need, unsigned lanes, bool& ok,
-                                          DeviceStats* stats) {
+                                          DeviceStats* stats, const FlowLimit& limit) {
     const unsigned full = 0xffffffffu;
     unsigned long long t0 = 0;
     for (uint32_t spins = 0;; ++spins) {
@@ -155,7 +154,7 @@ __device__ __forceinline__ bool flow_wait(const uint32_t* word, uint32_t need, u
             const unsigned long long now = global_ns();
             if (t0 == 0) t0 = now;
             bool stop = *(volatile unsigned int*)&stats->error_flags != 0u;
-            if (now - t0 > kFlowWaitNs) {
+            if (now - t0 > limit.wait_ns) {
                 atomicOr(&stats->error_flags, kErrFlowTimeout);
                 stop = true;
             }
@@ -168,7 +167,8 @@ __device__ __forceinline__ bool flow_wait(const uint32_t* word, uint32_t need, u
 // still short): returns once no lane has a pending word among those of `mask`.
 template <uint32_t N>
 __device__ __forceinline__ bool flow_wait_words(const uint32_t* progress, const uint2* words, uint32_t first,
-                                           uint32_t stride, unsigned& pending, unsigned mask, DeviceStats* stats) {
+                                           uint32_t stride, unsigned& pending, unsigned mask, DeviceStats* stats,
+                                           const FlowLimit& limit) {
     const unsigned full = 0xffffffffu;
     unsigned long long t0 = 0;
     for (uint32_t spins = 0;; ++spins) {
@@ -191,7 +191,7 @@ __device__ __forceinline__ bool flow_wait_words(const uint32_t* progress, const 
             const unsigned long long now = global_ns();
             if (t0 == 0) t0 = now;
             bool stop = *(volatile unsigned int*)&stats->error_flags != 0u;
-            if (now - t0 > kFlowWaitNs) {
+            if (now - t0 > limit.wait_ns) {
                 atomicOr(&stats->error_flags, kErrFlowTimeout);
                 stop = true;
             }
@@ -219,19 +219,32 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t b
 // Orders the generic proxy's view of global memory (sites that other SMs have written and this
 // thread has acquired) before the bulk copies that follow.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
-// Wait for the barrier's phase of the given parity (the copies are this team's own and always
-// arrive; a wait of seconds raises kErrFlowTimeout and gives up).
-__device__ __forceinline__ void mbar_wait(unsigned long long* bar, uint32_t parity, DeviceStats* stats) {
-    uint32_t done = 0;
-    for (uint32_t i = 0; i < 1u << 22; ++i) {
+// Wait for the barrier's phase of the given parity. False: the copies did not arrive within the
+// limit, and the caller gives the trial up. The barrier is then waited for once more as long, since the
+// block's shared memory must not be given back while copies into it are on their way.
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t parity, DeviceStats* stats,
+                                          const FlowLimit& limit) {
+    unsigned long long t0 = 0;
+    bool late = false;
+    for (uint32_t i = 0;; ++i) {
+        uint32_t done;
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
             : "=r"(done)
             : "r"(smem_addr(bar)), "r"(parity)
             : "memory");
-        if (done) return;
+        if (done) return !late;
+        if ((i & 15u) == 15u) {
+            const unsigned long long now = global_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > limit.wait_ns) {
+                if (late) return false;
+                atomicOr(&stats->error_flags, kErrFlowTimeout);
+                late = true;
+                t0 = now;
+            }
+        }
     }
-    atomicOr(&stats->error_flags, kErrFlowTimeout);
 }
 
 // One axis of wrap_inv, point_to_space and cell_offsets: the lanes of a warp that share a trial

@@ -239,6 +239,17 @@ __device__ __forceinline__ double soft_pair64(const Pair& P, double r2) {
     return GENERIC ? lj_pair64(P, r2) : lj_only64(P, r2);
 }
 
+// The time limit of a dataflow launch's waits (hmc_flow.cuh), and what a test of the limit holds back.
+enum : uint32_t {
+    kStallNone = 0,
+    kStallTrial = 1,  // the first trial is left out: the trials around it wait for its space in vain
+    kStallCopy = 2,   // Lennard-Jones: the staging barriers wait for bytes that nobody copies
+};
+struct FlowLimit {
+    unsigned long long wait_ns = 20ull * 1000 * 1000 * 1000;  // far beyond any trial
+    uint32_t stall = kStallNone;
+};
+
 // One sweep launch: counter, move and colour.
 struct Launch {
     uint64_t step;
@@ -256,6 +267,7 @@ struct Launch {
                                 // same sweep (this pass may start before it ends)
     uint32_t early_wait;        // 1: the previous launch is the rebuild's last kernel: launch
                                 // early but wait for it before reading anything
+    FlowLimit flow;             // dataflow launches
 };
 
 // Injected trials for the probe mode of the colour-pass kernels (hmc_eval_trials): trial i
@@ -438,7 +450,7 @@ cudaError_t launch_overlap_batch(int dim, const Batch& b, const Arrays& a, uint3
 // (round = kRoundFromDevice: round_end sets from Batch::round_dev), two kernels: the trials' random
 // draws, then the trials in dataflow order.
 cudaError_t launch_flow_batch_lj(int dim, bool fp32, const Batch& b, const Arrays& a, uint32_t round,
-                                 uint32_t round_end, cudaStream_t s, uint32_t variant = 0);
+                                 uint32_t round_end, const FlowLimit& limit, cudaStream_t s, uint32_t variant = 0);
 // coop selects the warp-cooperative pass (the per-lane pass otherwise).
 cudaError_t launch_sweep_sphere(int dim, bool fp32, const Geometry& g, const Arrays& a, const Pair& p,
                                 const Launch& l, bool coop, cudaStream_t s, uint32_t variant = 0);

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(128) k_draw_lj(Geometry g, Arrays A, Launch L,
         L.round_end += L.round;
     }
     const FlowRange f = flow_range(A.stats, L.round, L.round_end, 1u << DIM);
-    if (blockIdx.x == 0 && threadIdx.x == 0) A.stats->ticket = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.stats->ticket = L.flow.stall == kStallTrial ? 1u : 0u;
     const uint32_t stride = BATCH ? B.color_stride : g.color_stride;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += gridDim.x * blockDim.x) {
         uint32_t round, color, entry;
@@ -225,6 +225,7 @@ struct alignas(16) Team {
     double t[3], s[3];  // the trial site and (FP64) the current site
     int4 t32, s32;      // the same in fixed point (FP32)
     uint32_t n_parts, total, self, valid;
+    uint32_t lost;      // a thread's wait for staged sites ran out (mbar_wait)
     typename std::conditional<BATCH, Replica, uint32_t>::type rep;
 };
 
@@ -234,6 +235,11 @@ __device__ __forceinline__ void team_sync() {
         __syncwarp();
     else
         __syncthreads();  // a block is one team
+}
+// team_sync, and whether v holds in any thread of the team (the same answer for all).
+template <int W>
+__device__ __forceinline__ bool team_any(bool v) {
+    return W == 1 ? __any_sync(0xffffffffu, v) != 0 : __syncthreads_or(v) != 0;
 }
 
 // The stencil around space m into the team's scratch, by one warp, with the candidate number of slot k.
@@ -266,7 +272,7 @@ __device__ __forceinline__ void team_parts(const Geometry& g, const uint32_t* __
 // every copy is in flight at once, where a walk over the candidates in global memory waits for a
 // load per step or two.
 template <bool FP32, typename T>
-__device__ __forceinline__ void team_stage(const Arrays& A, uint32_t c0, uint32_t lane, T& S) {
+__device__ __forceinline__ void team_stage(const Arrays& A, uint32_t c0, uint32_t lane, T& S, const FlowLimit& limit) {
     using Site = typename T::Site;
     const Site* src;
     if constexpr (FP32)
@@ -274,7 +280,8 @@ __device__ __forceinline__ void team_stage(const Arrays& A, uint32_t c0, uint32_
     else
         src = A.sorted_s;
     const uint32_t c1 = min(c0 + kStage, S.total);
-    if (lane == 0) mbar_expect(&S.bar, (c1 - c0) * (uint32_t)sizeof(Site));
+    if (lane == 0)
+        mbar_expect(&S.bar, (c1 - c0) * (uint32_t)sizeof(Site) + (limit.stall == kStallCopy ? 16u : 0u));
     __syncwarp();
     if (lane < S.n_parts) {
         const StencilPart p = S.part[lane];
@@ -287,10 +294,11 @@ __device__ __forceinline__ void team_stage(const Arrays& A, uint32_t c0, uint32_
 // the staged candidates 32 at a time and list the pairs inside the cut-off band (1 in 6); the pair
 // energies are evaluated 32 listed pairs at a time, so that those ~60 instructions run with every
 // lane busy (two evaluations per trial instead of one per 32 candidates with five lanes). `phase`:
-// the parity of the staging barrier, the first chunk already on its way.
+// the parity of the staging barrier, the first chunk already on its way. False: a copy did not arrive
+// in time (mbar_wait) and there is no result, for the whole team.
 template <int DIM, int W, typename T>
-__device__ __forceinline__ void lj_delta32(const Geometry& g, const Arrays& A, const Pair& P, uint32_t lane, uint32_t warp, T& S,
-                                           uint32_t& phase, float& d32, float& bound) {
+__device__ __forceinline__ bool lj_delta32(const Geometry& g, const Arrays& A, const Pair& P, uint32_t lane, uint32_t warp, T& S,
+                                           uint32_t& phase, const FlowLimit& limit, float& d32, float& bound) {
     const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
     float2* list = S.list[warp].q32;
     const uint32_t total = S.total;
@@ -298,6 +306,7 @@ __device__ __forceinline__ void lj_delta32(const Geometry& g, const Arrays& A, c
     const float cut2 = P.lj_rcut2_hi32;
     float d = 0.f, err = 0.f, mag = 0.f;
     uint32_t listed = 0, rounds = 1;
+    bool lost = false;
     auto evaluate = [&](uint32_t at) {
         const float2 r2 = list[at];
         float e, x;
@@ -317,10 +326,12 @@ __device__ __forceinline__ void lj_delta32(const Geometry& g, const Arrays& A, c
 #pragma unroll 1
     for (uint32_t c0 = 0; c0 < total; c0 += kStage) {
         if (c0 > 0) {
-            team_sync<W>();  // the chunk before has been read
-            if (warp == 0) team_stage<true>(A, c0, lane, S);
+            lost = team_any<W>(W > 1 ? S.lost != 0u : lost);  // the chunk before has been read
+            if (lost) break;
+            if (warp == 0) team_stage<true>(A, c0, lane, S, limit);
         }
-        mbar_wait(&S.bar, phase, A.stats);
+        lost = !mbar_wait(&S.bar, phase, A.stats, limit);
+        if (W > 1 && lost) S.lost = 1u;
         phase ^= 1u;
         const uint32_t n = min(kStage, total - c0), self = S.self - c0;
 #pragma unroll 2
@@ -351,6 +362,9 @@ __device__ __forceinline__ void lj_delta32(const Geometry& g, const Arrays& A, c
     if (W > 1) {
         if (lane == 0) S.sum32[warp] = make_float2(d32, bound);
         team_sync<W>();
+    }
+    if (W > 1 ? S.lost != 0u : __any_sync(full, lost)) return false;
+    if (W > 1) {
         d32 = bound = 0.f;
 #pragma unroll
         for (int w = 0; w < W; ++w) {
@@ -359,6 +373,7 @@ __device__ __forceinline__ void lj_delta32(const Geometry& g, const Arrays& A, c
         }
     }
     bound += kU32 * fabsf(d32) + 1e-9f;
+    return true;
 }
 
 // FP64 energies of the trial site ta and of the current site tb against the stencil's candidates,
@@ -369,11 +384,11 @@ __device__ __forceinline__ void lj_delta32(const Geometry& g, const Arrays& A, c
 // INTERIOR: no space of the stencil is the first of an axis (which straddles the box boundary) or
 // reached across the wrap, and an axis has six spaces or more: every site of the stencil then lies
 // within 2 w <= L / 3 of the trial on each axis and any image at least 4 w away, so
-// ref_dist2 would choose the site itself.
+// ref_dist2 would choose the site itself. False: as lj_delta32.
 template <int DIM, bool GENERIC, bool INTERIOR, bool STAGED, int W, typename T>
-__device__ __forceinline__ void lj_energies64(const Geometry& g, const Arrays& A, const Pair& P, const double* ta,
+__device__ __forceinline__ bool lj_energies64(const Geometry& g, const Arrays& A, const Pair& P, const double* ta,
                                               const double* tb, uint32_t lane, uint32_t warp, T& S, uint32_t& phase,
-                                              double& ea, double& eb, double& mag) {
+                                              const FlowLimit& limit, double& ea, double& eb, double& mag) {
     const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
     const double cut2 = !GENERIC || P.penalty == 0u ? P.lj_rcut2 : (P.penalty == 1u ? P.op_rcut2 : P.uv_rcut2);
     double2* list = S.list[warp].q64;
@@ -402,10 +417,10 @@ __device__ __forceinline__ void lj_energies64(const Geometry& g, const Arrays& A
     for (uint32_t c0 = 0; c0 < total; c0 += kStage) {
         if constexpr (STAGED) {
             if (c0 > 0) {
-                team_sync<W>();  // the chunk before has been read
-                if (warp == 0) team_stage<false>(A, c0, lane, S);
+                if (team_any<W>(S.lost != 0u)) break;  // the chunk before has been read
+                if (warp == 0) team_stage<false>(A, c0, lane, S, limit);
             }
-            mbar_wait(&S.bar, phase, A.stats);
+            if (!mbar_wait(&S.bar, phase, A.stats, limit)) S.lost = 1u;
             phase ^= 1u;
         }
         const uint32_t n = min(kStage, total - c0), self = S.self - c0;
@@ -451,6 +466,9 @@ __device__ __forceinline__ void lj_energies64(const Geometry& g, const Arrays& A
             S.sum64[warp][2] = mag;
         }
         team_sync<W>();
+    }
+    if (STAGED && S.lost) return false;  // (the next wait lies behind another barrier)
+    if (W > 1) {
         ea = eb = mag = 0.0;
 #pragma unroll
         for (int w = 0; w < W; ++w) {
@@ -459,25 +477,27 @@ __device__ __forceinline__ void lj_energies64(const Geometry& g, const Arrays& A
             mag += S.sum64[w][2];
         }
     }
+    return true;
 }
 
 // The Metropolis test of the team's trial, slot k in space m (parallel_sweep.rs:267-268): FP32 sums
 // first (FP32), the FP64 sums when their bound could change the decision. The candidates of
-// the stencil in the team's scratch are on their way into its staging buffer.
+// the stencil in the team's scratch are on their way into its staging buffer. 1 accepts, 0 rejects;
+// -1: not decided, the launch is given up.
 template <int DIM, bool FP32, bool GENERIC, int W, typename T>
-__device__ __forceinline__ bool lj_decide(const Geometry& g, const Arrays& A, const Pair& P, double kt,
+__device__ __forceinline__ int lj_decide(const Geometry& g, const Arrays& A, const Pair& P, double kt,
                                           const uint32_t* m, uint32_t k, double u, float w_lo, float w_hi,
-                                          uint32_t lane, uint32_t warp, T& S, uint32_t& phase, PairStats& pst,
-                                          uint8_t& flags) {
+                                          uint32_t lane, uint32_t warp, T& S, uint32_t& phase, const FlowLimit& limit,
+                                          PairStats& pst, uint8_t& flags) {
     float d32 = 0.f;
     if constexpr (FP32) {
         float b;
-        lj_delta32<DIM, W>(g, A, P, lane, warp, S, phase, d32, b);
+        if (!lj_delta32<DIM, W>(g, A, P, lane, warp, S, phase, limit, d32, b)) return -1;
         if (lane == 0 && warp == 0) pst.checks += 2u * (S.total - 1u);
         const float lo = __fsub_rd(d32, b), hi = __fadd_ru(d32, b);
-        if (hi <= 0.f) return true;  // dU64 <= 0 for certain: accepted without a uniform
-        if (lo > 0.f && hi < w_lo) return true;
-        if (lo > 0.f && lo > w_hi) return false;
+        if (hi <= 0.f) return 1;  // dU64 <= 0 for certain: accepted without a uniform
+        if (lo > 0.f && hi < w_lo) return 1;
+        if (lo > 0.f && lo > w_hi) return 0;
         flags |= kTrialRechecked;  // (also where a sum is not finite: every comparison is false)
     }
     const double t[3] = {S.t[0], S.t[1], DIM == 3 ? S.t[2] : 0.0};
@@ -491,10 +511,14 @@ __device__ __forceinline__ bool lj_decide(const Geometry& g, const Arrays& A, co
 #pragma unroll
     for (int a = 0; a < DIM; ++a) interior = interior && g.shape[a] >= 6 && m[a] >= 2 && m[a] + 2 <= g.shape[a];
     double e_new, e_old, mag;
+    bool decided;
     if (!FP32 && interior)
-        lj_energies64<DIM, GENERIC, !FP32, !FP32, W>(g, A, P, t, si, lane, warp, S, phase, e_new, e_old, mag);
+        decided = lj_energies64<DIM, GENERIC, !FP32, !FP32, W>(g, A, P, t, si, lane, warp, S, phase, limit, e_new, e_old,
+                                                               mag);
     else
-        lj_energies64<DIM, GENERIC, false, !FP32, W>(g, A, P, t, si, lane, warp, S, phase, e_new, e_old, mag);
+        decided = lj_energies64<DIM, GENERIC, false, !FP32, W>(g, A, P, t, si, lane, warp, S, phase, limit, e_new, e_old,
+                                                               mag);
+    if (!decided) return -1;
     const double du = dsub(e_new, e_old);
     const double e0 = exp(ddiv(-du, kt));
     if (order_ambiguous(du, mag, S.total, u, kt, e0)) flags |= kTrialAmbiguous;
@@ -506,7 +530,7 @@ __device__ __forceinline__ bool lj_decide(const Geometry& g, const Arrays& A, co
         }
         if (flags & kTrialAmbiguous) pst.ambiguous++;
     }
-    return du <= 0.0 || u < e0;
+    return du <= 0.0 || u < e0 ? 1 : 0;
 }
 
 // The sweep: one team of W warps per trial in dataflow order (hmc_flow.cuh), all colour passes of
@@ -529,7 +553,10 @@ __global__ void __launch_bounds__(32 * WARPS, MINB)
     const uint32_t lane = threadIdx.x & 31u, axis = lane < DIM ? lane : 0u;
     const uint32_t warp = W == 1 ? 0u : threadIdx.x >> 5;  // within the team
     TeamT& S = s_team[W == 1 ? threadIdx.x >> 5 : 0u];
-    if (lane == 0 && warp == 0) mbar_init(&S.bar);
+    if (lane == 0 && warp == 0) {
+        mbar_init(&S.bar);
+        S.lost = 0;
+    }
     if (!INJ) {
         grid_dependency_wait();
         if (threadIdx.x == 0) {
@@ -590,11 +617,12 @@ __global__ void __launch_bounds__(32 * WARPS, MINB)
             float w_lo, w_hi;
             metropolis_bounds(u, L.kt, w_lo, w_hi);
             team_parts<DIM>(g0, A.cell_start, m, k, lane, S);
-            team_stage<FP32>(A, 0, lane, S);
-            const bool ok = lj_decide<DIM, FP32, GENERIC, W>(g0, A, P0, L.kt, m, k, u, w_lo, w_hi, lane, warp, S, phase,
-                                                             pst, flags);
+            team_stage<FP32>(A, 0, lane, S, L.flow);
+            const int decision = lj_decide<DIM, FP32, GENERIC, W>(g0, A, P0, L.kt, m, k, u, w_lo, w_hi, lane, warp, S,
+                                                                  phase, L.flow, pst, flags);
+            if (decision < 0) break;
             if (lane == 0) {
-                J.decisions[item] = ok;
+                J.decisions[item] = (uint8_t)decision;
                 J.flags[item] = flags;
             }
             __syncwarp();
@@ -642,7 +670,7 @@ __global__ void __launch_bounds__(32 * WARPS, MINB)
                 const uint32_t* word = A.progress + base + space;
                 bool ok = lane >= kNear;
                 team_parts<DIM>(g, A.cell_start + base, m, k, lane, S);
-                bool going = flow_wait(word, need, 1u << kOwn, ok, A.stats);
+                bool going = flow_wait(word, need, 1u << kOwn, ok, A.stats, L.flow);
                 __syncwarp();
                 const AxisGeometry ax = axis_geometry<DIM>(g, axis);
                 const double b = __ldcg(reinterpret_cast<const double*>(A.sorted_b + k) + axis);
@@ -661,21 +689,23 @@ __global__ void __launch_bounds__(32 * WARPS, MINB)
                     S.t[lane] = ta;
                     if (FP32) reinterpret_cast<int*>(&S.t32)[lane] = fixed_axis(ax.invL, ta);
                 }
-                if (inside && going) going = flow_wait(word, need, full, ok, A.stats);
+                if (inside && going) going = flow_wait(word, need, full, ok, A.stats, L.flow);
                 if (lane == 0) S.valid = going ? (inside ? 1u : 0u) : 2u;
                 __syncwarp();
                 if (inside && going) {
                     fence_proxy_async();
-                    team_stage<FP32>(A, 0, lane, S);
+                    team_stage<FP32>(A, 0, lane, S, L.flow);
                 }
             }
             team_sync<W>();
             const uint32_t valid = S.valid;
             if (valid == 2u) break;  // the launch is given up
             if (valid == 1u) {
-                if (lj_decide<DIM, FP32, GENERIC, W>(g, A, P, BATCH ? R->kt : L.kt, m, k, u, __uint_as_float(di.z),
-                                                     __uint_as_float(di.w), lane, warp, S, phase, pst, flags) &&
-                    warp == 0) {
+                const int decision =
+                    lj_decide<DIM, FP32, GENERIC, W>(g, A, P, BATCH ? R->kt : L.kt, m, k, u, __uint_as_float(di.z),
+                                                     __uint_as_float(di.w), lane, warp, S, phase, L.flow, pst, flags);
+                if (decision < 0) break;  // the whole team
+                if (decision > 0 && warp == 0) {
                     // update_body_properties: body = T, site = wrap(body)
                     const AxisGeometry ax = axis_geometry<DIM>(g, axis);
                     const double sv = wrap_axis(ax.L, ax.invL, ta);
@@ -927,8 +957,9 @@ cudaError_t launch_flow_lj(int dim, bool fp32, bool generic, const Geometry& g, 
 }
 
 cudaError_t launch_flow_batch_lj(int dim, bool fp32, const Batch& b, const Arrays& a, uint32_t round,
-                                 uint32_t round_end, cudaStream_t s, uint32_t variant) {
+                                 uint32_t round_end, const FlowLimit& limit, cudaStream_t s, uint32_t variant) {
     Launch l{};
+    l.flow = limit;
     l.round = round;
     l.round_end = round_end;
     return launch_flow(dim, true, lj_kernel(dim, fp32, false, true, variant, b.color_stride, (double)b.n_bodies / b.n_cells),

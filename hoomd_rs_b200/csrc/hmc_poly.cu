@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(128) k_draw_poly3(Geometry g, Arrays A, Launch
     grid_dependency_wait();
     allow_dependent_launch();
     const FlowRange f = flow_range(A.stats, L.round, L.round_end, 8);
-    if (blockIdx.x == 0 && threadIdx.x == 0) A.stats->ticket = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.stats->ticket = L.flow.stall == kStallTrial ? 1u : 0u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += gridDim.x * blockDim.x) {
         uint32_t round, color, entry;
         flow_item(f, i, round, color, entry);
@@ -882,7 +882,7 @@ __global__ void __launch_bounds__(32 * kWarps, MINB)
             if (sub + (kWarpsords - 1u) * kGroupLanes >= 27u) pending &= ~(1u << (kWarpsords - 1u));
             // the own space first: the proposal needs no other
             bool going = flow_wait_words<kWarpsords>(A.progress, S.near[grp], sub, kGroupLanes, pending,
-                                                 sub == kOwnLane ? kOwnBit : 0u, A.stats);
+                                                 sub == kOwnLane ? kOwnBit : 0u, A.stats, L.flow);
             __syncwarp();
             const AxisGeometry ax = axis_geometry<3>(g, axis);
             const uint32_t ma = axis == 0 ? m[0] : (axis == 1 ? m[1] : m[2]);
@@ -905,7 +905,8 @@ __global__ void __launch_bounds__(32 * kWarps, MINB)
             if (valid) ta = wrap_axis(ax.L, ax.invL, w1);  // the trial site T = wrap(W1)
             if (!valid) pending = 0;
             if (going)
-                going = flow_wait_words<kWarpsords>(A.progress, S.near[grp], sub, kGroupLanes, pending, ~0u, A.stats);
+                going = flow_wait_words<kWarpsords>(A.progress, S.near[grp], sub, kGroupLanes, pending, ~0u, A.stats,
+                                                    L.flow);
             if (!going) valid = false;
             if (__syncthreads_or(!going)) break;
             __syncwarp();

@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(128) k_draw_sphere(Geometry g, Arrays A, Launc
     grid_dependency_wait();
     allow_dependent_launch();
     const FlowRange f = flow_range(A.stats, L.round, L.round_end, 1u << DIM);
-    if (blockIdx.x == 0 && threadIdx.x == 0) A.stats->ticket = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.stats->ticket = L.flow.stall == kStallTrial ? 1u : 0u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < f.n; i += gridDim.x * blockDim.x) {
         uint32_t round, color, entry;
         flow_item(f, i, round, color, entry);
@@ -94,7 +94,7 @@ __device__ __forceinline__ double4 ldcg_site(const double4* p) { return ldcg4(p)
 // launch is given up.
 template <int N>
 __device__ __forceinline__ bool sphere_wait(const uint32_t* progress, const uint32_t* cell, const uint32_t* need,
-                                            unsigned pending, DeviceStats* stats) {
+                                            unsigned pending, DeviceStats* stats, const FlowLimit& limit) {
     const unsigned full = 0xffffffffu;
     unsigned long long t0 = 0;
     for (uint32_t spins = 0;; ++spins) {
@@ -110,7 +110,7 @@ __device__ __forceinline__ bool sphere_wait(const uint32_t* progress, const uint
             const unsigned long long now = global_ns();
             if (t0 == 0) t0 = now;
             bool stop = *(volatile unsigned int*)&stats->error_flags != 0u;
-            if (now - t0 > kFlowWaitNs) {
+            if (now - t0 > limit.wait_ns) {
                 atomicOr(&stats->error_flags, kErrFlowTimeout);
                 stop = true;
             }
@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(128, MINB) k_flow_sphere(Geometry g, Arrays A,
         if (INJ) {
             ta = wrap_axis(ax.L, ax.invL, x);  // T = wrap(W1), as delta_energy_one wraps the site
         } else {
-            if (round > f.r0 && !sphere_wait<1>(A.progress, &cell, &round, has ? 1u : 0u, A.stats)) break;  // given up
+            if (round > f.r0 && !sphere_wait<1>(A.progress, &cell, &round, has ? 1u : 0u, A.stats, L.flow))
+                break;  // given up
             const double b = has ? __ldcg(reinterpret_cast<const double*>(A.sorted_b + k) + axis) : 0.0;
             const double w1 = wrap_axis(ax.L, ax.invL, dadd(b, x));  // W1 = wrap(propose(..))
             const bool inside = axis_in_space(ax.origin, ax.width, ax.invW, ax.shape, ma, w1);
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(128, MINB) k_flow_sphere(Geometry g, Arrays A,
 #pragma unroll
             for (int i = 0; i < SP; ++i)
                 if (valid && R.end[i] > R.start[i] && R.need[i] > f.r0) pending |= 1u << i;
-            if (!sphere_wait<SP>(A.progress, R.cell, R.need, pending, A.stats)) break;  // given up
+            if (!sphere_wait<SP>(A.progress, R.cell, R.need, pending, A.stats, L.flow)) break;  // given up
         }
         // the first site of each space
         const Site* sites = FP32 ? reinterpret_cast<const Site*>(A.sorted_off) : reinterpret_cast<const Site*>(A.sorted_s);

@@ -56,7 +56,10 @@ typedef enum hmc_status {
     HMC_NAN_STATE = 5,            /* a non-finite coordinate was found */
     HMC_ITERATION_CAP = 6,        /* a bounded device loop reached its bound (an approximate
                                      separation, hmc_set_shape_overlap) */
-    HMC_TIMEOUT = 7,              /* reserved */
+    HMC_TIMEOUT = 7,              /* a trial of a dataflow sweep waited for its neighbours past the time
+                                     limit (20 s); part of the sweep is done and the counter has not
+                                     advanced: every body is where an accepted trial or the state
+                                     before put it, but set_state is needed to run the sweep again */
     HMC_CUDA_ERROR = 8,           /* a CUDA runtime call failed */
     HMC_OUT_OF_MEMORY = 9,
     HMC_NOT_SUPPORTED = 10,       /* combination not implemented */
