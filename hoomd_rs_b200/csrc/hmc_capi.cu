@@ -1316,6 +1316,7 @@ hmc_status hmc_sweep(hmc_system* s, const hmc_sweep_params* p, hmc_count* out) {
             if ((st = enqueue_sets(s, p, sp, L, guess, rounds))) return st;
             if (s->profiling) HMC_CUDA(cudaEventRecord(s->ev[3], s->stream));
             if ((st = read_stats(s))) return st;
+            if ((st = check_flags(s))) return st;  // (a wait that ran out in these sets)
         }
         if (s->profiling) {
             HMC_CUDA(cudaEventSynchronize(s->ev[3]));

@@ -111,3 +111,16 @@ def test_batches(ctx, captured, what, monkeypatch):
         assert all(np.array_equal(b.positions(k), fresh.positions(k)) for k in range(4))
     assert b.state(0)[1:] == fresh.state(0)[1:]
     sweep(fresh)
+
+
+@pytest.mark.parametrize("n_sweeps", [1, 3])
+@pytest.mark.parametrize("kind", ["lj", "cubes"])
+def test_a_wait_in_the_colour_sets_that_follow_the_count(ctx, kind, n_sweeps, monkeypatch):
+    """One colour set per launch: the sets beyond the host's guess are enqueued after a first look at the flags."""
+    def sweep(g):
+        g.sweep(TRANSLATE, 0.1, 1.0, FP32_RECHECK, n_sweeps=n_sweeps, increment_step=True)
+
+    monkeypatch.setenv("HMC_B200_FLOW_SETS", "1")
+    # cubes: 1,000 bodies in 6^3 spaces, five colour sets or more; the first sweep guesses two
+    g = stalled(lambda: system(ctx, kind), sweep, monkeypatch, "trial:3")
+    assert g.state()[1:] == system(ctx, kind).state()[1:]
