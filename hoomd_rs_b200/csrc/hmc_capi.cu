@@ -515,19 +515,46 @@ int32_t density_band(double bodies, double spaces) {
 }
 
 // Choices of hmc_autotune shared by every system and batch of the process, keyed by kernel
-// family, dimension, precision and density band.
+// family, dimension, precision, density band and size class.
 std::mutex g_variant_mutex;
-std::map<std::tuple<uint32_t, uint32_t, uint32_t, int32_t>, uint32_t> g_variant_cache;
+std::map<std::tuple<uint32_t, uint32_t, uint32_t, int32_t, uint32_t>, uint32_t> g_variant_cache;
 
-uint32_t cached_variant(uint32_t fam, uint32_t dim, bool fp32, int32_t band) {
+uint32_t cached_variant(uint32_t fam, uint32_t dim, bool fp32, int32_t band, uint32_t size) {
     std::lock_guard<std::mutex> lock(g_variant_mutex);
-    auto it = g_variant_cache.find(std::make_tuple(fam, dim, (uint32_t)fp32, band));
+    auto it = g_variant_cache.find(std::make_tuple(fam, dim, (uint32_t)fp32, band, size));
     return it == g_variant_cache.end() ? 0u : it->second;
 }
 
-void cache_variant(uint32_t fam, uint32_t dim, bool fp32, int32_t band, uint32_t v) {
+void cache_variant(uint32_t fam, uint32_t dim, bool fp32, int32_t band, uint32_t size, uint32_t v) {
     std::lock_guard<std::mutex> lock(g_variant_mutex);
-    g_variant_cache[std::make_tuple(fam, dim, (uint32_t)fp32, band)] = v;
+    g_variant_cache[std::make_tuple(fam, dim, (uint32_t)fp32, band, size)] = v;
+}
+
+// The size class of a recorded choice. Lennard-Jones variants are warps per trial, whose best number
+// goes with the trials of a colour: boxes for which the rule of variant 0 takes the same team share a
+// choice (at one density, 8 warps are fastest for 16,384 sites and take 2.3 times as long as 2 for
+// 262,144). The other families' variants (register caps, trials per warp) serve every size.
+uint32_t size_class(uint32_t fam, int dim, uint32_t list, uint64_t n, uint32_t cells) {
+    return fam == kFamLj || fam == kFamBatchLj ? lj_team_rule(dim, list, (double)n / std::max(1u, cells)) : 0u;
+}
+uint32_t size_class(const hmc_system* s, uint32_t fam) {
+    return size_class(fam, s->dim, s->geom.color_stride, s->n, s->geom.n_cells);
+}
+
+// Times variants 0 .. n-1 in turn: time(v, ms). Lennard-Jones: variant 0 is one of the others
+// (size_class), which is not timed again.
+template <typename Time>
+hmc_status time_variants(uint32_t fam, uint32_t size, uint32_t n, std::vector<double>& ms, Time&& time) {
+    ms.assign(n, 0.0);
+    hmc_status st = HMC_OK;
+    for (uint32_t v = 0; v < n && !st; ++v) {
+        const bool again = v > 0 && v == size && (fam == kFamLj || fam == kFamBatchLj);
+        if (again)
+            ms[v] = ms[0];
+        else
+            st = time(v, &ms[v]);
+    }
+    return st;
 }
 
 // Hard-sphere pass choices of hmc_autotune (true: the warp-cooperative pass), keyed by
@@ -552,8 +579,9 @@ void cache_pass(uint32_t dim, bool fp32, int32_t band, bool coop) {
 // The variant the next sweep of system s runs in this precision.
 uint32_t variant_of(const hmc_system* s, bool fp32) {
     if (s->variant[fp32] >= 0) return (uint32_t)s->variant[fp32];
-    return cached_variant(family_of(s, fp32), (uint32_t)s->dim, fp32,
-                          density_band((double)s->n, (double)s->geom.n_cells));
+    const uint32_t fam = family_of(s, fp32);
+    return cached_variant(fam, (uint32_t)s->dim, fp32, density_band((double)s->n, (double)s->geom.n_cells),
+                          size_class(s, fam));
 }
 
 // Kernels of one cell-list rebuild: bin, 2 scan passes (3 for grids of more than 2048 scan
@@ -1476,18 +1504,18 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
         const uint32_t fam = family_of(s, fp32);
         uint32_t n_var = 0;
         family_shapes(fam, &n_var);
-        ms.assign(n_var, 0.0);
-        for (uint32_t v = 0; v < n_var && !st; ++v) {
+        st = time_variants(fam, size_class(s, fam), n_var, ms, [&](uint32_t v, double* t) {
             s->variant[fp32] = (int32_t)v;
-            st = time_variant(s->stream, *p, sweeps, run, restore, &ms[v]);
-            if (!st && (!have || ms[v] < best_t)) {
+            return time_variant(s->stream, *p, sweeps, run, restore, t);
+        });
+        for (uint32_t v = 0; v < n_var && !st; ++v)
+            if (!have || ms[v] < best_t) {
                 have = true;
                 best_t = ms[v];
                 best = v;
                 best_fam = fam;
                 best_coop = coop;
             }
-        }
         if (!st && best_fam == fam && best_coop == coop) best_ms = ms;  // the chosen pass's times
     }
     hmc_status st2 = restore();
@@ -1507,7 +1535,7 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
         cache_pass((uint32_t)s->dim, fp32, band, best_coop);
     }
     s->variant[fp32] = (int32_t)best;
-    cache_variant(best_fam, (uint32_t)s->dim, fp32, band, best);
+    cache_variant(best_fam, (uint32_t)s->dim, fp32, band, size_class(s, best_fam), best);
     if (chosen) describe_variant(best_fam, best, chosen);
     if (ms_per_sweep) std::memcpy(ms_per_sweep, best_ms.data(), sizeof(double) * best_ms.size());
     return HMC_OK;
@@ -2866,9 +2894,13 @@ static uint32_t batch_family(const hmc_batch* bt) {
 
 // The variant the batch's next sweep runs: its own choice, else the cached one for its family,
 // dimension, precision and density band (all replicas' bodies over all their spaces), else 0.
+static uint32_t size_class(const hmc_batch* bt) {
+    return size_class(batch_family(bt), bt->dim, bt->b.color_stride, bt->n, bt->cells);
+}
 static uint32_t batch_variant_of(const hmc_batch* bt, bool fp32) {
     if (bt->variant[fp32] >= 0) return (uint32_t)bt->variant[fp32];
-    return cached_variant(batch_family(bt), (uint32_t)bt->dim, fp32, density_band((double)bt->n, (double)bt->cells));
+    return cached_variant(batch_family(bt), (uint32_t)bt->dim, fp32, density_band((double)bt->n, (double)bt->cells),
+                          size_class(bt));
 }
 
 hmc_status hmc_batch_sweep(hmc_batch* bt, const hmc_sweep_params* params, hmc_count* counts, hmc_count* total) {
@@ -3007,13 +3039,15 @@ hmc_status hmc_batch_autotune(hmc_batch* bt, const hmc_sweep_params* params, uin
         return hmc_batch_sweep(bt, ps.data(), nullptr, nullptr);
     };
     hmc_status st = e == cudaSuccess ? HMC_OK : fail(HMC_CUDA_ERROR, "batch autotune: %s", cudaGetErrorString(e));
-    std::vector<double> ms(n_var, 0.0);
+    std::vector<double> ms;
+    if (!st)
+        st = time_variants(fam, size_class(bt), n_var, ms, [&](uint32_t v, double* t) {
+            bt->variant[fp32] = (int32_t)v;
+            return time_variant(bt->stream, params[0], sweeps, run, restore, t);
+        });
     uint32_t best = 0;
-    for (uint32_t v = 0; v < n_var && !st; ++v) {
-        bt->variant[fp32] = (int32_t)v;
-        st = time_variant(bt->stream, params[0], sweeps, run, restore, &ms[v]);
-        if (!st && ms[v] < ms[best]) best = v;
-    }
+    for (uint32_t v = 1; v < n_var && !st; ++v)
+        if (ms[v] < ms[best]) best = v;
     hmc_status st2 = restore();
     if (bp) cudaFreeAsync(bp, bt->stream);
     cudaStreamSynchronize(bt->stream);
@@ -3022,7 +3056,7 @@ hmc_status hmc_batch_autotune(hmc_batch* bt, const hmc_sweep_params* params, uin
         return st ? st : st2;
     }
     bt->variant[fp32] = (int32_t)best;
-    cache_variant(fam, (uint32_t)bt->dim, fp32, density_band((double)bt->n, (double)bt->cells), best);
+    cache_variant(fam, (uint32_t)bt->dim, fp32, density_band((double)bt->n, (double)bt->cells), size_class(bt), best);
     if (chosen) describe_variant(fam, best, chosen);
     if (ms_per_sweep) std::memcpy(ms_per_sweep, ms.data(), sizeof(double) * n_var);
     return HMC_OK;

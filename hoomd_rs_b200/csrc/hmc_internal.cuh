@@ -463,6 +463,9 @@ cudaError_t launch_flow_trials_sphere(int dim, bool fp32, const Geometry& g, con
 cudaError_t launch_overlap_sphere(int dim, const Geometry& g, const Arrays& a, const Pair& p, uint32_t n,
                                   cudaStream_t s);
 // generic: the system's energy is not Shifted Lennard-Jones (the overlap penalty, Isotropic).
+// The variant (team size) that variant 0 of a box or batch runs: colour lists of `list` spaces, per_space
+// bodies a space.
+uint32_t lj_team_rule(int dim, uint32_t list, double per_space);
 // The colour sets [l.round, l.round_end), two kernels as in launch_flow_batch_lj.
 cudaError_t launch_flow_lj(int dim, bool fp32, bool generic, const Geometry& g, const Arrays& a, const Pair& p,
                            const Launch& l, cudaStream_t s, uint32_t variant = 0);

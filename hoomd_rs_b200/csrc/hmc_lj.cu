@@ -917,7 +917,7 @@ LjVariant lj_kernel(uint32_t v) {
 }
 LjVariant lj_kernel(int dim, bool fp32, bool generic, bool batch, uint32_t variant, uint32_t list, double per_space) {
     static_assert(n_shapes(kLjShapes) == 5 && n_shapes(kBatchLjShapes) == 5, "the rule and four kernels");
-    const uint32_t v = variant == 0 || variant > 4 ? lj_team_variant(list, per_space * (dim == 3 ? 27 : 9)) : variant;
+    const uint32_t v = variant == 0 || variant > 4 ? lj_team_rule(dim, list, per_space) : variant;
     if (batch) {
         if (dim == 2) return fp32 ? lj_kernel<2, true, false, true>(v) : lj_kernel<2, false, false, true>(v);
         return fp32 ? lj_kernel<3, true, false, true>(v) : lj_kernel<3, false, false, true>(v);
@@ -948,6 +948,10 @@ cudaError_t launch_flow(int dim, bool batch, const LjVariant& v, const Geometry&
     return cudaLaunchKernelEx(&pl.cfg, v.kernel, g, a, p, l, b, Injected{});
 }
 }  // namespace
+
+uint32_t lj_team_rule(int dim, uint32_t list, double per_space) {
+    return lj_team_variant(list, per_space * (dim == 3 ? 27 : 9));
+}
 
 cudaError_t launch_flow_lj(int dim, bool fp32, bool generic, const Geometry& g, const Arrays& a, const Pair& p,
                            const Launch& l, cudaStream_t s, uint32_t variant) {

@@ -284,7 +284,8 @@ hmc_status hmc_total_energy(hmc_system* sys, double* energy);
  * sweeps of the system in every variant of its pass (precision and move from params), each from
  * the same saved state, keeps the fastest for this system and records it for every system and
  * batch of the process with the same pass, dimension, precision and density band (bodies per
- * checkerboard space, in quarter octaves); the state and counter are restored afterwards. A
+ * checkerboard space, in quarter octaves), Lennard-Jones and Isotropic also of the same size class (boxes
+ * whose variant 0 takes the same team); the state and counter are restored afterwards. A
  * system without its own choice uses the recorded one for its band, else variant 0. */
 typedef struct hmc_launch_variant {
     uint32_t index;            /* in the variant table of the system's pass for this precision */
@@ -292,8 +293,7 @@ typedef struct hmc_launch_variant {
     uint32_t blocks_per_sm;    /* resident blocks per SM the kernel is compiled for */
     uint32_t trials_per_warp;  /* trials one warp takes at once (1: a lane or a warp per trial) */
     uint32_t own_steps;        /* warp-cooperative sphere pass: candidates per row a lane tests;
-                                  Lennard-Jones / Isotropic passes: 2 = two candidates per lane
-                                  and step */
+                                  Lennard-Jones / Isotropic: warps per trial, 0 = by the box's size */
 } hmc_launch_variant;
 /* index UINT32_MAX: the variant the next hmc_sweep in this precision runs. */
 hmc_status hmc_get_launch_variant(hmc_system* sys, uint32_t precision, uint32_t index, hmc_launch_variant* out);

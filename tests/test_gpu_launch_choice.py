@@ -1,0 +1,48 @@
+"""Where a launch choice applies: recorded ones to boxes of their size class, a system's own to its pass."""
+import numpy as np
+import pytest
+
+from hoomd_rs_b200 import (FP32_RECHECK, FP64, TRANSLATE, Batch, Context, Isotropic, LennardJones, Microstate,
+                           PairwiseCutoff, Periodic, Shifted, lattice)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    return Context(0)
+
+
+def lj(ctx, n, rho, dim=3, r_cut=2.5):
+    pos, L = lattice.lennard_jones_box(n, rho, dim, 7)
+    h = PairwiseCutoff(Isotropic(Shifted(LennardJones(1.0, 1.0), r_cut), r_cut))
+    return Microstate(ctx, Periodic(r_cut, [L] * dim), pos, h, seed=7)
+
+
+# (4,096 sites run 8 warps a trial, 200,000 two)
+@pytest.mark.parametrize("precision", [FP64, FP32_RECHECK])
+@pytest.mark.parametrize("rho", [0.72, 0.77, 0.84, 0.93, 1.02, 1.12])
+def test_a_recorded_team_stays_in_its_size_class(ctx, rho, precision):
+    small = lj(ctx, 4096, rho)
+    chosen, ms = small.autotune(TRANSLATE, 0.1, 1.0, precision, sweeps=2)
+    assert len(ms) == chosen["count"] == 5 and ms[chosen["index"]] == ms.min()
+    assert ms[0] in ms[1:]  # variant 0 is one of the teams, and not timed twice
+    assert lj(ctx, 4096, rho).launch_variant(precision)["index"] == chosen["index"]
+    assert lj(ctx, 200000, rho).launch_variant(precision)["index"] == 0
+    assert lj(ctx, 200000, rho, r_cut=2.7).launch_variant(precision)["index"] == 0
+
+
+@pytest.mark.parametrize("rho", [0.72, 0.84, 1.02])
+def test_a_recorded_batch_team_stays_in_its_size_class(ctx, rho):
+    def batch(n):
+        h = PairwiseCutoff(Isotropic(Shifted(LennardJones(1.0, 1.0), 2.5), 2.5))
+        pos, L = lattice.lennard_jones_box(n, rho, 3, 7)
+        return Batch(ctx, [{"boundary": Periodic(2.5, [L] * 3), "positions": pos, "seed": 7 + k, "hamiltonian": h}
+                           for k in range(2)])
+
+    small = batch(4096)
+    chosen, ms = small.autotune(0.1, FP32_RECHECK, sweeps=2, temperatures=np.ones(2))
+    assert ms[0] in ms[1:]
+    large = batch(100000)
+    chosen_large, ms = large.autotune(0.1, FP32_RECHECK, sweeps=1, temperatures=np.ones(2))
+    assert ms[0] in ms[1:]
