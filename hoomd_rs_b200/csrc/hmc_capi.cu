@@ -95,6 +95,7 @@ struct hmc_system {
     DeviceStats* host_slots = nullptr;  // pinned: per-sweep statistics of a pipelined call
     uint32_t slots_cap = 0;
     int32_t variant[2] = {-1, -1};  // launch variant per precision; -1: the cached choice or the default
+    uint32_t variant_family[2] = {0, 0};  // whose table variant indexes; not used while another family runs
     bool pdl = true;                // colour passes launch while the previous one finishes
     FlowLimit flow_limit;           // of the dataflow launches (flow_limit_from_env)
     uint32_t stall_set = 0;         // the colour set whose launch flow_limit.stall holds back
@@ -578,8 +579,9 @@ void cache_pass(uint32_t dim, bool fp32, int32_t band, bool coop) {
 
 // The variant the next sweep of system s runs in this precision.
 uint32_t variant_of(const hmc_system* s, bool fp32) {
-    if (s->variant[fp32] >= 0) return (uint32_t)s->variant[fp32];
     const uint32_t fam = family_of(s, fp32);
+    // (set_cooperative_pass, or a number of bodies that crosses sphere_flow's line, changes the family)
+    if (s->variant[fp32] >= 0 && s->variant_family[fp32] == fam) return (uint32_t)s->variant[fp32];
     return cached_variant(fam, (uint32_t)s->dim, fp32, density_band((double)s->n, (double)s->geom.n_cells),
                           size_class(s, fam));
 }
@@ -1415,6 +1417,7 @@ hmc_status hmc_set_launch_variant(hmc_system* s, uint32_t precision, uint32_t in
     family_shapes(family_of(s, fp32), &n);
     if (index != UINT32_MAX && index >= n) return fail(HMC_INVALID_ARGUMENT, "variant %u of %u", index, n);
     s->variant[fp32] = index == UINT32_MAX ? -1 : (int32_t)index;
+    s->variant_family[fp32] = family_of(s, fp32);
     return HMC_OK;
 }
 
@@ -1471,6 +1474,7 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
     const uint64_t step0 = s->step;
     const uint32_t substep0 = s->substep, guess0 = s->rounds_guess;
     const int32_t own0 = s->variant[fp32];
+    const uint32_t own_family0 = s->variant_family[fp32];
     double4 *bp = nullptr, *bq = nullptr;
     cudaError_t e = cudaMallocAsync((void**)&bp, sizeof(double4) * (n ? n : 1), s->stream);
     if (e == cudaSuccess && n)
@@ -1506,6 +1510,7 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
         family_shapes(fam, &n_var);
         st = time_variants(fam, size_class(s, fam), n_var, ms, [&](uint32_t v, double* t) {
             s->variant[fp32] = (int32_t)v;
+            s->variant_family[fp32] = fam;
             return time_variant(s->stream, *p, sweeps, run, restore, t);
         });
         for (uint32_t v = 0; v < n_var && !st; ++v)
@@ -1524,6 +1529,7 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
     cudaStreamSynchronize(s->stream);
     if (st || st2) {
         s->variant[fp32] = own0;
+        s->variant_family[fp32] = own_family0;
         s->coop[fp32] = coop_own0;
         s->coop_set[fp32] = coop_set0;
         return st ? st : st2;
@@ -1535,6 +1541,7 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
         cache_pass((uint32_t)s->dim, fp32, band, best_coop);
     }
     s->variant[fp32] = (int32_t)best;
+    s->variant_family[fp32] = best_fam;
     cache_variant(best_fam, (uint32_t)s->dim, fp32, band, size_class(s, best_fam), best);
     if (chosen) describe_variant(best_fam, best, chosen);
     if (ms_per_sweep) std::memcpy(ms_per_sweep, best_ms.data(), sizeof(double) * best_ms.size());

@@ -2,8 +2,8 @@
 import numpy as np
 import pytest
 
-from hoomd_rs_b200 import (FP32_RECHECK, FP64, TRANSLATE, Batch, Context, Isotropic, LennardJones, Microstate,
-                           PairwiseCutoff, Periodic, Shifted, lattice)
+from hoomd_rs_b200 import (FP32_RECHECK, FP64, TRANSLATE, Batch, Context, GrandCanonical, HardSphere, IsothermalIsofugacity,
+                           Isotropic, LennardJones, Microstate, PairwiseCutoff, Periodic, Shifted, lattice)
 
 pytestmark = pytest.mark.gpu
 
@@ -46,3 +46,40 @@ def test_a_recorded_batch_team_stays_in_its_size_class(ctx, rho):
     large = batch(100000)
     chosen_large, ms = large.autotune(0.1, FP32_RECHECK, sweeps=1, temperatures=np.ones(2))
     assert ms[0] in ms[1:]
+
+
+def spheres(ctx, n, precision, dim=3, phi=0.45):
+    pos, L = lattice.hard_sphere_box(n, phi, dim, 7)
+    return Microstate(ctx, Periodic(1.0, [L] * dim), pos, PairwiseCutoff(HardSphere(1.0)), seed=7)
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_RECHECK])
+def test_an_own_variant_stays_with_its_pass(ctx, precision):
+    """A small box's variant is one of the dataflow sweep; the colour passes' tables mean other shapes by it."""
+    g = spheres(ctx, 4096, precision)
+    flow = g.launch_variant(precision)
+    assert flow["trials_per_warp"] == 3
+    g.set_launch_variant(precision, 1)
+    assert g.launch_variant(precision) == dict(g.launch_variant(precision, 1))
+    for coop in (False, True):
+        g.set_cooperative_pass(precision, coop)
+        v = g.launch_variant(precision)
+        assert v["trials_per_warp"] == 1 and v["index"] == 0
+        g.set_launch_variant(precision, 2)
+        assert g.launch_variant(precision)["index"] == 2
+        g.set_cooperative_pass(precision, coop)  # the same pass again keeps it
+        assert g.launch_variant(precision)["index"] == 2
+    g.set_cooperative_pass(precision, False)
+    assert g.launch_variant(precision)["index"] == 0
+
+
+def test_an_own_variant_stays_with_its_pass_across_the_line(ctx):
+    """Removing bodies takes a box of more than 114,695 spheres to the dataflow sweeps."""
+    g = spheres(ctx, 114700, FP32_RECHECK)
+    assert g.launch_variant(FP32_RECHECK)["trials_per_warp"] == 1
+    g.set_launch_variant(FP32_RECHECK, 1)
+    GrandCanonical().apply(g, None, IsothermalIsofugacity(1.0, 0.0), 64)
+    assert len(g.positions()) < 114696
+    v = g.launch_variant(FP32_RECHECK)
+    assert v["trials_per_warp"] == 3 and v["index"] == 0
+    g.sweep(TRANSLATE, 0.1, 1.0, FP32_RECHECK, n_sweeps=1, increment_step=True)
