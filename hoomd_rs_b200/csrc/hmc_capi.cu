@@ -586,6 +586,18 @@ uint32_t variant_of(const hmc_system* s, bool fp32) {
                           size_class(s, fam));
 }
 
+// The indices that set and get take: the family's, and those of the colour pass that such a system ran
+// before it had dataflow sweeps (polyhedra, few spheres) or another default (FP64 disks), so that a
+// program that keeps an index goes on; beyond the family's table they stand for variant 0.
+uint32_t accepted_variants(const hmc_system* s, bool fp32) {
+    uint32_t n = 0;
+    family_shapes(family_of(s, fp32), &n);
+    if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON) return std::max(n, 3u);
+    if (s->interaction == HMC_HARD_SPHERE && !s->coop_set[fp32])
+        return std::max(n, fp32 ? n_shapes(kSphereDirectShapes) : n_shapes(kSphereCoopShapes));
+    return n;
+}
+
 // Kernels of one cell-list rebuild: bin, 2 scan passes (3 for grids of more than 2048 scan
 // blocks), scatter, space sort, gather.
 uint32_t rebuild_kernels(const hmc_system* s) {
@@ -1382,9 +1394,7 @@ hmc_status hmc_get_launch_variant(hmc_system* s, uint32_t precision, uint32_t in
     if (!s || !out) return fail(HMC_INVALID_ARGUMENT, "NULL argument");
     if (precision > HMC_FP32_RECHECK) return fail(HMC_INVALID_ARGUMENT, "precision");
     const bool fp32 = precision == HMC_FP32_RECHECK;
-    const uint32_t fam = family_of(s, fp32);
-    uint32_t n = 0;
-    family_shapes(fam, &n);
+    const uint32_t fam = family_of(s, fp32), n = accepted_variants(s, fp32);
     if (index != UINT32_MAX && index >= n) return fail(HMC_INVALID_ARGUMENT, "variant %u of %u", index, n);
     describe_variant(fam, index == UINT32_MAX ? variant_of(s, fp32) : index, out);
     return HMC_OK;
@@ -1413,10 +1423,11 @@ hmc_status hmc_set_launch_variant(hmc_system* s, uint32_t precision, uint32_t in
     if (!s) return fail(HMC_INVALID_ARGUMENT, "NULL argument");
     if (precision > HMC_FP32_RECHECK) return fail(HMC_INVALID_ARGUMENT, "precision");
     const bool fp32 = precision == HMC_FP32_RECHECK;
-    uint32_t n = 0;
-    family_shapes(family_of(s, fp32), &n);
+    uint32_t count = 0;
+    family_shapes(family_of(s, fp32), &count);
+    const uint32_t n = accepted_variants(s, fp32);
     if (index != UINT32_MAX && index >= n) return fail(HMC_INVALID_ARGUMENT, "variant %u of %u", index, n);
-    s->variant[fp32] = index == UINT32_MAX ? -1 : (int32_t)index;
+    s->variant[fp32] = index == UINT32_MAX ? -1 : (int32_t)(index < count ? index : 0u);
     s->variant_family[fp32] = family_of(s, fp32);
     return HMC_OK;
 }

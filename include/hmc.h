@@ -297,7 +297,10 @@ typedef struct hmc_launch_variant {
 } hmc_launch_variant;
 /* index UINT32_MAX: the variant the next hmc_sweep in this precision runs. */
 hmc_status hmc_get_launch_variant(hmc_system* sys, uint32_t precision, uint32_t index, hmc_launch_variant* out);
-/* index UINT32_MAX: drop the system's own choice (the recorded one for its band, else 0). */
+/* index UINT32_MAX: drop the system's own choice (the recorded one for its band, else 0). Indices up to 2
+ * (convex polyhedra; hard spheres in FP32) or 4 (hard spheres in FP64, no pass chosen) are taken where
+ * the table is shorter, and stand for variant 0 there. A choice holds while the system runs the pass that
+ * it was made for. */
 hmc_status hmc_set_launch_variant(hmc_system* sys, uint32_t precision, uint32_t index);
 /* Hard spheres and disks: which colour pass a precision runs, one lane per trial (cooperative = 0,
  * the FP32 default and the default of disks) or the warp-cooperative pass (1, the FP64 default in

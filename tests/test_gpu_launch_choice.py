@@ -2,8 +2,9 @@
 import numpy as np
 import pytest
 
-from hoomd_rs_b200 import (FP32_RECHECK, FP64, TRANSLATE, Batch, Context, GrandCanonical, HardSphere, IsothermalIsofugacity,
-                           Isotropic, LennardJones, Microstate, PairwiseCutoff, Periodic, Shifted, lattice)
+from hoomd_rs_b200 import (FP32_RECHECK, FP64, TRANSLATE, Batch, Context, ConvexPolyhedron, GrandCanonical, HardShape,
+                           HardSphere, HmcError, IsothermalIsofugacity, Isotropic, LennardJones, Microstate,
+                           PairwiseCutoff, Periodic, Shifted, lattice)
 
 pytestmark = pytest.mark.gpu
 
@@ -83,3 +84,40 @@ def test_an_own_variant_stays_with_its_pass_across_the_line(ctx):
     v = g.launch_variant(FP32_RECHECK)
     assert v["trials_per_warp"] == 3 and v["index"] == 0
     g.sweep(TRANSLATE, 0.1, 1.0, FP32_RECHECK, n_sweeps=1, increment_step=True)
+
+
+def cubes(ctx):
+    verts = np.array([[x, y, z] for x in (-0.5, 0.5) for y in (-0.5, 0.5) for z in (-0.5, 0.5)])
+    return Microstate(ctx, Periodic(3.0 ** 0.5, [12.5] * 3), lattice.cubic_lattice(1000, 12.5, 3, 7),
+                      PairwiseCutoff(HardShape(ConvexPolyhedron.with_vertices(verts))), seed=7)
+
+
+# The indices of the colour passes that these boxes ran before they had dataflow sweeps, or another
+# default pass: 3 shapes of polyhedra and of a lane per sphere, 5 of a warp per sphere.
+@pytest.mark.parametrize("make,precision,accepted", [
+    (cubes, FP32_RECHECK, 3), (cubes, FP64, 3),
+    (lambda ctx: spheres(ctx, 4096, FP32_RECHECK), FP32_RECHECK, 3), (lambda ctx: spheres(ctx, 4096, FP64), FP64, 5),
+    (lambda ctx: spheres(ctx, 100000, FP64, 2, 0.6), FP64, 5)])
+def test_a_kept_index_is_accepted(ctx, make, precision, accepted):
+    """An index beyond the table of the pass that runs now stands for variant 0."""
+    g = make(ctx)
+    count = g.launch_variant(precision)["count"]
+    for index in range(accepted):
+        g.set_launch_variant(precision, index)
+        want = index if index < count else 0
+        assert g.launch_variant(precision)["index"] == g.launch_variant(precision, index)["index"] == want
+    g.sweep(TRANSLATE, 0.1, 1.0, precision, n_sweeps=1, increment_step=True)
+    for refused in (accepted, 1000):
+        with pytest.raises(HmcError):
+            g.set_launch_variant(precision, refused)
+        with pytest.raises(HmcError):
+            g.launch_variant(precision, refused)
+
+
+@pytest.mark.parametrize("precision,coop,accepted", [(FP64, False, 3), (FP64, True, 5), (FP32_RECHECK, False, 3)])
+def test_a_pass_that_was_chosen_has_its_own_indices(ctx, precision, coop, accepted):
+    g = spheres(ctx, 4096, precision)
+    g.set_cooperative_pass(precision, coop)
+    g.set_launch_variant(precision, accepted - 1)
+    with pytest.raises(HmcError):
+        g.set_launch_variant(precision, accepted)
