@@ -209,11 +209,15 @@ __global__ void __launch_bounds__(128) k_draw_lj(Geometry g, Arrays A, Launch L,
 struct StencilPart {
     uint32_t base, end;
 };
-constexpr uint32_t kStage = 384;  // candidates staged at a time (a stencil of 2^19 sites at 0.8 holds ~345)
-template <bool FP32, bool BATCH, int W>
+constexpr int kStage = 384;  // candidates staged at a time (a stencil of 2^19 sites at 0.8 holds ~345)
+constexpr int kDirect = 0;   // of trials with few candidates: their lanes load the sites (lj_staging)
+template <bool FP32, bool BATCH, int W, int STAGE>
 struct alignas(16) Team {
+    // candidates between two staging steps; direct loads need none
+    static constexpr bool staged = STAGE > 0;
+    static constexpr uint32_t stage = staged ? STAGE : 0x80000000u;
     using Site = typename std::conditional<FP32, int4, double4>::type;
-    Site site[kStage];
+    Site site[staged ? STAGE : 1];
     union {
         float2 q32[64];
         double2 q64[64];
@@ -268,7 +272,7 @@ __device__ __forceinline__ void team_parts(const Geometry& g, const uint32_t* __
     __syncwarp();
 }
 
-// Candidates [c0, c0 + kStage) into the team's staging buffer by one warp, one bulk copy per part:
+// Candidates [c0, c0 + T::stage) into the team's staging buffer by one warp, one bulk copy per part:
 // every copy is in flight at once, where a walk over the candidates in global memory waits for a
 // load per step or two.
 template <bool FP32, typename T>
@@ -279,7 +283,7 @@ __device__ __forceinline__ void team_stage(const Arrays& A, uint32_t c0, uint32_
         src = reinterpret_cast<const Site*>(A.sorted_off);
     else
         src = A.sorted_s;
-    const uint32_t c1 = min(c0 + kStage, S.total);
+    const uint32_t c1 = min(c0 + T::stage, S.total);
     if (lane == 0)
         mbar_expect(&S.bar, (c1 - c0) * (uint32_t)sizeof(Site) + (limit.stall == kStallCopy ? 16u : 0u));
     __syncwarp();
@@ -305,7 +309,7 @@ __device__ __forceinline__ bool lj_delta32(const Geometry& g, const Arrays& A, c
     const int4 t32 = S.t32, s32 = S.s32;
     const float cut2 = P.lj_rcut2_hi32;
     float d = 0.f, err = 0.f, mag = 0.f;
-    uint32_t listed = 0, rounds = 1;
+    uint32_t listed = 0, rounds = 1, part = 0;
     bool lost = false;
     auto evaluate = [&](uint32_t at) {
         const float2 r2 = list[at];
@@ -324,20 +328,28 @@ __device__ __forceinline__ bool lj_delta32(const Geometry& g, const Arrays& A, c
         }
     };
 #pragma unroll 1
-    for (uint32_t c0 = 0; c0 < total; c0 += kStage) {
+    for (uint32_t c0 = 0; c0 < total; c0 += T::stage) {
         if (c0 > 0) {
             lost = team_any<W>(W > 1 ? S.lost != 0u : lost);  // the chunk before has been read
             if (lost) break;
             if (warp == 0) team_stage<true>(A, c0, lane, S, limit);
         }
-        lost = !mbar_wait(&S.bar, phase, A.stats, limit);
-        if (W > 1 && lost) S.lost = 1u;
-        phase ^= 1u;
-        const uint32_t n = min(kStage, total - c0), self = S.self - c0;
+        if constexpr (T::staged) {
+            lost = !mbar_wait(&S.bar, phase, A.stats, limit);
+            if (W > 1 && lost) S.lost = 1u;
+            phase ^= 1u;
+        }
+        const uint32_t n = min(T::stage, total - c0), self = S.self - c0;
 #pragma unroll 2
         for (uint32_t j0 = 32u * warp; j0 < n; j0 += 32u * W) {
             const uint32_t j = j0 + lane;
-            const int4 o = S.site[j];  // (j < kStage; stale beyond n)
+            int4 o;
+            if constexpr (T::staged) {
+                o = S.site[j];  // (j < T::stage; stale beyond n)
+            } else {
+                while (j < n && j >= S.part[part].end) ++part;
+                o = j < n ? __ldcg(reinterpret_cast<const int4*>(A.sorted_off) + (S.part[part].base + j)) : t32;
+            }
             const float rn = fixed_dist2<DIM>(g, t32, o), ro = fixed_dist2<DIM>(g, s32, o);
             const bool need = fminf(rn, ro) < cut2 && j < n && j != self;
             const unsigned b = __ballot_sync(full, need);
@@ -414,8 +426,8 @@ __device__ __forceinline__ bool lj_energies64(const Geometry& g, const Arrays& A
         return r2;
     };
 #pragma unroll 1
-    for (uint32_t c0 = 0; c0 < total; c0 += kStage) {
-        if constexpr (STAGED) {
+    for (uint32_t c0 = 0; c0 < total; c0 += T::stage) {
+        if constexpr (STAGED && T::staged) {
             if (c0 > 0) {
                 if (team_any<W>(S.lost != 0u)) break;  // the chunk before has been read
                 if (warp == 0) team_stage<false>(A, c0, lane, S, limit);
@@ -423,21 +435,21 @@ __device__ __forceinline__ bool lj_energies64(const Geometry& g, const Arrays& A
             if (!mbar_wait(&S.bar, phase, A.stats, limit)) S.lost = 1u;
             phase ^= 1u;
         }
-        const uint32_t n = min(kStage, total - c0), self = S.self - c0;
+        const uint32_t n = min(T::stage, total - c0), self = S.self - c0;
 #pragma unroll 1
         for (uint32_t j0 = 32u * warp; j0 < n; j0 += 32u * W) {
             const uint32_t j = j0 + lane;
             double rn = cut2, ro = cut2;
             if (j < n && j != self) {
                 double sv[3];
-                if constexpr (STAGED) {
+                if constexpr (STAGED && T::staged) {
                     const double4 v = S.site[j];
                     sv[0] = v.x, sv[1] = v.y, sv[2] = v.z;
                 } else {
                     while (c0 + j >= S.part[part].end) ++part;
-                    const double4 v = ldcg4(A.sorted_b + (S.part[part].base + c0 + j));
+                    const double4 v = ldcg4((STAGED ? A.sorted_s : A.sorted_b) + (S.part[part].base + c0 + j));
                     sv[0] = v.x, sv[1] = v.y, sv[2] = v.z;
-                    wrap_inv<DIM>(g.L, g.invL, sv);
+                    if (!STAGED) wrap_inv<DIM>(g.L, g.invL, sv);
                 }
                 rn = dist2(ta, sv);
                 ro = dist2(tb, sv);
@@ -455,6 +467,10 @@ __device__ __forceinline__ bool lj_energies64(const Geometry& g, const Arrays& A
         }
     }
     __syncwarp();
+    if (!T::staged && total <= 32u && listed == 0u) {  // no pair: sums of zeros
+        ea = eb = mag = 0.0;
+        return true;
+    }
     if (lane < listed) evaluate(lane);
     ea = warp_sum(a);
     eb = warp_sum(b);
@@ -467,7 +483,7 @@ __device__ __forceinline__ bool lj_energies64(const Geometry& g, const Arrays& A
         }
         team_sync<W>();
     }
-    if (STAGED && S.lost) return false;  // (the next wait lies behind another barrier)
+    if (STAGED && T::staged && S.lost) return false;  // (the next wait lies behind another barrier)
     if (W > 1) {
         ea = eb = mag = 0.0;
 #pragma unroll
@@ -520,8 +536,19 @@ __device__ __forceinline__ int lj_decide(const Geometry& g, const Arrays& A, con
                                                                mag);
     if (!decided) return -1;
     const double du = dsub(e_new, e_old);
-    const double e0 = exp(ddiv(-du, kt));
-    if (order_ambiguous(du, mag, S.total, u, kt, e0)) flags |= kTrialAmbiguous;
+    // order_ambiguous is false where dU lies well off 0 and u well off e0, or where no pair was in range:
+    // the tests here imply its own (mag >= |dU| and S.total < 2^24 make order_bound less than 1e-8 mag) and
+    // spare its divisions, and the exponential where dU < 0.
+    bool accept = du <= 0.0;
+    const double b = 1e-8 * mag;
+    const bool few = S.total < (1u << 24) && mag > 1e-200;
+    if (!(few && du < -b) && !(du == 0.0 && mag == 0.0 && u < 1.0 - 1e-15)) {
+        const double e0 = exp(ddiv(-du, kt));
+        if (!(few && du > b && b < 0.99e-3 * kt && fabs(u - e0) * kt > e0 * (4.1 * b + 1.1e-14 * kt)) &&
+            order_ambiguous(du, mag, S.total, u, kt, e0))
+            flags |= kTrialAmbiguous;
+        accept = accept || u < e0;
+    }
     if (lane == 0 && warp == 0) {
         if (FP32) {
             pst.rechecks++;
@@ -530,7 +557,7 @@ __device__ __forceinline__ int lj_decide(const Geometry& g, const Arrays& A, con
         }
         if (flags & kTrialAmbiguous) pst.ambiguous++;
     }
-    return du <= 0.0 || u < e0 ? 1 : 0;
+    return accept ? 1 : 0;
 }
 
 // The sweep: one team of W warps per trial in dataflow order (hmc_flow.cuh), all colour passes of
@@ -540,13 +567,13 @@ __device__ __forceinline__ int lj_decide(const Geometry& g, const Arrays& A, con
 // The proposal (B + displacement, W1 = wrap, the space check, T = wrap(W1), fixed-point site) and the
 // commit run on one lane per axis of the team's first warp; the proposal needs the own space's
 // last colour set only and is done before the wait for the neighbours.
-template <int DIM, bool FP32, bool GENERIC, bool BATCH, bool INJ, int WARPS, int MINB, int W>
+template <int DIM, bool FP32, bool GENERIC, bool BATCH, bool INJ, int WARPS, int MINB, int W, int STAGE>
 __global__ void __launch_bounds__(32 * WARPS, MINB)
     k_flow_lj(Geometry g0, Arrays A, Pair P0, Launch L, Batch B, Injected J) {
     static_assert(W == 1 || W == WARPS, "a team is a warp or a block");
     constexpr unsigned full = 0xffffffffu;
     constexpr uint32_t kTeams = WARPS / W, kNear = DIM == 3 ? 27u : 9u, kOwn = kNear / 2;
-    using TeamT = Team<FP32, BATCH, W>;
+    using TeamT = Team<FP32, BATCH, W, STAGE>;
     __shared__ TeamT s_team[kTeams];
     __shared__ FlowRange s_range;
     __shared__ uint32_t s_item[2];
@@ -692,9 +719,11 @@ __global__ void __launch_bounds__(32 * WARPS, MINB)
                 if (inside && going) going = flow_wait(word, need, full, ok, A.stats, L.flow);
                 if (lane == 0) S.valid = going ? (inside ? 1u : 0u) : 2u;
                 __syncwarp();
-                if (inside && going) {
-                    fence_proxy_async();
-                    team_stage<FP32>(A, 0, lane, S, L.flow);
+                if constexpr (TeamT::staged) {
+                    if (inside && going) {
+                        fence_proxy_async();
+                        team_stage<FP32>(A, 0, lane, S, L.flow);
+                    }
                 }
             }
             team_sync<W>();
@@ -904,27 +933,45 @@ uint32_t lj_team_variant(uint32_t list, double candidates) {
     const uint32_t by_steps = candidates < 128 ? 1u : (candidates < 192 ? 2u : (candidates < 256 ? 3u : 4u));
     return by_trials < by_steps ? by_trials : by_steps;
 }
+// How a one-warp trial gets its sites: staged, or (few candidates) loaded by its lanes, in a kernel for few
+// trials, which is not short of registers, or for many, nine blocks an SM. The staging buffers let an SM
+// hold 24 warps (FP64: 16), too few where a trial is short and a colour has more trials than that; and a
+// copy's way through the barrier is longer than a load. A sweep, us, FP64 (FP32) staged / few / many: 2-D
+// at density 0.3 (17 candidates), 800 spaces a colour 84 / 83 / 85 (81 / 79 / 80), 3,000 95 / 89 / 98
+// (88 / 88 / 94), 5,000 127 / 112 / 102 (102 / 107 / 100), 30,000 507 / 424 / 312 (358 / 401 / 291); 3-D at
+// 0.1 (43), 3,000 157 / 168 / 184 (141 / 145 / 160), 5,000 204 / 189 / 195 (159 / 175 / 171), 30,000
+// 1016 / 898 / 694 (715 / 822 / 627); 3-D at 0.03 (13), 3,000 114 / 109 / 120 (157 / 155 / 167). A launch per
+// colour pass took 318 (360), 729 (817) and 132 (327) us for the last of each.
+enum LjStaging { kLjStaged, kLjFew, kLjMany };
+LjStaging lj_staging(uint32_t list, double candidates) {
+    if (list >= 4500 && candidates <= 96) return kLjMany;
+    return candidates <= 24 ? kLjFew : kLjStaged;
+}
 template <int DIM, bool FP32, bool GENERIC, bool BATCH>
-LjVariant lj_kernel(uint32_t v) {
+LjVariant lj_kernel(uint32_t v, LjStaging sites) {
     // single-warp teams share a block: FP32 staging buffers of four, FP64 of two fit 48 KB
     constexpr int N = FP32 ? 4 : 2;
     switch (v) {
-        case 2: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 2, FP32 ? 12 : 8, 2>, 2, 2};
-        case 3: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 4, 6, 4>, 4, 4};
-        case 4: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 8, 3, 8>, 8, 8};
-        default: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, N, FP32 ? 6 : 8, 1>, N, 1};
+        case 2: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 2, FP32 ? 12 : 8, 2, kStage>, 2, 2};
+        case 3: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 4, 6, 4, kStage>, 4, 4};
+        case 4: return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 8, 3, 8, kStage>, 8, 8};
+        default:
+            if (sites == kLjMany) return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 4, 9, 1, kDirect>, 4, 1};
+            if (sites == kLjFew) return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, 4, 4, 1, kDirect>, 4, 1};
+            return {k_flow_lj<DIM, FP32, GENERIC, BATCH, false, N, FP32 ? 6 : 8, 1, kStage>, N, 1};
     }
 }
 LjVariant lj_kernel(int dim, bool fp32, bool generic, bool batch, uint32_t variant, uint32_t list, double per_space) {
     static_assert(n_shapes(kLjShapes) == 5 && n_shapes(kBatchLjShapes) == 5, "the rule and four kernels");
     const uint32_t v = variant == 0 || variant > 4 ? lj_team_rule(dim, list, per_space) : variant;
+    const LjStaging w = lj_staging(list, per_space * (dim == 3 ? 27 : 9));
     if (batch) {
-        if (dim == 2) return fp32 ? lj_kernel<2, true, false, true>(v) : lj_kernel<2, false, false, true>(v);
-        return fp32 ? lj_kernel<3, true, false, true>(v) : lj_kernel<3, false, false, true>(v);
+        if (dim == 2) return fp32 ? lj_kernel<2, true, false, true>(v, w) : lj_kernel<2, false, false, true>(v, w);
+        return fp32 ? lj_kernel<3, true, false, true>(v, w) : lj_kernel<3, false, false, true>(v, w);
     }
-    if (generic) return dim == 2 ? lj_kernel<2, false, true, false>(v) : lj_kernel<3, false, true, false>(v);
-    if (dim == 2) return fp32 ? lj_kernel<2, true, false, false>(v) : lj_kernel<2, false, false, false>(v);
-    return fp32 ? lj_kernel<3, true, false, false>(v) : lj_kernel<3, false, false, false>(v);
+    if (generic) return dim == 2 ? lj_kernel<2, false, true, false>(v, w) : lj_kernel<3, false, true, false>(v, w);
+    if (dim == 2) return fp32 ? lj_kernel<2, true, false, false>(v, w) : lj_kernel<2, false, false, false>(v, w);
+    return fp32 ? lj_kernel<3, true, false, false>(v, w) : lj_kernel<3, false, false, false>(v, w);
 }
 
 // The two kernels of a range of colour sets whose longest colour list has at most `list` entries.
@@ -986,10 +1033,10 @@ cudaError_t launch_trials_lj(int dim, bool fp32, const Geometry& g, const Arrays
     Launch l{};
     l.kt = kt;
     // single-warp teams, as the sweep's variant 1
-    const LjKernel k = dim == 2 ? (fp32 ? k_flow_lj<2, true, false, false, true, 4, 6, 1>
-                                        : k_flow_lj<2, false, true, false, true, 2, 8, 1>)
-                                : (fp32 ? k_flow_lj<3, true, false, false, true, 4, 6, 1>
-                                        : k_flow_lj<3, false, true, false, true, 2, 8, 1>);
+    const LjKernel k = dim == 2 ? (fp32 ? k_flow_lj<2, true, false, false, true, 4, 6, 1, kStage>
+                                        : k_flow_lj<2, false, true, false, true, 2, 8, 1, kStage>)
+                                : (fp32 ? k_flow_lj<3, true, false, false, true, 4, 6, 1, kStage>
+                                        : k_flow_lj<3, false, true, false, true, 2, 8, 1, kStage>);
     const uint32_t warps = fp32 ? 4u : 2u, n = (j.n + warps - 1) / warps;
     const uint32_t wave = (uint32_t)resident_wave((const void*)k, (int)(32 * warps));
     k<<<n < wave ? n : wave, 32 * warps, 0, s>>>(g, a, p, l, Batch{}, j);
