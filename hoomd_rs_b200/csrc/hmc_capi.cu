@@ -92,6 +92,7 @@ struct hmc_system {
     std::vector<void*> allocations;
     bool coop[2] = {true, false};  // warp-cooperative hard-sphere pass: [fp64, fp32]
     bool coop_set[2] = {false, false};  // coop chosen for this system (else the recorded choice)
+    bool flow_set[2] = {false, false};  // dataflow order chosen for this system by hmc_autotune
     DeviceStats* host_slots = nullptr;  // pinned: per-sweep statistics of a pipelined call
     uint32_t slots_cap = 0;
     int32_t variant[2] = {-1, -1};  // launch variant per precision; -1: the cached choice or the default
@@ -467,9 +468,22 @@ hmc_status flow_buffers(hmc_system* s) {
 // 254 / 302; 3-D FP64 200,003 495 / 345, 300,007 523 / 491, 500,009 572 / 793; 2-D FP32 16,384 77 / 71,
 // 50,021 80 / 99; 2-D FP64 16,384 87 / 71, 50,021 91 / 90, 100,003 95 / 128. The lines lie below
 // those points: at 114,688 and 262,144 bodies in 3-D, at 24,576 in 2-D.
-bool sphere_flow(const hmc_system* s, bool fp32) {
+bool few_spheres(const hmc_system* s, bool fp32) {
     const uint64_t most = s->dim == 2 ? 6144 : (fp32 ? 14336 : 32768);  // bodies per colour
-    return s->interaction == HMC_HARD_SPHERE && !s->coop_set[fp32] && (s->n >> s->dim) <= most;
+    return s->interaction == HMC_HARD_SPHERE && (s->n >> s->dim) <= most;
+}
+
+// How hard spheres run: colour passes with a lane or with a warp per trial, or in dataflow order.
+enum SphereForm : uint32_t { kFormLane, kFormWarp, kFormFlow, kFormNone };
+SphereForm recorded_form(const hmc_system* s, bool fp32);
+
+// Few spheres without a pass of their own: in dataflow order, unless hmc_autotune found a pass faster in a box like
+// this one.
+bool sphere_flow(const hmc_system* s, bool fp32) {
+    if (!few_spheres(s, fp32) || s->coop_set[fp32]) return false;
+    if (s->flow_set[fp32]) return true;
+    const SphereForm f = recorded_form(s, fp32);
+    return f == kFormNone || f == kFormFlow;
 }
 
 // Whether the system's sweeps run in dataflow order, and the colour sets one launch then holds.
@@ -562,10 +576,30 @@ hmc_status time_variants(uint32_t fam, uint32_t size, uint32_t n, std::vector<do
 // dimension, precision and density band; guarded by g_variant_mutex.
 std::map<std::tuple<uint32_t, uint32_t, int32_t>, bool> g_pass_cache;
 
+// The choices of few_spheres boxes, keyed by dimension, precision, density band and power of two of the
+// bodies: the three forms scale differently with the size.
+std::map<std::tuple<uint32_t, uint32_t, int32_t, uint32_t>, SphereForm> g_form_cache;
+std::atomic<bool> g_forms{false};  // whether it holds any: a sweep without a choice asks it
+std::tuple<uint32_t, uint32_t, int32_t, uint32_t> form_key(const hmc_system* s, bool fp32) {
+    return std::make_tuple((uint32_t)s->dim, (uint32_t)fp32, density_band((double)s->n, (double)s->geom.n_cells),
+                           s->n ? (uint32_t)std::ilogb((double)s->n) : 0u);
+}
+SphereForm recorded_form(const hmc_system* s, bool fp32) {
+    if (!g_forms.load(std::memory_order_acquire)) return kFormNone;
+    std::lock_guard<std::mutex> lock(g_variant_mutex);
+    auto it = g_form_cache.find(form_key(s, fp32));
+    return it == g_form_cache.end() ? kFormNone : it->second;
+}
+
 // Whether the next hard-sphere sweep of system s in this precision runs the warp-cooperative
-// pass: the system's own choice, else the recorded one for its band, else the default.
+// pass: the system's own choice, else the recorded one for its band, else the default. (For a box that runs
+// in dataflow order: the pass it would run instead.)
 bool coop_of(const hmc_system* s, bool fp32) {
     if (s->coop_set[fp32] || s->interaction != HMC_HARD_SPHERE) return s->coop[fp32];
+    if (few_spheres(s, fp32)) {
+        const SphereForm f = recorded_form(s, fp32);
+        if (f == kFormLane || f == kFormWarp) return f == kFormWarp;
+    }
     std::lock_guard<std::mutex> lock(g_variant_mutex);
     auto it = g_pass_cache.find(std::make_tuple((uint32_t)s->dim, (uint32_t)fp32,
                                                 density_band((double)s->n, (double)s->geom.n_cells)));
@@ -1113,8 +1147,9 @@ hmc_status hmc_increment_step(hmc_system* s) {
 }
 
 // How the sweeps of one call run: precision, launch variant and, for hard spheres, the pass.
+// Settled once per call: another thread's hmc_autotune may record a choice meanwhile.
 struct SweepPlan {
-    bool fp32, coop, poly2_fp32;
+    bool fp32, flow, coop, poly2_fp32;
     uint32_t variant;
 };
 
@@ -1122,6 +1157,7 @@ static SweepPlan sweep_plan(const hmc_system* s, const hmc_sweep_params* p) {
     SweepPlan sp{};
     sp.fp32 = p->precision == HMC_FP32_RECHECK;
     sp.variant = variant_of(s, sp.fp32);
+    sp.flow = flow_of(s, sp.fp32);
     sp.coop = coop_of(s, sp.fp32);
     sp.poly2_fp32 = sp.fp32 && sp.variant == 0;  // polygon variant 1: the FP64 pass in both modes
     return sp;
@@ -1130,7 +1166,7 @@ static SweepPlan sweep_plan(const hmc_system* s, const hmc_sweep_params* p) {
 // The cell-list rebuild of the current sweep; shapes read S in both modes, and the colour passes
 // do not read slot_of_body.
 static hmc_status sweep_rebuild(hmc_system* s, const SweepPlan& sp) {
-    if (flow_of(s, sp.fp32)) {
+    if (sp.flow) {
         hmc_status st = flow_buffers(s);
         if (st) return st;
     }
@@ -1154,7 +1190,7 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
                                uint32_t r1) {
     const bool fp32 = sp.fp32;
     const uint32_t colors = 1u << s->dim;
-    if (flow_of(s, fp32)) {
+    if (sp.flow) {
         const uint32_t sets = flow_sets(s);
         L.substep = s->substep;  // the kernels add the colour set
         for (uint32_t r = r0; r < r1; r += std::min(sets, r1 - r)) {
@@ -1210,8 +1246,8 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
 
 // The colour sets the host enqueues before it knows a sweep's count: the last sweep's, or all of
 // them where one dataflow launch runs however many there are.
-static uint32_t guessed_sets(const hmc_system* s, bool fp32) {
-    return flow_of(s, fp32) && flow_sets(s) == UINT32_MAX ? UINT32_MAX : std::max(1u, s->rounds_guess);
+static uint32_t guessed_sets(const hmc_system* s, const SweepPlan& sp) {
+    return sp.flow && flow_sets(s) == UINT32_MAX ? UINT32_MAX : std::max(1u, s->rounds_guess);
 }
 
 // A finished sweep into the call's Count and the system's Counter.
@@ -1263,7 +1299,7 @@ static hmc_status sweep_pipelined(hmc_system* s, const hmc_sweep_params* p, hmc_
             s->step = step0 + j;
             s->substep = j == 0 ? substep0 : 0u;
             if ((st = sweep_rebuild(s, sp))) break;
-            if (j == 0) guess = guessed_sets(s, sp.fp32);
+            if (j == 0) guess = guessed_sets(s, sp);
             Launch L = sweep_launch(s, p);
             if ((st = enqueue_sets(s, p, sp, L, 0, guess))) break;
             cudaError_t e = launch_sweep_guard(s->arr.stats, guess, s->arr.abort_word, s->stream);
@@ -1345,7 +1381,7 @@ hmc_status hmc_sweep(hmc_system* s, const hmc_sweep_params* p, hmc_count* out) {
         // The rounds (while count.total() < N, :402-418) are known on the device after the
         // rebuild; the host enqueues the previous sweep's number of colour sets without
         // waiting, the kernels skip sets beyond the true count, and any missing sets follow.
-        const uint32_t guess = s->n == 0 ? 0u : guessed_sets(s, sp.fp32);
+        const uint32_t guess = s->n == 0 ? 0u : guessed_sets(s, sp);
         if ((st = enqueue_sets(s, p, sp, L, 0, guess))) return st;
         // the passes' end is recorded before the host waits for the counts, so that profiling adds
         // no host round trip to the sweep
@@ -1369,7 +1405,7 @@ hmc_status hmc_sweep(hmc_system* s, const hmc_sweep_params* p, hmc_count* out) {
             s->prof.rebuild_launches += rebuild_kernels(s);
             s->prof.sweep_ms += t_sweep;
             // a dataflow launch holds several colour passes
-            s->prof.sweep_launches += flow_of(s, sp.fp32) ? (guess == UINT32_MAX ? 1u : std::max(rounds, guess))
+            s->prof.sweep_launches += sp.flow ? (guess == UINT32_MAX ? 1u : std::max(rounds, guess))
                                                  : (uint64_t)std::max(rounds, guess) * colors;
             s->prof.sweeps += 1;
         }
@@ -1408,6 +1444,7 @@ hmc_status hmc_set_cooperative_pass(hmc_system* s, uint32_t precision, uint32_t 
     if (coop_of(s, fp32) != (cooperative != 0)) s->variant[fp32] = -1;  // the other pass has its own variants
     s->coop[fp32] = cooperative != 0;
     s->coop_set[fp32] = true;
+    s->flow_set[fp32] = false;
     return HMC_OK;
 }
 
@@ -1477,9 +1514,20 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
     HMC_CUDA(cudaSetDevice(s->ctx->device));
     const bool fp32 = p->precision == HMC_FP32_RECHECK;
     // hard spheres without a pass chosen for the system: both passes (a lane or a warp per
-    // trial) and each one's variants, the current pass first
-    const bool coop0 = coop_of(s, fp32), coop_set0 = s->coop_set[fp32], coop_own0 = s->coop[fp32];
-    const bool both = s->interaction == HMC_HARD_SPHERE && !coop_set0 && !sphere_flow(s, fp32);
+    // trial), few spheres in dataflow order too, and each one's variants, the current form first
+    const bool coop_set0 = s->coop_set[fp32], coop_own0 = s->coop[fp32], flow_set0 = s->flow_set[fp32];
+    std::vector<SphereForm> forms = {kFormNone};  // as the system runs now
+    const bool choose = s->interaction == HMC_HARD_SPHERE && !coop_set0;
+    if (choose) {
+        forms = {coop_of(s, fp32) ? kFormWarp : kFormLane, coop_of(s, fp32) ? kFormLane : kFormWarp};
+        if (few_spheres(s, fp32)) forms.insert(sphere_flow(s, fp32) ? forms.begin() : forms.end(), kFormFlow);
+    }
+    auto run_as = [&](SphereForm f) {
+        if (f == kFormNone) return;
+        s->coop[fp32] = f == kFormFlow ? coop_own0 : f == kFormWarp;
+        s->coop_set[fp32] = f != kFormFlow;
+        s->flow_set[fp32] = f == kFormFlow;
+    };
     // the state to start every variant from
     const uint64_t n = s->n;
     const uint64_t step0 = s->step;
@@ -1508,18 +1556,20 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
     hmc_status st = e == cudaSuccess ? HMC_OK : fail(HMC_CUDA_ERROR, "autotune: %s", cudaGetErrorString(e));
     std::vector<double> ms, best_ms;
     uint32_t best = 0, best_fam = family_of(s, fp32);
-    bool best_coop = coop0, have = false;
+    SphereForm best_form = kFormNone;
+    bool have = false;
     double best_t = 0.0;
-    for (int k = 0; k < (both ? 2 : 1) && !st; ++k) {
-        const bool coop = k == 0 ? coop0 : !coop0;
-        if (both) {
-            s->coop[fp32] = coop;
-            s->coop_set[fp32] = true;
-        }
+    for (SphereForm form : forms) {
+        if (st) break;
+        run_as(form);
         const uint32_t fam = family_of(s, fp32);
         uint32_t n_var = 0;
         family_shapes(fam, &n_var);
         st = time_variants(fam, size_class(s, fam), n_var, ms, [&](uint32_t v, double* t) {
+            if (have && v > 0 && ms[0] > 1.5 * best_t) {  // no variant of this form will be the fastest
+                *t = ms[0];
+                return HMC_OK;
+            }
             s->variant[fp32] = (int32_t)v;
             s->variant_family[fp32] = fam;
             return time_variant(s->stream, *p, sweeps, run, restore, t);
@@ -1530,9 +1580,9 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
                 best_t = ms[v];
                 best = v;
                 best_fam = fam;
-                best_coop = coop;
+                best_form = form;
             }
-        if (!st && best_fam == fam && best_coop == coop) best_ms = ms;  // the chosen pass's times
+        if (!st && best_fam == fam) best_ms = ms;  // the chosen pass's times
     }
     hmc_status st2 = restore();
     if (bp) cudaFreeAsync(bp, s->stream);
@@ -1543,13 +1593,19 @@ hmc_status hmc_autotune(hmc_system* s, const hmc_sweep_params* p, uint32_t sweep
         s->variant_family[fp32] = own_family0;
         s->coop[fp32] = coop_own0;
         s->coop_set[fp32] = coop_set0;
+        s->flow_set[fp32] = flow_set0;
         return st ? st : st2;
     }
     const int32_t band = density_band((double)s->n, (double)s->geom.n_cells);
-    if (both) {  // the pass chosen becomes the system's own, and the recorded one for its band
-        s->coop[fp32] = best_coop;
-        s->coop_set[fp32] = true;
-        cache_pass((uint32_t)s->dim, fp32, band, best_coop);
+    if (choose) {  // the form chosen becomes the system's own, and the recorded one for boxes like it
+        run_as(best_form);
+        if (few_spheres(s, fp32)) {
+            std::lock_guard<std::mutex> lock(g_variant_mutex);
+            g_form_cache[form_key(s, fp32)] = best_form;
+            g_forms.store(true, std::memory_order_release);
+        } else {
+            cache_pass((uint32_t)s->dim, fp32, band, best_form == kFormWarp);
+        }
     }
     s->variant[fp32] = (int32_t)best;
     s->variant_family[fp32] = best_fam;

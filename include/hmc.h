@@ -313,7 +313,8 @@ hmc_status hmc_set_launch_variant(hmc_system* sys, uint32_t precision, uint32_t 
 hmc_status hmc_set_cooperative_pass(hmc_system* sys, uint32_t precision, uint32_t cooperative);
 hmc_status hmc_get_cooperative_pass(hmc_system* sys, uint32_t precision, uint32_t* cooperative);
 /* Hard spheres and disks without a pass set by hmc_set_cooperative_pass: hmc_autotune times the
- * variants of both passes and keeps the fastest pass and variant (and records both).
+ * variants of both passes, with few bodies those of the dataflow sweeps too, and keeps the fastest pass and
+ * variant (and records both; with few bodies for boxes with the same power of two of bodies).
  * ms_per_sweep (may be NULL): chosen->count entries, the mean time of one sweep per variant of
  * the chosen pass. */
 hmc_status hmc_autotune(hmc_system* sys, const hmc_sweep_params* params, uint32_t sweeps, hmc_launch_variant* chosen,

@@ -121,3 +121,29 @@ def test_a_pass_that_was_chosen_has_its_own_indices(ctx, precision, coop, accept
     g.set_launch_variant(precision, accepted - 1)
     with pytest.raises(HmcError):
         g.set_launch_variant(precision, accepted)
+
+
+@pytest.mark.parametrize("n,phi,precision", [(250000, 0.02, FP64), (4096, 0.45, FP32_RECHECK), (4096, 0.45, FP64)])
+def test_autotune_of_few_spheres_chooses_among_three_forms(ctx, n, phi, precision):
+    """Dilute boxes near the dataflow sweeps' line run a colour pass a third faster; small ones do not."""
+    g = spheres(ctx, n, precision, phi=phi)
+    g.sweep(TRANSLATE, 0.1, 1.0, precision, n_sweeps=2, increment_step=True)
+    before = g.state()
+    chosen, ms = g.autotune(TRANSLATE, 0.1, 1.0, precision, sweeps=4)
+    assert len(ms) == chosen["count"] and ms[chosen["index"]] == ms.min()
+    flow = chosen["trials_per_warp"] == 3
+    assert flow == (n == 4096)
+    after = g.state()
+    assert np.array_equal(before[0], after[0]) and before[1:] == after[1:]
+    twin, other = spheres(ctx, n, precision, phi=phi), spheres(ctx, 2000, precision, phi=phi)
+    assert twin.launch_variant(precision) == g.launch_variant(precision) == chosen
+    assert other.launch_variant(precision)["trials_per_warp"] == 3  # another size has its own choice
+    for s in (g, twin):
+        s.set_state(*before)
+    counts = [s.sweep(TRANSLATE, 0.1, 1.0, precision, n_sweeps=2, increment_step=True) for s in (g, twin)]
+    assert counts[0].accepted == counts[1].accepted and np.array_equal(g.positions(), twin.positions())
+    # tuning again starts from the choice, and a pass that is set by hand is the only one tuned
+    again, _ = g.autotune(TRANSLATE, 0.1, 1.0, precision, sweeps=2)
+    assert (again["trials_per_warp"] == 3) == flow
+    g.set_cooperative_pass(precision, True)
+    assert g.autotune(TRANSLATE, 0.1, 1.0, precision, sweeps=1)[0]["count"] == 5
