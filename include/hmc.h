@@ -307,9 +307,9 @@ hmc_status hmc_set_launch_variant(hmc_system* sys, uint32_t precision, uint32_t 
  * 3-D). Both make the same pair tests, so the trajectory does not depend on the choice; the launch
  * variants are those of the chosen pass. A system without its own choice runs the one hmc_autotune
  * recorded for its dimension, precision and density band, else the default; with few bodies (up to
- * 114,688 spheres in FP32, 262,144 in FP64, 24,576 disks) it runs its sweeps in dataflow order, one
- * launch for all colour passes, with launch variants of its own. HMC_NOT_SUPPORTED for other
- * interactions. */
+ * 114,688 spheres in FP32, 262,144 in FP64, 24,576 disks; fewer where most spaces are empty) it runs its
+ * sweeps in dataflow order, one launch for all colour passes, with launch variants of its own.
+ * HMC_NOT_SUPPORTED for other interactions. */
 hmc_status hmc_set_cooperative_pass(hmc_system* sys, uint32_t precision, uint32_t cooperative);
 hmc_status hmc_get_cooperative_pass(hmc_system* sys, uint32_t precision, uint32_t* cooperative);
 /* Hard spheres and disks without a pass set by hmc_set_cooperative_pass: hmc_autotune times the

@@ -147,3 +147,17 @@ def test_autotune_of_few_spheres_chooses_among_three_forms(ctx, n, phi, precisio
     assert (again["trials_per_warp"] == 3) == flow
     g.set_cooperative_pass(precision, True)
     assert g.autotune(TRANSLATE, 0.1, 1.0, precision, sweeps=1)[0]["count"] == 5
+
+
+# bodies, packing fraction: on both sides of the dataflow sweeps' line, which falls with the density
+@pytest.mark.parametrize("dim,n,phi,precision,flow", [
+    (3, 114000, 0.45, FP32_RECHECK, True), (3, 114000, 0.05, FP32_RECHECK, False), (3, 60000, 0.03, FP32_RECHECK, True),
+    (3, 250000, 0.45, FP64, True), (3, 250000, 0.11, FP64, False), (3, 60000, 0.03, FP64, True),
+    (2, 24000, 0.5, FP64, True), (2, 24000, 0.06, FP64, False), (2, 5000, 0.06, FP64, True)])
+def test_the_line_falls_with_the_density(ctx, dim, n, phi, precision, flow):
+    g = spheres(ctx, n, precision, dim, phi)
+    assert (g.launch_variant(precision)["trials_per_warp"] == 3) == flow
+    o = spheres(ctx, n, precision, dim, phi)
+    o.set_cooperative_pass(precision, True)  # the other form
+    counts = [s.sweep(TRANSLATE, 0.2, 1.0, precision, n_sweeps=2, increment_step=True) for s in (g, o)]
+    assert counts[0].accepted == counts[1].accepted and np.array_equal(g.positions(), o.positions())
