@@ -1204,6 +1204,7 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
         for (uint32_t r = r0; r < r1; r += std::min(sets, r1 - r)) {
             L.round = r;
             L.round_end = r + std::min(sets, r1 - r);
+            L.overlap_previous = s->pdl ? 1u : 0u;
             L.flow = flow_limit_of(s->flow_limit, s->stall_set, L.round, L.round_end);
             // the overlap penalty and Isotropic have no FP32 path: FP64 in both modes
             if (s->interaction == HMC_HARD_SPHERE)

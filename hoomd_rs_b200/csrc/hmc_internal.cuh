@@ -264,7 +264,8 @@ struct Launch {
     double kt;            // Isothermal temperature
     uint32_t n_bodies;
     uint32_t overlap_previous;  // 1: the previous launch on the stream is a colour pass of the
-                                // same sweep (this pass may start before it ends)
+                                // same sweep (this pass may start before it ends), or a dataflow
+                                // launch's two kernels may each start before the kernel ahead ends
     uint32_t early_wait;        // 1: the previous launch is the rebuild's last kernel: launch
                                 // early but wait for it before reading anything
     FlowLimit flow;             // dataflow launches

@@ -986,12 +986,12 @@ cudaError_t launch_flow(int dim, bool batch, const LjVariant& v, const Geometry&
     const uint64_t entries = ((uint64_t)list << dim) * 16u;
     uint64_t blocks = (entries + 127) / 128;
     const uint64_t wave_d = (uint64_t)resident_wave((const void*)d);
-    PassLaunch pd((uint32_t)(blocks < wave_d ? blocks : wave_d), true, s);
+    PassLaunch pd((uint32_t)(blocks < wave_d ? blocks : wave_d), l.overlap_previous != 0, s);
     cudaError_t e = cudaLaunchKernelEx(&pd.cfg, d, g, a, l, b);
     if (e != cudaSuccess) return e;
     blocks = ((uint64_t)list * 2 * v.team + v.warps - 1) / v.warps;
     const uint64_t wave = (uint64_t)resident_wave((const void*)v.kernel, (int)(32 * v.warps));
-    PassLaunch pl((uint32_t)(blocks < wave ? blocks : wave), true, s, 32 * v.warps);
+    PassLaunch pl((uint32_t)(blocks < wave ? blocks : wave), l.overlap_previous != 0, s, 32 * v.warps);
     return cudaLaunchKernelEx(&pl.cfg, v.kernel, g, a, p, l, b, Injected{});
 }
 }  // namespace
@@ -1011,6 +1011,7 @@ cudaError_t launch_flow_batch_lj(int dim, bool fp32, const Batch& b, const Array
                                  uint32_t round_end, const FlowLimit& limit, cudaStream_t s, uint32_t variant) {
     Launch l{};
     l.flow = limit;
+    l.overlap_previous = 1;
     l.round = round;
     l.round_end = round_end;
     return launch_flow(dim, true, lj_kernel(dim, fp32, false, true, variant, b.color_stride, (double)b.n_bodies / b.n_cells),

@@ -1488,7 +1488,7 @@ cudaError_t launch_flow_poly(bool fp32, const Geometry& g, const Arrays& a, cons
     const uint64_t entries = (uint64_t)g.color_stride * 8u * 4u;
     uint64_t blocks = (entries + 127) / 128;
     const uint64_t wave_d = (uint64_t)resident_wave((const void*)k_draw_poly3);
-    PassLaunch pd((uint32_t)(blocks < wave_d ? blocks : wave_d), true, s);
+    PassLaunch pd((uint32_t)(blocks < wave_d ? blocks : wave_d), l.overlap_previous != 0, s);
     cudaError_t e = cudaLaunchKernelEx(&pd.cfg, k_draw_poly3, g, a, l, rot);
     if (e != cudaSuccess) return e;
     // the compiled launch variants, in the order of kPolyShapes
@@ -1498,7 +1498,7 @@ cudaError_t launch_flow_poly(bool fp32, const Geometry& g, const Arrays& a, cons
     const PolyKernel k = kernels[fp32][variant < 2 ? variant : 0];
     const uint64_t wave = (uint64_t)resident_wave((const void*)k, 32 * kWarps);
     blocks = ((uint64_t)g.color_stride * 2 + kWarps * kGroup - 1) / (kWarps * kGroup);  // warps for two colours' units
-    PassLaunch pl((uint32_t)(blocks < wave ? blocks : wave), true, s, 32 * kWarps);
+    PassLaunch pl((uint32_t)(blocks < wave ? blocks : wave), l.overlap_previous != 0, s, 32 * kWarps);
     return cudaLaunchKernelEx(&pl.cfg, k, g, a, PolyShape{verts, nv, rcut2, rcut2_hi32, site_error(g)}, l, rot,
                               Injected{});
 }

@@ -304,7 +304,7 @@ cudaError_t launch(const Geometry& g, const Arrays& a, const Pair& p, const Laun
     const auto d = k_draw_sphere<DIM>;
     const uint64_t per_set = (uint64_t)g.color_stride << DIM, wave_d = (uint64_t)resident_wave((const void*)d);
     uint64_t blocks = (2u * per_set + 127u) / 128u;
-    PassLaunch pd((uint32_t)(blocks < wave_d ? blocks : wave_d), true, s);
+    PassLaunch pd((uint32_t)(blocks < wave_d ? blocks : wave_d), l.overlap_previous != 0, s);
     cudaError_t e = cudaLaunchKernelEx(&pd.cfg, d, g, a, l);
     if (e != cudaSuccess) return e;
     // the compiled launch variants, in the order of kSphereFlowShapes
@@ -315,7 +315,7 @@ cudaError_t launch(const Geometry& g, const Arrays& a, const Pair& p, const Laun
     // warps for the trials of two colours, at most one resident wave
     blocks = ((uint64_t)g.color_stride * 2u + 4u * kTrials - 1u) / (4u * kTrials);
     const uint64_t wave = (uint64_t)resident_wave((const void*)k);
-    PassLaunch pl((uint32_t)(blocks < wave ? blocks : wave), true, s);
+    PassLaunch pl((uint32_t)(blocks < wave ? blocks : wave), l.overlap_previous != 0, s);
     return cudaLaunchKernelEx(&pl.cfg, k, g, a, p, l, Injected{});
 }
 
