@@ -120,6 +120,7 @@ struct hmc_system {
     uint32_t n_vertices = 0;
     double poly_rcut2 = 0.0;
     float poly_rcut2_hi32 = 0.f;
+    float poly_bound_scale = 1.f;  // fp32_band_scale
     bool polygon() const {
         return interaction == HMC_HARD_CONVEX_POLYGON || interaction == HMC_HARD_CONVEX_SURFACE_MESH_2D;
     }
@@ -302,6 +303,7 @@ void pair_setup(hmc_system* s) {
         s->pair.sigma2 = s->poly_rcut2;  // the FP32 prefilter threshold reuses the sphere bound
         sphere_bound(s);
         s->poly_rcut2_hi32 = s->pair.sig2_hi32;
+        s->poly_bound_scale = (float)fp32_band_scale();
         if (s->arr.fixed_sites) {
             // fixed-point sites: the r^2 bound of lj_setup_for at the circumsphere distance, twice
             const double u32 = std::ldexp(1.0, -24), u64 = std::ldexp(1.0, -53), r = std::sqrt(s->poly_rcut2);
@@ -1211,7 +1213,8 @@ static hmc_status enqueue_sets(hmc_system* s, const hmc_sweep_params* p, const S
                 HMC_CUDA(launch_flow_sphere(s->dim, fp32, s->geom, s->arr, s->pair, L, s->stream, sp.variant));
             else if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON)
                 HMC_CUDA(launch_flow_poly(fp32, s->geom, s->arr, s->verts, s->n_vertices, s->poly_rcut2,
-                                          s->poly_rcut2_hi32, L, p->move == HMC_ROTATE, s->stream, sp.variant));
+                                          s->poly_rcut2_hi32, s->poly_bound_scale, L, p->move == HMC_ROTATE, s->stream,
+                                          sp.variant));
             else
                 HMC_CUDA(launch_flow_lj(s->dim, fp32 && s->soft_fp32(), !s->soft_fp32(), s->geom, s->arr, s->pair, L,
                                     s->stream, sp.variant));
@@ -2467,8 +2470,8 @@ hmc_status hmc_eval_trials(hmc_system* s, const hmc_injected_move* moves, uint64
         if (s->soft())
             e = launch_trials_lj(s->dim, fp32 && s->soft_fp32(), s->geom, s->arr, s->pair, temperature, j, s->stream);
         else if (s->oriented())
-            e = launch_trials_poly(fp32, s->geom, s->arr, s->verts, s->n_vertices, s->poly_rcut2, s->poly_rcut2_hi32, j,
-                                   s->stream);
+            e = launch_trials_poly(fp32, s->geom, s->arr, s->verts, s->n_vertices, s->poly_rcut2, s->poly_rcut2_hi32,
+                                   s->poly_bound_scale, j, s->stream);
         else if (sphere_flow(s, fp32))
             e = launch_flow_trials_sphere(s->dim, fp32, s->geom, s->arr, s->pair, j, s->stream);
         else

@@ -515,8 +515,8 @@ cudaError_t launch_energy_lj(int dim, const Geometry& g, const Arrays& a, const 
                              cudaStream_t s);
 // Hard convex polyhedra: the colour sets [l.round, l.round_end), two kernels as in launch_flow_lj.
 cudaError_t launch_flow_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
-                             double rcut2, float rcut2_hi32, const Launch& l, bool rotate, cudaStream_t s,
-                             uint32_t variant = 0);
+                             double rcut2, float rcut2_hi32, float bound_scale, const Launch& l, bool rotate,
+                             cudaStream_t s, uint32_t variant = 0);
 cudaError_t launch_eval_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
                              double rcut2, float rcut2_hi32, const uint64_t* bodies, const double4* trial,
                              const double4* trial_q, uint32_t n, uint8_t* decisions, cudaStream_t s);
@@ -640,7 +640,7 @@ cudaError_t launch_trials_sphere(int dim, bool fp32, bool coop, const Geometry& 
 cudaError_t launch_trials_lj(int dim, bool fp32, const Geometry& g, const Arrays& a, const Pair& p, double kt,
                              const Injected& j, cudaStream_t s);
 cudaError_t launch_trials_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
-                               double rcut2, float rcut2_hi32, const Injected& j, cudaStream_t s);
+                               double rcut2, float rcut2_hi32, float bound_scale, const Injected& j, cudaStream_t s);
 // The sequential-stream tuner (TuneJob), one warp per job (jobs in device memory): hard spheres,
 // Lennard-Jones / overlap penalty, convex polyhedra, convex polygons (sat: separating axes).
 cudaError_t launch_tune_stream_sphere(int dim, TuneJob* jobs, uint32_t n_jobs, cudaStream_t s);

@@ -232,6 +232,7 @@ struct PolyShape {
     double rcut2;     // (R_a + R_b)^2
     float rcut2_hi32; // FP32 threshold: at or above this, outside the circumsphere for certain
     float site_err;   // per-axis error of a displacement of fixed-point sites beyond its FP32 roundings
+    float bound_scale;  // widens the FP32 bounds of the pair tests (1; tests: HMC_B200_FP32_BAND_SCALE)
 };
 
 __device__ __forceinline__ bool warp_any(bool v) { return __any_sync(0xffffffffu, v); }
@@ -357,6 +358,7 @@ struct ShapeTable {
     double v[32][3];
     uint32_t nv;
     float vmax;
+    float bound_scale;  // PolyShape's
 };
 
 // ConvexPolytope::support_mapping (support above): which vertex has the first maximum of ((v0 n0) + v1
@@ -406,7 +408,7 @@ __device__ __forceinline__ V3 pair_support(const ShapeTable& T, const M3& q, con
             mine = p > first ? i : mine;
             first = fmaxf(first, p);
         }
-        const float gap = 64.f * 5.9604645e-8f * 1.01f * T.vmax * (fabsf((float)n.x) + fabsf((float)n.y) + fabsf((float)n.z)) + 1e-35f;
+        const float gap = 64.f * 5.9604645e-8f * 1.01f * T.bound_scale * T.vmax * (fabsf((float)n.x) + fabsf((float)n.y) + fabsf((float)n.z)) + 1e-35f;
         if (!(first - second > gap)) mine = support64(T, dir);
     } else {
         mine = support64(T, dir);
@@ -523,7 +525,7 @@ __device__ __forceinline__ bool separated32(const ShapeTable& T, float dx, float
         hb = fmaxf(hb, v.x * bx + v.y * by + v.z * bz);
     }
     const float D = fabsf(dx) + fabsf(dy) + fabsf(dz);
-    const float scale = si * (si * D + 3.f * T.vmax * (1.f + si * sj));
+    const float scale = T.bound_scale * si * (si * D + 3.f * T.vmax * (1.f + si * sj));
     return vx * vx + vy * vy + vz * vz - ha - hb > scale * (128.f * 5.9604645e-8f * D + 6.f * site_err);
 }
 
@@ -807,7 +809,7 @@ __global__ void __launch_bounds__(32 * kWarps, MINB)
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(full, vmax, o));
-        if (threadIdx.x == 0) T.vmax = vmax, T.nv = sh.nv;
+        if (threadIdx.x == 0) T.vmax = vmax, T.nv = sh.nv, T.bound_scale = sh.bound_scale;
     }
     if (!INJ) {
         grid_dependency_wait();
@@ -1420,7 +1422,7 @@ cudaError_t launch_serial_poly(const Geometry& g, const Arrays& a, const double4
     const SerialGrid G = make_grid(3, nc, w, cap, size, items, cell_of, site);
     cudaError_t e = build_grid(3, g, a, G, l.n_bodies, s);
     if (e != cudaSuccess || l.n_bodies == 0) return e;
-    k_serial_poly3<<<1, 32, 0, s>>>(g, a, G, PolyShape{verts, nv, rcut2, 0.f, 0.f}, l, rotate ? 1u : 0u, mask);
+    k_serial_poly3<<<1, 32, 0, s>>>(g, a, G, PolyShape{verts, nv, rcut2, 0.f, 0.f, 1.f}, l, rotate ? 1u : 0u, mask);
     return cudaGetLastError();
 }
 
@@ -1467,7 +1469,7 @@ cudaError_t launch_quick_insert_poly3(const Geometry& g, const Arrays& a, const 
 cudaError_t launch_tune_stream_poly(TuneJob* jobs, uint32_t n_jobs, const double4* verts, uint32_t nv, double rcut2,
                                     cudaStream_t s) {
     if (n_jobs == 0) return cudaSuccess;
-    k_tune_stream_poly3<<<n_jobs, 32, 0, s>>>(jobs, n_jobs, PolyShape{verts, nv, rcut2, 0.f, 0.f});
+    k_tune_stream_poly3<<<n_jobs, 32, 0, s>>>(jobs, n_jobs, PolyShape{verts, nv, rcut2, 0.f, 0.f, 1.f});
     return cudaGetLastError();
 }
 
@@ -1481,8 +1483,8 @@ using PolyKernel = void (*)(Geometry, Arrays, PolyShape, Launch, uint32_t, Injec
 }  // namespace
 
 cudaError_t launch_flow_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
-                             double rcut2, float rcut2_hi32, const Launch& l, bool rotate, cudaStream_t s,
-                             uint32_t variant) {
+                             double rcut2, float rcut2_hi32, float bound_scale, const Launch& l, bool rotate,
+                             cudaStream_t s, uint32_t variant) {
     if (l.n_active == 0) return cudaSuccess;
     const uint32_t rot = rotate ? 1u : 0u;
     const uint64_t entries = (uint64_t)g.color_stride * 8u * 4u;
@@ -1499,16 +1501,17 @@ cudaError_t launch_flow_poly(bool fp32, const Geometry& g, const Arrays& a, cons
     const uint64_t wave = (uint64_t)resident_wave((const void*)k, 32 * kWarps);
     blocks = ((uint64_t)g.color_stride * 2 + kWarps * kGroup - 1) / (kWarps * kGroup);  // warps for two colours' units
     PassLaunch pl((uint32_t)(blocks < wave ? blocks : wave), l.overlap_previous != 0, s, 32 * kWarps);
-    return cudaLaunchKernelEx(&pl.cfg, k, g, a, PolyShape{verts, nv, rcut2, rcut2_hi32, site_error(g)}, l, rot,
+    return cudaLaunchKernelEx(&pl.cfg, k, g, a, PolyShape{verts, nv, rcut2, rcut2_hi32, site_error(g), bound_scale}, l, rot,
                               Injected{});
 }
 
 cudaError_t launch_trials_poly(bool fp32, const Geometry& g, const Arrays& a, const double4* verts, uint32_t nv,
-                               double rcut2, float rcut2_hi32, const Injected& j, cudaStream_t s) {
+                               double rcut2, float rcut2_hi32, float bound_scale, const Injected& j, cudaStream_t s) {
     if (j.n == 0) return cudaSuccess;
     const PolyKernel k = fp32 ? k_flow_poly3<true, true, 1> : k_flow_poly3<false, true, 1>;
     const uint32_t wave = (uint32_t)resident_wave((const void*)k), n = (j.n + 4 * kGroup - 1) / (4 * kGroup);
-    k<<<n < wave ? n : wave, 128, 0, s>>>(g, a, PolyShape{verts, nv, rcut2, rcut2_hi32, site_error(g)}, Launch{}, 0u, j);
+    k<<<n < wave ? n : wave, 128, 0, s>>>(
+        g, a, PolyShape{verts, nv, rcut2, rcut2_hi32, site_error(g), bound_scale}, Launch{}, 0u, j);
     return cudaGetLastError();
 }
 
@@ -1516,7 +1519,7 @@ cudaError_t launch_eval_poly(bool fp32, const Geometry& g, const Arrays& a, cons
                              double rcut2, float rcut2_hi32, const uint64_t* bodies, const double4* trial,
                              const double4* trial_q, uint32_t n, uint8_t* decisions, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    PolyShape sh{verts, nv, rcut2, rcut2_hi32, 0.f};
+    PolyShape sh{verts, nv, rcut2, rcut2_hi32, 0.f, 1.f};
     const uint32_t blocks = (n + 3) / 4;
     if (fp32)
         k_eval_poly3<true><<<blocks, 128, 0, s>>>(g, a, sh, bodies, trial, trial_q, n, decisions);
