@@ -387,10 +387,10 @@ struct PairLane {
 
 // composite_support_mapping (xenocollide.rs:318-328) in direction n by the two lanes of a pair test:
 // role 0 finds the trial shape's vertex in direction -n, role 1 the other's in direction q^T n.
-// FP32: the vertex is looked for in FP32 first: with |v_a| <= vmax, vertices and direction components
-// rounded once and three roundings per sum, a product is off by at most 6 u32 vmax |n|_1 (role 1:
-// |q^T n|_1 <= sqrt(3) |n|_1: by 11), so a maximum ahead of the runner-up by more than
-// 64 u32 vmax |n|_1 is the FP64 maximum too; else (ties, as along the edges of a portal) the FP64
+// FP32: the vertex is looked for in FP32 first: with |v_a| <= vmax, vertices and the components of the
+// direction d that is searched rounded once and three roundings per sum, a product is off by at most
+// 6 u32 vmax |d|_1, so a maximum ahead of the runner-up by more than 64 u32 vmax |d|_1 is the FP64
+// maximum too (also where d = q^T n of a versor that is not of unit length is longer than n); else (ties, as along the edges of a portal) the FP64
 // products decide. FP32 takes 8 instructions per vertex against 17 (FP64 issues at half rate).
 template <bool FP32>
 __device__ __forceinline__ V3 pair_support(const ShapeTable& T, const M3& q, const V3& vij, const V3& n, uint32_t role,
@@ -408,7 +408,7 @@ __device__ __forceinline__ V3 pair_support(const ShapeTable& T, const M3& q, con
             mine = p > first ? i : mine;
             first = fmaxf(first, p);
         }
-        const float gap = 64.f * 5.9604645e-8f * 1.01f * T.bound_scale * T.vmax * (fabsf((float)n.x) + fabsf((float)n.y) + fabsf((float)n.z)) + 1e-35f;
+        const float gap = 64.f * 5.9604645e-8f * 1.01f * T.bound_scale * T.vmax * (fabsf(x) + fabsf(y) + fabsf(z)) + 1e-35f;
         if (!(first - second > gap)) mine = support64(T, dir);
     } else {
         mine = support64(T, dir);

@@ -44,3 +44,22 @@ def test_wide_bounds_leave_the_trajectory(ctx, name, verts, spacing, monkeypatch
     for g, _ in runs[1:]:
         assert np.array_equal(g.positions(), wide.positions())
         assert np.array_equal(g.orientations(), wide.orientations())
+
+
+@pytest.mark.parametrize("scale", [0.8, 1.0, 1.25])
+def test_versors_of_other_lengths(ctx, scale):
+    """Orientations are taken as they are given; the bounds hold for versors that are not of unit length too."""
+    n, L = 343, 7 * 1.9
+    pos = lattice.cubic_lattice(n, L, 3, 23, jitter=0.05)
+    q = np.random.default_rng(3).normal(size=(n, 4))
+    q *= scale / np.linalg.norm(q, axis=1)[:, None]
+    h = PairwiseCutoff(HardShape(ConvexPolyhedron.with_vertices(BOX)))
+    runs = []
+    for precision in (FP64, FP32_RECHECK):
+        g = Microstate(ctx, Periodic(3.0 ** 0.5, [L] * 3), pos, h, seed=23)
+        g.set_state(pos, 0, 0, orientations=q)
+        counts = [g.sweep(m, x, 1.0, precision, n_sweeps=3, increment_step=True)
+                  for m, x in ((TRANSLATE, 0.4), (ROTATE, 0.5))]
+        runs.append(([(c.accepted, c.rejected) for c in counts], g.positions(), g.orientations()))
+    assert runs[0][0] == runs[1][0]
+    assert np.array_equal(runs[0][1], runs[1][1]) and np.array_equal(runs[0][2], runs[1][2])
