@@ -1018,7 +1018,8 @@ __global__ void __launch_bounds__(256) k_order_spaces(Arrays A, uint32_t n_cells
     grid_dependency_wait();  // rebuild kernels run back to back: the previous one has ended here
     allow_dependent_launch();
     const unsigned full = 0xffffffffu;
-    const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    // (2^31 spaces take 2^36 threads: the space from the block's number, not from the thread's)
+    const uint32_t c = blockIdx.x * (256u / 32u) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (c >= n_cells) return;
     const uint32_t s = A.cell_start[c], n = A.cell_start[c + 1] - s;
     if (n < 2u) return;
