@@ -321,6 +321,18 @@ void pair_setup(hmc_system* s) {
     }
 }
 
+// The rounds' trial moves, by space, of the passes with lanes per trial: polygons, and polyhedra under the
+// approximate overlap (the sweeps of hard polyhedra keep theirs in the draws).
+hmc_status trial_arrays(hmc_system* s, uint64_t cells) {
+    Arrays& A = s->arr;
+    hmc_status st;
+    if ((!s->polygon() && !s->shape_soft) || A.trial_o || A.trial_q) return HMC_OK;
+    dfree(s, &A.trial_t);
+    dfree(s, &A.trial_k);
+    if ((st = dalloc(s, &A.trial_t, cells)) || (st = dalloc(s, &A.trial_k, cells))) return st;
+    return s->polygon() ? dalloc(s, &A.trial_o, cells) : dalloc(s, &A.trial_q, cells);
+}
+
 // The periodic box and its checkerboard: Periodic::new's range check (boundary/periodic.rs:
 // 97-107) and HypercuboidCheckerboard::compute_dimensions (hypercuboid.rs:188-228). The
 // checkerboard arrays grow when the box needs more spaces than they hold.
@@ -375,16 +387,11 @@ hmc_status setup_geometry(hmc_system* s, const double* L) {
         if ((st = dalloc(s, &A.cell_count, cells)) || (st = dalloc(s, &A.cell_start, cells + 1)) ||
             (st = dalloc(s, &A.block_sums, (size_t)scan_blocks * 9)) || (st = dalloc(s, &A.color_cells, cells)))
             return st;
-        if (s->oriented()) {  // the rounds' trial moves of the passes with lanes per trial
-            dfree(s, &A.trial_t);
-            dfree(s, &A.trial_o);
-            dfree(s, &A.trial_k);
-            dfree(s, &A.trial_q);
-            if ((st = dalloc(s, &A.trial_t, cells)) || (st = dalloc(s, &A.trial_o, cells)) ||
-                (st = dalloc(s, &A.trial_k, cells)))
-                return st;
-            if (s->interaction == HMC_HARD_CONVEX_POLYHEDRON && (st = dalloc(s, &A.trial_q, cells))) return st;
-        }
+        dfree(s, &A.trial_t);
+        dfree(s, &A.trial_o);
+        dfree(s, &A.trial_k);
+        dfree(s, &A.trial_q);
+        if ((st = trial_arrays(s, cells))) return st;
         s->cells_alloc = cells;
     }
     s->geom = g;
@@ -2101,8 +2108,12 @@ hmc_status hmc_set_shape_overlap(hmc_system* s, const hmc_shape_overlap_params* 
     so.half_k = 0.5 * p->penalty_k;
     so.shoulder = p->penalty_shoulder;
     so.max_steps = (uint32_t)steps;
+    HMC_CUDA(cudaSetDevice(s->ctx->device));
+    const bool soft0 = s->shape_soft;
     s->shape_soft = true;
-    return HMC_OK;
+    hmc_status st = trial_arrays(s, s->cells_alloc);
+    if (st) s->shape_soft = soft0;
+    return st;
 }
 
 hmc_status hmc_set_box(hmc_system* s, const double* edge_lengths) {
