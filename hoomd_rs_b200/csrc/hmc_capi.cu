@@ -2585,7 +2585,7 @@ hmc_status batch_rebuild(hmc_batch* bt, bool write_s) {
     if (st) return st;
     HMC_CUDA(cudaMemsetAsync(bt->arr.stats, 0, sizeof(DeviceStats), bt->stream));
     HMC_CUDA(launch_rebuild_batch(bt->dim, bt->b, bt->arr, (uint32_t)bt->n, write_s, bt->stream));
-    bt->kernel_launches += bt->n > 0 ? 6 : 2;  // bin, 2 scan passes, scatter, space sort, gather
+    bt->kernel_launches += rebuild_batch_kernels(bt->b, (uint32_t)bt->n);
     return HMC_OK;
 }
 
@@ -2735,9 +2735,9 @@ hmc_status batch_sweep_captured(hmc_batch* bt, const hmc_sweep_params& p0, bool 
     HMC_CUDA(cudaStreamSynchronize(bt->stream));
     std::memcpy(bt->rep.data(), bt->rep_pinned, sizeof(Replica) * bt->n_rep);
     const BatchSweepTotals& t = *bt->host_totals;
-    // kernels: origins, the rebuild's six, rounds, the first test and the end per sweep; the
+    // kernels: origins, the rebuild's, rounds, the first test and the end per sweep; the
     // colour passes and the step per colour set
-    const uint64_t per_sweep = bt->n > 0 ? 10 : 6;
+    const uint64_t per_sweep = 4 + rebuild_batch_kernels(bt->b, (uint32_t)bt->n);
     bt->kernel_launches += per_sweep * p0.n_sweeps + t.set_launches * (batch_set_kernels(bt) + 1);
     const uint32_t f = t.error_flags;
     if (f & kErrNonFinite) return fail(HMC_NAN_STATE, "a body position is not finite");

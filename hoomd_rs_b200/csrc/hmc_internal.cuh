@@ -442,6 +442,7 @@ cudaError_t launch_batch_sweep_end(const Batch& b, Replica* rep, const DeviceSta
                                    unsigned long long* rep_counts, BatchSweepTotals* totals, bool increment_step,
                                    uint32_t sets, cudaStream_t s);
 // Batches of replicas: the rebuild and the hard-sphere colour pass over all replicas at once.
+uint32_t rebuild_batch_kernels(const Batch& b, uint32_t n);  // kernels that launch_rebuild_batch launches
 cudaError_t launch_rebuild_batch(int dim, const Batch& b, const Arrays& a, uint32_t n, bool write_s, cudaStream_t s);
 cudaError_t launch_sweep_batch(int dim, bool fp32, const Batch& b, const Arrays& a, uint32_t color, uint32_t round,
                                uint32_t max_active, bool overlap_previous, bool early_wait, cudaStream_t s,

@@ -1041,6 +1041,7 @@ __global__ void __launch_bounds__(256) k_order_spaces(Arrays A, uint32_t n_cells
     }
 }
 constexpr uint32_t kWideSpaces = 4;  // bodies per space from which a warp orders a space
+inline bool wide_spaces(uint32_t n, uint32_t n_cells) { return n / kWideSpaces >= n_cells; }
 
 // Per space: order its bodies by index (the order update_checkerboard pushes them,
 // parallel_sweep.rs:194-200, which IndexedRandom::choose indexes), and (lists) list it under its
@@ -1857,7 +1858,7 @@ cudaError_t launch_rebuild(int dim, const Geometry& g, const Arrays& a, uint32_t
     if (n == 0) return cudaSuccess;
     if ((e = launch_chained(k_scatter, blocks_for(n, kBodyThreads), kBodyThreads, true, s, a, n)) != cudaSuccess) return e;
     const uint32_t cb = blocks_for(g.n_cells, kCellThreads), gb = blocks_for(n, kBodyThreads);
-    const bool wide = !lists && n / kWideSpaces >= g.n_cells;
+    const bool wide = !lists && wide_spaces(n, g.n_cells);
     if (wide && (e = launch_chained(k_order_spaces, blocks_for(g.n_cells, 8), 256, true, s, a, g.n_cells)) != cudaSuccess)
         return e;
     if (dim == 2) {
@@ -1868,6 +1869,12 @@ cudaError_t launch_rebuild(int dim, const Geometry& g, const Arrays& a, uint32_t
     if (!wide && (e = launch_chained(k_cells<3>, cb, kCellThreads, true, s, g, a, lists)) != cudaSuccess) return e;
     return launch_chained(gather_kernel<3>(a.fixed_sites != 0, write_s, write_slots),
                           gb, kBodyThreads, true, s, g, a, n);
+}
+
+uint32_t rebuild_batch_kernels(const Batch& b, uint32_t n) {
+    if (n == 0) return 2;  // the scan
+    // bin, 2 scan passes (3 for large grids), (wide spaces) order, lists, scatter, gather
+    return 6u + (wide_spaces(n, b.n_cells) ? 1u : 0u) + (blocks_for(b.n_cells, kScanTile) > kScanDirectBlocks ? 1u : 0u);
 }
 
 cudaError_t launch_rebuild_batch(int dim, const Batch& b, const Arrays& a, uint32_t n, bool write_s, cudaStream_t s) {
@@ -1885,7 +1892,7 @@ cudaError_t launch_rebuild_batch(int dim, const Batch& b, const Arrays& a, uint3
     if ((e = launch_chained(k_scatter, blocks_for(n, 256), 256, true, s, a, n)) != cudaSuccess) return e;
     const uint32_t cb = blocks_for(b.n_cells, kCellThreads), gb = blocks_for(n, 256);
     // (k_cells_batch then finds the spaces in order and lists them)
-    if (n / kWideSpaces >= b.n_cells &&
+    if (wide_spaces(n, b.n_cells) &&
         (e = launch_chained(k_order_spaces, blocks_for(b.n_cells, 8), 256, true, s, a, b.n_cells)) != cudaSuccess)
         return e;
     if (dim == 2) {
