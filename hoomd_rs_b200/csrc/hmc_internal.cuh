@@ -77,14 +77,15 @@ struct Arrays {
     uint32_t* abort_word;    // pipelined sweeps: nonzero once a sweep stopped the call (may be null)
     const double* zig_x;     // ziggurat tables (257 each)
     const double* zig_f;
-    // A round's trial moves, one per colour-list entry (shapes: k_propose_poly3/2 write them
-    // before the round's colour passes, which give each trial several lanes): trial site T = wrap(W1) and
-    // the Metropolis uniform in trial_t, T's FP32 offsets in trial_o, the chosen slot in trial_k
-    // (kNoTrial when the move leaves its space or the entry is empty).
+    // A round's trial moves, one per colour-list entry (polygons, and polyhedra under the approximate
+    // overlap: k_propose_poly2/3 write them before the round's colour passes, which give each trial several
+    // lanes; else null): trial site T = wrap(W1) and the Metropolis uniform in trial_t (2-D: the uniform in .z,
+    // the angle in .w), T's FP32 offsets in trial_o, the chosen slot in trial_k (kNoTrial when the move
+    // leaves its space or the entry is empty).
     double4* trial_t;        // [cells]
-    float4* trial_o;         // [cells]
+    float4* trial_o;         // [cells] polygons
     uint32_t* trial_k;       // [cells]
-    double4* trial_q;        // [cells] shapes: the proposed versor (2-D: the angle in .x)
+    double4* trial_q;        // [cells] polyhedra: the proposed versor
     // Dataflow launches (hmc_flow.cuh): what the random streams of a launch's trials give, by trial
     // number (draw_d: displacement and uniform, draw_i: slot, space, uniform's bounds), and the
     // colour sets each space has finished (~0 for an empty space).
@@ -315,7 +316,7 @@ struct TuneJob {
 // Launch variants of the colour-pass kernels (the autotuner's search space, hmc_autotune): each
 // variant is a compiled instantiation; index 0 of every table is the default. blocks_per_sm is
 // the resident-block target the kernel is compiled for (its register cap), trials_per_warp the
-// trials a warp of the packed polyhedron pass takes, own_steps the candidates per row a lane of
+// trials a warp takes (polyhedra, polygons, small boxes of spheres), own_steps the candidates per row a lane of
 // the warp-cooperative sphere pass tests before handing the rest to its warp. Every variant makes
 // the same pair tests and decisions, so the trajectory does not depend on the choice.
 struct LaunchShape {
@@ -342,7 +343,7 @@ constexpr uint32_t n_shapes(const LaunchShape (&)[N]) {
 
 // Blocks in one resident wave of a kernel with `threads` per block on the current device (SMs x
 // resident blocks per SM), cached per kernel.
-int resident_wave(const void* kernel, int threads = 128, size_t dynamic_bytes = 0);
+int resident_wave(const void* kernel, int threads = 128);
 
 // Launch configuration of a colour pass: 128 threads per block; overlap = programmatic
 // dependent launch after the previous colour pass of the same sweep (the kernel waits with
@@ -633,9 +634,8 @@ cudaError_t launch_pack_positions(int dim, const double4* body_pos, double* pack
 // (angles, 2-D), FP32 site versors (n x 4), in body order.
 cudaError_t launch_gsd_encode(int dim, int ori_kind, const Geometry& g, const double4* body_pos,
                               const double4* body_ori, uint64_t n, float* pos, float* ori, cudaStream_t s);
-// Injected trials through the colour-pass kernels themselves (the probe mode, Injected): the
-// hard-sphere passes (FP32: the per-lane pass, FP64: the warp-cooperative pass, or the one
-// `coop` names), the Lennard-Jones and overlap-penalty passes, the packed polyhedron pass.
+// Injected trials through the sweeps' kernels themselves (the probe mode, Injected): the hard-sphere
+// colour pass that `coop` names, the Lennard-Jones / Isotropic and the polyhedron dataflow kernels.
 cudaError_t launch_trials_sphere(int dim, bool fp32, bool coop, const Geometry& g, const Arrays& a, const Pair& p,
                                  const Injected& j, cudaStream_t s);
 cudaError_t launch_trials_lj(int dim, bool fp32, const Geometry& g, const Arrays& a, const Pair& p, double kt,

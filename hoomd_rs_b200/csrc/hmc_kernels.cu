@@ -1009,8 +1009,9 @@ __device__ __forceinline__ uint32_t append_by_color(DeviceStats* stats, bool has
 
 constexpr int kCellThreads = 512;  // 1024: 71.7 us per 2^20-sphere rebuild, 512: 70.7 us
 
-// The same order by a warp per space, for spaces of several bodies (soft potentials: 10 to 20): a lane per
-// body, which counts the lower indices of its space. A thread per space (k_cells) sorts those by
+// The bodies of a space in the order of their indices (k_cells) by a warp per space, for spaces of several
+// bodies (soft potentials: 10 to 20): a lane per body, which counts the lower indices of its space; beyond
+// 32 bodies one lane sorts them. A thread per space (k_cells) sorts those by
 // insertion, a chain of loads and stores as long as the square of their number: 2^17 sites, 14 a space,
 // 58 -> 4.6 us; 2^19 10 us; ten sweeps of 2^19 sites 14.0 -> 13.7 ms, of 20,011 7.76 -> 7.47 ms. With one
 // or two bodies a space (hard shapes) a warp would have little to share.
@@ -2015,7 +2016,7 @@ SphereKernel coop_kernel(int dim, bool fp32, uint32_t v) {
 
 }  // namespace
 
-int resident_wave(const void* kernel, int threads, size_t dynamic_bytes) {
+int resident_wave(const void* kernel, int threads) {
     static std::mutex mu;
     static std::unordered_map<const void*, int> cache;
     int dev = 0;
@@ -2026,7 +2027,7 @@ int resident_wave(const void* kernel, int threads, size_t dynamic_bytes) {
     if (it != cache.end()) return it->second;
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, dynamic_bytes) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess) {
         cudaGetLastError();
         per_sm = 1;
     }

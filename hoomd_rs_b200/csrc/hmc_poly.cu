@@ -270,11 +270,11 @@ __device__ __forceinline__ bool poly_overlaps(const Geometry& g, const Arrays& A
     return false;
 }
 
-// A round's trial moves of convex polyhedra for every colour list (generate_trial_moves,
-// parallel_sweep.rs:231-278, up to delta_energy_one), one thread per trial: the chosen body,
-// Translate (Ball::sample) or Rotate<Versor>, W1 = wrap(propose(..)), the space check, the trial
-// site T = wrap(W1) and its FP32 offsets; the packed pass reads them instead of computing each
-// move on the 8 lanes of its group.
+// A round's trial moves of convex polyhedra under the approximate overlap for every colour list
+// (generate_trial_moves, parallel_sweep.rs:231-278, up to delta_energy_one), one thread per trial: the
+// chosen body, Translate (Ball::sample) or Rotate<Versor>, W1 = wrap(propose(..)), the space check, the
+// trial site T = wrap(W1) and the Metropolis uniform; k_sweep_poly3_soft, which gives a trial a warp, reads
+// them instead of computing each move in 32 lanes.
 __global__ void __launch_bounds__(128) k_propose_poly3(Geometry g, Arrays A, Launch L, uint32_t rotate) {
     const DeviceStats* st = A.stats;
     if (st->error_flags != 0u || L.round >= st->rounds) return;
@@ -789,9 +789,9 @@ template <bool FP32, bool INJ, int MINB>
 __global__ void __launch_bounds__(32 * kWarps, MINB)
     k_flow_poly3(Geometry g, Arrays A, PolyShape sh, Launch L, uint32_t rotate, Injected J) {
     constexpr unsigned full = 0xffffffffu;
-    // each lane polls up to kWarpsords of its trial's 27 progress words: word sub + i lanes, i < kWarpsords;
+    // each lane polls up to kWords of its trial's 27 progress words: word sub + i lanes, i < kWords;
     // the own space's is word 13
-    constexpr uint32_t kWarpsords = (27 + kGroupLanes - 1) / kGroupLanes;
+    constexpr uint32_t kWords = (27 + kGroupLanes - 1) / kGroupLanes;
     constexpr uint32_t kOwnLane = 13 % kGroupLanes, kOwnBit = 1u << (13 / kGroupLanes);
     __shared__ PolyTeam s_team[kWarps];
     __shared__ uint32_t s_unit;
@@ -880,10 +880,10 @@ __global__ void __launch_bounds__(32 * kWarps, MINB)
         __syncwarp();
         if constexpr (!INJ) {
             unsigned pending = 0;
-            if (valid) pending = (1u << kWarpsords) - 1u;
-            if (sub + (kWarpsords - 1u) * kGroupLanes >= 27u) pending &= ~(1u << (kWarpsords - 1u));
+            if (valid) pending = (1u << kWords) - 1u;
+            if (sub + (kWords - 1u) * kGroupLanes >= 27u) pending &= ~(1u << (kWords - 1u));
             // the own space first: the proposal needs no other
-            bool going = flow_wait_words<kWarpsords>(A.progress, S.near[grp], sub, kGroupLanes, pending,
+            bool going = flow_wait_words<kWords>(A.progress, S.near[grp], sub, kGroupLanes, pending,
                                                  sub == kOwnLane ? kOwnBit : 0u, A.stats, L.flow);
             __syncwarp();
             const AxisGeometry ax = axis_geometry<3>(g, axis);
@@ -907,7 +907,7 @@ __global__ void __launch_bounds__(32 * kWarps, MINB)
             if (valid) ta = wrap_axis(ax.L, ax.invL, w1);  // the trial site T = wrap(W1)
             if (!valid) pending = 0;
             if (going)
-                going = flow_wait_words<kWarpsords>(A.progress, S.near[grp], sub, kGroupLanes, pending, ~0u, A.stats,
+                going = flow_wait_words<kWords>(A.progress, S.near[grp], sub, kGroupLanes, pending, ~0u, A.stats,
                                                     L.flow);
             if (!going) valid = false;
             if (__syncthreads_or(!going)) break;

@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(32) k_tune_stream_poly2(TuneJob* jobs, uint32_
 // A round's trial moves of convex polygons for every colour list, one thread per trial: the
 // chosen body, Translate (Ball::sample) or Rotate<Angle> (theta += Uniform(-a, a), rotate/angle.rs:
 // 46-55), W1 = wrap(propose(..)), the space check, T = wrap(W1) with the angle in .w, and T's FP32
-// offsets; the packed pass reads them instead of computing each move on the 8 lanes of its group.
+// offsets; the passes read them instead of computing each move in all the lanes of its trial.
 template <bool FP32>
 __global__ void __launch_bounds__(128) k_propose_poly2(Geometry g, Arrays A, Launch L, uint32_t rotate,
                                                        uint32_t soft) {

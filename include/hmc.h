@@ -257,7 +257,7 @@ hmc_status hmc_eval_moves(hmc_system* sys, const hmc_injected_move* moves, uint6
 /* The colour pass's own decision for injected trial moves: the kernel that hmc_sweep runs for
  * the system's interaction and `precision` (hard spheres: the dataflow sweep of a small box, the
  * per-lane or the warp-cooperative pass; Lennard-Jones and the overlap penalty: teams of warps per
- * trial; convex polyhedra: the packed pass) takes each move in place of a drawn trial
+ * trial; convex polyhedra: the dataflow sweep) takes each move in place of a drawn trial
  * (generate_trial_moves, parallel_sweep.rs:231-278) and writes its decision instead of
  * committing it; the state does not change. The checkerboard is the one the next hmc_sweep lays
  * out (update_checkerboard, parallel_sweep.rs:176-201: origin from the system's counter).
@@ -280,7 +280,9 @@ hmc_status hmc_total_energy(hmc_system* sys, double* energy);
  * hard spheres in dataflow order: 3) and, for the warp-cooperative FP64 sphere pass, the candidates per stencil row a lane tests before
  * handing the rest to its warp; for convex polygons in HMC_FP32_RECHECK, variant 1 runs the FP64
  * pass instead of the FP32 prefilter. All take the same decisions, so the trajectory is the same
- * in every variant; only the speed differs, by shape and density. hmc_autotune times `sweeps`
+ * in every variant; only the speed differs, by shape and density. (Lennard-Jones and Isotropic: the FP64 sums
+ * add their terms in an order that goes with the variant, so this holds for every decision that no order of
+ * the terms can change; hmc_count's order_ambiguous counts the others.) hmc_autotune times `sweeps`
  * sweeps of the system in every variant of its pass (precision and move from params), each from
  * the same saved state, keeps the fastest for this system and records it for every system and
  * batch of the process with the same pass, dimension, precision and density band (bodies per
