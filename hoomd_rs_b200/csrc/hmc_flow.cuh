@@ -219,32 +219,37 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t b
 // Orders the generic proxy's view of global memory (sites that other SMs have written and this
 // thread has acquired) before the bulk copies that follow.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
-// Wait for the barrier's phase of the given parity. False: the copies did not arrive within the
-// limit, and the caller gives the trial up. The barrier is then waited for once more as long, since the
+__device__ __forceinline__ bool mbar_try(unsigned long long* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    return done != 0u;
+}
+// Wait for the barrier's phase of the given parity. Where the copies do not arrive within the limit `lost`
+// is set, and the caller gives the trial up; the barrier is then waited for once more as long, since the
 // block's shared memory must not be given back while copies into it are on their way.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t parity, DeviceStats* stats,
-                                          const FlowLimit& limit) {
-    unsigned long long t0 = 0;
+static __device__ __noinline__ void mbar_wait_long(unsigned long long* bar, uint32_t parity, DeviceStats* stats,
+                                                   unsigned long long wait_ns, uint32_t* lost) {
+    unsigned long long t0 = global_ns();
     bool late = false;
-    for (uint32_t i = 0;; ++i) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done)
-            : "r"(smem_addr(bar)), "r"(parity)
-            : "memory");
-        if (done) return !late;
-        if ((i & 15u) == 15u) {
-            const unsigned long long now = global_ns();
-            if (t0 == 0) t0 = now;
-            if (now - t0 > limit.wait_ns) {
-                if (late) return false;
-                atomicOr(&stats->error_flags, kErrFlowTimeout);
-                late = true;
-                t0 = now;
-            }
-        }
+    while (!mbar_try(bar, parity)) {
+        const unsigned long long now = global_ns();
+        if (now - t0 <= wait_ns) continue;
+        if (late) return;
+        atomicOr(&stats->error_flags, kErrFlowTimeout);
+        *lost = 1u;
+        late = true;
+        t0 = now;
     }
+}
+__device__ __forceinline__ void mbar_wait(unsigned long long* bar, uint32_t parity, DeviceStats* stats,
+                                          const FlowLimit& limit, uint32_t* lost) {
+    for (uint32_t i = 0; i < 16u; ++i)  // (a try suspends the warp for a while)
+        if (mbar_try(bar, parity)) return;
+    mbar_wait_long(bar, parity, stats, limit.wait_ns, lost);
 }
 
 // One axis of wrap_inv, point_to_space and cell_offsets: the lanes of a warp that share a trial

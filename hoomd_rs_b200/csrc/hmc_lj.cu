@@ -298,10 +298,11 @@ __device__ __forceinline__ void team_stage(const Arrays& A, uint32_t c0, uint32_
 // the staged candidates 32 at a time and list the pairs inside the cut-off band (1 in 6); the pair
 // energies are evaluated 32 listed pairs at a time, so that those ~60 instructions run with every
 // lane busy (two evaluations per trial instead of one per 32 candidates with five lanes). `phase`:
-// the parity of the staging barrier, the first chunk already on its way. False: a copy did not arrive
-// in time (mbar_wait) and there is no result, for the whole team.
+// the parity of the staging barrier, the first chunk already on its way. Where a copy does not arrive in
+// time (mbar_wait) S.lost is set before a barrier of the team, and the caller drops the result: the next
+// wait lies behind another barrier, so all threads read the same.
 template <int DIM, int W, typename T>
-__device__ __forceinline__ bool lj_delta32(const Geometry& g, const Arrays& A, const Pair& P, uint32_t lane, uint32_t warp, T& S,
+__device__ __forceinline__ void lj_delta32(const Geometry& g, const Arrays& A, const Pair& P, uint32_t lane, uint32_t warp, T& S,
                                            uint32_t& phase, const FlowLimit& limit, float& d32, float& bound) {
     const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
     float2* list = S.list[warp].q32;
@@ -310,7 +311,6 @@ __device__ __forceinline__ bool lj_delta32(const Geometry& g, const Arrays& A, c
     const float cut2 = P.lj_rcut2_hi32;
     float d = 0.f, err = 0.f, mag = 0.f;
     uint32_t listed = 0, rounds = 1, part = 0;
-    bool lost = false;
     auto evaluate = [&](uint32_t at) {
         const float2 r2 = list[at];
         float e, x;
@@ -330,13 +330,11 @@ __device__ __forceinline__ bool lj_delta32(const Geometry& g, const Arrays& A, c
 #pragma unroll 1
     for (uint32_t c0 = 0; c0 < total; c0 += T::stage) {
         if (c0 > 0) {
-            lost = team_any<W>(W > 1 ? S.lost != 0u : lost);  // the chunk before has been read
-            if (lost) break;
+            if (team_any<W>(S.lost != 0u)) break;  // the chunk before has been read
             if (warp == 0) team_stage<true>(A, c0, lane, S, limit);
         }
         if constexpr (T::staged) {
-            lost = !mbar_wait(&S.bar, phase, A.stats, limit);
-            if (W > 1 && lost) S.lost = 1u;
+            mbar_wait(&S.bar, phase, A.stats, limit, &S.lost);
             phase ^= 1u;
         }
         const uint32_t n = min(T::stage, total - c0), self = S.self - c0;
@@ -374,9 +372,6 @@ __device__ __forceinline__ bool lj_delta32(const Geometry& g, const Arrays& A, c
     if (W > 1) {
         if (lane == 0) S.sum32[warp] = make_float2(d32, bound);
         team_sync<W>();
-    }
-    if (W > 1 ? S.lost != 0u : __any_sync(full, lost)) return false;
-    if (W > 1) {
         d32 = bound = 0.f;
 #pragma unroll
         for (int w = 0; w < W; ++w) {
@@ -385,7 +380,6 @@ __device__ __forceinline__ bool lj_delta32(const Geometry& g, const Arrays& A, c
         }
     }
     bound += kU32 * fabsf(d32) + 1e-9f;
-    return true;
 }
 
 // FP64 energies of the trial site ta and of the current site tb against the stencil's candidates,
@@ -396,9 +390,9 @@ __device__ __forceinline__ bool lj_delta32(const Geometry& g, const Arrays& A, c
 // INTERIOR: no space of the stencil is the first of an axis (which straddles the box boundary) or
 // reached across the wrap, and an axis has six spaces or more: every site of the stencil then lies
 // within 2 w <= L / 3 of the trial on each axis and any image at least 4 w away, so
-// ref_dist2 would choose the site itself. False: as lj_delta32.
+// ref_dist2 would choose the site itself.
 template <int DIM, bool GENERIC, bool INTERIOR, bool STAGED, int W, typename T>
-__device__ __forceinline__ bool lj_energies64(const Geometry& g, const Arrays& A, const Pair& P, const double* ta,
+__device__ __forceinline__ void lj_energies64(const Geometry& g, const Arrays& A, const Pair& P, const double* ta,
                                               const double* tb, uint32_t lane, uint32_t warp, T& S, uint32_t& phase,
                                               const FlowLimit& limit, double& ea, double& eb, double& mag) {
     const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
@@ -432,7 +426,7 @@ __device__ __forceinline__ bool lj_energies64(const Geometry& g, const Arrays& A
                 if (team_any<W>(S.lost != 0u)) break;  // the chunk before has been read
                 if (warp == 0) team_stage<false>(A, c0, lane, S, limit);
             }
-            if (!mbar_wait(&S.bar, phase, A.stats, limit)) S.lost = 1u;
+            mbar_wait(&S.bar, phase, A.stats, limit, &S.lost);
             phase ^= 1u;
         }
         const uint32_t n = min(T::stage, total - c0), self = S.self - c0;
@@ -469,7 +463,7 @@ __device__ __forceinline__ bool lj_energies64(const Geometry& g, const Arrays& A
     __syncwarp();
     if (!T::staged && total <= 32u && listed == 0u) {  // no pair: sums of zeros
         ea = eb = mag = 0.0;
-        return true;
+        return;
     }
     if (lane < listed) evaluate(lane);
     ea = warp_sum(a);
@@ -482,9 +476,6 @@ __device__ __forceinline__ bool lj_energies64(const Geometry& g, const Arrays& A
             S.sum64[warp][2] = mag;
         }
         team_sync<W>();
-    }
-    if (STAGED && T::staged && S.lost) return false;  // (the next wait lies behind another barrier)
-    if (W > 1) {
         ea = eb = mag = 0.0;
 #pragma unroll
         for (int w = 0; w < W; ++w) {
@@ -493,27 +484,26 @@ __device__ __forceinline__ bool lj_energies64(const Geometry& g, const Arrays& A
             mag += S.sum64[w][2];
         }
     }
-    return true;
 }
 
 // The Metropolis test of the team's trial, slot k in space m (parallel_sweep.rs:267-268): FP32 sums
 // first (FP32), the FP64 sums when their bound could change the decision. The candidates of
-// the stencil in the team's scratch are on their way into its staging buffer. 1 accepts, 0 rejects;
-// -1: not decided, the launch is given up.
+// the stencil in the team's scratch are on their way into its staging buffer; not decided where S.lost
+// is set then.
 template <int DIM, bool FP32, bool GENERIC, int W, typename T>
-__device__ __forceinline__ int lj_decide(const Geometry& g, const Arrays& A, const Pair& P, double kt,
+__device__ __forceinline__ bool lj_decide(const Geometry& g, const Arrays& A, const Pair& P, double kt,
                                           const uint32_t* m, uint32_t k, double u, float w_lo, float w_hi,
                                           uint32_t lane, uint32_t warp, T& S, uint32_t& phase, const FlowLimit& limit,
                                           PairStats& pst, uint8_t& flags) {
     float d32 = 0.f;
     if constexpr (FP32) {
         float b;
-        if (!lj_delta32<DIM, W>(g, A, P, lane, warp, S, phase, limit, d32, b)) return -1;
+        lj_delta32<DIM, W>(g, A, P, lane, warp, S, phase, limit, d32, b);
         if (lane == 0 && warp == 0) pst.checks += 2u * (S.total - 1u);
         const float lo = __fsub_rd(d32, b), hi = __fadd_ru(d32, b);
-        if (hi <= 0.f) return 1;  // dU64 <= 0 for certain: accepted without a uniform
-        if (lo > 0.f && hi < w_lo) return 1;
-        if (lo > 0.f && lo > w_hi) return 0;
+        if (hi <= 0.f) return true;  // dU64 <= 0 for certain: accepted without a uniform
+        if (lo > 0.f && hi < w_lo) return true;
+        if (lo > 0.f && lo > w_hi) return false;
         flags |= kTrialRechecked;  // (also where a sum is not finite: every comparison is false)
     }
     const double t[3] = {S.t[0], S.t[1], DIM == 3 ? S.t[2] : 0.0};
@@ -527,14 +517,10 @@ __device__ __forceinline__ int lj_decide(const Geometry& g, const Arrays& A, con
 #pragma unroll
     for (int a = 0; a < DIM; ++a) interior = interior && g.shape[a] >= 6 && m[a] >= 2 && m[a] + 2 <= g.shape[a];
     double e_new, e_old, mag;
-    bool decided;
     if (!FP32 && interior)
-        decided = lj_energies64<DIM, GENERIC, !FP32, !FP32, W>(g, A, P, t, si, lane, warp, S, phase, limit, e_new, e_old,
-                                                               mag);
+        lj_energies64<DIM, GENERIC, !FP32, !FP32, W>(g, A, P, t, si, lane, warp, S, phase, limit, e_new, e_old, mag);
     else
-        decided = lj_energies64<DIM, GENERIC, false, !FP32, W>(g, A, P, t, si, lane, warp, S, phase, limit, e_new, e_old,
-                                                               mag);
-    if (!decided) return -1;
+        lj_energies64<DIM, GENERIC, false, !FP32, W>(g, A, P, t, si, lane, warp, S, phase, limit, e_new, e_old, mag);
     const double du = dsub(e_new, e_old);
     // order_ambiguous is false where dU lies well off 0 and u well off e0, or where no pair was in range:
     // the tests here imply its own (mag >= |dU| and S.total < 2^24 make order_bound less than 1e-8 mag) and
@@ -557,7 +543,7 @@ __device__ __forceinline__ int lj_decide(const Geometry& g, const Arrays& A, con
         }
         if (flags & kTrialAmbiguous) pst.ambiguous++;
     }
-    return accept ? 1 : 0;
+    return accept;
 }
 
 // The sweep: one team of W warps per trial in dataflow order (hmc_flow.cuh), all colour passes of
@@ -645,11 +631,11 @@ __global__ void __launch_bounds__(32 * WARPS, MINB)
             metropolis_bounds(u, L.kt, w_lo, w_hi);
             team_parts<DIM>(g0, A.cell_start, m, k, lane, S);
             team_stage<FP32>(A, 0, lane, S, L.flow);
-            const int decision = lj_decide<DIM, FP32, GENERIC, W>(g0, A, P0, L.kt, m, k, u, w_lo, w_hi, lane, warp, S,
-                                                                  phase, L.flow, pst, flags);
-            if (decision < 0) break;
+            const bool accept = lj_decide<DIM, FP32, GENERIC, W>(g0, A, P0, L.kt, m, k, u, w_lo, w_hi, lane, warp, S,
+                                                                 phase, L.flow, pst, flags);
+            if (S.lost) break;
             if (lane == 0) {
-                J.decisions[item] = (uint8_t)decision;
+                J.decisions[item] = accept;
                 J.flags[item] = flags;
             }
             __syncwarp();
@@ -730,11 +716,11 @@ __global__ void __launch_bounds__(32 * WARPS, MINB)
             const uint32_t valid = S.valid;
             if (valid == 2u) break;  // the launch is given up
             if (valid == 1u) {
-                const int decision =
+                const bool accept =
                     lj_decide<DIM, FP32, GENERIC, W>(g, A, P, BATCH ? R->kt : L.kt, m, k, u, __uint_as_float(di.z),
                                                      __uint_as_float(di.w), lane, warp, S, phase, L.flow, pst, flags);
-                if (decision < 0) break;  // the whole team
-                if (decision > 0 && warp == 0) {
+                if (TeamT::staged && S.lost) break;  // not decided, the whole team gives up
+                if (accept && warp == 0) {
                     // update_body_properties: body = T, site = wrap(body)
                     const AxisGeometry ax = axis_geometry<DIM>(g, axis);
                     const double sv = wrap_axis(ax.L, ax.invL, ta);
