@@ -478,15 +478,15 @@ hmc_status flow_buffers(hmc_system* s) {
 // 500,009 572 / 793; 2-D FP32 16,384 77 / 71, 50,021 80 / 99; 2-D FP64 16,384 87 / 71, 50,021 91 / 90,
 // 100,003 95 / 128. The lines lie below those points: at 114,688 and 262,144 bodies in 3-D, at 24,576
 // in 2-D. Where spaces are empty a lane has few pairs to test and its pass gains, while a trial in dataflow
-// order keeps its waits: 3-D FP32 114,000 bodies at 0.30 213 / 197, 0.10 185 / 198, 0.02 130 / 144, 50,021 at
-// 0.02 100 / 90; FP64 262,000 at 0.45 464 / 422, 0.30 399 / 421, 0.10 297 / 408, 150,000 at 0.10 258 / 251, 0.02
-// 141 / 169, 50,021 at 0.02 100 / 87; 2-D 24,500 at 0.20 68 / 69, 0.05 52 / 58, 4,096 at 0.05 47 / 44. So the lines
-// fall with the bodies per space (0.04 at 0.02 in 3-D, 0.19 at 0.10, 0.57 at 0.30).
+// order keeps its waits: against the default pass, 3-D FP32 114,000 bodies at 0.30 213 / 197, 0.10 185 / 198,
+// 0.02 131 / 144, 50,021 at 0.02 104 / 90; FP64 262,000 at 0.30 511 / 421, 0.10 310 / 408, 150,000 at 0.10
+// 284 / 251, 0.02 141 / 169, 50,021 at 0.02 100 / 87; 2-D 24,500 at 0.20 68 / 69, 0.05 53 / 58, 4,096 at 0.05
+// 47 / 44. So the lines fall with the bodies per space (0.04 at 0.02 in 3-D, 0.19 at 0.10, 0.57 at 0.30).
 bool few_spheres(const hmc_system* s, bool fp32) {
     const double per_space = (double)s->n / std::max(1u, s->geom.n_cells);
     const double most = s->dim == 2 ? std::min(6144.0, 2000.0 + 14000.0 * per_space)  // bodies per colour
                         : fp32      ? std::min(14336.0, 10000.0 + 14000.0 * per_space)
-                                    : std::min(32768.0, 9000.0 + 37000.0 * per_space);
+                                    : std::min(32768.0, 8000.0 + 65000.0 * per_space);
     return s->interaction == HMC_HARD_SPHERE && (double)(s->n >> s->dim) <= most;
 }
 

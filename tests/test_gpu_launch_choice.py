@@ -152,7 +152,7 @@ def test_autotune_of_few_spheres_chooses_among_three_forms(ctx, n, phi, precisio
 # bodies, packing fraction: on both sides of the dataflow sweeps' line, which falls with the density
 @pytest.mark.parametrize("dim,n,phi,precision,flow", [
     (3, 114000, 0.45, FP32_RECHECK, True), (3, 114000, 0.05, FP32_RECHECK, False), (3, 60000, 0.03, FP32_RECHECK, True),
-    (3, 250000, 0.45, FP64, True), (3, 250000, 0.11, FP64, False), (3, 60000, 0.03, FP64, True),
+    (3, 250000, 0.45, FP64, True), (3, 260000, 0.30, FP64, True), (3, 250000, 0.11, FP64, False), (3, 60000, 0.03, FP64, True),
     (2, 24000, 0.5, FP64, True), (2, 24000, 0.06, FP64, False), (2, 5000, 0.06, FP64, True)])
 def test_the_line_falls_with_the_density(ctx, dim, n, phi, precision, flow):
     g = spheres(ctx, n, precision, dim, phi)
