@@ -17,9 +17,9 @@
 //
 // Bound: the dependent chain of a trial (L2 latency of the staging copies, the acquire and release
 // of the progress words, FP64 wraps) and issue slots; DRAM is idle (the state stays in L2).
-// Measured, ten sweeps with the frame's copy: 2^19 sites FP32 29.3 -> 14.0 ms, 20,011 sites FP64
-// 18.3 -> 7.8 ms, 64 replicas of 8,192 FP32 43.7 -> 21.8 ms, against one launch per colour pass
-// with a warp per trial.
+// Measured, ten sweeps with the frame's copy: 2^19 sites FP32 29.4 -> 13.7 ms, 20,011 sites FP64
+// 18.3 -> 6.9 ms, 64 replicas of 8,192 FP32 44.0 -> 21.3 ms, against one launch per colour pass
+// with a warp per trial. (Trials with few candidates: lj_staging.)
 #include <cuda_runtime.h>
 
 #include <type_traits>

@@ -783,8 +783,8 @@ __device__ __forceinline__ void poly_parts(const Geometry& g, const Arrays& A, c
 // some 2,000 instructions; with every warp at its own place among them the schedulers found no
 // instruction in a third of the cycles, so the block's warps take the steps together (a barrier before
 // each): 24.6 -> 20.9 ms on 2^18 cubes at packing fraction 0.55, ten sweeps of each move (FP32;
-// FP64 44.7 -> 30.6). One launch per colour pass with four trials per warp and a lane per pair test:
-// 42.0 ms (FP64 44.3).
+// FP64 44.7 -> 30.6; the sweeps alone, 22.5 with the frame's copy). One launch per colour pass with four
+// trials per warp and a lane per pair test: 42.0 ms (FP64 44.3).
 template <bool FP32, bool INJ, int MINB>
 __global__ void __launch_bounds__(32 * kWarps, MINB)
     k_flow_poly3(Geometry g, Arrays A, PolyShape sh, Launch L, uint32_t rotate, Injected J) {
